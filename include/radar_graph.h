@@ -447,7 +447,10 @@ typedef enum rg_option {
    * variants push in dense iterations (dense_forward), push-pull pulls.
    * 1: dense iterations pull in every variant (no atomics; BFS exits at the
    * first frontier neighbour; Radii and multi-source BFS OR every neighbour's
-   * mask).  Results are identical either way. */
+   * mask).  Results are identical either way.  rg_bfs, and the other apps on
+   * graphs of up to a few million edges, run their levels in one launch that
+   * pulls dense iterations in every variant, whatever this option says; while
+   * rg_set_trace is on they run level by level. */
   RG_OPT_DIRECTION = 0,
   /* hub copies per CTA for HUBDUP/RADAR; 0 = as many as the budget allows */
   RG_OPT_HUB_SLOTS = 1,

@@ -55,7 +55,9 @@ void kt_end(cudaStream_t st);
 struct CallTimer {
   rg_graph* g;
   explicit CallTimer(rg_graph* gr);
-  rg_status stop();
+  rg_status mark();    // the device work ends here
+  rg_status finish();  // once the stream has passed the mark: fills g_timing
+  rg_status stop();    // mark, wait, finish
 };
 
 int device_sms();     // of the calling thread's current device

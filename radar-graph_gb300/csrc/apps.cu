@@ -18,6 +18,7 @@
 
 #include "app_common.cuh"
 #include "engine.cuh"
+#include "fused.cuh"
 #include "rg_device.cuh"
 
 namespace rg {
@@ -53,10 +54,20 @@ CallTimer::CallTimer(rg_graph* gr) : g(gr) {
   cudaEventRecord(ctx().ev0, ctx().stream);
 }
 
-rg_status CallTimer::stop() {
+rg_status CallTimer::mark() {
   Ctx& c = ctx();
   RG_CUDA(cudaEventRecord(c.ev1, c.stream));
-  RG_CUDA(cudaEventSynchronize(c.ev1));
+  return RG_OK;
+}
+
+rg_status CallTimer::stop() {
+  RG_TRY(mark());
+  RG_CUDA(cudaEventSynchronize(ctx().ev1));
+  return finish();
+}
+
+rg_status CallTimer::finish() {
+  Ctx& c = ctx();
   float ms = 0;
   RG_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
   g_timing.total_ms = ms;
@@ -195,6 +206,11 @@ rg_status bfs_run(rg_graph* g, int variant, uint32_t root_orig, uint32_t* h_pare
   OptScope opt_scope(g, kAppBfs);
   Ctx* cx = nullptr;
   RG_TRY(get_ctx(&cx));
+  if (fused_fits(g, kFusedBfsEdges)) {
+    bool done = false;
+    RG_TRY(bfs_fused_run(g, root_orig, h_parents, h_depth, rounds_out, reached_out, d_depth_out, &done));
+    if (done) return RG_OK;
+  }
   cudaStream_t st = cx->stream;
   const int64_t n = g->n;
   static thread_local BfsState S;
@@ -334,6 +350,11 @@ rg_status bc_run(rg_graph* g, int variant, const uint32_t* src_orig, int nsrc, d
   OptScope opt_scope(g, kAppBc);
   Ctx* cx = nullptr;
   RG_TRY(get_ctx(&cx));
+  if (nsrc > 0 && fused_fits(g, kFusedBcEdges)) {
+    bool done = false;
+    RG_TRY(bc_fused_run(g, src_orig, nsrc, h_deps, levels_out, d_deps_out, &done));
+    if (done) return RG_OK;
+  }
   cudaStream_t st = cx->stream;
   const int64_t n = g->n;
   const int64_t nwords = (n + 31) / 32;
@@ -559,6 +580,22 @@ rg_status radii_run(rg_graph* g, int variant, const uint32_t* seeds_orig, int k,
   OptScope opt_scope(g, kAppRadii);
   Ctx* cx = nullptr;
   RG_TRY(get_ctx(&cx));
+  if (fused_fits(g, kFusedRadiiEdges)) {
+    // each seed once, the largest bit on a repeat (as the seeding loop below)
+    uint32_t v[64];
+    unsigned long long mk[64];
+    int u = 0;
+    for (int i = 0; i < k; i++) {
+      if (seeds_orig[i] >= (uint64_t)g->n) return fail(RG_EINVAL, "vertex id %u >= n", seeds_orig[i]);
+      const int j = (int)(std::find(v, v + u, seeds_orig[i]) - v);
+      v[j] = seeds_orig[i];
+      mk[j] = 1ull << i;
+      u = std::max(u, j + 1);
+    }
+    bool done = false;
+    RG_TRY(radii_fused_run(g, v, mk, u, h_radii, rounds_out, d_radii_out, &done));
+    if (done) return RG_OK;
+  }
   cudaStream_t st = cx->stream;
   const int64_t n = g->n;
   static thread_local RadiiState S;

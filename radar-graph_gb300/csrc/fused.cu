@@ -1,0 +1,1365 @@
+// Whole traversals in one launch.
+//
+// A level-by-level run costs six or seven launches and a host round trip per
+// level (about 30 us), whatever the level holds; on graphs up to a few
+// million edges that is most of a call.  Here one cooperative launch runs
+// every level: its CTAs keep the frontier on the device, meet at a grid
+// barrier (about 1.3 us over the whole chip, a __syncthreads for the smallest
+// graphs, which get one CTA) and take every decision from counters that all of
+// them read after the barrier.  What bounds a small graph now is the chain of
+// dependent loads of a level, about 5 us with its barrier (BFS, R-MAT edge
+// factor 16: 2^10 vertices 182 -> 31 us, 2^16 298 -> 46 us); a large one is bound
+// by its pulls' gathers, as level by level (2^24: 973 -> 560 us; the compactions
+// between the levels are gone).
+//
+// The frontier is two unordered queues: vertices of degree <= kSmallDeg, four
+// lanes each, and pieces of at most kPiece edges of the larger ones, a warp
+// each, so a hub and a leaf cost the same per edge.  Winners are collected in a
+// per-warp shared-memory buffer and appended with one counter update per flush.
+//
+// Every wait is bounded: a CTA that waits too long raises `fail` and returns,
+// the host sees that the run did not finish and answers level by level.
+
+#include <cuda_runtime.h>
+#include <string.h>
+
+#include <algorithm>
+#include <atomic>
+
+#include "fused.cuh"
+#include "pr_exact.cuh"
+
+namespace rg {
+
+namespace {
+
+constexpr int kFT = 1024;             // threads per CTA, one CTA per SM
+constexpr int kFWarps = kFT / 32;
+constexpr uint32_t kSmallDeg = 32;    // at most this degree: four lanes per vertex
+constexpr uint32_t kPiece = 128;      // edges per piece of a larger vertex
+constexpr int kFlushAt = 64;          // winners a warp collects before it appends them
+constexpr int kBuf = kFlushAt + 32;
+constexpr unsigned kAll = 0xffffffffu;
+constexpr unsigned kSpinLimit = 1u << 21;  // polls of the grid barrier: a second or two
+
+// One level's frontier: queue lengths, members and their degree sum.
+struct Slot {
+  unsigned int ns, nl, count, pad;
+  unsigned long long degsum, pad2;
+};
+
+// A 128-bit sum that CTAs add to without waiting for a carry: 43-bit limbs in
+// 64-bit words, so up to 2^21 additions fit.
+struct L1Sum {
+  unsigned long long limb[4];  // the fourth is padding
+  __device__ __forceinline__ void add(const U128& x) {
+    constexpr unsigned long long kMask = (1ull << 43) - 1;
+    atomicAdd(&limb[0], x.lo & kMask);
+    atomicAdd(&limb[1], ((x.lo >> 43) | (x.hi << 21)) & kMask);
+    atomicAdd(&limb[2], x.hi >> 22);
+  }
+  __device__ __forceinline__ U128 read() const {
+    const unsigned long long a = __ldcg(&limb[0]), b = __ldcg(&limb[1]), c = __ldcg(&limb[2]);
+    U128 s{a, 0ull};
+    add128(s, U128{b << 43, b >> 21});
+    add128(s, U128{0ull, c << 22});
+    return s;
+  }
+};
+
+// Zeroed before every launch.
+struct Ctl {
+  unsigned int bar, fail;
+  unsigned int pad[14];
+  Slot lv[4];
+};
+
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// A member of the next frontier and its edges.
+struct Member {
+  uint32_t v, b, e;
+};
+
+// What a CTA shares: its members' totals, what the last barrier completed and
+// the barrier's verdict.
+struct Shared {
+  unsigned int count;
+  unsigned long long degsum;
+  Slot slot;  // the frontier that the last barrier completed
+  U128 l1;    // the sum that it completed (PageRank)
+  int ok;
+};
+
+__device__ __forceinline__ Slot read_slot(const Slot* s) {
+  Slot r;
+  r.ns = __ldcg(&s->ns);
+  r.nl = __ldcg(&s->nl);
+  r.count = __ldcg(&s->count);
+  r.degsum = __ldcg(&s->degsum);
+  return r;
+}
+
+struct Grid {
+  Ctl* ctl;
+  Shared* sh;
+  unsigned target;
+
+  // All CTAs meet; this CTA's totals go into `slot` first (null: dropped) and the
+  // completed slot comes back in sh->slot (and the completed sum `l1` in sh->l1).  What
+  // any thread wrote before is visible to every thread after.  False: the wait
+  // ran out.
+  __device__ __forceinline__ bool sync(Slot* slot = nullptr, const L1Sum* l1 = nullptr) {
+    __syncthreads();
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+      if (slot && sh->count) {
+        atomicAdd(&slot->count, sh->count);
+        atomicAdd(&slot->degsum, sh->degsum);
+      }
+      sh->count = 0;
+      sh->degsum = 0;
+      int ok = 1;
+      if (gridDim.x > 1) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->bar) : "memory");
+        unsigned spins = 0;
+        while ((int)(ld_acquire(&ctl->bar) - target) < 0) {
+          if (++spins > kSpinLimit) {
+            atomicExch(&ctl->fail, 1u);
+            ok = 0;
+            break;
+          }
+        }
+      } else {
+        __threadfence();
+      }
+      if (l1) sh->l1 = l1->read();
+      if (slot) sh->slot = read_slot(slot);  // once per CTA: thousands of warps would queue on its line
+      sh->ok = ok;
+    }
+    __syncthreads();
+    return sh->ok != 0;
+  }
+};
+
+// An entry: a vertex, the edges [y, z) of it that the entry stands for, and in w
+// twice the vertex's number of entries, plus 1 on its first.
+struct Queues {
+  uint4* small;  // whole vertices
+  uint4* large;  // pieces
+};
+
+// Appends a warp's n collected winners (buf) to the next frontier's queues and
+// adds their number and degrees to the CTA's totals.  kEmpty: vertices without
+// edges are queued too (the caller visits every member).
+template <bool kEmpty>
+__device__ __noinline__ void flush_winners(const Member* buf, int n, uint4* qs, uint4* ql, Slot* slot, uint32_t sbase,
+                                           uint32_t lbase, Shared* sh) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();
+  uint32_t v[kBuf / 32], b[kBuf / 32], d[kBuf / 32];
+  unsigned small_total = 0;
+  unsigned long long degsum = 0;
+#pragma unroll
+  for (int i = 0; i < kBuf / 32; i++) {
+    v[i] = 0;
+    d[i] = 0;
+    b[i] = 0;
+    const bool in = i * 32 + lane < n;
+    if (in) {
+      const Member x = buf[i * 32 + lane];
+      v[i] = x.v;
+      b[i] = x.b;
+      d[i] = x.e - x.b;
+      degsum += d[i];
+    }
+    small_total += __popc(__ballot_sync(kAll, d[i] <= kSmallDeg && (kEmpty ? in : d[i] > 0)));
+  }
+  degsum = warp_sum(degsum);
+  unsigned at = 0;
+  if (lane == 0) {
+    atomicAdd(&sh->count, (unsigned)n);
+    atomicAdd(&sh->degsum, degsum);
+    if (small_total) at = atomicAdd(&slot->ns, small_total);
+  }
+  at = __shfl_sync(kAll, at, 0) + sbase;
+#pragma unroll
+  for (int i = 0; i < kBuf / 32; i++) {
+    const bool is = d[i] <= kSmallDeg && (kEmpty ? i * 32 + lane < n : d[i] > 0);
+    const unsigned m = __ballot_sync(kAll, is);
+    if (is) qs[at + __popc(m & ((1u << lane) - 1u))] = make_uint4(v[i], b[i], b[i] + d[i], 3u);
+    at += __popc(m);
+    if (__any_sync(kAll, d[i] > kSmallDeg)) {
+      const unsigned pieces = d[i] > kSmallDeg ? (d[i] + kPiece - 1) / kPiece : 0;
+      unsigned inc = pieces;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned t = __shfl_up_sync(kAll, inc, o);
+        if (lane >= o) inc += t;
+      }
+      unsigned lat = 0;
+      if (lane == 31) lat = atomicAdd(&slot->nl, inc);
+      lat = __shfl_sync(kAll, lat, 31) + lbase;
+      // every lane writes every 32nd piece; its vertex is the first whose pieces
+      // end past it (a hub's hundreds of pieces cost the warp no more than as
+      // many vertices with one)
+      const unsigned total = __shfl_sync(kAll, inc, 31);
+      for (unsigned p0 = 0; p0 < total; p0 += 32) {
+        const unsigned p = p0 + lane;
+        int j = 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          if (__shfl_sync(kAll, inc, j + o - 1) <= p) j += o;
+        }
+        j &= 31;  // (past the last piece: unused)
+        const uint32_t jv = __shfl_sync(kAll, v[i], j), jb = __shfl_sync(kAll, b[i], j);
+        const uint32_t jend = jb + __shfl_sync(kAll, d[i], j);
+        const unsigned np = __shfl_sync(kAll, pieces, j), k = p - (__shfl_sync(kAll, inc, j) - np);
+        if (p < total) {
+          const uint32_t y = jb + k * kPiece;
+          ql[lat + p] = make_uint4(jv, y, min(y + kPiece, jend), 2 * np + (k == 0 ? 1u : 0u));
+        }
+      }
+    }
+  }
+  __syncwarp();
+}
+
+// A warp's winners on their way into the next frontier's queues.
+template <bool kEmpty>
+struct Appender {
+  Member* buf;
+  Shared* sh;
+  int n;
+
+  // b, e: v's edges (the caller loads them beside the update that decides
+  // `won`, so that an append waits for no memory)
+  __device__ __forceinline__ void add(bool won, uint32_t v, uint32_t b, uint32_t e, const Queues& q, Slot* slot,
+                                      uint32_t sbase, uint32_t lbase) {
+    const unsigned m = __ballot_sync(kAll, won);
+    if (!m) return;
+    if (won) buf[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = Member{v, b, e};
+    n += __popc(m);
+    if (n >= kFlushAt) finish(q, slot, sbase, lbase);
+  }
+
+  __device__ __forceinline__ void finish(const Queues& q, Slot* slot, uint32_t sbase, uint32_t lbase) {
+    if (n) flush_winners<kEmpty>(buf, n, q.small, q.large, slot, sbase, lbase, sh);
+    n = 0;
+  }
+};
+
+// fn(lane has an edge, source, neighbour) over every edge of a frontier, all
+// lanes of a warp together, four edges per lane in flight.
+template <class Fn>
+__device__ __forceinline__ void expand(const DevGraph& g, const Queues& q, uint32_t sbase, uint32_t ns, uint32_t lbase,
+                                       uint32_t nl, Fn&& fn) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t warp = (uint32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);  // neighbours on other SMs
+  const uint32_t nwarps = gridDim.x * kFWarps;
+  for (uint32_t i = warp; i < nl; i += nwarps) {
+    const uint4 it = q.large[lbase + i];
+    uint32_t d[4];
+    bool in[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t e = it.y + 32 * k + lane;
+      in[k] = e < it.z;
+      d[k] = in[k] ? g.adj[e] : 0u;
+    }
+    fn(in, it.x, d);
+  }
+  const uint32_t groups = (ns + 7) / 8;
+  for (uint32_t i = warp; i < groups; i += nwarps) {
+    const uint32_t j = i * 8 + (lane >> 2);
+    const uint4 it = j < ns ? q.small[sbase + j] : make_uint4(0, 0, 0, 0);
+    const uint32_t s = it.x, b = it.y, end = it.z;
+    for (uint32_t e0 = b + (lane & 3); __any_sync(kAll, e0 < end); e0 += 16) {
+      uint32_t d[4];
+      bool in[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint32_t e = e0 + 4 * k;
+        in[k] = e < end;
+        d[k] = in[k] ? g.adj[e] : 0u;
+      }
+      fn(in, s, d);
+    }
+  }
+}
+
+__device__ __forceinline__ void begin(Grid& grid, Shared* sh, Ctl* ctl) {
+  grid.ctl = ctl;
+  grid.sh = sh;
+  grid.target = 0;
+  if (threadIdx.x == 0) {
+    sh->count = 0;
+    sh->degsum = 0;
+    sh->ok = 1;
+  }
+  __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// BFS (BFS.C:122-188)
+// ---------------------------------------------------------------------------
+struct BfsArgs {
+  DevGraph out, in;  // push and pull lists
+  const uint32_t* new_ids;  // null: not sorted
+  uint32_t root;            // original id
+  int64_t threshold;
+  uint32_t* vis[2];   // visited bitmaps, (n+31)/32 words
+  int32_t* depth;
+  uint32_t* parents;  // null: not wanted
+  int32_t* depth_out;  // original-id order; null: not wanted (or not sorted)
+  Queues q[2];
+  Ctl* ctl;
+  volatile uint64_t* info;  // mapped: rounds, reached, edges, done
+};
+
+// A push level claims vertices with an atomicOr on the visited bitmap; a pull
+// level reads one bitmap and writes the other (a visited in-neighbour of an
+// unvisited vertex is in the frontier, so visited is all a pull has to test).
+__global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
+  __shared__ Shared sh;
+  __shared__ Member buf[kFWarps][kBuf];
+  Grid grid;
+  Appender<false> ap{buf[threadIdx.x >> 5], &sh, 0};
+  begin(grid, &sh, A.ctl);
+  const uint32_t n = A.out.n, nwords = (n + 31) / 32;
+  const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
+  const int lane = threadIdx.x & 31;
+  const uint32_t warp = tid >> 5, nwarps = nthreads >> 5;
+  const uint32_t root = A.new_ids ? A.new_ids[A.root] : A.root;
+  for (uint32_t i = tid; i < n; i += nthreads) {
+    A.depth[i] = i == root ? 0 : -1;
+    if (A.parents) A.parents[i] = i == root ? root : kNone;
+  }
+  for (uint32_t w = tid; w < nwords; w += nthreads) A.vis[0][w] = w == root >> 5 ? 1u << (root & 31) : 0u;
+  if (warp == 0) {
+    ap.add(lane == 0, root, A.out.off[root], A.out.off[root + 1], A.q[0], &A.ctl->lv[0], 0, 0);
+    ap.finish(A.q[0], &A.ctl->lv[0], 0, 0);
+  }
+  if (!grid.sync(&A.ctl->lv[0])) return;
+  int cv = 0;             // the bitmap that is current
+  int cq = 0;             // the queue pair that holds the frontier
+  bool queued = true;
+  int32_t level = 0;
+  unsigned long long reached = 0, edges = 0;
+  for (;;) {
+    Slot* cs = &A.ctl->lv[level % 3];
+    Slot* ns = &A.ctl->lv[(level + 1) % 3];
+    Slot c = sh.slot;
+    if (c.count == 0) break;
+    reached += c.count;
+    edges += c.degsum;
+    if (tid == 0) A.ctl->lv[(level + 2) % 3] = Slot{};
+    const bool pull = (int64_t)(c.count + c.degsum) > A.threshold && c.degsum > 0;
+    level++;
+    uint32_t* vis = A.vis[cv];
+    if (pull) {
+      uint32_t* nvis = A.vis[cv ^ 1];
+      unsigned count = 0;
+      unsigned long long degsum = 0;
+      for (uint32_t w = warp; w < nwords; w += nwarps) {
+        const uint32_t seen = vis[w];
+        const uint32_t v = w * 32 + lane;
+        const bool want = v < n && !((seen >> lane) & 1u);
+        uint32_t b = 0, e = 0, from = kNone;
+        if (want) {
+          b = A.in.off[v];
+          e = A.in.off[v + 1];
+        }
+        // each lane tries its first 16 neighbours, four at a time; the lists
+        // that are longer are then read by the whole warp, one at a time
+        const uint32_t stop = min(e, b + 16);
+        for (; b < stop && from == kNone; b += 4) {
+          uint32_t u[4];
+          bool hit[4];
+#pragma unroll
+          for (int k = 0; k < 4; k++) u[k] = b + k < e ? A.in.adj[b + k] : kNone;
+#pragma unroll
+          for (int k = 0; k < 4; k++) hit[k] = u[k] != kNone && bit_test(vis, u[k]);
+#pragma unroll
+          for (int k = 3; k >= 0; k--) {
+            if (hit[k]) from = u[k];
+          }
+        }
+        unsigned rest = __ballot_sync(kAll, from == kNone && b < e);
+        while (rest) {
+          const int j = __ffs(rest) - 1;
+          rest &= rest - 1;
+          const uint32_t jb = __shfl_sync(kAll, b, j), je = __shfl_sync(kAll, e, j);
+          for (uint32_t x = jb; x < je; x += 32) {
+            const uint32_t u = x + lane < je ? A.in.adj[x + lane] : kNone;
+            const unsigned hits = __ballot_sync(kAll, u != kNone && bit_test(vis, u));
+            if (hits) {
+              const uint32_t f = __shfl_sync(kAll, u, __ffs(hits) - 1);
+              if (lane == j) from = f;
+              break;
+            }
+          }
+        }
+        const bool won = from != kNone;
+        const unsigned now = __ballot_sync(kAll, won);
+        if (lane == 0) nvis[w] = seen | now;
+        if (won) {
+          A.depth[v] = level;
+          if (A.parents) A.parents[v] = from;
+          count++;
+          degsum += A.out.off[v + 1] - A.out.off[v];
+        }
+      }
+      count = __reduce_add_sync(kAll, count);
+      if (count) {
+        degsum = warp_sum(degsum);
+        if (lane == 0) {
+          atomicAdd(&sh.count, count);
+          atomicAdd(&sh.degsum, degsum);
+        }
+      }
+      cv ^= 1;
+      queued = false;
+    } else {
+      if (!queued) {  // after a pull: the frontier is what it added to the bitmap
+        const uint32_t* old = A.vis[cv ^ 1];
+        for (uint32_t w = warp; w < nwords; w += nwarps) {
+          const uint32_t x = vis[w] & ~old[w];
+          if (!x) continue;
+          const uint32_t v = min(w * 32 + lane, n - 1);
+          ap.add((x >> lane) & 1u, v, A.out.off[v], A.out.off[v + 1], A.q[cq], cs, 0, 0);
+        }
+        ap.finish(A.q[cq], cs, 0, 0);
+        if (!grid.sync()) return;  // (its members were counted by the pull)
+        c = read_slot(cs);
+        queued = true;
+      }
+      const Queues nq = A.q[cq ^ 1];
+      expand(A.out, A.q[cq], 0, c.ns, 0, c.nl, [&](const bool (&in)[4], uint32_t s, const uint32_t (&d)[4]) {
+        bool won[4];
+        uint32_t b[4] = {}, e[4] = {};
+#pragma unroll
+        for (int k = 0; k < 4; k++) won[k] = in[k] && !bit_test(vis, d[k]);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          if (won[k]) {
+            const uint32_t bit = 1u << (d[k] & 31);
+            b[k] = A.out.off[d[k]];
+            e[k] = A.out.off[d[k] + 1];
+            won[k] = !(atomicOr(vis + (d[k] >> 5), bit) & bit);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          if (won[k]) {
+            A.depth[d[k]] = level;
+            if (A.parents) A.parents[d[k]] = s;
+          }
+          ap.add(won[k], d[k], b[k], e[k], nq, ns, 0, 0);
+        }
+      });
+      ap.finish(nq, ns, 0, 0);
+      cq ^= 1;
+    }
+    if (!grid.sync(ns)) return;
+  }
+  if (A.depth_out) {
+    for (uint32_t i = tid; i < n; i += nthreads) A.depth_out[i] = A.depth[A.new_ids ? A.new_ids[i] : i];
+  }
+  if (tid == 0) {
+    A.info[0] = (uint64_t)level;
+    A.info[1] = reached;
+    A.info[2] = edges;
+    __threadfence_system();
+    A.info[3] = 1;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// BC, one source (BC-manyiter-v2.C:205-367)
+// ---------------------------------------------------------------------------
+struct BcArgs {
+  DevGraph g;  // the lists the forward phase pushes along (the backward phase reads them the other way)
+  const uint32_t* new_ids;
+  uint32_t source;   // original id
+  int32_t* lvl;
+  double *sigma, *deps;
+  double* deps_out;  // original-id order after the last source; null otherwise
+  Queues q;          // every level's frontier, one after another
+  uint32_t *first_small, *first_large;  // per level, levels + 1 entries
+  bool first_source;
+  Ctl* ctl;
+  volatile uint64_t* info;  // mapped, summed over the sources: levels, edges, done
+};
+
+// Forward: sigma is pushed along the frontier's edges to vertices of the next
+// level.  Backward: every vertex sums the dependencies of its successors, so
+// only the pieces of large vertices need an atomic add.
+__global__ void __launch_bounds__(kFT, 1) bc_fused(BcArgs A) {
+  __shared__ Shared sh;
+  __shared__ Member buf[kFWarps][kBuf];
+  Grid grid;
+  Appender<true> ap{buf[threadIdx.x >> 5], &sh, 0};
+  begin(grid, &sh, A.ctl);
+  const uint32_t n = A.g.n;
+  const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
+  const int lane = threadIdx.x & 31;
+  const uint32_t src = A.new_ids ? A.new_ids[A.source] : A.source;
+  for (uint32_t i = tid; i < n; i += nthreads) {
+    A.lvl[i] = i == src ? 0 : -1;
+    A.sigma[i] = i == src ? 1.0 : 0.0;
+    if (A.first_source) A.deps[i] = 0.0;
+  }
+  if ((tid >> 5) == 0) {
+    ap.add(lane == 0, src, A.g.off[src], A.g.off[src + 1], A.q, &A.ctl->lv[0], 0, 0);
+    ap.finish(A.q, &A.ctl->lv[0], 0, 0);
+  }
+  if (!grid.sync(&A.ctl->lv[0])) return;
+  uint32_t sbase = 0, lbase = 0;
+  int32_t level = 0;
+  unsigned long long edges = 0;
+  for (;;) {
+    Slot* ns = &A.ctl->lv[(level + 1) % 3];
+    const Slot c = sh.slot;
+    if (tid == 0) {
+      A.first_small[level] = sbase;
+      A.first_large[level] = lbase;
+    }
+    if (c.count == 0) break;
+    edges += c.degsum;
+    if (tid == 0) A.ctl->lv[(level + 2) % 3] = Slot{};
+    level++;
+    const uint32_t sn = sbase + c.ns, ln = lbase + c.nl;  // where the next level's entries begin
+    expand(A.g, A.q, sbase, c.ns, lbase, c.nl, [&](const bool (&in)[4], uint32_t s, const uint32_t (&d)[4]) {
+      int32_t l[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) l[k] = in[k] ? A.lvl[d[k]] : -2;
+      const double x = A.sigma[s];
+      uint32_t b[4] = {}, e[4] = {};
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        if (l[k] == -1) {
+          b[k] = A.g.off[d[k]];
+          e[k] = A.g.off[d[k] + 1];
+          l[k] = atomicCAS(A.lvl + d[k], -1, level);
+        } else if (l[k] != level) {
+          l[k] = -2;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) {  // l: -1 reached here first, level reached by another edge, else not next
+        if (l[k] >= -1) atomicAdd(A.sigma + d[k], x);
+        ap.add(l[k] == -1, d[k], b[k], e[k], A.q, ns, sn, ln);
+      }
+    });
+    ap.finish(A.q, ns, sn, ln);
+    sbase = sn;
+    lbase = ln;
+    if (!grid.sync(ns)) return;
+  }
+  // sbase, lbase: the ends of the last level's entries; first_* are written by
+  // thread 0 above, so every CTA waits once before it reads them
+  if (!grid.sync()) return;
+  const uint32_t gwarp = (uint32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+  const uint32_t nwarps = gridDim.x * kFWarps;
+  for (int32_t r = level - 1; r >= 0; r--) {
+    const uint32_t s0 = A.first_small[r], s1 = A.first_small[r + 1];
+    const uint32_t l0 = A.first_large[r], l1 = A.first_large[r + 1];
+    const bool deepest = r == level - 1;  // its vertices have no successors: 1/sigma alone
+    for (uint32_t i = l0 + gwarp; i < l1; i += nwarps) {
+      const uint4 it = A.q.large[i];
+      double acc = 0.0;
+      if (!deepest) {
+        uint32_t d[4];
+        int32_t l[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) d[k] = it.y + 32 * k + lane < it.z ? A.g.adj[it.y + 32 * k + lane] : kNone;
+#pragma unroll
+        for (int k = 0; k < 4; k++) l[k] = d[k] != kNone ? A.lvl[d[k]] : -2;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          if (l[k] == r + 1) acc += A.deps[d[k]];
+        }
+      }
+      acc = warp_sum(acc);
+      if (lane == 0) {
+        if (it.w & 1u) acc += 1.0 / A.sigma[it.x];
+        atomicAdd(A.deps + it.x, acc);
+      }
+    }
+    const uint32_t groups = (s1 - s0 + 7) / 8;
+    for (uint32_t i = gwarp; i < groups; i += nwarps) {
+      const uint32_t j = s0 + i * 8 + (lane >> 2);
+      const uint4 it = j < s1 ? A.q.small[j] : make_uint4(0, 0, 0, 0);
+      const uint32_t s = it.x, b = it.y, end = it.z;
+      double acc = 0.0;
+      for (uint32_t e0 = b + (lane & 3); !deepest && __any_sync(kAll, e0 < end); e0 += 16) {
+        uint32_t d[4];
+        int32_t l[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) d[k] = e0 + 4 * k < end ? A.g.adj[e0 + 4 * k] : kNone;
+#pragma unroll
+        for (int k = 0; k < 4; k++) l[k] = d[k] != kNone ? A.lvl[d[k]] : -2;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          if (l[k] == r + 1) acc += A.deps[d[k]];
+        }
+      }
+      acc += __shfl_xor_sync(kAll, acc, 1);
+      acc += __shfl_xor_sync(kAll, acc, 2);
+      if (j < s1 && (lane & 3) == 0) A.deps[s] += 1.0 / A.sigma[s] + acc;
+    }
+    if (!grid.sync()) return;
+  }
+  // D = (D - 1/sigma) / (1/sigma), as bc_final forms it (unreached: NaN)
+  if (A.deps_out) {
+    for (uint32_t i = tid; i < n; i += nthreads) {
+      const uint32_t v = A.new_ids ? A.new_ids[i] : i;
+      const double s = A.sigma[v];
+      A.deps_out[i] = (A.deps[v] - 1 / s) * s;
+    }
+  } else {
+    for (uint32_t i = tid; i < n; i += nthreads) {
+      const double s = A.sigma[i];
+      A.deps[i] = (A.deps[i] - 1 / s) * s;
+    }
+  }
+  if (tid == 0) {
+    A.info[0] += (uint64_t)level;
+    A.info[1] += edges;
+    __threadfence_system();
+    A.info[3] += 1;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Radii (Radii.C:140-218)
+// ---------------------------------------------------------------------------
+struct RadiiArgs {
+  DevGraph out, in;
+  const uint32_t* chunk_v;  // the pull lists' partition
+  uint32_t nchunks;
+  const uint32_t* new_ids;
+  uint32_t seed[64];  // original ids, each once
+  unsigned long long mask[64];
+  int k;
+  int64_t threshold;
+  unsigned long long *vis, *nvis;
+  int32_t* radii;
+  int32_t* radii_out;  // original-id order; null: not wanted (or not sorted)
+  uint32_t* bits;
+  Queues q[2];
+  Ctl* ctl;
+  volatile uint64_t* info;  // mapped: rounds, edges, -, done
+};
+
+__device__ __forceinline__ void radii_flush(const RadiiArgs& A, uint32_t row, unsigned long long part) {
+  const unsigned long long w = part & ~A.vis[row];
+  if (!w) return;
+  atomicOr(A.nvis + row, w);
+  bit_set(A.bits, row);
+}
+
+// Rounds push over the queue or, dense ones, pull every row's neighbour masks
+// (4 edges per lane, one segmented OR scan per 128 edges, as mask_pull_sweep
+// with shorter steps: a small graph has more warps than 512-edge chunks).  A
+// vertex pass after either makes the new masks current and queues the vertices
+// that grew.
+__global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ RadiiArgs A) {
+  __shared__ Shared sh;
+  __shared__ Member buf[kFWarps][kBuf];
+  Grid grid;
+  Appender<true> ap{buf[threadIdx.x >> 5], &sh, 0};
+  begin(grid, &sh, A.ctl);
+  const uint32_t n = A.out.n, nwords = (n + 31) / 32;
+  const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
+  const int lane = threadIdx.x & 31;
+  const uint32_t warp = tid >> 5, nwarps = nthreads >> 5;
+  for (uint32_t i = tid; i < n; i += nthreads) {
+    A.vis[i] = 0ull;
+    A.nvis[i] = 0ull;
+    A.radii[i] = -1;
+  }
+  for (uint32_t w = tid; w < nwords; w += nthreads) A.bits[w] = 0u;
+  unsigned long long full = 0ull;  // the bits that can spread: seeds with out-edges
+  for (int j = lane; j < A.k; j += 32) {
+    const uint32_t v = A.new_ids ? A.new_ids[A.seed[j]] : A.seed[j];
+    if (A.out.off[v + 1] > A.out.off[v]) full |= A.mask[j];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) full |= __shfl_xor_sync(kAll, full, o);
+  if (!grid.sync()) return;
+  if (warp == 0) {
+    for (int j0 = 0; j0 < 64; j0 += 32) {
+      const int j = j0 + lane;
+      uint32_t v = 0;
+      if (j < A.k) {
+        v = A.new_ids ? A.new_ids[A.seed[j]] : A.seed[j];
+        A.vis[v] = A.nvis[v] = A.mask[j];
+        A.radii[v] = 0;
+      }
+      ap.add(j < A.k, v, A.out.off[v], A.out.off[v + 1], A.q[0], &A.ctl->lv[0], 0, 0);
+    }
+    ap.finish(A.q[0], &A.ctl->lv[0], 0, 0);
+  }
+  if (!grid.sync(&A.ctl->lv[0])) return;
+  int cq = 0;
+  int32_t round = 0;
+  unsigned long long edges = 0;
+  for (;;) {
+    Slot* ns = &A.ctl->lv[(round + 1) % 3];
+    const Slot c = sh.slot;
+    if (c.count == 0) break;
+    edges += c.degsum;
+    if (tid == 0) A.ctl->lv[(round + 2) % 3] = Slot{};
+    round++;
+    const Queues nq = A.q[cq ^ 1];
+    if ((int64_t)(c.count + c.degsum) > A.threshold && A.in.m > 0) {
+      const uint32_t steps = (A.in.m + 127) / 128;
+      const uint32_t gwarp = (uint32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+      for (uint32_t t = gwarp; t < steps; t += nwarps) {
+        const uint32_t e = t * 128 + lane * 4;
+        const uint32_t ch = t / (kSweepChunk / 128);
+        uint32_t row = kNone;
+        unsigned long long part = 0ull;
+        if (e < A.in.m) {
+          const uint4 w = __ldg(reinterpret_cast<const uint4*>(A.in.adj + e));  // adj is padded past m
+          const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+          row = upper_index(A.in.off, A.chunk_v[ch], A.chunk_v[ch + 1], e);
+          uint32_t r = row, nxt = A.in.off[r + 1], rows[4];
+          bool need[4];
+          bool open = full == 0ull || (A.vis[r] & full) != full;
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            if (e + k < A.in.m && e + k >= nxt) {
+              do { r++; nxt = A.in.off[r + 1]; } while (e + k >= nxt);
+              open = full == 0ull || (A.vis[r] & full) != full;
+            }
+            rows[k] = r;
+            need[k] = e + k < A.in.m && open;
+          }
+          unsigned long long x[4];
+#pragma unroll
+          for (int k = 0; k < 4; k++) x[k] = need[k] ? A.vis[u[k]] : 0ull;
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            if (rows[k] != row) {
+              radii_flush(A, row, part);
+              part = 0ull;
+              row = rows[k];
+            }
+            part |= x[k];
+          }
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const unsigned long long p = __shfl_up_sync(kAll, part, o);
+          const uint32_t tr = __shfl_up_sync(kAll, row, o);
+          if (lane >= o && tr == row) part |= p;
+        }
+        const uint32_t next_row = __shfl_down_sync(kAll, row, 1);
+        if (row != kNone && (lane == 31 || next_row != row)) radii_flush(A, row, part);
+      }
+      if (!grid.sync()) return;
+      for (uint32_t w = warp; w < nwords; w += nwarps) {
+        const uint32_t x = A.bits[w];
+        if (!x) continue;
+        const uint32_t v = min(w * 32 + lane, n - 1);
+        const bool in = (x >> lane) & 1u;
+        if (in) {
+          A.radii[v] = round;
+          A.vis[v] = A.nvis[v];
+        }
+        if (lane == 0) A.bits[w] = 0u;
+        ap.add(in, v, A.out.off[v], A.out.off[v + 1], nq, ns, 0, 0);
+      }
+      ap.finish(nq, ns, 0, 0);
+      if (!grid.sync(ns)) return;
+    } else {
+      expand(A.out, A.q[cq], 0, c.ns, 0, c.nl, [&](const bool (&in)[4], uint32_t s, const uint32_t (&d)[4]) {
+        unsigned long long vd[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) vd[k] = in[k] ? A.vis[d[k]] : ~0ull;
+        const unsigned long long ms = A.vis[s];
+        bool won[4];
+        uint32_t b[4] = {}, e[4] = {};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const unsigned long long w = ms & ~vd[k];
+          won[k] = w != 0ull;
+          if (w) {
+            atomicOr(A.nvis + d[k], w);
+            won[k] = A.radii[d[k]] != round;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          if (won[k]) {
+            b[k] = A.out.off[d[k]];
+            e[k] = A.out.off[d[k] + 1];
+            won[k] = atomicExch(A.radii + d[k], round) != round;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) ap.add(won[k], d[k], b[k], e[k], nq, ns, 0, 0);
+      });
+      ap.finish(nq, ns, 0, 0);
+      if (!grid.sync(ns)) return;
+      const Slot nx = sh.slot;
+      for (uint32_t i = tid; i < nx.ns; i += nthreads) {
+        const uint32_t v = nq.small[i].x;
+        A.vis[v] = A.nvis[v];
+      }
+      for (uint32_t i = tid; i < nx.nl; i += nthreads) {
+        const uint4 it = nq.large[i];
+        if (it.w & 1u) A.vis[it.x] = A.nvis[it.x];
+      }
+      if (!grid.sync()) return;
+    }
+    cq ^= 1;
+  }
+  if (A.radii_out) {
+    for (uint32_t i = tid; i < n; i += nthreads) A.radii_out[i] = A.radii[A.new_ids ? A.new_ids[i] : i];
+  }
+  if (tid == 0) {
+    A.info[0] = (uint64_t)round;
+    A.info[1] = edges;
+    __threadfence_system();
+    A.info[3] = 1;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// PageRank (PageRank.C:120-189), the exact-sum pull of pagerank.cu
+// ---------------------------------------------------------------------------
+struct PrArgs {
+  DevGraph in;
+  const uint32_t* out_off;
+  const uint32_t* chunk_v;
+  const uint32_t* new_ids;
+  uint32_t* lane_row;    // the row of every lane's first edge
+  U128 *opens, *closes;  // per warp step: the piece of the row that goes on past it, and of the one that began before it
+  double* p;
+  double* contrib[2];  // read by even and by odd iterations
+  unsigned long long* rmag;
+  double* ranks_out;  // original-id order; null: not wanted (or not sorted)
+  L1Sum* l1;          // per iteration
+  uint32_t row_weight;  // a row counts as this many edges when rows are shared out
+  int64_t max_iters;
+  double p0, added;
+  Ctl* ctl;
+  volatile uint64_t* info;  // mapped: iterations run, last L1 (2 words), done, broke
+};
+
+constexpr uint32_t kPrStep = 128;  // edges per warp step, four per lane
+
+// PR_Vertex_F, the L1 term and the next contribution of one vertex.
+__device__ __forceinline__ void pr_vertex(const PrArgs& A, uint32_t v, const U128& sum, uint32_t deg, double* next,
+                                          U128& l1) {
+  const bool has = (sum.lo | sum.hi) != 0ull;
+  const double pn = has ? fma(kPrDamp, fx_to_double(sum), A.added) : A.added;
+  const double po = A.p[v];
+  if (bits_of(po) != bits_of(pn)) add128(l1, fx_from_double(fabs(po - pn)));
+  A.p[v] = pn;
+  // p'/deg by degree class (pr_quotient's; the reciprocals are written by this
+  // kernel, so they are read as plain memory)
+  if (deg == 0) next[v] = 0.0;
+  else if ((deg & (deg - 1)) == 0) next[v] = double_of(bits_of(pn) - ((unsigned long long)(31 - __clz(deg)) << 52));
+  else next[v] = div_by_magic(pn, deg, A.rmag[v]);
+}
+
+// One warp step: edges [s0, s0 + kPrStep) that lie in [elo, ehi), the edges of
+// the CTA's rows.  pr_pull_sweep's step with four edges per lane (a small graph
+// has few steps, so short ones keep more warps busy) and the row of a lane's
+// first edge read instead of searched for.  A row inside the step is stored to
+// acc; a row that it shares with other steps leaves its piece in opens (it
+// begins here) or closes (it began before), which the row's thread adds up.
+__device__ __forceinline__ void pr_step(const PrArgs& A, const double* c, uint32_t s0, uint32_t elo, uint32_t ehi,
+                                        const uint32_t* rows, U128* acc, uint32_t lo, U128* opens, U128* closes) {
+  const int lane = threadIdx.x & 31;
+  const DevGraph& g = A.in;
+  const uint32_t e = s0 + lane * 4, begin = max(s0, elo);
+  uint32_t row = kNone, head_row = kNone;
+  U128 part{0ull, 0ull}, head{0ull, 0ull};
+  bool cont = false;
+  if (e < ehi && e + 4 > elo) {
+    const uint4 w = __ldg(reinterpret_cast<const uint4*>(g.adj + e));  // adj is padded past m
+    uint32_t v = rows[lane];
+    const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+    double x[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) x[j] = e + j >= elo && e + j < ehi ? c[u[j]] : 0.0;
+    uint32_t nxt = g.off[v + 1];
+    const bool before = g.off[v] < e;
+    row = v;
+    bool at_first = true;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t ee = e + j;
+      if (ee < elo || ee >= ehi) continue;
+      if (ee >= nxt) {
+        if (at_first && before) {
+          head = part;
+          head_row = row;
+        } else {
+          acc[row - lo] = part;
+        }
+        at_first = false;
+        part = U128{0ull, 0ull};
+        do { v++; nxt = g.off[v + 1]; } while (ee >= nxt);
+        row = v;
+      }
+      add128(part, fx_from_double(x[j]));
+    }
+    cont = nxt > e + 4;
+  }
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const U128 y = shfl_up128(part, o);
+    const uint32_t tr = __shfl_up_sync(kAll, row, o);
+    if (lane >= o && tr == row) add128(part, y);
+  }
+  const U128 prev = shfl_up128(part, 1);
+  const uint32_t prev_row = __shfl_up_sync(kAll, row, 1);
+  if (head_row != kNone) {
+    if (lane > 0 && prev_row == head_row) add128(head, prev);
+    if (g.off[head_row] >= begin) acc[head_row - lo] = head;
+    else *closes = head;
+  }
+  if (row != kNone && (!cont || lane == 31)) {
+    const bool here = g.off[row] >= begin;
+    if (!here) *closes = part;
+    else if (cont) *opens = part;
+    else acc[row - lo] = part;
+  }
+}
+
+// Each CTA owns a run of rows of about the same number of edges and rows and
+// keeps their sums in shared memory, so an iteration is one pass over its
+// edges, one over its rows and one grid barrier: contributions are read from
+// one array and written to the other.  The sums are exact (pr_exact.cuh).
+__global__ void __launch_bounds__(kFT, 1) pagerank_fused(const __grid_constant__ PrArgs A) {
+  __shared__ Shared sh;
+  __shared__ uint32_t s_range[2];
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  U128* acc = reinterpret_cast<U128*>(smem_raw);
+  Grid grid;
+  begin(grid, &sh, A.ctl);
+  const uint32_t n = A.in.n, m = A.in.m;
+  const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x < 2) {  // first row whose edges and rows before reach this CTA's (and the next one's) share
+    const uint64_t want = ((uint64_t)m + (uint64_t)n * A.row_weight) * (blockIdx.x + threadIdx.x) / gridDim.x;
+    uint32_t lo = 0, hi = n;
+    while (lo < hi) {
+      const uint32_t mid = lo + (hi - lo) / 2;
+      if (A.in.off[mid] + (uint64_t)mid * A.row_weight >= want) hi = mid;
+      else lo = mid + 1;
+    }
+    s_range[threadIdx.x] = lo;
+  }
+  __syncthreads();
+  const uint32_t lo = s_range[0], hi = s_range[1];
+  const uint32_t elo = A.in.off[lo], ehi = A.in.off[hi], base = elo & ~3u;
+  const uint32_t steps = ehi > elo ? (ehi - base + kPrStep - 1) / kPrStep : 0;
+  // the CTA's part of the per-lane and per-step arrays: CTAs share at most one
+  // group of four edges, so shifting each by one keeps them apart
+  uint32_t* rows = A.lane_row + (base / 4 + blockIdx.x * 32);
+  U128* opens = A.opens + (base / kPrStep + 2 * blockIdx.x);
+  U128* closes = A.closes + (base / kPrStep + 2 * blockIdx.x);
+  for (uint32_t v = lo + threadIdx.x; v < hi; v += kFT) {
+    A.p[v] = A.p0;
+    const uint32_t d = A.out_off[v + 1] - A.out_off[v];
+    const unsigned long long R = (d & (d - 1)) ? recip_magic(d) : 0ull;
+    A.contrib[0][v] = deg_quotient(A.p0, d, R);
+    A.rmag[v] = R;
+  }
+  for (uint32_t i = threadIdx.x; i < steps * 32; i += kFT) {
+    const uint32_t e = max(base + i * 4, elo);
+    if (e < ehi) {
+      const uint32_t ch = e / kSweepChunk;
+      rows[i] = upper_index(A.in.off, A.chunk_v[ch], A.chunk_v[ch + 1], e);
+    }
+  }
+  for (int64_t i = tid; i < A.max_iters; i += nthreads) A.l1[i] = L1Sum{};
+  if (!grid.sync()) return;
+  const U128 eps = pr_eps_fx();
+  U128 last{0ull, 0ull};
+  int64_t it = 0;
+  bool broke = false;
+  while (it < A.max_iters && !broke) {
+    const double* c = A.contrib[it & 1];
+    double* next = A.contrib[(it & 1) ^ 1];
+    for (uint32_t t = warp; t < steps; t += kFWarps) {
+      pr_step(A, c, base + t * kPrStep, elo, ehi, rows + t * 32, acc, lo, opens + t, closes + t);
+    }
+    __syncthreads();
+    U128 local{0ull, 0ull};
+    for (uint32_t v0 = lo + warp * 32; v0 < hi; v0 += kFT) {
+      const uint32_t v = v0 + lane;
+      U128 sum{0ull, 0ull};
+      uint32_t first = 0, end = 0;  // steps whose `closes` hold pieces of the row
+      if (v < hi) {
+        const uint32_t b = A.in.off[v], e = A.in.off[v + 1];
+        if (e > b) {
+          const uint32_t s1 = (b - base) / kPrStep, s2 = (e - 1 - base) / kPrStep;
+          sum = s1 == s2 ? acc[v - lo] : opens[s1];
+          first = s1 + 1;
+          end = s2 + 1;
+        }
+      }
+      unsigned many = __ballot_sync(kAll, end > first + 8);  // long rows: the warp adds their pieces together
+      while (many) {
+        const int j = __ffs(many) - 1;
+        many &= many - 1;
+        const uint32_t jf = __shfl_sync(kAll, first, j), je = __shfl_sync(kAll, end, j);
+        U128 s{0ull, 0ull};
+        for (uint32_t k = jf + lane; k < je; k += 32) add128(s, closes[k]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          add128(s, U128{__shfl_xor_sync(kAll, s.lo, o), __shfl_xor_sync(kAll, s.hi, o)});
+        }
+        if (lane == j) {
+          add128(sum, s);
+          first = end;
+        }
+      }
+      for (; first < end; first++) add128(sum, closes[first]);
+      if (v < hi) pr_vertex(A, v, sum, A.out_off[v + 1] - A.out_off[v], next, local);
+    }
+    const U128 t = block_sum128(local);
+    if (threadIdx.x == 0 && (t.lo | t.hi)) A.l1[it].add(t);
+    if (!grid.sync(nullptr, A.l1 + it)) return;
+    last = sh.l1;
+    broke = less128(last, eps);
+    it++;
+  }
+  if (A.ranks_out) {
+    for (uint32_t i = tid; i < n; i += nthreads) A.ranks_out[i] = A.p[A.new_ids ? A.new_ids[i] : i];
+  }
+  if (tid == 0) {
+    A.info[0] = (uint64_t)it;
+    A.info[1] = last.lo;
+    A.info[2] = last.hi;
+    A.info[4] = broke ? 1 : 0;
+    __threadfence_system();
+    A.info[3] = 1;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------
+// The largest in-degree of g (found once per graph); n if it cannot be found.
+__global__ void find_max_degree(const uint32_t* __restrict__ off, uint32_t n, unsigned int* out) {
+  unsigned int mx = 0;
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+    mx = max(mx, off[v + 1] - off[v]);
+  }
+  mx = __reduce_max_sync(kAll, mx);
+  if ((threadIdx.x & 31) == 0) atomicMax(out, mx);
+}
+
+int64_t max_in_degree(const rg_graph* g, cudaStream_t st) {
+  if (!g->directed) return g->max_deg;
+  int64_t v = g->max_in_deg.load(std::memory_order_relaxed);
+  if (v >= 0) return v;
+  unsigned int* d = reinterpret_cast<unsigned int*>(ctx().ws.counters.as<uint64_t>() + 8);  // a free scratch word
+  uint32_t h = 0;
+  cudaError_t e = cudaMemsetAsync(d, 0, 4, st);
+  if (e == cudaSuccess) {
+    find_max_degree<<<64, 256, 0, st>>>(g->in_view().off, (uint32_t)g->n, d);
+    e = cudaGetLastError();
+  }
+  if (e != cudaSuccess || read_small(d, &h, 4, st) != RG_OK) {
+    cudaGetLastError();
+    return g->n;  // too large a row for the one-launch path
+  }
+  g->max_in_deg.store(h, std::memory_order_relaxed);
+  return h;
+}
+
+struct FusedState {
+  DevBuf ctl, bits0, bits1, i32a, i32b, f64a, f64b, f64c, u64a, u64b, row, opens, closes, l1, out;
+  DevBuf qs0, qs1, ql0, ql1, first_s, first_l;
+};
+thread_local FusedState S;
+
+int fused_grid(int64_t work, int64_t per_cta) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(device_sms(), work / per_cta));
+}
+
+template <class K, class Args>
+rg_status launch_fused(K kern, const Args& args, int grid, size_t dyn, size_t most_dyn, cudaStream_t st) {
+  static std::atomic<uint64_t> checked{0};
+  RG_TRY(once_per_device(checked, [&]() -> rg_status {
+    // one CTA per SM must fit, with all the dynamic shared memory it may ask for
+    if (most_dyn) {
+      static std::atomic<uint64_t> limit_set{0};
+      RG_TRY(allow_max_dyn_smem(limit_set, kern));
+    }
+    int per_sm = 0;
+    RG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFT, most_dyn));
+    return per_sm > 0 ? RG_OK : fail(RG_ECUDA, "one-launch traversal does not fit an SM");
+  }));
+  RG_CUDA(cudaMemsetAsync(args.ctl, 0, sizeof(Ctl), st));
+  void* p[] = {const_cast<Args*>(&args)};
+  kt_begin(st);
+  RG_CUDA(cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(kFT), p, dyn, st));
+  kt_end(st);
+  g_timing.kernel_launches++;
+  g_timing.edge_launches++;
+  return RG_OK;
+}
+
+rg_status queue_pair(int64_t n, int64_t m, DevBuf& s, DevBuf& l, Queues* q) {
+  RG_TRY(s.reserve(16 * (size_t)(n + 32)));
+  // pieces: one per started kPiece edges of every vertex above kSmallDeg
+  RG_TRY(l.reserve(16 * (size_t)(std::min<int64_t>(n, m / (kSmallDeg + 1)) + m / kPiece + 64)));
+  *q = Queues{s.as<uint4>(), l.as<uint4>()};
+  return RG_OK;
+}
+
+int64_t dense_threshold(const rg_graph* g) { return g->m / std::max<int64_t>(g_opts.dense_div, 1); }
+
+// The results of a finished launch on their way to the caller: `dev_out`
+// (device, original ids) and `host_out`.  `internal` holds them by internal
+// id, `ordered` (when the launch wrote it) by original id.
+template <class T>
+rg_status deliver(rg_graph* g, const T* internal, const T* ordered, T* host_out, T* dev_out, cudaStream_t st) {
+  const T* src = ordered ? ordered : internal;
+  if (dev_out && dev_out != src) RG_CUDA(cudaMemcpyAsync(dev_out, src, sizeof(T) * g->n, cudaMemcpyDeviceToDevice, st));
+  if (!host_out) return RG_OK;
+  if (g_opts.async_results) {
+    return download_async<T>(host_out, g->n, st, [&](T* stage) -> rg_status {
+      RG_CUDA(cudaMemcpyAsync(stage, src, sizeof(T) * g->n, cudaMemcpyDeviceToDevice, st));
+      return RG_OK;
+    });
+  }
+  RG_CUDA(cudaMemcpyAsync(host_out, src, sizeof(T) * g->n, cudaMemcpyDeviceToHost, st));
+  return RG_OK;
+}
+
+}  // namespace
+
+bool fused_fits(const rg_graph* g, int64_t max_edges) {
+  return g->m <= max_edges && g->n <= max_edges && !g_trace_on;
+}
+
+rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t* h_depth,
+                        int64_t* rounds_out, int64_t* reached_out, int32_t* d_depth_out, bool* done) {
+  Ctx& cx = ctx();
+  cudaStream_t st = cx.stream;
+  const int64_t n = g->n, m = g->m, nwords = (n + 31) / 32;
+  BfsArgs A;
+  RG_TRY(S.ctl.reserve(sizeof(Ctl)));
+  RG_TRY(S.bits0.reserve(4 * nwords));
+  RG_TRY(S.bits1.reserve(4 * nwords));
+  RG_TRY(S.i32a.reserve(4 * n));
+  if (h_parents) RG_TRY(S.i32b.reserve(4 * n));
+  RG_TRY(queue_pair(n, m, S.qs0, S.ql0, &A.q[0]));
+  RG_TRY(queue_pair(n, m, S.qs1, S.ql1, &A.q[1]));
+  const bool order = g->sorted && (h_depth || d_depth_out);
+  if (order && !d_depth_out) RG_TRY(S.out.reserve(4 * n));
+  A.out = g->view();
+  A.in = g->in_view();
+  A.new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
+  A.root = root;
+  A.threshold = dense_threshold(g);
+  A.vis[0] = S.bits0.as<uint32_t>();
+  A.vis[1] = S.bits1.as<uint32_t>();
+  A.depth = S.i32a.as<int32_t>();
+  A.parents = h_parents ? S.i32b.as<uint32_t>() : nullptr;
+  A.depth_out = order ? (d_depth_out ? d_depth_out : S.out.as<int32_t>()) : nullptr;
+  A.ctl = S.ctl.as<Ctl>();
+  A.info = cx.ws.h_info_dev;
+  volatile uint64_t* info = cx.ws.h_info;
+  info[3] = 0;
+  CallTimer timer(g);
+  RG_TRY(launch_fused(bfs_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
+  RG_TRY(timer.mark());
+  RG_TRY(deliver<int32_t>(g, A.depth, A.depth_out, h_depth, d_depth_out, st));
+  DevBuf tmp(true, st);  // parents by original id
+  RG_TRY(download_orig<uint32_t>(g, A.parents, h_parents, tmp, st));
+  RG_CUDA(cudaStreamSynchronize(st));
+  RG_TRY(timer.finish());
+  *done = info[3] == 1;
+  if (!*done) return RG_OK;
+  g_timing.edges_traversed = (int64_t)info[2];
+  g_timing.algorithmic_bytes =
+      4 * g_timing.edges_traversed + 4 * (n + 1) + 4 * n + 2 * ((n + 7) / 8) * (int64_t)info[0];
+  if (rounds_out) *rounds_out = (int64_t)info[0];
+  if (reached_out) *reached_out = (int64_t)info[1];
+  return RG_OK;
+}
+
+rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* h_deps, int64_t* levels_out,
+                       double* d_deps_out, bool* done) {
+  Ctx& cx = ctx();
+  cudaStream_t st = cx.stream;
+  const int64_t n = g->n, m = g->m;
+  BcArgs A;
+  RG_TRY(S.ctl.reserve(sizeof(Ctl)));
+  RG_TRY(S.i32a.reserve(4 * n));
+  RG_TRY(S.f64a.reserve(8 * n));
+  RG_TRY(S.f64b.reserve(8 * n));
+  RG_TRY(queue_pair(n, m, S.qs0, S.ql0, &A.q));
+  RG_TRY(S.first_s.reserve(4 * (n + 2)));
+  RG_TRY(S.first_l.reserve(4 * (n + 2)));
+  const bool order = g->sorted && (h_deps || d_deps_out);
+  if (order && !d_deps_out) RG_TRY(S.f64c.reserve(8 * n));
+  A.new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
+  A.lvl = S.i32a.as<int32_t>();
+  A.sigma = S.f64a.as<double>();
+  A.deps = S.f64b.as<double>();
+  A.first_small = S.first_s.as<uint32_t>();
+  A.first_large = S.first_l.as<uint32_t>();
+  A.ctl = S.ctl.as<Ctl>();
+  A.info = cx.ws.h_info_dev;
+  volatile uint64_t* info = cx.ws.h_info;
+  info[0] = info[1] = info[3] = 0;
+  CallTimer timer(g);
+  double* ordered = order ? (d_deps_out ? d_deps_out : S.f64c.as<double>()) : nullptr;
+  for (int it = 0; it < nsrc; it++) {
+    // the reference transposes a directed graph after every source
+    A.g = it % 2 == 1 ? g->in_view() : g->view();
+    A.source = src_orig[it];
+    A.first_source = it == 0;
+    A.deps_out = it == nsrc - 1 ? ordered : nullptr;
+    RG_TRY(launch_fused(bc_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
+  }
+  RG_TRY(timer.mark());
+  RG_TRY(deliver<double>(g, A.deps, ordered, h_deps, d_deps_out, st));
+  RG_CUDA(cudaStreamSynchronize(st));
+  RG_TRY(timer.finish());
+  *done = info[3] == (uint64_t)nsrc;
+  if (!*done) return RG_OK;
+  g_timing.edges_traversed = (int64_t)info[1];
+  g_timing.algorithmic_bytes =
+      4 * g_timing.edges_traversed + (int64_t)nsrc * (8 * (n + 1) + 8 * n + n + 16 * n + 8 * n);
+  if (levels_out) *levels_out = (int64_t)info[0];
+  return RG_OK;
+}
+
+rg_status radii_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int k,
+                          int32_t* h_radii, int64_t* rounds_out, int32_t* d_radii_out, bool* done) {
+  Ctx& cx = ctx();
+  cudaStream_t st = cx.stream;
+  const int64_t n = g->n, m = g->m;
+  RadiiArgs A;
+  RG_TRY(S.ctl.reserve(sizeof(Ctl)));
+  RG_TRY(S.bits0.reserve(4 * ((n + 31) / 32)));
+  RG_TRY(S.u64a.reserve(8 * n));
+  RG_TRY(S.u64b.reserve(8 * n));
+  RG_TRY(S.i32a.reserve(4 * n));
+  RG_TRY(queue_pair(n, m, S.qs0, S.ql0, &A.q[0]));
+  RG_TRY(queue_pair(n, m, S.qs1, S.ql1, &A.q[1]));
+  const bool order = g->sorted && (h_radii || d_radii_out);
+  if (order && !d_radii_out) RG_TRY(S.out.reserve(4 * n));
+  A.out = g->view();
+  A.in = g->in_view();
+  A.chunk_v = g->in_chunks();
+  A.nchunks = (uint32_t)g->nchunks;
+  A.new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
+  A.k = k;
+  for (int i = 0; i < k; i++) {
+    A.seed[i] = seeds[i];
+    A.mask[i] = masks[i];
+  }
+  A.threshold = dense_threshold(g);
+  A.vis = S.u64a.as<unsigned long long>();
+  A.nvis = S.u64b.as<unsigned long long>();
+  A.radii = S.i32a.as<int32_t>();
+  A.radii_out = order ? (d_radii_out ? d_radii_out : S.out.as<int32_t>()) : nullptr;
+  A.bits = S.bits0.as<uint32_t>();
+  A.ctl = S.ctl.as<Ctl>();
+  A.info = cx.ws.h_info_dev;
+  volatile uint64_t* info = cx.ws.h_info;
+  info[3] = 0;
+  CallTimer timer(g);
+  RG_TRY(launch_fused(radii_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
+  RG_TRY(timer.mark());
+  RG_TRY(deliver<int32_t>(g, A.radii, A.radii_out, h_radii, d_radii_out, st));
+  RG_CUDA(cudaStreamSynchronize(st));
+  RG_TRY(timer.finish());
+  *done = info[3] == 1;
+  if (!*done) return RG_OK;
+  g_timing.edges_traversed = (int64_t)info[1];
+  g_timing.algorithmic_bytes = 4 * g_timing.edges_traversed + 16 * n + 4 * n;
+  if (rounds_out) *rounds_out = (int64_t)info[0];
+  return RG_OK;
+}
+
+rg_status pagerank_fused_run(rg_graph* g, int64_t max_iters, double* h_ranks, int64_t* iters_out, double* l1_out,
+                             bool* done) {
+  Ctx& cx = ctx();
+  cudaStream_t st = cx.stream;
+  const int64_t n = g->n, m = g->m;
+  PrArgs A;
+  const int grid = fused_grid(m + n, kFusedPrEdgesPerCta);
+  // a row counts as `weight` edges: as few as keep a CTA's rows in its shared
+  // memory (share / weight of them at most).  `share`: the edges of a CTA, but
+  // for its last row
+  const int64_t room = kFusedPrRows - 4 - n / grid;
+  if (room <= 0) return RG_OK;
+  const int64_t weight = m / grid / room + 1;
+  const int64_t share = (m + weight * n + grid - 1) / grid;
+  const int64_t rows = std::min<int64_t>(n, share / weight + 2);
+  A.row_weight = (uint32_t)weight;
+  // a row is not shared between CTAs: one with far more edges than a CTA's
+  // share would hold the others up
+  if (rows > kFusedPrRows || max_in_degree(g, st) > 2 * share) return RG_OK;
+  RG_TRY(S.ctl.reserve(sizeof(Ctl)));
+  RG_TRY(S.row.reserve(4 * (size_t)(m / 4 + 32 * (grid + 2) + 64)));
+  RG_TRY(S.opens.reserve(sizeof(U128) * (size_t)(m / kPrStep + 2 * grid + 4)));
+  RG_TRY(S.closes.reserve(sizeof(U128) * (size_t)(m / kPrStep + 2 * grid + 4)));
+  RG_TRY(S.f64a.reserve(8 * n));
+  RG_TRY(S.f64b.reserve(8 * n));
+  RG_TRY(S.u64b.reserve(8 * n));
+  RG_TRY(S.u64a.reserve(8 * n));
+  RG_TRY(S.l1.reserve(sizeof(L1Sum) * std::max<int64_t>(max_iters, 1)));
+  const bool order = g->sorted && h_ranks;
+  if (order) RG_TRY(S.f64c.reserve(8 * n));
+  A.in = g->in_view();
+  A.out_off = g->off.as<uint32_t>();
+  A.chunk_v = g->in_chunks();
+  A.new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
+  A.lane_row = S.row.as<uint32_t>();
+  A.opens = S.opens.as<U128>();
+  A.closes = S.closes.as<U128>();
+  A.p = S.f64a.as<double>();
+  A.contrib[0] = S.f64b.as<double>();
+  A.contrib[1] = S.u64b.as<double>();
+  A.rmag = S.u64a.as<unsigned long long>();
+  A.ranks_out = order ? S.f64c.as<double>() : nullptr;
+  A.l1 = S.l1.as<L1Sum>();
+  A.max_iters = max_iters;
+  A.p0 = 1 / (double)n;
+  A.added = (1 - kPrDamp) * (1 / (double)n);
+  A.ctl = S.ctl.as<Ctl>();
+  A.info = cx.ws.h_info_dev;
+  volatile uint64_t* info = cx.ws.h_info;
+  info[3] = 0;
+  CallTimer timer(g);
+  RG_TRY(launch_fused(pagerank_fused, A, grid, sizeof(U128) * (size_t)rows, sizeof(U128) * kFusedPrRows, st));
+  RG_TRY(timer.mark());
+  RG_TRY(deliver<double>(g, A.p, A.ranks_out, h_ranks, nullptr, st));
+  RG_CUDA(cudaStreamSynchronize(st));
+  RG_TRY(timer.finish());
+  *done = info[3] == 1;
+  if (!*done) return RG_OK;
+  const int64_t run = (int64_t)info[0];
+  const bool broke = info[4] != 0;
+  g_timing.edge_launches = run;
+  g_timing.edges_traversed = m * run;
+  g_timing.algorithmic_bytes = (4 * m + 4 * (n + 1) + 16 * n) * run;
+  if (iters_out) *iters_out = broke ? run : max_iters + 1;
+  if (l1_out) *l1_out = max_iters ? fx_to_double(U128{info[1], info[2]}) : 0.0;
+  return RG_OK;
+}
+
+}  // namespace rg

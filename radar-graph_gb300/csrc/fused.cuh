@@ -1,0 +1,104 @@
+// Whole traversals in one launch (fused.cu), and the PageRank device helpers
+// that its kernels share with the sweeps of pagerank.cu.
+#pragma once
+
+#include "app_common.cuh"
+#include "pr_exact.cuh"
+
+namespace rg {
+
+// A CTA of a one-launch traversal is given at least this many edges (and
+// vertices): 2048 and 8192 measured within 3 % at 2^14 vertices and 10-20 %
+// apart at 2^10, the smaller the better for BC and Radii, the same for BFS.
+constexpr int64_t kFusedEdgesPerCta = 4096;
+
+// The one-launch PageRank is a chain of dependent loads per step, so smaller
+// CTAs pay for longer (2^14 vertices, 4.4e5 edges, 20 iterations: 236 us a
+// call with 8192 edges per CTA, 189 with 4096, 153 with 2048, 148 with 1024).
+constexpr int64_t kFusedPrEdgesPerCta = 1024;
+
+// Rows of a CTA of the one-launch PageRank (16 bytes of shared memory each).
+constexpr int64_t kFusedPrRows = 12000;
+
+// Largest graphs (edges, and vertices) that take the one-launch path, by app.
+// Device time against the level-by-level run, R-MAT edge factor 16, degree
+// sorted (in brackets: uniform, unsorted), us:
+//   BFS       2^10 vertices 31 / 182, 2^16 46 / 298, 2^20 95 / 415 (167 / 402),
+//             2^24 560 / 973 (1823 / 2972): every size
+//   BC        2^10 54 / 250, 2^18 204 / 527 (302 / 496), 2^20 576 / 720
+//             (934 / 855), 2^22 1928 / 1569: the line lies between 8e6 and 3.3e7
+//             edges, where the larger grids of the sweeps win
+//   Radii     2^10 71 / 309, 2^18 303 / 584 (340 / 517), 2^20 790 / 792
+//             (1015 / 953): the same line
+//   PageRank  20 iterations: 2^10 97 / 217, 2^16 304 / 481 (183 / 220), 2^17
+//             546 / 648 (298 / 342), 2^18 1337 / 1033 (573 / 532): 4e6 edges
+constexpr int64_t kFusedBfsEdges = INT64_MAX;
+constexpr int64_t kFusedBcEdges = 3 << 23;
+constexpr int64_t kFusedRadiiEdges = 3 << 23;
+constexpr int64_t kFusedPagerankEdges = 5 << 20;
+
+// Whether a call on g may take the one-launch path: small enough, and no
+// per-level records (rg_set_trace) are asked for.
+bool fused_fits(const rg_graph* g, int64_t max_edges);
+
+// Each sets *done when the launch answered the call; otherwise (its bounded
+// waits ran out) the caller answers level by level.
+rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t* h_depth,
+                        int64_t* rounds_out, int64_t* reached_out, int32_t* d_depth_out, bool* done);
+rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* h_deps, int64_t* levels_out,
+                       double* d_deps_out, bool* done);
+// seeds: original ids, each once, with its mask
+rg_status radii_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int k,
+                          int32_t* h_radii, int64_t* rounds_out, int32_t* d_radii_out, bool* done);
+rg_status pagerank_fused_run(rg_graph* g, int64_t max_iters, double* h_ranks, int64_t* iters_out, double* l1_out,
+                             bool* done);
+
+constexpr double kPrDamp = 0.85;  // PageRank.C:126
+
+// acc[v] += x for a 128-bit sum shared with other warps: the low word's
+// atomic returns the old value, so the carry out of it is known and goes into
+// the high word.  Every carry is counted once, so the final sum is exact.
+__device__ __forceinline__ void atomic_add128(U128* p, const U128& x) {
+  const unsigned long long old = atomicAdd(&p->lo, x.lo);
+  const unsigned long long hi = x.hi + (old + x.lo < old ? 1ull : 0ull);
+  if (hi) atomicAdd(&p->hi, hi);
+}
+
+__device__ __forceinline__ void store128(U128* p, const U128& x) {
+  asm volatile("st.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(x.lo), "l"(x.hi) : "memory");
+}
+
+__device__ __forceinline__ U128 shfl_up128(const U128& x, int o) {
+  return U128{__shfl_up_sync(0xffffffffu, x.lo, o), __shfl_up_sync(0xffffffffu, x.hi, o)};
+}
+
+__device__ __forceinline__ U128 block_sum128(U128 v) {
+  __shared__ U128 ws[32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    add128(v, U128{__shfl_xor_sync(0xffffffffu, v.lo, o), __shfl_xor_sync(0xffffffffu, v.hi, o)});
+  }
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+  __syncthreads();
+  U128 t{0ull, 0ull};
+  if (threadIdx.x < 32) {
+    if (threadIdx.x < (blockDim.x >> 5)) t = ws[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      add128(t, U128{__shfl_xor_sync(0xffffffffu, t.lo, o), __shfl_xor_sync(0xffffffffu, t.hi, o)});
+    }
+  }
+  return t;  // valid in thread 0
+}
+
+// p'/deg, the IEEE quotient of PR_F (PageRank.C:48), by degree class (the
+// deg_quotient classes): the integer reciprocal is read only for degrees
+// that need it, and degree-sorted graphs keep whole warps in one class.
+__device__ __forceinline__ double pr_quotient(double pn, uint32_t d, const unsigned long long* __restrict__ rmag,
+                                              int64_t v) {
+  if (d == 0) return 0.0;
+  if ((d & (d - 1)) == 0) return double_of(bits_of(pn) - ((unsigned long long)(31 - __clz(d)) << 52));
+  return div_by_magic(pn, d, rmag[v]);
+}
+
+}  // namespace rg

@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "app_common.cuh"
+#include "fused.cuh"
 #include "pr_exact.cuh"
 
 namespace rg {
@@ -39,58 +40,11 @@ namespace {
 
 constexpr int kSweepThreads = 1024;  // push sweep CTA (one per SM with hub copies)
 constexpr int kPullThreads = 256;
-constexpr double kDamp = 0.85;       // PageRank.C:126
 constexpr uint32_t kNoRow = 0xFFFFFFFFu;
 
 // L1 of the previous iteration (exact) below 1e-7: this iteration is skipped.
 __device__ __forceinline__ bool converged(const U128* l1_prev) {
   return l1_prev != nullptr && less128(*l1_prev, pr_eps_fx());
-}
-
-// acc[v] += x for a 128-bit sum shared with other warps: the low word's
-// atomic returns the old value, so the carry out of it is known and goes into
-// the high word.  Every carry is counted once, so the final sum is exact.
-__device__ __forceinline__ void atomic_add128(U128* p, const U128& x) {
-  const unsigned long long old = atomicAdd(&p->lo, x.lo);
-  const unsigned long long hi = x.hi + (old + x.lo < old ? 1ull : 0ull);
-  if (hi) atomicAdd(&p->hi, hi);
-}
-
-__device__ __forceinline__ void store128(U128* p, const U128& x) {
-  asm volatile("st.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(x.lo), "l"(x.hi) : "memory");
-}
-
-__device__ __forceinline__ U128 shfl_up128(const U128& x, int o) {
-  return U128{__shfl_up_sync(0xffffffffu, x.lo, o), __shfl_up_sync(0xffffffffu, x.hi, o)};
-}
-
-__device__ __forceinline__ U128 block_sum128(U128 v) {
-  __shared__ U128 ws[32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    add128(v, U128{__shfl_xor_sync(0xffffffffu, v.lo, o), __shfl_xor_sync(0xffffffffu, v.hi, o)});
-  }
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
-  __syncthreads();
-  U128 t{0ull, 0ull};
-  if (threadIdx.x < 32) {
-    if (threadIdx.x < (blockDim.x >> 5)) t = ws[threadIdx.x];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      add128(t, U128{__shfl_xor_sync(0xffffffffu, t.lo, o), __shfl_xor_sync(0xffffffffu, t.hi, o)});
-    }
-  }
-  return t;  // valid in thread 0
-}
-
-// p'/deg, the IEEE quotient of PR_F (PageRank.C:48), by degree class (the
-// deg_quotient classes): the integer reciprocal is read only for degrees
-// that need it, and degree-sorted graphs keep whole warps in one class.
-__device__ __forceinline__ double pr_quotient(double pn, uint32_t d, const unsigned long long* __restrict__ rmag,
-                                              int64_t v) {
-  if (d == 0) return 0.0;
-  if ((d & (d - 1)) == 0) return double_of(bits_of(pn) - ((unsigned long long)(31 - __clz(d)) << 52));
-  return div_by_magic(pn, d, rmag[v]);
 }
 
 // p = 1/n, contrib = p/deg (PageRank.C:126-138), rmag = the integer
@@ -390,7 +344,7 @@ __global__ void __launch_bounds__(256) pr_finalize(uint32_t n, const uint32_t* _
       accd[v] = 0.0;
     }
     // fma(0.85, 0, added) is `added` exactly: vertices without in-edges skip it
-    const double pn = has ? fma(kDamp, sum, added) : added;
+    const double pn = has ? fma(kPrDamp, sum, added) : added;
     const double po = p[v];
     if (bits_of(po) != bits_of(pn)) add128(local, fx_from_double(fabs(po - pn)));
     p[v] = pn;
@@ -422,6 +376,11 @@ rg_status pagerank_run(rg_graph* g, int variant, int64_t max_iters, double* h_ra
   OptScope opt_scope(g, kAppPagerank);
   Ctx* cx = nullptr;
   RG_TRY(get_ctx(&cx));
+  if (max_iters > 0 && fused_fits(g, kFusedPagerankEdges)) {
+    bool done = false;
+    RG_TRY(pagerank_fused_run(g, max_iters, h_ranks, iters_out, l1_out, &done));
+    if (done) return RG_OK;
+  }
   cudaStream_t st = cx->stream;
   const int64_t n = g->n;
   static thread_local PrState S;
@@ -433,7 +392,7 @@ rg_status pagerank_run(rg_graph* g, int variant, int64_t max_iters, double* h_ra
   RG_TRY(S.out.reserve(8 * n));
   // the reference's constants (PageRank.C:126-138)
   const double p0 = 1 / (double)n;
-  const double added = (1 - kDamp) * (1 / (double)n);
+  const double added = (1 - kPrDamp) * (1 / (double)n);
   // hub set-up (host side, before the timed span).  The full sweeps run one
   // CTA per SM, so their hub copies may use the whole shared memory.
   // hub copies only with a shared-memory budget; the push kernel's hub mode is

@@ -194,6 +194,8 @@ size_t working_bytes(const rg_graph* g, int kind, int k) {
     while (W < k) W *= 2;
     return (size_t)(16 * W + 8 * k + 40) * n;
   }
+  // one BFS: two queues of vertices and of 128-edge pieces (16 bytes each) beside the depths
+  if (k == 1) return 88 * n + (size_t)g->m / 4;
   return (size_t)(8 * k + 40) * n;  // masks, depth rows and their original-order copy, two frontiers
 }
 
