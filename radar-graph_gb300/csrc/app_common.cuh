@@ -152,6 +152,7 @@ rg_status download_async(T* h_out, int64_t count, cudaStream_t st, Fill fill) {
   cudaStream_t cs = nullptr;
   RG_TRY(copy_stream(&cs));
   DevBuf stage(true, cs);
+  stage.on_stream = false;  // filled on `st`
   RG_TRY(stage.reserve(sizeof(T) * (size_t)count));
   RG_TRY(fill(stage.as<T>()));
   cudaEvent_t ev = nullptr;

@@ -19,7 +19,9 @@
 #include <thread>
 #include <vector>
 
+#include "app_common.cuh"
 #include "rg_device.cuh"
+#include "sort.cuh"
 
 namespace rg {
 
@@ -50,7 +52,9 @@ rg_status DevBuf::reserve(size_t b) {
   if (b <= bytes && p) return RG_OK;
   release();
   size_t want = b < 256 ? 256 : b;
-  if (pooled) {  // usable from every stream once the allocating stream has it
+  if (pooled && on_stream) {  // used and released in its stream's order
+    RG_CUDA(cudaMallocAsync(&p, want, free_stream));
+  } else if (pooled) {  // usable from every stream once the allocating stream has it
     RG_CUDA(cudaMallocAsync(&p, want, 0));
     RG_CUDA(cudaStreamSynchronize(0));
   } else {
@@ -773,79 +777,20 @@ extern "C" rg_status rg_graph_download(const rg_graph* g, uint32_t* h_off, uint3
 // ---------------------------------------------------------------------------
 namespace rg {
 
-constexpr int kSortThreads = 256;
-constexpr int kSortSub = 16;  // sub-tiles per block
-constexpr int kSortTile = kSortThreads * kSortSub;
-
-// key[i] = ~deg(id), val[i] = id with ids laid out in DESCENDING order.
-__global__ void sort_init(const uint32_t* __restrict__ off, uint32_t n, uint32_t* key, uint32_t* val) {
+// (~deg(id), id) with ids laid out in DESCENDING order.
+__global__ void sort_init(const uint32_t* __restrict__ off, uint32_t n, uint64_t* __restrict__ key) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
-    uint32_t v = n - 1 - (uint32_t)i;
-    key[i] = ~(off[v + 1] - off[v]);
-    val[i] = v;
+    const uint32_t v = n - 1 - (uint32_t)i;
+    key[i] = ((uint64_t)~(off[v + 1] - off[v]) << 32) | v;
   }
 }
 
-__global__ void sort_hist(const uint32_t* __restrict__ key, int64_t n, int shift, int64_t nblocks,
-                          uint32_t* __restrict__ hist) {
-  __shared__ uint32_t h[256];
-  h[threadIdx.x] = 0;
-  __syncthreads();
-  int64_t base = (int64_t)blockIdx.x * kSortTile;
-  for (int s = 0; s < kSortSub; s++) {
-    int64_t i = base + (int64_t)s * kSortThreads + threadIdx.x;
-    if (i < n) atomicAdd(&h[(key[i] >> shift) & 255u], 1u);
-  }
-  __syncthreads();
-  hist[(int64_t)threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
-}
-
-// Stable scatter: sub-tiles in order, threads in order within a sub-tile.
-__global__ void sort_scatter(const uint32_t* __restrict__ key, const uint32_t* __restrict__ val, int64_t n,
-                             int shift, int64_t nblocks, const uint32_t* __restrict__ hist_scan,
-                             uint32_t* __restrict__ key_out, uint32_t* __restrict__ val_out) {
-  constexpr int kWarps = kSortThreads / 32;
-  __shared__ uint32_t running[256];
-  __shared__ uint32_t wcount[kWarps][257];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  running[threadIdx.x] = hist_scan[(int64_t)threadIdx.x * nblocks + blockIdx.x];
-  int64_t base = (int64_t)blockIdx.x * kSortTile;
-  for (int s = 0; s < kSortSub; s++) {
-    for (int d = threadIdx.x; d < kWarps * 257; d += kSortThreads) (&wcount[0][0])[d] = 0;
-    __syncthreads();
-    int64_t i = base + (int64_t)s * kSortThreads + threadIdx.x;
-    bool valid = i < n;
-    uint32_t k = valid ? key[i] : 0, v = valid ? val[i] : 0;
-    uint32_t digit = valid ? ((k >> shift) & 255u) : 256u;
-    uint32_t peers = __match_any_sync(0xffffffffu, digit);
-    uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-    if (rank == 0) wcount[w][digit] = __popc(peers);
-    __syncthreads();
-    uint32_t pos = 0;
-    if (valid) {
-      pos = running[digit] + rank;
-      for (int ww = 0; ww < w; ww++) pos += wcount[ww][digit];
-    }
-    __syncthreads();
-    {
-      uint32_t t = 0;
-      for (int ww = 0; ww < kWarps; ww++) t += wcount[ww][threadIdx.x];
-      running[threadIdx.x] += t;
-    }
-    if (valid) {
-      key_out[pos] = k;
-      val_out[pos] = v;
-    }
-    __syncthreads();
-  }
-}
-
-__global__ void rank_to_ids(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ off, uint32_t n,
+__global__ void rank_to_ids(const uint64_t* __restrict__ sorted, const uint32_t* __restrict__ off, uint32_t n,
                             uint32_t* __restrict__ new_ids, uint32_t* __restrict__ new_deg) {
   int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r < n) {
-    uint32_t v = sorted_ids[r];
+    const uint32_t v = (uint32_t)sorted[r];
     new_ids[v] = (uint32_t)r;
     new_deg[r] = off[v + 1] - off[v];
   }
@@ -906,11 +851,11 @@ __global__ void __launch_bounds__(256) relabel_sweep(DevGraph g, const uint32_t*
 }  // namespace rg
 
 // in-degree of each rank's vertex (a directed graph's new in-lists)
-__global__ void rank_in_deg(const uint32_t* __restrict__ sorted_ids, const uint32_t* __restrict__ in_off, uint32_t n,
+__global__ void rank_in_deg(const uint64_t* __restrict__ sorted, const uint32_t* __restrict__ in_off, uint32_t n,
                             uint32_t* __restrict__ new_in_deg) {
   int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r < n) {
-    const uint32_t v = sorted_ids[r];
+    const uint32_t v = (uint32_t)sorted[r];
     new_in_deg[r] = in_off[v + 1] - in_off[v];
   }
 }
@@ -927,30 +872,25 @@ static rg_status degree_sort_impl(const rg_graph* g, bool by_out, rg_graph** out
   cudaStream_t st = c->stream;
   Workspace& ws = c->ws;
   // temporaries from the stream-ordered pool, released in order on `st`
-  DevBuf k0{true, st}, v0{true, st}, k1{true, st}, v1{true, st}, hist{true, st}, new_deg{true, st}, bad{true, st};
+  DevBuf k0{true, st}, k1{true, st}, new_deg{true, st}, bad{true, st};
   RG_TRY(bad.reserve(16));
-  RG_CUDA(cudaMemsetAsync(bad.p, 0, 4, st));
-  const int64_t nblocks = (n + kSortTile - 1) / kSortTile;
-  RG_TRY(k0.reserve(4 * n)); RG_TRY(v0.reserve(4 * n));
-  RG_TRY(k1.reserve(4 * n)); RG_TRY(v1.reserve(4 * n));
-  RG_TRY(hist.reserve(4 * (256 * nblocks + 1)));
+  RG_CUDA(cudaMemsetAsync(bad.p, 0, 8, st));
+  RG_TRY(k0.reserve(8 * n));
+  RG_TRY(k1.reserve(8 * n));
   sort_init<<<(unsigned)((n + 255) / 256), 256, 0, st>>>((by_in ? g->in_off : g->off).as<uint32_t>(), (uint32_t)n,
-                                                        k0.as<uint32_t>(), v0.as<uint32_t>());
+                                                        k0.as<uint64_t>());
   // ~deg differs from 0xFFFFFFFF only in the low bits that max_deg spans
   // (in-degrees: all 32 bits, their maximum is not kept)
   int bits = 0;
   while (bits < 32 && (g->max_deg >> bits) != 0) bits++;
   if (by_in) bits = 32;
-  int passes = (bits + 7) / 8;
-  uint32_t *ka = k0.as<uint32_t>(), *va = v0.as<uint32_t>(), *kb = k1.as<uint32_t>(), *vb = v1.as<uint32_t>();
-  for (int p = 0; p < passes; p++) {
-    int shift = 8 * p;
-    sort_hist<<<(unsigned)nblocks, kSortThreads, 0, st>>>(ka, n, shift, nblocks, hist.as<uint32_t>());
-    RG_TRY(scan_u32(ws, hist.as<uint32_t>(), hist.as<uint32_t>(), 256 * nblocks, st));
-    sort_scatter<<<(unsigned)nblocks, kSortThreads, 0, st>>>(ka, va, n, shift, nblocks, hist.as<uint32_t>(), kb,
-                                                             vb);
-    std::swap(ka, kb);
-    std::swap(va, vb);
+  uint64_t *order = k0.as<uint64_t>(), *other = k1.as<uint64_t>();
+  SortScratch sort(st);
+  if (bits > 0) {
+    RG_TRY(sort_begin(sort, n, sort_passes(32, 32 + bits), st));
+    RG_TRY(sort_count(sort, order, n, 32, 32 + bits, st));
+    RG_TRY(sort_run(sort, &order, &other, n, 32, 32 + bits, st));
+    RG_CUDA(cudaMemcpyAsync(bad.as<unsigned int>() + 1, sort_failed(sort), 4, cudaMemcpyDeviceToDevice, st));
   }
   RG_CUDA(cudaGetLastError());
   rg_graph* ng = nullptr;
@@ -963,7 +903,7 @@ static rg_status degree_sort_impl(const rg_graph* g, bool by_out, rg_graph** out
     delete ng;
     return s;
   }
-  rank_to_ids<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(va, g->off.as<uint32_t>(), (uint32_t)n,
+  rank_to_ids<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(order, g->off.as<uint32_t>(), (uint32_t)n,
                                                           ng->new_ids.as<uint32_t>(), new_deg.as<uint32_t>());
   if ((s = scan_u32(ws, new_deg.as<uint32_t>(), ng->off.as<uint32_t>(), n, st)) != RG_OK) {
     delete ng;
@@ -975,7 +915,7 @@ static rg_status degree_sort_impl(const rg_graph* g, bool by_out, rg_graph** out
       delete ng;
       return s;
     }
-    rank_in_deg<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(va, g->in_off.as<uint32_t>(), (uint32_t)n,
+    rank_in_deg<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(order, g->in_off.as<uint32_t>(), (uint32_t)n,
                                                             new_deg.as<uint32_t>());
     if ((s = scan_u32(ws, new_deg.as<uint32_t>(), ng->in_off.as<uint32_t>(), n, st)) != RG_OK) {
       delete ng;
@@ -997,15 +937,19 @@ static rg_status degree_sort_impl(const rg_graph* g, bool by_out, rg_graph** out
   }
   cudaError_t e = cudaMemsetAsync(ng->adj.as<uint32_t>() + m, 0, 32, st);
   if (e == cudaSuccess && g->directed) e = cudaMemsetAsync(ng->in_adj.as<uint32_t>() + m, 0, 32, st);
-  unsigned int h_bad = 0;
+  unsigned int h_bad[2] = {0, 0};
   if (e == cudaSuccess) e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&h_bad, bad.p, 4, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h_bad, bad.p, 8, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
     delete ng;
     return cuda_fail(e, "degree sort", __FILE__, __LINE__);
   }
-  if (h_bad) {
+  if (h_bad[1]) {
+    delete ng;
+    return fail(RG_ECUDA, "rg_graph_degree_sort: the sort did not finish");
+  }
+  if (h_bad[0]) {
     delete ng;
     return fail(RG_EINVAL, "rg_graph_degree_sort: a neighbour id is >= n");
   }
@@ -1031,50 +975,180 @@ extern "C" rg_status rg_graph_degree_sort_by(const rg_graph* g, int by_out_degre
 
 // ---------------------------------------------------------------------------
 // CSR construction on the device (the symmetric loader's clean-up, IO.h:429-474,
-// for an edge list): both directions of every edge become directed entries
-// (a, b); two stable radix sorts order them by (a, b); self loops and repeats
-// are dropped; a scan compacts the survivors into the neighbour array, and
-// each vertex's offset is the position of its first entry.  The result is
-// bit-identical to rg_csr_from_edges.
+// for an edge list): both directions of every edge become 64-bit entries
+// a << bits | b (ids < 2^bits), which one radix sort orders by (a, b); self
+// loops and repeats are dropped while the survivors are written to the neighbour
+// array, and each vertex's offset is the place of its first entry.  The result
+// is bit-identical to rg_csr_from_edges.
 // ---------------------------------------------------------------------------
 namespace rg {
 
-__global__ void csr_keep(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, int64_t k,
-                         uint32_t* __restrict__ keep) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < k; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t ai = a[i], bi = b[i];
-    keep[i] = (ai != bi && (i == 0 || a[i - 1] != ai || b[i - 1] != bi)) ? 1u : 0u;
-  }
-}
-
-__global__ void csr_compact(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
-                            const uint32_t* __restrict__ keep, const uint32_t* __restrict__ pos, int64_t k,
-                            uint32_t* __restrict__ a_out, uint32_t* __restrict__ adj) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < k; i += (int64_t)gridDim.x * blockDim.x) {
-    if (keep[i]) {
-      a_out[pos[i]] = a[i];
-      adj[pos[i]] = b[i];
-    }
-  }
-}
-
-// off[v] = first position whose source is >= v, for v in [0, n]: position p
-// (0 <= p <= m) fills the vertices between the previous source and its own.
-__global__ void csr_offsets(const uint32_t* __restrict__ a, int64_t m, int64_t n, uint32_t* __restrict__ off) {
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p <= m; p += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t lo = p == 0 ? 0 : (int64_t)a[p - 1] + 1;
-    const int64_t hi = p == m ? n : min((int64_t)a[p], n);  // ids are < n; never write past off[n]
-    for (int64_t v = lo; v <= hi; v++) off[v] = (uint32_t)p;
-  }
-}
-
-__global__ void max_value(const uint32_t* __restrict__ x, int64_t k, unsigned int* out) {
+// Entries from an edge list, their digit counts (passes of the sort on `hi`
+// bits) and the largest id.  src and dst may be page-locked host memory, read
+// once over the host link.  kWide: both are 16-byte aligned.
+template <bool kWide>
+__global__ void __launch_bounds__(256) csr_pack(const uint32_t* __restrict__ src, const uint32_t* __restrict__ dst,
+                                                int64_t ne, int bits, bool both, uint64_t* __restrict__ key, int hi,
+                                                int passes, uint32_t* hist, unsigned int* max_id) {
+  __shared__ uint32_t sh[kMaxSortPasses * 256];
+  sort_zero(sh, passes);
   unsigned int mx = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < k; i += (int64_t)gridDim.x * blockDim.x) {
-    mx = max(mx, x[i]);
+  auto one = [&](int64_t i, uint32_t a, uint32_t b) {
+    mx = max(mx, max(a, b));
+    const uint64_t k0 = ((uint64_t)a << bits) | b;
+    key[i] = k0;
+    sort_count_key(sh, k0, 0, hi, passes);
+    if (both) {
+      const uint64_t k1 = ((uint64_t)b << bits) | a;
+      key[ne + i] = k1;
+      sort_count_key(sh, k1, 0, hi, passes);
+    }
+  };
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
+  if (kWide) {
+    for (int64_t q = t; q * 4 < ne; q += nt) {
+      if (q * 4 + 4 <= ne) {
+        const uint4 a = __ldg(reinterpret_cast<const uint4*>(src) + q), b = __ldg(reinterpret_cast<const uint4*>(dst) + q);
+        one(q * 4, a.x, b.x);
+        one(q * 4 + 1, a.y, b.y);
+        one(q * 4 + 2, a.z, b.z);
+        one(q * 4 + 3, a.w, b.w);
+      } else {
+        for (int64_t i = q * 4; i < ne; i++) one(i, src[i], dst[i]);
+      }
+    }
+  } else {
+    for (int64_t i = t; i < ne; i += nt) one(i, src[i], dst[i]);
   }
-  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, mx);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((threadIdx.x & 31) == 0) atomicMax(max_id, mx);
+  sort_flush(sh, hist, passes);
+}
+
+// Sorted entries -> neighbour array and offsets.  kClean drops self loops and
+// repeats (the first of equal entries stays).  Entry i keeps its place when
+// `keep`; csr_count gives the kept entries of each tile, csr_emit, from their
+// scan (whose last word is their total), writes them and the offsets.
+constexpr int kCsrThreads = 256, kCsrItems = 8, kCsrTile = kCsrThreads * kCsrItems;
+
+template <bool kClean>
+__device__ __forceinline__ bool csr_keep(uint64_t x, uint64_t prev, bool has_prev, int bits) {
+  const uint64_t mask = (1ull << bits) - 1;
+  return !kClean || ((x >> bits) != (x & mask) && (!has_prev || x != prev));
+}
+
+template <bool kClean>
+__global__ void __launch_bounds__(kCsrThreads) csr_count(const uint64_t* __restrict__ key, int64_t k, int bits,
+                                                         uint32_t* __restrict__ tile_count) {
+  const int64_t t0 = (int64_t)blockIdx.x * kCsrTile;
+  uint32_t c = 0;
+#pragma unroll 4
+  for (int s = 0; s < kCsrItems; s++) {
+    const int64_t i = t0 + s * kCsrThreads + threadIdx.x;
+    if (i < k) c += csr_keep<kClean>(key[i], i ? key[i - 1] : 0ull, i > 0, bits);
+  }
+  __shared__ uint32_t tot;
+  block_exclusive_sum<kCsrThreads>(c, &tot);
+  if (threadIdx.x == 0) tile_count[blockIdx.x] = tot;
+}
+
+template <bool kClean>
+__global__ void __launch_bounds__(kCsrThreads) csr_emit(const uint64_t* __restrict__ key, int64_t k, int bits,
+                                                        const uint32_t* __restrict__ tile_first, int64_t n,
+                                                        uint32_t* __restrict__ off, uint32_t* __restrict__ adj) {
+  // a warp's sub-tile of kCsrItems x 32 entries, 32 at a time: writes stay coalesced
+  __shared__ uint32_t wsum[kCsrThreads / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t t0 = (int64_t)blockIdx.x * kCsrTile + (int64_t)w * kCsrItems * 32;
+  uint64_t x[kCsrItems], prev[kCsrItems];
+  unsigned kept[kCsrItems];
+  uint32_t c = 0;
+#pragma unroll
+  for (int s = 0; s < kCsrItems; s++) {
+    const int64_t i = t0 + s * 32 + lane;
+    x[s] = i < k ? key[i] : 0ull;
+    prev[s] = i > 0 && i <= k ? key[i - 1] : 0ull;
+  }
+#pragma unroll
+  for (int s = 0; s < kCsrItems; s++) {
+    const int64_t i = t0 + s * 32 + lane;
+    kept[s] = __ballot_sync(0xffffffffu, i < k && csr_keep<kClean>(x[s], prev[s], i > 0, bits));
+    c += __popc(kept[s]);
+  }
+  if (lane == 0) wsum[w] = c;
+  __syncthreads();
+  uint32_t at = tile_first[blockIdx.x];
+  for (int j = 0; j < w; j++) at += wsum[j];
+  const uint64_t mask = (1ull << bits) - 1;
+#pragma unroll
+  for (int s = 0; s < kCsrItems; s++) {
+    const int64_t i = t0 + s * 32 + lane;
+    const uint32_t pos = at + __popc(kept[s] & ((1u << lane) - 1u));
+    if ((kept[s] >> lane) & 1u) adj[pos] = (uint32_t)(x[s] & mask);
+    // offsets of the rows that begin at this entry: its own and the empty ones
+    // before it (and, past the last entry, up to n); runs of more than a few by
+    // the whole warp
+    int64_t from = 0, to = -1;
+    if (i < k) {
+      from = i ? (int64_t)(prev[s] >> bits) + 1 : 0;
+      to = min((int64_t)(x[s] >> bits), n);  // ids are < n; never write past off[n]
+      if (to - from < 8) {
+        for (int64_t v = from; v <= to; v++) off[v] = pos;
+        to = from - 1;
+      }
+    }
+    for (unsigned runs = __ballot_sync(0xffffffffu, to >= from); runs; runs &= runs - 1) {
+      const int j = __ffs(runs) - 1;
+      const int64_t f = __shfl_sync(0xffffffffu, from, j), l = __shfl_sync(0xffffffffu, to, j);
+      const uint32_t p = __shfl_sync(0xffffffffu, pos, j);
+      for (int64_t v = f + lane; v <= l; v += 32) off[v] = p;
+    }
+    at += __popc(kept[s]);
+  }
+  // rows past the last entry's: the block that holds it
+  if (blockIdx.x == gridDim.x - 1) {
+    const int64_t last = min((int64_t)(key[k - 1] >> bits), n);
+    const uint32_t end = tile_first[gridDim.x];
+    for (int64_t v = last + 1 + threadIdx.x; v <= n; v += kCsrThreads) off[v] = end;
+  }
+}
+
+// off and adj of the sorted entries; *m_out entries survive.  `adj` is sized
+// here, from the count (one host sync, which also reads the sort's failure flag
+// and, unless null, the largest id).
+template <bool kClean>
+static rg_status csr_from_sorted(Workspace& ws, const uint64_t* key, int64_t k, int bits, int64_t n, DevBuf& off,
+                                 DevBuf& adj, int64_t* m_out, const uint32_t* failed, const unsigned int* max_id,
+                                 const char* who, cudaStream_t st) {
+  const int64_t tiles = (k + kCsrTile - 1) / kCsrTile;
+  DevBuf first(true, st), back(true, st);
+  RG_TRY(first.reserve(4 * (size_t)(tiles + 1)));
+  RG_TRY(back.reserve(16));
+  csr_count<kClean><<<(unsigned)tiles, kCsrThreads, 0, st>>>(key, k, bits, first.as<uint32_t>());
+  RG_TRY(scan_u32(ws, first.as<uint32_t>(), first.as<uint32_t>(), tiles, st));
+  uint32_t h[3] = {0, 0, 0};  // entries, sort failure, largest id
+  uint32_t* b = back.as<uint32_t>();
+  RG_CUDA(cudaMemcpyAsync(b, first.as<uint32_t>() + tiles, 4, cudaMemcpyDeviceToDevice, st));
+  RG_CUDA(cudaMemcpyAsync(b + 1, failed, 4, cudaMemcpyDeviceToDevice, st));
+  if (max_id) RG_CUDA(cudaMemcpyAsync(b + 2, max_id, 4, cudaMemcpyDeviceToDevice, st));
+  RG_TRY(read_small(b, h, max_id ? 12 : 8, st));
+  if (max_id && h[2] >= (uint64_t)n) return fail(RG_EINVAL, "edge endpoint %u >= n", h[2]);
+  if (h[1]) return fail(RG_ECUDA, "%s: the sort did not finish", who);
+  *m_out = (int64_t)h[0];
+  RG_TRY(off.reserve(4 * (size_t)(n + 1)));
+  RG_TRY(adj.reserve(4 * (size_t)(*m_out + 8)));
+  csr_emit<kClean><<<(unsigned)tiles, kCsrThreads, 0, st>>>(key, k, bits, first.as<uint32_t>(), n, off.as<uint32_t>(),
+                                                            adj.as<uint32_t>());
+  RG_CUDA(cudaMemsetAsync(adj.as<uint32_t>() + *m_out, 0, 32, st));
+  RG_CUDA(cudaGetLastError());
+  return RG_OK;
+}
+
+rg_status csr_from_sorted_rows(Workspace& ws, const uint64_t* key, int64_t k, int bits, int64_t n, bool clean,
+                               DevBuf& off, DevBuf& adj, int64_t* kept, const SortScratch& sort, const char* who,
+                               cudaStream_t st) {
+  auto fn = clean ? csr_from_sorted<true> : csr_from_sorted<false>;
+  return fn(ws, key, k, bits, n, off, adj, kept, sort_failed(sort), nullptr, who, st);
 }
 
 __global__ void max_degree(const uint32_t* __restrict__ off, int64_t n, unsigned int* out) {
@@ -1086,35 +1160,19 @@ __global__ void max_degree(const uint32_t* __restrict__ off, int64_t n, unsigned
   if ((threadIdx.x & 31) == 0) atomicMax(out, mx);
 }
 
-// Stable LSD radix sort of k (key, val) pairs on the `bits` low key bits;
-// the result ends in (key, val) (the buffers are swapped as needed).
-static rg_status radix_pairs(Workspace& ws, DevBuf& key, DevBuf& val, DevBuf& key2, DevBuf& val2, int64_t k, int bits,
-                             DevBuf& hist, cudaStream_t st) {
-  const int64_t nblocks = (k + kSortTile - 1) / kSortTile;
-  RG_TRY(hist.reserve(4 * (256 * nblocks + 1)));
-  uint32_t *ka = key.as<uint32_t>(), *va = val.as<uint32_t>(), *kb = key2.as<uint32_t>(), *vb = val2.as<uint32_t>();
-  const int passes = (bits + 7) / 8;
-  for (int p = 0; p < passes; p++) {
-    sort_hist<<<(unsigned)nblocks, kSortThreads, 0, st>>>(ka, k, 8 * p, nblocks, hist.as<uint32_t>());
-    RG_TRY(scan_u32(ws, hist.as<uint32_t>(), hist.as<uint32_t>(), 256 * nblocks, st));
-    sort_scatter<<<(unsigned)nblocks, kSortThreads, 0, st>>>(ka, va, k, 8 * p, nblocks, hist.as<uint32_t>(), kb, vb);
-    std::swap(ka, kb);
-    std::swap(va, vb);
-  }
-  RG_CUDA(cudaGetLastError());
-  if (passes % 2) {  // the sorted pairs are in the second buffers: swap ownership
-    std::swap(key.p, key2.p);
-    std::swap(key.bytes, key2.bytes);
-    std::swap(val.p, val2.p);
-    std::swap(val.bytes, val2.bytes);
-  }
-  return RG_OK;
-}
-
 }  // namespace rg
 
 namespace rg {
 rg_status build_in_lists(rg_graph* g, cudaStream_t st);
+}
+
+// The device's address of page-locked host memory (false: pageable).
+static bool host_on_device(const uint32_t* h, const uint32_t** d) {
+  cudaPointerAttributes pa;
+  const bool ok = cudaPointerGetAttributes(&pa, h) == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer;
+  cudaGetLastError();  // an unregistered pointer is not an error here
+  if (ok) *d = static_cast<const uint32_t*>(pa.devicePointer);
+  return ok;
 }
 
 // Shared by the symmetric and directed builders.  Symmetric: entries
@@ -1134,82 +1192,63 @@ static rg_status create_from_edges(const char* who, int64_t n, int64_t num_edges
   cudaStream_t st = c->stream;
   int sms = 0;
   RG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-  // temporaries from the pool
-  DevBuf a{true, st}, b{true, st}, a2{true, st}, b2{true, st}, hist{true, st}, info{true, st};
-  RG_TRY(a.reserve(4 * (size_t)k));
-  RG_TRY(b.reserve(4 * (size_t)k));
-  RG_TRY(a2.reserve(4 * (size_t)k));
-  RG_TRY(b2.reserve(4 * (size_t)k));
-  RG_TRY(info.reserve(8));
-  const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-  if (num_edges > 0) {
-    RG_CUDA(cudaMemcpyAsync(a.as<uint32_t>(), src, 4 * num_edges, kind, st));
-    RG_CUDA(cudaMemcpyAsync(b.as<uint32_t>(), dst, 4 * num_edges, kind, st));
-    if (!directed) {
-      RG_CUDA(cudaMemcpyAsync(a.as<uint32_t>() + num_edges, dst, 4 * num_edges, kind, st));
-      RG_CUDA(cudaMemcpyAsync(b.as<uint32_t>() + num_edges, src, 4 * num_edges, kind, st));
-    }
-  }
-  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((k + 255) / 256, (int64_t)sms * 32));
-  if (k > 0) {  // every id must be < n: the offsets below are indexed by them
-    uint32_t mx_id = 0;
-    RG_CUDA(cudaMemsetAsync(info.p, 0, 4, st));
-    max_value<<<blocks, 256, 0, st>>>(a.as<uint32_t>(), k, info.as<unsigned int>());
-    RG_CUDA(cudaGetLastError());
-    RG_CUDA(cudaMemcpyAsync(&mx_id, info.p, 4, cudaMemcpyDeviceToHost, st));
-    RG_CUDA(cudaStreamSynchronize(st));
-    if (mx_id >= (uint64_t)n) return fail(RG_EINVAL, "edge endpoint %u >= n", mx_id);
-  }
   int bits = 1;
   while (bits < 32 && ((uint64_t)(n - 1) >> bits) != 0) bits++;
-  uint32_t* keep = a2.as<uint32_t>();
-  uint32_t* src_c = b2.as<uint32_t>();  // compacted sources
-  DevBuf scan{true, st};                 // exclusive scan of keep, k+1 entries
-  int64_t m = 0;
-  if (k > 0) {
-    // by (a, b): stable sort on b, then on a
-    RG_TRY(radix_pairs(c->ws, b, a, b2, a2, k, bits, hist, st));
-    RG_TRY(radix_pairs(c->ws, a, b, a2, b2, k, bits, hist, st));
-    keep = a2.as<uint32_t>();  // a2/b2 are free again after the sorts
-    src_c = b2.as<uint32_t>();
-    csr_keep<<<blocks, 256, 0, st>>>(a.as<uint32_t>(), b.as<uint32_t>(), k, keep);
-    RG_CUDA(cudaGetLastError());
-    RG_TRY(scan.reserve(4 * (size_t)(k + 1)));
-    RG_TRY(scan_u32(c->ws, keep, scan.as<uint32_t>(), k, st));
-    uint32_t m32 = 0;
-    RG_CUDA(cudaMemcpyAsync(&m32, scan.as<uint32_t>() + k, 4, cudaMemcpyDeviceToHost, st));
-    RG_CUDA(cudaStreamSynchronize(st));
-    m = (int64_t)m32;
-  }
   rg_graph* g = nullptr;
   RG_TRY(new_graph(&g));
   g->n = n;
-  g->m = m;
-  rg_status s;
-  if ((s = g->off.reserve(4 * (n + 1))) != RG_OK || (s = g->adj.reserve(4 * (m + 8))) != RG_OK) {
+  rg_status s = RG_OK;
+  uint32_t mx = 0;
+  {
+    // temporaries from the pool
+    DevBuf k0{true, st}, k1{true, st}, info{true, st};
+    SortScratch sort(st);
+    const int hi = 2 * bits, passes = sort_passes(0, hi);
+    auto fill = [&]() -> rg_status {
+      RG_TRY(info.reserve(8));
+      RG_CUDA(cudaMemsetAsync(info.p, 0, 8, st));
+      if (k == 0) {
+        RG_TRY(g->off.reserve(4 * (n + 1)));
+        RG_TRY(g->adj.reserve(32));
+        RG_CUDA(cudaMemsetAsync(g->off.p, 0, 4 * (n + 1), st));
+        RG_CUDA(cudaMemsetAsync(g->adj.p, 0, 32, st));
+        return RG_OK;
+      }
+      RG_TRY(k0.reserve(8 * (size_t)k));
+      RG_TRY(k1.reserve(8 * (size_t)k + 16));
+      RG_TRY(sort_begin(sort, k, passes, st));
+      const uint32_t *d_src = src, *d_dst = dst;
+      if (!on_device && !(host_on_device(src, &d_src) && host_on_device(dst, &d_dst))) {
+        // pageable: copied (into the sort's second buffer, free until its first pass)
+        uint32_t* c2 = k1.as<uint32_t>();
+        RG_CUDA(cudaMemcpyAsync(c2, src, 4 * num_edges, cudaMemcpyHostToDevice, st));
+        RG_CUDA(cudaMemcpyAsync(c2 + ((num_edges + 3) & ~3ll), dst, 4 * num_edges, cudaMemcpyHostToDevice, st));
+        d_src = c2;
+        d_dst = c2 + ((num_edges + 3) & ~3ll);
+      }
+      const bool wide = (((uintptr_t)d_src | (uintptr_t)d_dst) & 15u) == 0;
+      const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((num_edges + 1023) / 1024, (int64_t)sms * 8));
+      auto pack = wide ? csr_pack<true> : csr_pack<false>;
+      pack<<<(unsigned)blocks, 256, 0, st>>>(d_src, d_dst, num_edges, bits, !directed, k0.as<uint64_t>(), hi, passes,
+                                             sort_counts(sort), info.as<unsigned int>());
+      RG_CUDA(cudaGetLastError());
+      uint64_t *key = k0.as<uint64_t>(), *other = k1.as<uint64_t>();
+      RG_TRY(sort_run(sort, &key, &other, k, 0, hi, st));
+      return csr_from_sorted<true>(c->ws, key, k, bits, n, g->off, g->adj, &g->m, sort_failed(sort),
+                                   info.as<unsigned int>(), who, st);
+    };
+    s = fill();
+    if (s == RG_OK) {
+      const int dblocks = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sms * 16));
+      max_degree<<<dblocks, 256, 0, st>>>(g->off.as<uint32_t>(), n, info.as<unsigned int>() + 1);
+      cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) s = cuda_fail(e, "device CSR build", __FILE__, __LINE__);
+      else s = read_small(info.as<unsigned int>() + 1, &mx, 4, st);
+    }
+  }
+  if (s != RG_OK) {
     delete g;
     return s;
-  }
-  cudaError_t e = cudaSuccess;
-  if (k > 0) {
-    csr_compact<<<blocks, 256, 0, st>>>(a.as<uint32_t>(), b.as<uint32_t>(), keep, scan.as<uint32_t>(), k, src_c,
-                                       g->adj.as<uint32_t>());
-  }
-  const int oblocks = (int)std::max<int64_t>(1, std::min<int64_t>((m + 1 + 255) / 256, (int64_t)sms * 32));
-  csr_offsets<<<oblocks, 256, 0, st>>>(src_c, m, n, g->off.as<uint32_t>());
-  e = cudaMemsetAsync(g->adj.as<uint32_t>() + m, 0, 32, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(info.p, 0, 4, st);
-  if (e == cudaSuccess) {
-    const int dblocks = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)sms * 16));
-    max_degree<<<dblocks, 256, 0, st>>>(g->off.as<uint32_t>(), n, info.as<unsigned int>());
-    e = cudaGetLastError();
-  }
-  uint32_t mx = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&mx, info.p, 4, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) {
-    delete g;
-    return cuda_fail(e, "device CSR build", __FILE__, __LINE__);
   }
   g->max_deg = mx;  // host degree array: on first full use (host_arrays)
   if ((s = finish_graph(g)) != RG_OK) { delete g; return s; }
@@ -1243,8 +1282,11 @@ extern "C" rg_status rg_graph_create_directed_from_edges(int64_t n, int64_t num_
 // ---------------------------------------------------------------------------
 namespace rg {
 
-__global__ void __launch_bounds__(256) expand_rows(DevGraph g, const uint32_t* __restrict__ chunk_v,
-                                                   uint32_t nchunks, uint32_t* __restrict__ row) {
+// Entries target << bits | source in list order, and their digit counts.
+__global__ void __launch_bounds__(256) in_entries(DevGraph g, const uint32_t* __restrict__ chunk_v, uint32_t nchunks,
+                                                  int bits, uint64_t* __restrict__ key, int passes, uint32_t* hist) {
+  __shared__ uint32_t sh[kMaxSortPasses * 256];
+  sort_zero(sh, passes);
   const int lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -1253,39 +1295,41 @@ __global__ void __launch_bounds__(256) expand_rows(DevGraph g, const uint32_t* _
     for (int r = 0; r < kSweepChunk / 32; r++) {
       const uint32_t e = c * kSweepChunk + r * 32 + lane;
       if (e >= g.m) break;
-      row[e] = upper_index(g.off, vlo, vhi, e);
+      const uint64_t k = ((uint64_t)g.adj[e] << bits) | upper_index(g.off, vlo, vhi, e);
+      key[e] = k;
+      sort_count_key(sh, k, bits, 2 * bits, passes);
     }
   }
+  sort_flush(sh, hist, passes);
 }
 
 rg_status build_in_lists(rg_graph* g, cudaStream_t st) {
   const int64_t n = g->n, m = g->m;
-  RG_TRY(g->in_off.reserve(4 * (n + 1)));
-  RG_TRY(g->in_adj.reserve(4 * (m + 8)));
-  RG_CUDA(cudaMemsetAsync(g->in_adj.as<uint32_t>() + m, 0, 32, st));
-  int sms = 0;
-  RG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device));
   if (m == 0) {
+    RG_TRY(g->in_off.reserve(4 * (n + 1)));
+    RG_TRY(g->in_adj.reserve(32));
     RG_CUDA(cudaMemsetAsync(g->in_off.p, 0, 4 * (n + 1), st));
+    RG_CUDA(cudaMemsetAsync(g->in_adj.p, 0, 32, st));
     return RG_OK;
   }
-  DevBuf key{true, st}, val{true, st}, key2{true, st}, val2{true, st}, hist{true, st};
-  RG_TRY(key.reserve(4 * (size_t)m));
-  RG_TRY(val.reserve(4 * (size_t)m));
-  RG_TRY(key2.reserve(4 * (size_t)m));
-  RG_TRY(val2.reserve(4 * (size_t)m));
-  RG_CUDA(cudaMemcpyAsync(key.p, g->adj.p, 4 * m, cudaMemcpyDeviceToDevice, st));
-  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((g->nchunks * 32 + 255) / 256, (int64_t)sms * 8));
-  expand_rows<<<(unsigned)blocks, 256, 0, st>>>(g->view(), g->chunk_v.as<uint32_t>(), (uint32_t)g->nchunks,
-                                                val.as<uint32_t>());
-  RG_CUDA(cudaGetLastError());
+  int sms = 0;
+  RG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device));
   int bits = 1;
   while (bits < 32 && ((uint64_t)(n - 1) >> bits) != 0) bits++;
-  RG_TRY(radix_pairs(ctx().ws, key, val, key2, val2, m, bits, hist, st));
-  RG_CUDA(cudaMemcpyAsync(g->in_adj.p, val.p, 4 * m, cudaMemcpyDeviceToDevice, st));
-  const int oblocks = (int)std::max<int64_t>(1, std::min<int64_t>((m + 1 + 255) / 256, (int64_t)sms * 32));
-  csr_offsets<<<oblocks, 256, 0, st>>>(key.as<uint32_t>(), m, n, g->in_off.as<uint32_t>());
+  const int passes = sort_passes(bits, 2 * bits);
+  DevBuf k0{true, st}, k1{true, st};
+  SortScratch sort(st);
+  RG_TRY(k0.reserve(8 * (size_t)m));
+  RG_TRY(k1.reserve(8 * (size_t)m));
+  RG_TRY(sort_begin(sort, m, passes, st));
+  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((g->nchunks * 32 + 255) / 256, (int64_t)sms * 8));
+  in_entries<<<(unsigned)blocks, 256, 0, st>>>(g->view(), g->chunk_v.as<uint32_t>(), (uint32_t)g->nchunks, bits,
+                                               k0.as<uint64_t>(), passes, sort_counts(sort));
   RG_CUDA(cudaGetLastError());
+  uint64_t *key = k0.as<uint64_t>(), *other = k1.as<uint64_t>();
+  RG_TRY(sort_run(sort, &key, &other, m, bits, 2 * bits, st));
+  int64_t kept = 0;
+  RG_TRY(csr_from_sorted_rows(ctx().ws, key, m, bits, n, false, g->in_off, g->in_adj, &kept, sort, "in-lists", st));
   RG_CUDA(cudaStreamSynchronize(st));
   return RG_OK;
 }

@@ -68,8 +68,10 @@ struct DevBuf {
   size_t bytes = 0;
   bool pooled = false;
   cudaStream_t free_stream = nullptr;  // pooled: the release is ordered after this stream's work
+  bool on_stream = false;  // pooled: only free_stream's work uses it, so it is allocated in that order too, without a sync
   DevBuf() = default;
-  explicit DevBuf(bool from_pool, cudaStream_t stream = nullptr) : pooled(from_pool), free_stream(stream) {}
+  explicit DevBuf(bool from_pool, cudaStream_t stream = nullptr)
+      : pooled(from_pool), free_stream(stream), on_stream(stream != nullptr) {}
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() { release(); }
