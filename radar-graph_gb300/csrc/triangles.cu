@@ -1,152 +1,266 @@
 // Triangle counting (GAP tc_local, src/*/GAP/src/tc_local.cc:49-157) on the
 // device.
 //
-// The graph is relabelled by degree (descending, ties by descending id, the
-// order of builder.h:247-282 and of the degree sort) with every neighbour
-// list sorted ascending; a triangle is then counted once, as u > v > w: for
-// every edge (u, v) with v < u, the common neighbours w < v of u and v are
-// found by merging u's list before v with v's list below v (or, when one is
-// far longer, by searching the short one's elements in it).  In this order
-// both lists hold only higher-degree neighbours, so they stay short even on
-// skewed graphs.  Per-vertex counts (triangles containing each vertex) are
-// returned by original id; the counts of the H highest-degree vertices
-// (ids < H) are kept per CTA in shared memory and merged once per CTA -- the
-// RADAR variant's per-thread copies of triangles[u] for u < numHubs
-// (tc_local.cc:54-96).
+// In degree order (descending, ties by descending id, the order of
+// builder.h:247-282 and of the degree sort) every vertex u keeps its lower list
+// L(u): its neighbours below u, ascending.  A triangle is counted once, as
+// u > v > w: for every v in L(u) the common members of L(u) and L(v) (all of
+// them below v).  Lower lists hold only higher-degree neighbours, so they stay
+// short on skewed graphs.  Per-vertex counts (triangles containing each vertex)
+// are returned by original id; counts of the w's among the first ids are kept
+// per CTA in shared memory and merged once per CTA -- the RADAR variant's
+// per-thread copies of triangles[u] for u < numHubs (tc_local.cc:54-96).
+//
+// The lower lists come from one stable sort: walking the rows v in order and
+// keeping the neighbours u > v yields the pairs (u, v) ordered by v, so sorting
+// them by u alone leaves every list ascending.
 
 #include <cuda_runtime.h>
 
 #include <algorithm>
 
 #include "app_common.cuh"
+#include "sort.cuh"
 
 namespace rg {
 
 namespace {
 
-// a[j] = source row of edge j, b[j] = neighbour (edge-balanced: each warp owns
-// kSweepChunk consecutive edges and finds their rows from the chunk starts)
-__global__ void __launch_bounds__(256) expand_entries(DevGraph g, const uint32_t* __restrict__ chunk_v,
-                                                      uint32_t nchunks, uint32_t* __restrict__ a,
-                                                      uint32_t* __restrict__ b) {
+constexpr unsigned kAll = 0xffffffffu;
+
+// The pairs (u, v), u > v, of a symmetric graph, ordered by v: counted per
+// kSweepChunk edges (a warp each; rows from the chunk starts), then written as
+// u << bits | v at the chunk's place with the digit counts of the sort by u.
+template <bool kEmit>
+__global__ void __launch_bounds__(256) upper_pairs(DevGraph g, const uint32_t* __restrict__ chunk_v, uint32_t nchunks,
+                                                   uint32_t* __restrict__ count, const uint32_t* __restrict__ place,
+                                                   int bits, uint64_t* __restrict__ key, int passes, uint32_t* hist) {
+  __shared__ uint32_t sh[kEmit ? kMaxSortPasses * 256 : 1];
+  if (kEmit) sort_zero(sh, passes);
   const int lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t c = warp; c < nchunks; c += nwarps) {
     const uint32_t vlo = chunk_v[c], vhi = chunk_v[c + 1];
+    uint32_t n = 0, at = kEmit ? place[c] : 0;
     for (int r = 0; r < kSweepChunk / 32; r++) {
       const uint32_t e = c * kSweepChunk + r * 32 + lane;
-      if (e >= g.m) break;
-      a[e] = upper_index(g.off, vlo, vhi, e);
-      b[e] = g.adj[e];
+      const uint32_t v = e < g.m ? upper_index(g.off, vlo, vhi, e) : 0, u = e < g.m ? g.adj[e] : 0;
+      const unsigned keep = __ballot_sync(kAll, u > v);
+      if (kEmit && u > v) {
+        const uint64_t k = ((uint64_t)u << bits) | v;
+        key[at + __popc(keep & ((1u << lane) - 1u))] = k;
+        sort_count_key(sh, k, bits, 2 * bits, passes);
+      }
+      at += __popc(keep);
+      n += __popc(keep);
     }
+    if (!kEmit && lane == 0) count[c] = n;
   }
+  if (kEmit) sort_flush(sh, hist, passes);
 }
 
-// lower[u] = number of u's (sorted) neighbours below u
-__global__ void lower_degrees(DevGraph g, uint32_t* __restrict__ lower) {
-  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < g.n; u += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t lo = g.off[u], hi = g.off[u + 1];
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (g.adj[mid] < (uint32_t)u) lo = mid + 1;
-      else hi = mid;
-    }
-    lower[u] = lo - g.off[u];
-  }
-}
+constexpr int kTcThreads = 512;
+constexpr int kTcWarps = kTcThreads / 32;
+constexpr uint32_t kMarkIds = 16384;  // ids with a bit in a warp's marks (2 KiB)
+constexpr uint32_t kHubIds = 4096;    // ids with a counter per CTA (16 KiB)
 
-template <bool kHub>
-__global__ void __launch_bounds__(256) count_triangles(DevGraph g, const uint32_t* __restrict__ chunk_v,
-                                                       uint32_t nchunks, const uint32_t* __restrict__ lower,
-                                                       unsigned long long* tri, uint32_t H,
-                                                       unsigned long long* total) {
+constexpr uint32_t kTake = 4;
+
+struct TcShared {
+  uint32_t mark[kTcWarps][kMarkIds / 32];
+  uint32_t hub[kHubIds];
+  uint32_t found[kTcWarps][32];  // per edge of a warp's group
+};
+
+// A warp takes 32 edges at a time, one per lane, in the order of the graph's rows
+// v; the neighbours u > v count.
+//  * Where one of L(v) and L(u) is far shorter than the other (or v is past the
+//    ids that a bitmap covers), its members are searched in the other; the searches of all such edges are
+//    dealt out to the lanes together, so a tail vertex with two or three lower
+//    neighbours does not idle a warp.
+//  * Otherwise, v being a high-degree vertex, L(v) is marked in the warp's bitmap,
+//    once for all of a row's edges, and L(u) streamed against it as far as v: 32
+//    members per load where a search step gathers 32 lines.  (Marking L(u) and
+//    streaming L(v) reads 2.7 times as much on R-MAT s18: the members of L(u)
+//    below v are few where v is a hub, all of L(v) are not.)
+// What bounds it is the streamed members: a bitmap lookup each and a shared-memory
+// add per triangle.  R-MAT, 2e5 vertices, 3.6e6 edges, 8e7 triangles: 4061 us by
+// a merge or search per lane, 880 us streaming L(v) at half the occupancy.
+// A w meets a given edge at most once, so a CTA adds at most 32 per group to a
+// hub counter: fewer than 2^32 over the fewer than 2^27 groups of any graph.
+__global__ void __launch_bounds__(kTcThreads, 4) count_triangles(DevGraph g, const uint32_t* __restrict__ chunk_v,
+                                                                const uint32_t* __restrict__ off,
+                                                                const uint32_t* __restrict__ adj, unsigned int* next,
+                                                                unsigned long long* tri, unsigned long long* total) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  unsigned long long* hs = reinterpret_cast<unsigned long long*>(smem_raw);
-  if (kHub) {
-    for (uint32_t h = threadIdx.x; h < H; h += blockDim.x) hs[h] = 0ull;
-    __syncthreads();
-  }
-  const int lane = threadIdx.x & 31;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  unsigned long long found = 0;
-  for (uint32_t c = warp; c < nchunks; c += nwarps) {
-    const uint32_t vlo = chunk_v[c], vhi = chunk_v[c + 1];
-    for (int r = 0; r < kSweepChunk / 32; r++) {
-      const uint32_t e = c * kSweepChunk + r * 32 + lane;
-      if (e >= g.m) break;
-      const uint32_t u = upper_index(g.off, vlo, vhi, e);
-      const uint32_t v = g.adj[e];
-      if (v >= u) continue;  // each triangle once: u > v > w
-      // u's neighbours before v (all < v) against v's neighbours below v:
-      // merged, unless one list is far longer -- then each element of the
-      // short one is searched in the long one (min * log(max) steps)
-      uint32_t sa = g.off[u], ea = e, sb = g.off[v], eb = g.off[v] + lower[v];
-      if (ea - sa > eb - sb) {
-        const uint32_t t0 = sa, t1 = ea;
-        sa = sb;
-        ea = eb;
-        sb = t0;
-        eb = t1;
-      }
-      uint32_t cnt = 0;
-      if (eb - sb > 16 * (ea - sa)) {
-        uint32_t lo = sb;  // the short list ascends: each search starts past the last one
-        for (uint32_t i = sa; i < ea && lo < eb; i++) {
-          const uint32_t x = g.adj[i];
-          uint32_t hi = eb;
-          while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (g.adj[mid] < x) lo = mid + 1;
-            else hi = mid;
-          }
-          if (lo < eb && g.adj[lo] == x) {
-            cnt++;
-            if (kHub && x < H) atomicAdd(hs + x, 1ull);
-            else atomicAdd(tri + x, 1ull);
-            lo++;
-          }
-        }
-      } else {
-        uint32_t ia = sa, ib = sb;
-        while (ia < ea && ib < eb) {
-          const uint32_t x = g.adj[ia], y = g.adj[ib];
-          if (x == y) {
-            cnt++;
-            if (kHub && x < H) atomicAdd(hs + x, 1ull);
-            else atomicAdd(tri + x, 1ull);
-            ia++;
-            ib++;
-          } else if (x < y) {
-            ia++;
-          } else {
-            ib++;
-          }
-        }
-      }
-      if (cnt) {
-        if (kHub && u < H) atomicAdd(hs + u, (unsigned long long)cnt);
-        else atomicAdd(tri + u, (unsigned long long)cnt);
-        if (kHub && v < H) atomicAdd(hs + v, (unsigned long long)cnt);
-        else atomicAdd(tri + v, (unsigned long long)cnt);
-        found += cnt;
+  TcShared& S = *reinterpret_cast<TcShared*>(smem_raw);
+  for (uint32_t i = threadIdx.x; i < kTcWarps * (kMarkIds / 32); i += kTcThreads) (&S.mark[0][0])[i] = 0u;
+  for (uint32_t i = threadIdx.x; i < kHubIds; i += kTcThreads) S.hub[i] = 0u;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t* mark = S.mark[w];
+  uint32_t* found = S.found[w];
+  const uint32_t groups = (g.m + 31) / 32;
+  unsigned long long sum = 0;
+  auto hit = [&](uint32_t x) {
+    if (x < kHubIds) atomicAdd(S.hub + x, 1u);
+    else atomicAdd(tri + x, 1ull);
+  };
+  uint32_t t = 0, end = 0;
+  for (;; t++) {
+    if (t >= end) {  // groups are taken kTake at a time: one counter serves every warp
+      if (lane == 0) t = atomicAdd(next, (unsigned)kTake);
+      t = __shfl_sync(kAll, t, 0);
+      if (t >= groups) break;
+      end = min(t + kTake, groups);
+    }
+    const uint32_t e = t * 32 + lane, ch = t / (kSweepChunk / 32);
+    uint32_t u = 0, v = 0, a = 0, la = 0, b = 0, lb = 0;
+    if (e < g.m) {
+      u = g.adj[e];
+      v = upper_index(g.off, chunk_v[ch], chunk_v[ch + 1], e);
+      if (u > v) {
+        b = off[v];
+        lb = off[v + 1] - b;
+        a = off[u];
+        la = lb ? min(off[u + 1] - a, v) : 0u;  // at least L(u)'s members below v
       }
     }
-  }
-  found = warp_sum(found);
-  if (lane == 0 && found) atomicAdd(total, found);
-  if (kHub) {
-    __syncthreads();
-    for (uint32_t h = threadIdx.x; h < H; h += blockDim.x) {
-      if (hs[h]) atomicAdd(tri + h, hs[h]);
+    const uint32_t lo = min(la, lb), hi = max(la, lb);
+    if (!__any_sync(kAll, lo > 0)) continue;
+    found[lane] = 0u;
+    const bool search = lo > 0 && (lo <= 8 || lo * 32 <= hi || v >= kMarkIds);
+    // searches: item t of the group's concatenated short lists
+    uint32_t inc = search ? lo : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(kAll, inc, o);
+      if (lane >= o) inc += x;
     }
+    const uint32_t items = __shfl_sync(kAll, inc, 31);
+    const uint32_t sp = la <= lb ? a : b, lp = la <= lb ? b : a;  // where the short and the long list begin
+    __syncwarp();
+    for (uint32_t i0 = 0; i0 < items; i0 += 32) {
+      const uint32_t i = i0 + lane;
+      int j = 0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        if (__shfl_sync(kAll, inc, j + o - 1) <= i) j += o;
+      }
+      j &= 31;
+      const uint32_t js = __shfl_sync(kAll, sp, j), jl = __shfl_sync(kAll, lp, j), jh = __shfl_sync(kAll, hi, j);
+      const uint32_t jn = __shfl_sync(kAll, lo, j), first = __shfl_sync(kAll, inc, j) - jn;
+      if (i < items) {
+        const uint32_t x = adj[js + (i - first)];
+        uint32_t l = 0, h = jh;
+        while (l < h) {
+          const uint32_t mid = (l + h) >> 1;
+          if (adj[jl + mid] < x) l = mid + 1;
+          else h = mid;
+        }
+        if (l < jh && adj[jl + l] == x) {
+          atomicAdd(found + j, 1u);
+          hit(x);
+        }
+      }
+    }
+    __syncwarp();
+    uint32_t marked = kNone, mb = 0, mn = 0;  // the v whose list is marked
+    auto unmark = [&] {
+      __syncwarp();
+      for (uint32_t i = lane; i < mn; i += 32) mark[adj[mb + i] >> 5] = 0u;
+      __syncwarp();
+    };
+    for (unsigned todo = __ballot_sync(kAll, lo > 0 && !search); todo; todo &= todo - 1) {
+      const int j = __ffs(todo) - 1;
+      const uint32_t jv = __shfl_sync(kAll, v, j), ja = __shfl_sync(kAll, a, j), jn = __shfl_sync(kAll, la, j);
+      if (jv != marked) {
+        unmark();
+        marked = jv;
+        mb = __shfl_sync(kAll, b, j);
+        mn = __shfl_sync(kAll, lb, j);
+        for (uint32_t i = lane; i < mn; i += 32) {  // v < kMarkIds, so every member has a bit
+          const uint32_t x = adj[mb + i];
+          atomicOr(mark + (x >> 5), 1u << (x & 31));
+        }
+        __syncwarp();
+      }
+      uint32_t c = 0;
+      for (uint32_t i0 = 0; i0 < jn; i0 += 128) {
+        uint32_t x[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) x[k] = i0 + 32 * k + lane < jn ? adj[ja + i0 + 32 * k + lane] : kNone;
+        if (__shfl_sync(kAll, x[0], 0) >= jv) break;  // the rest lies above v
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          if (x[k] < jv && ((mark[x[k] >> 5] >> (x[k] & 31)) & 1u)) {
+            c++;
+            hit(x[k]);
+          }
+        }
+      }
+      c = __reduce_add_sync(kAll, c);
+      if (lane == j) found[lane] += c;
+    }
+    unmark();
+    const uint32_t c = found[lane];
+    const uint32_t v0 = __shfl_sync(kAll, v, 0);
+    if (c) atomicAdd(tri + u, (unsigned long long)c);
+    if (__all_sync(kAll, v == v0 || c == 0)) {  // one row: one add for it
+      const uint32_t cs = __reduce_add_sync(kAll, c);
+      if (lane == 0 && cs) atomicAdd(tri + v0, (unsigned long long)cs);
+    } else if (c) {
+      atomicAdd(tri + v, (unsigned long long)c);
+    }
+    sum += c;
+    __syncwarp();
+  }
+  sum = warp_sum(sum);
+  if (lane == 0 && sum) atomicAdd(total, sum);
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < min(kHubIds, g.n); i += kTcThreads) {
+    if (S.hub[i]) atomicAdd(tri + i, (unsigned long long)S.hub[i]);
   }
 }
 
 struct TcState {
-  DevBuf a, b, lower, tri, total, out;
+  DevBuf tri, total, out;
 };
+
+// Lower lists of the degree-ordered graph rs, and their members' count.
+rg_status lower_lists(rg_graph* rs, DevBuf& off, DevBuf& adj, int64_t* entries, cudaStream_t st) {
+  const int64_t n = rs->n;
+  const uint32_t nchunks = (uint32_t)rs->nchunks;
+  int bits = 1;
+  while (bits < 32 && ((uint64_t)(n - 1) >> bits) != 0) bits++;
+  const int passes = sort_passes(bits, 2 * bits);
+  DevBuf place(true, st), k0(true, st), k1(true, st);
+  SortScratch sort(st);
+  RG_TRY(place.reserve(4 * ((size_t)nchunks + 1)));
+  uint32_t* pl = place.as<uint32_t>();
+  const unsigned blocks =
+      (unsigned)std::max<int64_t>(1, std::min<int64_t>((rs->nchunks * 32 + 255) / 256, (int64_t)device_sms() * 8));
+  upper_pairs<false><<<blocks, 256, 0, st>>>(rs->view(), rs->chunk_v.as<uint32_t>(), nchunks, pl, nullptr, bits,
+                                             nullptr, passes, nullptr);
+  RG_CUDA(cudaGetLastError());
+  RG_TRY(scan_u32(ctx().ws, pl, pl, nchunks, st));
+  uint32_t k = 0;
+  RG_TRY(read_small(pl + nchunks, &k, 4, st));
+  *entries = k;
+  if (k == 0) return RG_OK;
+  RG_TRY(k0.reserve(8 * (size_t)k));
+  RG_TRY(k1.reserve(8 * (size_t)k));
+  RG_TRY(sort_begin(sort, k, passes, st));
+  upper_pairs<true><<<blocks, 256, 0, st>>>(rs->view(), rs->chunk_v.as<uint32_t>(), nchunks, nullptr, pl, bits,
+                                            k0.as<uint64_t>(), passes, sort_counts(sort));
+  RG_CUDA(cudaGetLastError());
+  uint64_t *key = k0.as<uint64_t>(), *other = k1.as<uint64_t>();
+  RG_TRY(sort_run(sort, &key, &other, k, bits, 2 * bits, st));
+  g_timing.kernel_launches += 3 + passes;
+  // (repeats are dropped, as the loaders drop them)
+  return csr_from_sorted_rows(ctx().ws, key, k, bits, n, true, off, adj, entries, sort, "lower lists", st);
+}
 
 }  // namespace
 
@@ -159,6 +273,11 @@ rg_status triangle_run(rg_graph* g, uint64_t* h_counts, uint64_t* total_out) {
   const int64_t n = g->n, m = g->m;
   static thread_local TcState S;
   CallTimer timer(g);
+  RG_TRY(S.tri.reserve(8 * (size_t)n));
+  RG_TRY(S.total.reserve(16));
+  RG_TRY(S.out.reserve(8 * (size_t)n));
+  unsigned long long* tri = S.tri.as<unsigned long long>();
+  unsigned long long* total = S.total.as<unsigned long long>();
   // degree order (the relabelled graph of the sort, or g itself when sorted)
   rg_graph* rs = g;
   rg_graph* tmp = nullptr;
@@ -166,77 +285,38 @@ rg_status triangle_run(rg_graph* g, uint64_t* h_counts, uint64_t* total_out) {
     RG_TRY(rg_graph_degree_sort(g, &tmp, nullptr));
     rs = tmp;
   }
-  // neighbour lists sorted: the device CSR builder over rs's entries (every
-  // entry appears twice after symmetrising; the repeats are dropped)
-  rg_graph* gt = nullptr;
-  rg_status s = RG_OK;
-  if (m > 0) {
-    s = S.a.reserve(4 * (size_t)m);
-    if (s == RG_OK) s = S.b.reserve(4 * (size_t)m);
-    if (s == RG_OK) {
-      const int64_t blocks = std::min<int64_t>((rs->nchunks * 32 + 255) / 256, (int64_t)device_sms() * 8);
-      expand_entries<<<(unsigned)std::max<int64_t>(blocks, 1), 256, 0, st>>>(
-          rs->view(), rs->chunk_v.as<uint32_t>(), (uint32_t)rs->nchunks, S.a.as<uint32_t>(), S.b.as<uint32_t>());
-      const cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) s = cuda_fail(e, "expand_entries", __FILE__, __LINE__);
-    }
-    if (s == RG_OK) s = rg_graph_create_from_edges(n, m, S.a.as<uint32_t>(), S.b.as<uint32_t>(), 1, &gt);
-  } else {
-    s = rg_graph_create_from_edges(n, 0, nullptr, nullptr, 1, &gt);
-  }
-  if (s != RG_OK) {
-    if (tmp) rg_graph_free(tmp);
-    return s;
-  }
-  auto cleanup = [&]() {
-    rg_graph_free(gt);
-    if (tmp) rg_graph_free(tmp);
-  };
-  if ((s = S.lower.reserve(4 * (size_t)n)) != RG_OK || (s = S.tri.reserve(8 * (size_t)n)) != RG_OK ||
-      (s = S.total.reserve(8)) != RG_OK || (s = S.out.reserve(8 * (size_t)n)) != RG_OK) {
-    cleanup();
-    return s;
-  }
-  unsigned long long* tri = S.tri.as<unsigned long long>();
-  unsigned long long* total = S.total.as<unsigned long long>();
-  cudaError_t e = cudaMemsetAsync(tri, 0, 8 * n, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(total, 0, 8, st);
-  if (e == cudaSuccess && gt->m > 0) {
-    const int vblocks = (int)std::min<int64_t>((n + 255) / 256, (int64_t)device_sms() * 16);
-    lower_degrees<<<vblocks, 256, 0, st>>>(gt->view(), S.lower.as<uint32_t>());
-    // hub counters: as many of the first ids as a CTA's shared memory holds
-    const bool hubs = g_opts.hub_smem_kb > 0;
-    const uint32_t H = hubs ? (uint32_t)std::min<int64_t>(n, g_opts.hub_smem_kb * 1024 / 8) : 0;
-    auto kern = hubs ? count_triangles<true> : count_triangles<false>;
-    const size_t dyn = 8 * (size_t)H;
-    static std::atomic<uint64_t> limit_set[2];  // count_triangles<false>, <true>
-    e = allow_max_dyn_smem(limit_set[hubs ? 1 : 0], kern) == RG_OK ? cudaSuccess : cudaErrorInvalidValue;
-    int per_sm = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, dyn);
-    const int64_t grid = std::min<int64_t>((gt->nchunks * 32 + 255) / 256, (int64_t)device_sms() * std::max(per_sm, 1));
-    if (e == cudaSuccess) {
+  uint64_t t = 0;
+  auto count = [&]() -> rg_status {
+    RG_CUDA(cudaMemsetAsync(tri, 0, 8 * n, st));
+    RG_CUDA(cudaMemsetAsync(total, 0, 16, st));
+    DevBuf off(true, st), adj(true, st);
+    int64_t k = 0;
+    if (m > 0) RG_TRY(lower_lists(rs, off, adj, &k, st));
+    if (k > 0) {
+      static std::atomic<uint64_t> limit_set{0};
+      RG_TRY(allow_max_dyn_smem(limit_set, count_triangles));
+      const int64_t grid = std::min<int64_t>((m + 32 * kTcWarps - 1) / (32 * kTcWarps), (int64_t)device_sms() * 4);
       kt_begin(st);
-      kern<<<(unsigned)std::max<int64_t>(grid, 1), 256, dyn, st>>>(gt->view(), gt->chunk_v.as<uint32_t>(),
-                                                                    (uint32_t)gt->nchunks, S.lower.as<uint32_t>(),
-                                                                    tri, H, total);
+      count_triangles<<<(unsigned)grid, kTcThreads, sizeof(TcShared), st>>>(
+          rs->view(), rs->chunk_v.as<uint32_t>(), off.as<uint32_t>(), adj.as<uint32_t>(),
+          (unsigned int*)(total + 1), tri, total);
       kt_end(st);
-      e = cudaGetLastError();
-      g_timing.kernel_launches += 2;
+      RG_CUDA(cudaGetLastError());
+      g_timing.kernel_launches++;
       g_timing.edge_launches++;
     }
-  }
-  uint64_t t = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&t, total, 8, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess && h_counts) {  // by original id: rs's permutation maps g's ids to gt's
-    const int64_t blocks = std::min<int64_t>((n + 255) / 256, (int64_t)device_sms() * 32);
-    gather_kernel<unsigned long long><<<(unsigned)blocks, 256, 0, st>>>(
-        tri, (g->sorted ? g : rs)->new_ids.as<uint32_t>(), n, S.out.as<unsigned long long>());
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h_counts, S.out.p, 8 * n, cudaMemcpyDeviceToHost, st);
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cleanup();
-  if (e != cudaSuccess) return cuda_fail(e, "triangle count", __FILE__, __LINE__);
+    if (h_counts) {  // by original id: rs's permutation maps g's ids to the order's
+      const int64_t blocks = std::min<int64_t>((n + 255) / 256, (int64_t)device_sms() * 32);
+      gather_kernel<unsigned long long><<<(unsigned)blocks, 256, 0, st>>>(tri, rs->new_ids.as<uint32_t>(), n,
+                                                                          S.out.as<unsigned long long>());
+      RG_CUDA(cudaGetLastError());
+      RG_CUDA(cudaMemcpyAsync(h_counts, S.out.p, 8 * n, cudaMemcpyDeviceToHost, st));
+    }
+    return read_small(total, &t, 8, st);
+  };
+  const rg_status s = count();
+  if (tmp) rg_graph_free(tmp);
+  RG_TRY(s);
   RG_TRY(timer.stop());
   g_timing.edges_traversed = m;
   if (total_out) *total_out = t;
