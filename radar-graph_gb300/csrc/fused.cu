@@ -42,10 +42,12 @@ constexpr int kBuf = kFlushAt + 32;
 constexpr unsigned kAll = 0xffffffffu;
 constexpr unsigned kSpinLimit = 1u << 21;  // polls of the grid barrier: a second or two
 
-// One level's frontier: queue lengths, members and their degree sum.
+// One level's frontier: queue lengths, members and their degree sum
+// (PageRankDelta: and the round's L1).
 struct Slot {
   unsigned int ns, nl, count, pad;
-  unsigned long long degsum, pad2;
+  unsigned long long degsum;
+  double l1;
 };
 
 // A 128-bit sum that CTAs add to without waiting for a carry: 43-bit limbs in
@@ -101,6 +103,7 @@ __device__ __forceinline__ Slot read_slot(const Slot* s) {
   r.nl = __ldcg(&s->nl);
   r.count = __ldcg(&s->count);
   r.degsum = __ldcg(&s->degsum);
+  r.l1 = __ldcg(&s->l1);
   return r;
 }
 
@@ -1052,6 +1055,191 @@ __global__ void __launch_bounds__(kFT, 1) pagerank_fused(const __grid_constant__
 }
 
 // ---------------------------------------------------------------------------
+// PageRankDelta (PageRankDelta.C:98-155)
+// ---------------------------------------------------------------------------
+struct PrdArgs {
+  DevGraph out, in;
+  const uint32_t* new_ids;
+  double *p, *ngh, *c;
+  uint32_t* bits;  // the frontier, as the last filter left it
+  Queues rows;     // every row with in-edges (whole runs only)
+  Queues q[2];
+  int64_t start;   // rounds already run level by level (0: a whole run)
+  int64_t max_iters;
+  int64_t threshold;
+  bool allow_pull;
+  double one_over_n, added;
+  double* ranks_out;  // original-id order; null: not wanted (or not sorted)
+  Ctl* ctl;
+  volatile uint64_t* info;  // mapped: rounds, L1 (bits), edges, done
+};
+
+// A round pushes the frontier's contributions or, a dense one, sums every row's
+// (c is 0 outside the frontier); a filter pass over the vertices then forms the
+// next frontier as prd_filter does, skipping words that nothing reached and that
+// held no member.  A run can be taken over after its dense first rounds, which
+// large graphs sweep with a launch of their own.
+__global__ void __launch_bounds__(kFT, 1) prd_fused(const __grid_constant__ PrdArgs A) {
+  __shared__ Shared sh;
+  __shared__ Member buf[kFWarps][kBuf];
+  __shared__ double s_l1[kFWarps];
+  Grid grid;
+  Appender<false> ap{buf[threadIdx.x >> 5], &sh, 0};
+  begin(grid, &sh, A.ctl);
+  const uint32_t n = A.out.n, nwords = (n + 31) / 32;
+  const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t warp = tid >> 5, nwarps = nthreads >> 5;
+  uint32_t rs = 0, rl = 0;  // entries of the row queues
+  if (A.start == 0) {
+    for (uint32_t w = warp; w < nwords; w += nwarps) {
+      const bool in = w * 32 + lane < n;
+      const uint32_t v = in ? w * 32 + lane : n - 1;
+      if (in) {
+        A.p[v] = 0.0;
+        A.ngh[v] = 0.0;
+        const uint32_t d = A.out.off[v + 1] - A.out.off[v];
+        A.c[v] = d ? A.one_over_n / d : 0.0;
+      }
+      if (lane == 0) A.bits[w] = 0u;
+      const uint32_t b = A.in.off[v], e = A.in.off[v + 1];
+      ap.add(in && e > b, v, b, e, A.rows, &A.ctl->lv[3], 0, 0);
+    }
+    ap.finish(A.rows, &A.ctl->lv[3], 0, 0);
+    if (!grid.sync()) return;
+    const Slot r = read_slot(&A.ctl->lv[3]);
+    rs = r.ns;
+    rl = r.nl;
+    if (threadIdx.x == 0) {
+      sh.slot = Slot{};  // every vertex starts in the frontier
+      sh.slot.count = n;
+      sh.slot.degsum = A.out.m;
+    }
+    __syncthreads();
+  } else {
+    for (uint32_t w = warp; w < nwords; w += nwarps) {
+      const uint32_t x = A.bits[w];
+      if (!x) continue;
+      const uint32_t v = min(w * 32 + lane, n - 1);
+      ap.add((x >> lane) & 1u, v, A.out.off[v], A.out.off[v + 1], A.q[0], &A.ctl->lv[0], 0, 0);
+    }
+    ap.finish(A.q[0], &A.ctl->lv[0], 0, 0);
+    if (!grid.sync(&A.ctl->lv[0])) return;
+  }
+  int cq = 0;
+  int64_t k = 0, round = A.start;  // k: rounds of this launch
+  unsigned long long edges = 0;
+  double l1 = 0.0;
+  while (round++ < A.max_iters) {
+    const Slot c = sh.slot;
+    Slot* ns = &A.ctl->lv[(k + 1) % 3];
+    if (tid == 0) A.ctl->lv[(k + 2) % 3] = Slot{};
+    k++;
+    edges += c.degsum;
+    const bool whole = A.start == 0 && k == 1;  // the queue does not hold the first frontier of a whole run
+    if (whole || (A.start == 0 && A.allow_pull && (int64_t)(c.count + c.degsum) > A.threshold)) {
+      const uint32_t gwarp = (uint32_t)(wid * gridDim.x + blockIdx.x);
+      for (uint32_t i = gwarp; i < rl; i += nwarps) {
+        const uint4 it = A.rows.large[i];
+        uint32_t u[4];
+        double x[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) u[j] = it.y + 32 * j + lane < it.z ? A.in.adj[it.y + 32 * j + lane] : kNone;
+#pragma unroll
+        for (int j = 0; j < 4; j++) x[j] = u[j] != kNone ? A.c[u[j]] : 0.0;
+        const double s = warp_sum((x[0] + x[1]) + (x[2] + x[3]));
+        if (lane == 0) {
+          if (it.w == 3u) A.ngh[it.x] = s;  // the row's only piece
+          else if (s != 0.0) atomicAdd(A.ngh + it.x, s);
+        }
+      }
+      for (uint32_t i = gwarp; i < (rs + 7) / 8; i += nwarps) {
+        const uint32_t j = i * 8 + (lane >> 2);
+        const uint4 it = j < rs ? A.rows.small[j] : make_uint4(0, 0, 0, 0);
+        double s = 0.0;
+        for (uint32_t e0 = it.y + (lane & 3); __any_sync(kAll, e0 < it.z); e0 += 16) {
+          uint32_t u[4];
+          double x[4];
+#pragma unroll
+          for (int q = 0; q < 4; q++) u[q] = e0 + 4 * q < it.z ? A.in.adj[e0 + 4 * q] : kNone;
+#pragma unroll
+          for (int q = 0; q < 4; q++) x[q] = u[q] != kNone ? A.c[u[q]] : 0.0;
+          s += (x[0] + x[1]) + (x[2] + x[3]);
+        }
+        s += __shfl_xor_sync(kAll, s, 1);
+        s += __shfl_xor_sync(kAll, s, 2);
+        if (j < rs && (lane & 3) == 0) A.ngh[it.x] = s;
+      }
+    } else {
+      expand(A.out, A.q[cq], 0, c.ns, 0, c.nl, [&](const bool (&in)[4], uint32_t s, const uint32_t (&d)[4]) {
+        const double x = A.c[s];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          if (in[j]) atomicAdd(A.ngh + d[j], x);
+        }
+      });
+    }
+    if (!grid.sync()) return;
+    const Queues nq = A.q[cq ^ 1];
+    double local = 0.0;
+    for (uint32_t w = warp; w < nwords; w += nwarps) {
+      const bool in = w * 32 + lane < n;
+      const uint32_t v = in ? w * 32 + lane : n - 1;
+      const double g = in ? A.ngh[v] : 0.0;
+      const uint32_t old = A.bits[w];
+      // nothing arrived and nobody was active: delta is 0, the vertex stays as it is
+      if (round > 1 && !old && !__any_sync(kAll, g != 0.0)) continue;
+      bool act = false;
+      uint32_t b = 0, e = 0;
+      if (in) {
+        b = A.out.off[v];
+        e = A.out.off[v + 1];
+        double pv = A.p[v], d;
+        if (round == 1) {  // PageRankDelta.C:46-61
+          d = __dadd_rn(__dmul_rn(kPrDamp, g), A.added);
+          pv = __dadd_rn(pv, d);
+          d = __dsub_rn(d, A.one_over_n);
+          act = fabs(d) > __dmul_rn(kPrdEps2, pv);
+          A.p[v] = pv;
+        } else {  // PageRankDelta.C:63-76
+          d = __dmul_rn(g, kPrDamp);
+          act = fabs(d) > __dmul_rn(kPrdEps2, pv);
+          if (act) A.p[v] = __dadd_rn(pv, d);
+        }
+        A.ngh[v] = 0.0;
+        A.c[v] = (act && e > b) ? __ddiv_rn(d, (double)(e - b)) : 0.0;
+        local += fabs(d);
+      }
+      const unsigned now = __ballot_sync(kAll, act);
+      if (lane == 0) A.bits[w] = now;
+      ap.add(act, v, b, e, nq, ns, 0, 0);
+    }
+    ap.finish(nq, ns, 0, 0);
+    local = warp_sum(local);
+    if (lane == 0) s_l1[wid] = local;
+    __syncthreads();
+    if (wid == 0) {
+      const double t = warp_sum(s_l1[lane]);
+      if (lane == 0 && t != 0.0) atomicAdd(&ns->l1, t);
+    }
+    if (!grid.sync(ns)) return;
+    l1 = sh.slot.l1;
+    if (l1 < kPrdEps) break;  // PageRankDelta.C:144
+    cq ^= 1;
+  }
+  if (A.ranks_out) {
+    for (uint32_t i = tid; i < n; i += nthreads) A.ranks_out[i] = A.p[A.new_ids ? A.new_ids[i] : i];
+  }
+  if (tid == 0) {
+    A.info[0] = (uint64_t)round;
+    A.info[1] = bits_of(l1);
+    A.info[2] = edges;
+    __threadfence_system();
+    A.info[3] = 1;
+  }
+}
+
+// ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
 // The largest in-degree of g (found once per graph); n if it cannot be found.
@@ -1085,7 +1273,7 @@ int64_t max_in_degree(const rg_graph* g, cudaStream_t st) {
 
 struct FusedState {
   DevBuf ctl, bits0, bits1, i32a, i32b, f64a, f64b, f64c, u64a, u64b, row, opens, closes, l1, out;
-  DevBuf qs0, qs1, ql0, ql1, first_s, first_l;
+  DevBuf qs0, qs1, qs2, ql0, ql1, ql2, first_s, first_l;
 };
 thread_local FusedState S;
 
@@ -1359,6 +1547,45 @@ rg_status pagerank_fused_run(rg_graph* g, int64_t max_iters, double* h_ranks, in
   g_timing.algorithmic_bytes = (4 * m + 4 * (n + 1) + 16 * n) * run;
   if (iters_out) *iters_out = broke ? run : max_iters + 1;
   if (l1_out) *l1_out = max_iters ? fx_to_double(U128{info[1], info[2]}) : 0.0;
+  return RG_OK;
+}
+
+rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max_iters, double* p, double* ngh,
+                        double* c, uint32_t* bits, double* ranks_out, int64_t* rounds, double* l1, bool* done) {
+  Ctx& cx = ctx();
+  cudaStream_t st = cx.stream;
+  const int64_t n = g->n, m = g->m;
+  PrdArgs A;
+  RG_TRY(S.ctl.reserve(sizeof(Ctl)));
+  RG_TRY(queue_pair(n, m, S.qs0, S.ql0, &A.q[0]));
+  RG_TRY(queue_pair(n, m, S.qs1, S.ql1, &A.q[1]));
+  if (start == 0) RG_TRY(queue_pair(n, m, S.qs2, S.ql2, &A.rows));
+  else A.rows = Queues{};
+  A.out = g->view();
+  A.in = g->in_view();
+  A.new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
+  A.p = p;
+  A.ngh = ngh;
+  A.c = c;
+  A.bits = bits;
+  A.start = start;
+  A.max_iters = max_iters;
+  A.threshold = dense_threshold(g);
+  A.allow_pull = allow_pull;
+  A.one_over_n = 1 / (double)n;
+  A.added = (1 - kPrDamp) * A.one_over_n;
+  A.ranks_out = ranks_out;
+  A.ctl = S.ctl.as<Ctl>();
+  A.info = cx.ws.h_info_dev;
+  volatile uint64_t* info = cx.ws.h_info;
+  info[3] = 0;
+  RG_TRY(launch_fused(prd_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
+  RG_CUDA(cudaStreamSynchronize(st));
+  *done = info[3] == 1;
+  if (!*done) return RG_OK;
+  *rounds = (int64_t)info[0];
+  *l1 = double_of(info[1]);
+  g_timing.edges_traversed += (int64_t)info[2];
   return RG_OK;
 }
 

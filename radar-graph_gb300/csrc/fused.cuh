@@ -32,10 +32,14 @@ constexpr int64_t kFusedPrRows = 12000;
 //             (1015 / 953): the same line
 //   PageRank  20 iterations: 2^10 97 / 217, 2^16 304 / 481 (183 / 220), 2^17
 //             546 / 648 (298 / 342), 2^18 1337 / 1033 (573 / 532): 4e6 edges
+//   PageRankDelta  whole, against dense rounds swept and the rest handed over:
+//             2^10 139 / 398 (85 / 238), 2^18 494 / 688 (332 / 440), 2^19
+//             774 / 815 (605 / 598), 2^20 1441 / 1164 (1146 / 872): 1.7e7 edges
 constexpr int64_t kFusedBfsEdges = INT64_MAX;
 constexpr int64_t kFusedBcEdges = 3 << 23;
 constexpr int64_t kFusedRadiiEdges = 3 << 23;
 constexpr int64_t kFusedPagerankEdges = 5 << 20;
+constexpr int64_t kFusedPrdEdges = 1 << 24;
 
 // Whether a call on g may take the one-launch path: small enough, and no
 // per-level records (rg_set_trace) are asked for.
@@ -53,7 +57,21 @@ rg_status radii_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned lon
 rg_status pagerank_fused_run(rg_graph* g, int64_t max_iters, double* h_ranks, int64_t* iters_out, double* l1_out,
                              bool* done);
 
+// PageRankDelta from round `start` on (0: a whole run, which initialises p, ngh
+// and c itself; else p, c and the frontier's bits as the filter of round `start`
+// left them, ngh 0).  Synchronises; *rounds as the reference counts them.
+// ranks_out (device, original ids) may be null.
+rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max_iters, double* p, double* ngh,
+                        double* c, uint32_t* bits, double* ranks_out, int64_t* rounds, double* l1, bool* done);
+
 constexpr double kPrDamp = 0.85;  // PageRank.C:126
+constexpr double kPrdEps = 0.0000001, kPrdEps2 = 0.01;  // PageRankDelta.C:103-104
+
+// The exact pull of pagerank.cu over signed contributions (PageRankDelta's):
+// acc[v] = sum of c over v's in-neighbours as a 128-bit two's complement fixed
+// point number.  acc must be 0 in the rows that cross a step of kExactStep edges.
+constexpr uint32_t kExactStep = 512;
+rg_status exact_pull_signed(rg_graph* g, const double* c, U128* acc, cudaStream_t st);
 
 // acc[v] += x for a 128-bit sum shared with other warps: the low word's
 // atomic returns the old value, so the carry out of it is known and goes into

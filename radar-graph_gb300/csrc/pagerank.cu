@@ -139,7 +139,8 @@ __global__ void __launch_bounds__(kSweepThreads) pr_push_sweep(DevGraph g, const
 // kCache (degree-sorted graphs): the contributions of the H hubs (ids < H)
 // are copied into shared memory once per CTA -- RADAR's duplication of hub
 // data, used here for the reads of a pull instead of the writes of a push.
-template <bool kCache, int kItems, int kMode>
+// kSigned: the contributions may be negative (PageRankDelta's).
+template <bool kCache, int kItems, int kMode, bool kSigned = false>
 __global__ void __launch_bounds__(kCache ? 1024 : kPullThreads)
     pr_pull_sweep(DevGraph g, const uint32_t* __restrict__ chunk_v, uint32_t nchunks,
                   const double* __restrict__ contrib, U128* acc, uint32_t H, const U128* l1_prev) {
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(kCache ? 1024 : kPullThreads)
               do { v++; nxt = g.off[v + 1]; } while (ee >= nxt);
               row = v;
             }
-            add128(part, fx_from_double(x[j]));
+            add128(part, kSigned ? fx_from_signed(x[j]) : fx_from_double(x[j]));
           }
         }
         cont = nxt > e + kItems;
@@ -367,6 +368,32 @@ struct PrState {
 };
 
 }  // namespace
+
+rg_status exact_pull_signed(rg_graph* g, const double* c, U128* acc, cudaStream_t st) {
+  auto kern = pr_pull_sweep<false, 16, 1, true>;
+  static std::atomic<uint64_t> carveout_set{0};
+  RG_TRY(once_per_device(carveout_set, [&]() -> rg_status {
+    RG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 0));
+    return RG_OK;
+  }));
+  static std::atomic<int> resident{0};
+  int per_sm = resident.load(std::memory_order_relaxed);
+  if (!per_sm) {
+    RG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kPullThreads, 0));
+    per_sm = std::max(per_sm, 1);
+    resident.store(per_sm, std::memory_order_relaxed);
+  }
+  const int64_t grid = std::min<int64_t>((int64_t)device_sms() * per_sm,
+                                         std::max<int64_t>((g->nchunks * 32 + kPullThreads - 1) / kPullThreads, 1));
+  static_assert(kExactStep == 32 * 16, "a warp step of 16 edges per lane");
+  kt_begin(st);
+  kern<<<(unsigned)grid, kPullThreads, 0, st>>>(g->in_view(), g->in_chunks(), (uint32_t)g->nchunks, c, acc, 0u, nullptr);
+  kt_end(st);
+  RG_CUDA(cudaGetLastError());
+  g_timing.kernel_launches++;
+  g_timing.edge_launches++;
+  return RG_OK;
+}
 
 rg_status pagerank_run(rg_graph* g, int variant, int64_t max_iters, double* h_ranks, int64_t* iters_out,
                        double* l1_out, uint32_t hub_h) {

@@ -80,6 +80,18 @@ __host__ __device__ __forceinline__ U128 fx_from_double(double x) {
   return U128{0ull, 0ull};
 }
 
+// The same for x in (-8, 8), as a two's complement number (PageRankDelta's
+// contributions: at least 0.01 (0.15/n)/deg in size, which is above 2^-72).
+__host__ __device__ __forceinline__ U128 fx_from_signed(double x) {
+  const unsigned long long b = bits_of(x);
+  U128 m = fx_from_double(double_of(b & ~(1ull << 63)));
+  if (b >> 63) {
+    m.lo = ~m.lo + 1ull;
+    m.hi = ~m.hi + (m.lo == 0ull ? 1ull : 0ull);
+  }
+  return m;
+}
+
 // s * 2^-124 rounded to the nearest double, ties to even.
 __host__ __device__ __forceinline__ double fx_to_double(const U128& s) {
   int t;  // position of the leading one
@@ -107,6 +119,14 @@ __host__ __device__ __forceinline__ double fx_to_double(const U128& s) {
   }
   const unsigned long long ex = (unsigned long long)(t - kPrFrac + 1023);
   return double_of((ex << 52) | (M & 0xFFFFFFFFFFFFFull));
+}
+
+// fx_to_double of a two's complement number.
+__host__ __device__ __forceinline__ double fx_to_signed(U128 s) {
+  if (!(s.hi >> 63)) return fx_to_double(s);
+  s.lo = ~s.lo + 1ull;
+  s.hi = ~s.hi + (s.lo == 0ull ? 1ull : 0ull);
+  return -fx_to_double(s);
 }
 
 __host__ __device__ __forceinline__ int clz32(uint32_t x) {
