@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "app_common.cuh"
+#include "fused.cuh"
 
 namespace rg {
 namespace {
@@ -386,6 +387,23 @@ rg_status bc_multi_run(rg_graph* g, const uint32_t* src_orig, int k, double* h_o
   RG_TRY(get_ctx(&cx));
   cudaStream_t st = cx->stream;
   const int64_t n = g->n;
+  if (fused_fits(g, kFusedBcRowsEdges / k)) {
+    DevBuf rows(true, st);
+    if (!d_out) RG_TRY(rows.reserve(8 * (size_t)n * k));
+    double* out = d_out ? d_out : rows.as<double>();
+    CallTimer timer(g);
+    bool done = false;
+    int64_t levels = 0;
+    RG_TRY(bc_rows_fused_run(g, src_orig, k, out, &levels, &done));
+    if (done) {
+      RG_TRY(timer.stop());
+      if (h_out) RG_CUDA(cudaMemcpyAsync(h_out, out, 8 * (size_t)n * k, cudaMemcpyDeviceToHost, st));
+      RG_CUDA(cudaStreamSynchronize(st));
+      g_timing.algorithmic_bytes = 4 * g_timing.edges_traversed + (int64_t)k * 16 * n + 24 * n;
+      if (levels_out) *levels_out = levels - 1;
+      return RG_OK;
+    }
+  }
   const int64_t nwords = (n + 31) / 32;
   const int kk = (k + 3) & ~3;
   const size_t cells = (size_t)n * kk;

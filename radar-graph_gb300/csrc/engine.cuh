@@ -503,11 +503,18 @@ __global__ void __launch_bounds__(kThreads) push_lbs(DevGraph g, const uint32_t*
 // segmented OR scan per warp step, one atomicOr and activation per row piece
 // that adds bits.
 // ---------------------------------------------------------------------------
-static __device__ __forceinline__ void mask_flush(const unsigned long long* __restrict__ visited,
-                                            unsigned long long* next_visited, uint32_t* next_bits, uint32_t row,
-                                            unsigned long long part) {
+// kStable: no launch in flight writes the masks, so they are read through the
+// read-only path; a kernel that also writes them (between barriers) reads plain.
+template <bool kStable>
+static __device__ __forceinline__ unsigned long long mask_load(const unsigned long long* p) {
+  return kStable ? __ldg(p) : *p;
+}
+
+template <bool kStable>
+static __device__ __forceinline__ void mask_flush(const unsigned long long* visited, unsigned long long* next_visited,
+                                                  uint32_t* next_bits, uint32_t row, unsigned long long part) {
   if (!part) return;
-  const unsigned long long vd = __ldg(visited + row);
+  const unsigned long long vd = mask_load<kStable>(visited + row);
   const unsigned long long w = part & ~vd;
   if (!w) return;
   atomicOr(next_visited + row, w);
@@ -521,87 +528,94 @@ static __device__ __forceinline__ void mask_flush(const unsigned long long* __re
 // gathered: in the last dense rounds that is most of the graph (RMAT s22,
 // 64 samples: 64 % of the edges in round 4, 99.8 % in round 5), and the hub
 // rows, which hold the most edges, fill first.  full = 0 gathers every row.
+template <int kItems, bool kStable>
+static __device__ __forceinline__ void mask_pull_chunk(const DevGraph& g, uint32_t c, uint32_t vlo, uint32_t vhi,
+                                                       const unsigned long long* visited,
+                                                       unsigned long long* next_visited, uint32_t* next_bits,
+                                                       unsigned long long full) {
+  static_assert(kItems == 8 || kItems == 16, "8 or 16 edges per lane");
+  constexpr int kStep = 32 * kItems;
+  constexpr int kBatch = 8;  // gathers in flight per lane at a time
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int r = 0; r < kSweepChunk / kStep; r++) {
+    const uint32_t e = c * kSweepChunk + r * kStep + lane * kItems;
+    uint32_t row = kNone;
+    unsigned long long part = 0;
+    if (e < g.m) {
+      uint32_t v = upper_index(g.off, vlo, vhi, e);
+      uint32_t nxt = g.off[v + 1];
+      // the rows of the lane's edges first, then gathers only for rows
+      // that can still grow.  8 edges per lane keep the rows in registers;
+      // 16 walk them again while accumulating (the offsets hit L1), which
+      // keeps the kernel at 8 gathers and 8 row ids per lane
+      constexpr bool kKeepRows = kItems <= 8;
+      uint32_t rowi[kKeepRows ? kItems : 1];
+      unsigned need = 0;
+      {
+        uint32_t rv = v, rn = nxt;
+        bool open = full == 0ull || (mask_load<kStable>(visited + rv) & full) != full;
+#pragma unroll
+        for (int i = 0; i < kItems; i++) {
+          const uint32_t ee = e + i;
+          if (ee < g.m && ee >= rn) {
+            do { rv++; rn = g.off[rv + 1]; } while (ee >= rn);
+            open = full == 0ull || (mask_load<kStable>(visited + rv) & full) != full;
+          }
+          if (kKeepRows) rowi[kKeepRows ? i : 0] = rv;
+          if (ee < g.m && open) need |= 1u << i;
+        }
+      }
+      row = v;
+#pragma unroll
+      for (int b = 0; b < kItems; b += kBatch) {
+        if (e + b >= g.m) break;
+        // this batch's neighbour ids (in bounds: adj is padded by 8
+        // entries and the batch starts before m)
+        const U32x8 w = ld_stream_v8(g.adj + e + b);
+        unsigned long long x[kBatch];
+#pragma unroll
+        for (int j = 0; j < kBatch; j++) x[j] = ((need >> (b + j)) & 1u) ? mask_load<kStable>(visited + w.v[j]) : 0ull;
+#pragma unroll
+        for (int j = 0; j < kBatch; j++) {
+          const int i = b + j;
+          const uint32_t ee = e + i;
+          if (ee >= g.m) break;
+          const bool ends = kKeepRows ? rowi[kKeepRows ? i : 0] != row : ee >= nxt;
+          if (ends) {
+            mask_flush<kStable>(visited, next_visited, next_bits, row, part);  // a row piece that ends in this lane
+            part = 0;
+            if (kKeepRows) {
+              row = rowi[kKeepRows ? i : 0];
+            } else {
+              do { v++; nxt = g.off[v + 1]; } while (ee >= nxt);
+              row = v;
+            }
+          }
+          part |= x[j];
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, part, o);
+      const uint32_t tr = __shfl_up_sync(0xffffffffu, row, o);
+      if (lane >= o && tr == row) part |= t;
+    }
+    const uint32_t next_row = __shfl_down_sync(0xffffffffu, row, 1);
+    if (row != kNone && (lane == 31 || next_row != row)) mask_flush<kStable>(visited, next_visited, next_bits, row, part);
+  }
+}
+
 template <int kItems>
 static __global__ void __launch_bounds__(256) mask_pull_sweep(DevGraph g, const uint32_t* __restrict__ chunk_v,
                                                         uint32_t nchunks, const unsigned long long* __restrict__ visited,
                                                         unsigned long long* next_visited, uint32_t* next_bits,
                                                         unsigned long long full) {
-  static_assert(kItems == 8 || kItems == 16, "8 or 16 edges per lane");
-  constexpr int kStep = 32 * kItems;
-  constexpr int kBatch = 8;  // gathers in flight per lane at a time
-  const int lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t c = warp; c < nchunks; c += nwarps) {
-    const uint32_t vlo = chunk_v[c], vhi = chunk_v[c + 1];
-#pragma unroll
-    for (int r = 0; r < kSweepChunk / kStep; r++) {
-      const uint32_t e = c * kSweepChunk + r * kStep + lane * kItems;
-      uint32_t row = kNone;
-      unsigned long long part = 0;
-      if (e < g.m) {
-        uint32_t v = upper_index(g.off, vlo, vhi, e);
-        uint32_t nxt = g.off[v + 1];
-        // the rows of the lane's edges first, then gathers only for rows
-        // that can still grow.  8 edges per lane keep the rows in registers;
-        // 16 walk them again while accumulating (the offsets hit L1), which
-        // keeps the kernel at 8 gathers and 8 row ids per lane
-        constexpr bool kKeepRows = kItems <= 8;
-        uint32_t rowi[kKeepRows ? kItems : 1];
-        unsigned need = 0;
-        {
-          uint32_t rv = v, rn = nxt;
-          bool open = full == 0ull || (__ldg(visited + rv) & full) != full;
-#pragma unroll
-          for (int i = 0; i < kItems; i++) {
-            const uint32_t ee = e + i;
-            if (ee < g.m && ee >= rn) {
-              do { rv++; rn = g.off[rv + 1]; } while (ee >= rn);
-              open = full == 0ull || (__ldg(visited + rv) & full) != full;
-            }
-            if (kKeepRows) rowi[kKeepRows ? i : 0] = rv;
-            if (ee < g.m && open) need |= 1u << i;
-          }
-        }
-        row = v;
-#pragma unroll
-        for (int b = 0; b < kItems; b += kBatch) {
-          if (e + b >= g.m) break;
-          // this batch's neighbour ids (in bounds: adj is padded by 8
-          // entries and the batch starts before m)
-          const U32x8 w = ld_stream_v8(g.adj + e + b);
-          unsigned long long x[kBatch];
-#pragma unroll
-          for (int j = 0; j < kBatch; j++) x[j] = ((need >> (b + j)) & 1u) ? __ldg(visited + w.v[j]) : 0ull;
-#pragma unroll
-          for (int j = 0; j < kBatch; j++) {
-            const int i = b + j;
-            const uint32_t ee = e + i;
-            if (ee >= g.m) break;
-            const bool ends = kKeepRows ? rowi[kKeepRows ? i : 0] != row : ee >= nxt;
-            if (ends) {
-              mask_flush(visited, next_visited, next_bits, row, part);  // a row piece that ends in this lane
-              part = 0;
-              if (kKeepRows) {
-                row = rowi[kKeepRows ? i : 0];
-              } else {
-                do { v++; nxt = g.off[v + 1]; } while (ee >= nxt);
-                row = v;
-              }
-            }
-            part |= x[j];
-          }
-        }
-      }
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long t = __shfl_up_sync(0xffffffffu, part, o);
-        const uint32_t tr = __shfl_up_sync(0xffffffffu, row, o);
-        if (lane >= o && tr == row) part |= t;
-      }
-      const uint32_t next_row = __shfl_down_sync(0xffffffffu, row, 1);
-      if (row != kNone && (lane == 31 || next_row != row)) mask_flush(visited, next_visited, next_bits, row, part);
-    }
+    mask_pull_chunk<kItems, true>(g, c, chunk_v[c], chunk_v[c + 1], visited, next_visited, next_bits, full);
   }
 }
 

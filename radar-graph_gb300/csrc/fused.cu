@@ -488,40 +488,42 @@ __global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
 struct BcArgs {
   DevGraph g;  // the lists the forward phase pushes along (the backward phase reads them the other way)
   const uint32_t* new_ids;
-  uint32_t source;   // original id
+  uint32_t source[64];  // original ids
+  int k;
+  bool rows;  // k independent sources, source s to row s of deps_out; else one source, whose dependencies add to deps
   int32_t* lvl;
   double *sigma, *deps;
-  double* deps_out;  // original-id order after the last source; null otherwise
+  double* deps_out;  // original-id order; null: deps keeps the result
   Queues q;          // every level's frontier, one after another
   uint32_t *first_small, *first_large;  // per level, levels + 1 entries
+  size_t n_small, n_large;              // a group's share of the queues
   bool first_source;
   Ctl* ctl;
-  volatile uint64_t* info;  // mapped, summed over the sources: levels, edges, done
+  volatile uint64_t* info;  // mapped, four words per source (or summed over the calls): levels, edges, -, done
 };
 
 // Forward: sigma is pushed along the frontier's edges to vertices of the next
 // level.  Backward: every vertex sums the dependencies of its successors, so
-// only the pieces of large vertices need an atomic add.
-__global__ void __launch_bounds__(kFT, 1) bc_fused(BcArgs A) {
-  __shared__ Shared sh;
-  __shared__ Member buf[kFWarps][kBuf];
-  Grid grid;
-  Appender<true> ap{buf[threadIdx.x >> 5], &sh, 0};
-  begin(grid, &sh, A.ctl);
+// only the pieces of large vertices need an atomic add.  The CTAs of one
+// blockIdx.y are a group with arrays and a barrier of its own; independent
+// sources are dealt out to the groups, whose waits and loads overlap.
+__device__ bool bc_source(const BcArgs& A, int s, Grid& grid, Appender<true>& ap, Shared& sh) {
   const uint32_t n = A.g.n;
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
   const int lane = threadIdx.x & 31;
-  const uint32_t src = A.new_ids ? A.new_ids[A.source] : A.source;
+  const uint32_t src = A.new_ids ? A.new_ids[A.source[s]] : A.source[s];
   for (uint32_t i = tid; i < n; i += nthreads) {
     A.lvl[i] = i == src ? 0 : -1;
     A.sigma[i] = i == src ? 1.0 : 0.0;
     if (A.first_source) A.deps[i] = 0.0;
   }
   if ((tid >> 5) == 0) {
+    if (lane < 3) A.ctl->lv[lane] = Slot{};
+    __syncwarp();
     ap.add(lane == 0, src, A.g.off[src], A.g.off[src + 1], A.q, &A.ctl->lv[0], 0, 0);
     ap.finish(A.q, &A.ctl->lv[0], 0, 0);
   }
-  if (!grid.sync(&A.ctl->lv[0])) return;
+  if (!grid.sync(&A.ctl->lv[0])) return false;
   uint32_t sbase = 0, lbase = 0;
   int32_t level = 0;
   unsigned long long edges = 0;
@@ -562,11 +564,11 @@ __global__ void __launch_bounds__(kFT, 1) bc_fused(BcArgs A) {
     ap.finish(A.q, ns, sn, ln);
     sbase = sn;
     lbase = ln;
-    if (!grid.sync(ns)) return;
+    if (!grid.sync(ns)) return false;
   }
   // sbase, lbase: the ends of the last level's entries; first_* are written by
   // thread 0 above, so every CTA waits once before it reads them
-  if (!grid.sync()) return;
+  if (!grid.sync()) return false;
   const uint32_t gwarp = (uint32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
   const uint32_t nwarps = gridDim.x * kFWarps;
   for (int32_t r = level - 1; r >= 0; r--) {
@@ -616,26 +618,55 @@ __global__ void __launch_bounds__(kFT, 1) bc_fused(BcArgs A) {
       acc += __shfl_xor_sync(kAll, acc, 2);
       if (j < s1 && (lane & 3) == 0) A.deps[s] += 1.0 / A.sigma[s] + acc;
     }
-    if (!grid.sync()) return;
+    if (!grid.sync()) return false;
   }
   // D = (D - 1/sigma) / (1/sigma), as bc_final forms it (unreached: NaN)
   if (A.deps_out) {
+    double* out = A.deps_out + (A.rows ? (size_t)s * n : 0);
     for (uint32_t i = tid; i < n; i += nthreads) {
       const uint32_t v = A.new_ids ? A.new_ids[i] : i;
-      const double s = A.sigma[v];
-      A.deps_out[i] = (A.deps[v] - 1 / s) * s;
+      const double x = A.sigma[v];
+      out[i] = (A.deps[v] - 1 / x) * x;
     }
   } else {
     for (uint32_t i = tid; i < n; i += nthreads) {
-      const double s = A.sigma[i];
-      A.deps[i] = (A.deps[i] - 1 / s) * s;
+      const double x = A.sigma[i];
+      A.deps[i] = (A.deps[i] - 1 / x) * x;
     }
   }
   if (tid == 0) {
-    A.info[0] += (uint64_t)level;
-    A.info[1] += edges;
+    volatile uint64_t* f = A.info + (A.rows ? 4 * s : 0);
+    f[0] += (uint64_t)level;
+    f[1] += edges;
     __threadfence_system();
-    A.info[3] += 1;
+    f[3] += 1;
+  }
+  return true;
+}
+
+__global__ void __launch_bounds__(kFT, 1) bc_fused(const __grid_constant__ BcArgs P) {
+  __shared__ Shared sh;
+  __shared__ Member buf[kFWarps][kBuf];
+  __shared__ BcArgs A;  // with the group's own arrays
+  if (threadIdx.x == 0) {
+    const size_t n = P.g.n, y = blockIdx.y;
+    A = P;
+    A.lvl += y * n;
+    A.sigma += y * n;
+    A.deps += y * n;
+    A.q.small += y * P.n_small;
+    A.q.large += y * P.n_large;
+    A.first_small += y * (n + 2);
+    A.first_large += y * (n + 2);
+    A.ctl += y;
+  }
+  __syncthreads();
+  Grid grid;
+  Appender<true> ap{buf[threadIdx.x >> 5], &sh, 0};
+  begin(grid, &sh, A.ctl);
+  for (int s = blockIdx.y; s < P.k; s += gridDim.y) {
+    if (!bc_source(A, s, grid, ap, sh)) return;
+    if (s + (int)gridDim.y < P.k && !grid.sync()) return;  // the arrays are free for the next source
   }
 }
 
@@ -649,16 +680,68 @@ struct RadiiArgs {
   const uint32_t* new_ids;
   uint32_t seed[64];  // original ids, each once
   unsigned long long mask[64];
-  int k;
+  int k;  // seeds
   int64_t threshold;
   unsigned long long *vis, *nvis;
   int32_t* radii;
   int32_t* radii_out;  // original-id order; null: not wanted (or not sorted)
   uint32_t* bits;
   Queues q[2];
+  // multi-source BFS: bit q of plane p of v is bit p of v's depth from source q
+  unsigned long long* planes;
+  int32_t* depths;  // sources rows of n, original-id order
+  int sources;
   Ctl* ctl;
   volatile uint64_t* info;  // mapped: rounds, edges, -, done
 };
+// Chunks of kSweepChunk edges per warp from which a dense round takes them whole
+// (16 edges per lane, a quarter of the scans) instead of in steps of 128.
+constexpr uint32_t kWideChunks = 2;
+constexpr int kPlanes = 6;  // depths up to 63; deeper searches run level by level
+
+// The vertex's new mask becomes current.
+template <bool kDepths>
+__device__ __forceinline__ void radii_advance(const RadiiArgs& A, uint32_t v, int32_t round) {
+  const unsigned long long now = A.nvis[v];
+  if (kDepths) {
+    const unsigned long long w = now & ~A.vis[v];
+#pragma unroll
+    for (int p = 0; p < kPlanes; p++) {
+      if ((round >> p) & 1) A.planes[(size_t)p * A.out.n + v] |= w;
+    }
+  }
+  A.vis[v] = now;
+}
+
+// The depth rows from the planes: a warp takes 32 vertices and writes one whole
+// line per source (a depth stored where it is found costs a line each, and a fill
+// of every row before).
+template <int kUsed>
+__device__ __forceinline__ void write_depths(const RadiiArgs& A) {
+  const uint32_t n = A.out.n;
+  const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
+  for (uint32_t i = tid; i < n; i += nthreads) {
+    const uint32_t v = A.new_ids ? A.new_ids[i] : i;
+    const unsigned long long seen = A.vis[v];
+    unsigned long long pl[kUsed];
+#pragma unroll
+    for (int p = 0; p < kUsed; p++) pl[p] = A.planes[(size_t)p * n + v];
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+      uint32_t s = (uint32_t)(seen >> (32 * half)), x[kUsed];
+#pragma unroll
+      for (int p = 0; p < kUsed; p++) x[p] = (uint32_t)(pl[p] >> (32 * half));
+      const int end = min(32, A.sources - 32 * half);
+      int32_t* row = A.depths + (size_t)(32 * half) * n + i;
+      for (int q = 0; q < end; q++, row += n) {
+        uint32_t d = 0;
+#pragma unroll
+        for (int p = 0; p < kUsed; p++) d |= ((x[p] >> q) & 1u) << p;
+        *row = (s >> q) & 1u ? (int32_t)d : -1;
+      }
+    }
+  }
+}
 
 __device__ __forceinline__ void radii_flush(const RadiiArgs& A, uint32_t row, unsigned long long part) {
   const unsigned long long w = part & ~A.vis[row];
@@ -671,7 +754,9 @@ __device__ __forceinline__ void radii_flush(const RadiiArgs& A, uint32_t row, un
 // (4 edges per lane, one segmented OR scan per 128 edges, as mask_pull_sweep
 // with shorter steps: a small graph has more warps than 512-edge chunks).  A
 // vertex pass after either makes the new masks current and queues the vertices
-// that grew.
+// that grew.  kDepths: the same propagation, one bit per source, is a
+// multi-source BFS (BFS.C); the bits that arrive in a round have that depth.
+template <bool kDepths>
 __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ RadiiArgs A) {
   __shared__ Shared sh;
   __shared__ Member buf[kFWarps][kBuf];
@@ -720,11 +805,24 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
     edges += c.degsum;
     if (tid == 0) A.ctl->lv[(round + 2) % 3] = Slot{};
     round++;
+    if (kDepths) {
+      if (round >> kPlanes) return;  // too deep: answered level by level
+      if ((round & (round - 1)) == 0) {  // the first round of a plane (a barrier lies before its first use)
+        unsigned long long* pl = A.planes + (size_t)(31 - __clz(round)) * n;
+        for (uint32_t i = tid; i < n; i += nthreads) pl[i] = 0ull;
+      }
+    }
     const Queues nq = A.q[cq ^ 1];
     if ((int64_t)(c.count + c.degsum) > A.threshold && A.in.m > 0) {
       const uint32_t steps = (A.in.m + 127) / 128;
       const uint32_t gwarp = (uint32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
-      for (uint32_t t = gwarp; t < steps; t += nwarps) {
+      const bool wide = A.nchunks >= kWideChunks * nwarps;
+      if (wide) {
+        for (uint32_t c = gwarp; c < A.nchunks; c += nwarps) {
+          mask_pull_chunk<16, false>(A.in, c, A.chunk_v[c], A.chunk_v[c + 1], A.vis, A.nvis, A.bits, full);
+        }
+      }
+      for (uint32_t t = gwarp; t < steps && !wide; t += nwarps) {
         const uint32_t e = t * 128 + lane * 4;
         const uint32_t ch = t / (kSweepChunk / 128);
         uint32_t row = kNone;
@@ -775,7 +873,7 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
         const bool in = (x >> lane) & 1u;
         if (in) {
           A.radii[v] = round;
-          A.vis[v] = A.nvis[v];
+          radii_advance<kDepths>(A, v, round);
         }
         if (lane == 0) A.bits[w] = 0u;
         ap.add(in, v, A.out.off[v], A.out.off[v + 1], nq, ns, 0, 0);
@@ -814,16 +912,25 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
       if (!grid.sync(ns)) return;
       const Slot nx = sh.slot;
       for (uint32_t i = tid; i < nx.ns; i += nthreads) {
-        const uint32_t v = nq.small[i].x;
-        A.vis[v] = A.nvis[v];
+        radii_advance<kDepths>(A, nq.small[i].x, round);
       }
       for (uint32_t i = tid; i < nx.nl; i += nthreads) {
         const uint4 it = nq.large[i];
-        if (it.w & 1u) A.vis[it.x] = A.nvis[it.x];
+        if (it.w & 1u) radii_advance<kDepths>(A, it.x, round);
       }
       if (!grid.sync()) return;
     }
     cq ^= 1;
+  }
+  if (kDepths) {
+    switch (32 - __clz(round)) {
+      case 1: write_depths<1>(A); break;
+      case 2: write_depths<2>(A); break;
+      case 3: write_depths<3>(A); break;
+      case 4: write_depths<4>(A); break;
+      case 5: write_depths<5>(A); break;
+      default: write_depths<6>(A); break;
+    }
   }
   if (A.radii_out) {
     for (uint32_t i = tid; i < n; i += nthreads) A.radii_out[i] = A.radii[A.new_ids ? A.new_ids[i] : i];
@@ -1272,7 +1379,7 @@ int64_t max_in_degree(const rg_graph* g, cudaStream_t st) {
 }
 
 struct FusedState {
-  DevBuf ctl, bits0, bits1, i32a, i32b, f64a, f64b, f64c, u64a, u64b, row, opens, closes, l1, out;
+  DevBuf ctl, bits0, bits1, i32a, i32b, f64a, f64b, f64c, u64a, u64b, row, opens, closes, l1, planes, out;
   DevBuf qs0, qs1, qs2, ql0, ql1, ql2, first_s, first_l;
 };
 thread_local FusedState S;
@@ -1282,7 +1389,7 @@ int fused_grid(int64_t work, int64_t per_cta) {
 }
 
 template <class K, class Args>
-rg_status launch_fused(K kern, const Args& args, int grid, size_t dyn, size_t most_dyn, cudaStream_t st) {
+rg_status launch_fused(K kern, const Args& args, dim3 grid, size_t dyn, size_t most_dyn, cudaStream_t st) {
   static std::atomic<uint64_t> checked{0};
   RG_TRY(once_per_device(checked, [&]() -> rg_status {
     // one CTA per SM must fit, with all the dynamic shared memory it may ask for
@@ -1294,20 +1401,24 @@ rg_status launch_fused(K kern, const Args& args, int grid, size_t dyn, size_t mo
     RG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFT, most_dyn));
     return per_sm > 0 ? RG_OK : fail(RG_ECUDA, "one-launch traversal does not fit an SM");
   }));
-  RG_CUDA(cudaMemsetAsync(args.ctl, 0, sizeof(Ctl), st));
+  RG_CUDA(cudaMemsetAsync(args.ctl, 0, sizeof(Ctl) * grid.y, st));
   void* p[] = {const_cast<Args*>(&args)};
   kt_begin(st);
-  RG_CUDA(cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(kFT), p, dyn, st));
+  RG_CUDA(cudaLaunchCooperativeKernel((const void*)kern, grid, dim3(kFT), p, dyn, st));
   kt_end(st);
   g_timing.kernel_launches++;
   g_timing.edge_launches++;
   return RG_OK;
 }
 
-rg_status queue_pair(int64_t n, int64_t m, DevBuf& s, DevBuf& l, Queues* q) {
-  RG_TRY(s.reserve(16 * (size_t)(n + 32)));
-  // pieces: one per started kPiece edges of every vertex above kSmallDeg
-  RG_TRY(l.reserve(16 * (size_t)(std::min<int64_t>(n, m / (kSmallDeg + 1)) + m / kPiece + 64)));
+size_t small_entries(int64_t n) { return (size_t)(n + 32); }
+// pieces: one per started kPiece edges of every vertex above kSmallDeg
+size_t large_entries(int64_t n, int64_t m) {
+  return (size_t)(std::min<int64_t>(n, m / (kSmallDeg + 1)) + m / kPiece + 64);
+}
+rg_status queue_pair(int64_t n, int64_t m, DevBuf& s, DevBuf& l, Queues* q, int groups = 1) {
+  RG_TRY(s.reserve(16 * small_entries(n) * groups));
+  RG_TRY(l.reserve(16 * large_entries(n, m) * groups));
   *q = Queues{s.as<uint4>(), l.as<uint4>()};
   return RG_OK;
 }
@@ -1385,37 +1496,52 @@ rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t
   return RG_OK;
 }
 
+namespace {
+
+// The arrays of `groups` groups of bc_fused.
+rg_status bc_arrays(const rg_graph* g, int groups, BcArgs* A) {
+  const int64_t n = g->n, m = g->m;
+  RG_TRY(S.ctl.reserve(sizeof(Ctl) * groups));
+  RG_TRY(S.i32a.reserve(4 * (size_t)n * groups));
+  RG_TRY(S.f64a.reserve(8 * (size_t)n * groups));
+  RG_TRY(S.f64b.reserve(8 * (size_t)n * groups));
+  RG_TRY(queue_pair(n, m, S.qs0, S.ql0, &A->q, groups));
+  RG_TRY(S.first_s.reserve(4 * (size_t)(n + 2) * groups));
+  RG_TRY(S.first_l.reserve(4 * (size_t)(n + 2) * groups));
+  A->n_small = small_entries(n);
+  A->n_large = large_entries(n, m);
+  A->new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
+  A->lvl = S.i32a.as<int32_t>();
+  A->sigma = S.f64a.as<double>();
+  A->deps = S.f64b.as<double>();
+  A->first_small = S.first_s.as<uint32_t>();
+  A->first_large = S.first_l.as<uint32_t>();
+  A->ctl = S.ctl.as<Ctl>();
+  return RG_OK;
+}
+
+}  // namespace
+
 rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* h_deps, int64_t* levels_out,
                        double* d_deps_out, bool* done) {
   Ctx& cx = ctx();
   cudaStream_t st = cx.stream;
   const int64_t n = g->n, m = g->m;
   BcArgs A;
-  RG_TRY(S.ctl.reserve(sizeof(Ctl)));
-  RG_TRY(S.i32a.reserve(4 * n));
-  RG_TRY(S.f64a.reserve(8 * n));
-  RG_TRY(S.f64b.reserve(8 * n));
-  RG_TRY(queue_pair(n, m, S.qs0, S.ql0, &A.q));
-  RG_TRY(S.first_s.reserve(4 * (n + 2)));
-  RG_TRY(S.first_l.reserve(4 * (n + 2)));
+  RG_TRY(bc_arrays(g, 1, &A));
   const bool order = g->sorted && (h_deps || d_deps_out);
   if (order && !d_deps_out) RG_TRY(S.f64c.reserve(8 * n));
-  A.new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
-  A.lvl = S.i32a.as<int32_t>();
-  A.sigma = S.f64a.as<double>();
-  A.deps = S.f64b.as<double>();
-  A.first_small = S.first_s.as<uint32_t>();
-  A.first_large = S.first_l.as<uint32_t>();
-  A.ctl = S.ctl.as<Ctl>();
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = cx.ws.h_info;
   info[0] = info[1] = info[3] = 0;
   CallTimer timer(g);
   double* ordered = order ? (d_deps_out ? d_deps_out : S.f64c.as<double>()) : nullptr;
+  A.k = 1;
+  A.rows = false;
   for (int it = 0; it < nsrc; it++) {
     // the reference transposes a directed graph after every source
     A.g = it % 2 == 1 ? g->in_view() : g->view();
-    A.source = src_orig[it];
+    A.source[0] = src_orig[it];
     A.first_source = it == 0;
     A.deps_out = it == nsrc - 1 ? ordered : nullptr;
     RG_TRY(launch_fused(bc_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
@@ -1433,43 +1559,92 @@ rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* 
   return RG_OK;
 }
 
+// k independent sources, row q of `out` (device, original ids) from source q.
+rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double* out, int64_t* levels_out,
+                            bool* done) {
+  Ctx& cx = ctx();
+  cudaStream_t st = cx.stream;
+  const int64_t n = g->n, m = g->m;
+  // every source gets a group while there are SMs for it, and the group the
+  // SMs that are left, up to what one traversal can use
+  const int groups = std::min(k, device_sms());
+  const int width = std::min(fused_grid(m + n, kFusedEdgesPerCta), std::max(1, device_sms() / groups));
+  BcArgs A;
+  RG_TRY(bc_arrays(g, groups, &A));
+  A.g = g->view();
+  for (int q = 0; q < k; q++) A.source[q] = src_orig[q];
+  A.k = k;
+  A.rows = true;
+  A.first_source = true;
+  A.deps_out = out;
+  A.info = reinterpret_cast<volatile uint64_t*>(cx.ws.h_small_dev);
+  volatile uint64_t* info = reinterpret_cast<volatile uint64_t*>(cx.ws.h_small);
+  for (int i = 0; i < 4 * k; i++) info[i] = 0;
+  RG_TRY(launch_fused(bc_fused, A, dim3(width, groups), 0, 0, st));
+  RG_CUDA(cudaStreamSynchronize(st));
+  int64_t levels = 0;
+  for (int q = 0; q < k; q++) {
+    if (info[4 * q + 3] != 1) return RG_OK;
+    levels = std::max(levels, (int64_t)info[4 * q]);
+    g_timing.edges_traversed += (int64_t)info[4 * q + 1];
+  }
+  *done = true;
+  *levels_out = levels;
+  return RG_OK;
+}
+
+namespace {
+
+// What Radii and multi-source BFS share; seeds: original ids, each once.
+rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int k, RadiiArgs* A) {
+  const int64_t n = g->n, m = g->m;
+  RG_TRY(S.ctl.reserve(sizeof(Ctl)));
+  RG_TRY(S.bits0.reserve(4 * ((n + 31) / 32)));
+  RG_TRY(S.u64a.reserve(8 * n));
+  RG_TRY(S.u64b.reserve(8 * n));
+  RG_TRY(S.i32a.reserve(4 * n));
+  RG_TRY(queue_pair(n, m, S.qs0, S.ql0, &A->q[0]));
+  RG_TRY(queue_pair(n, m, S.qs1, S.ql1, &A->q[1]));
+  A->out = g->view();
+  A->in = g->in_view();
+  A->chunk_v = g->in_chunks();
+  A->nchunks = (uint32_t)g->nchunks;
+  A->new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
+  A->k = k;
+  for (int i = 0; i < k; i++) {
+    A->seed[i] = seeds[i];
+    A->mask[i] = masks[i];
+  }
+  A->threshold = dense_threshold(g);
+  A->vis = S.u64a.as<unsigned long long>();
+  A->nvis = S.u64b.as<unsigned long long>();
+  A->radii = S.i32a.as<int32_t>();
+  A->radii_out = nullptr;
+  A->bits = S.bits0.as<uint32_t>();
+  A->planes = nullptr;
+  A->depths = nullptr;
+  A->sources = 0;
+  A->ctl = S.ctl.as<Ctl>();
+  A->info = ctx().ws.h_info_dev;
+  ctx().ws.h_info[3] = 0;
+  return RG_OK;
+}
+
+}  // namespace
+
 rg_status radii_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int k,
                           int32_t* h_radii, int64_t* rounds_out, int32_t* d_radii_out, bool* done) {
   Ctx& cx = ctx();
   cudaStream_t st = cx.stream;
   const int64_t n = g->n, m = g->m;
   RadiiArgs A;
-  RG_TRY(S.ctl.reserve(sizeof(Ctl)));
-  RG_TRY(S.bits0.reserve(4 * ((n + 31) / 32)));
-  RG_TRY(S.u64a.reserve(8 * n));
-  RG_TRY(S.u64b.reserve(8 * n));
-  RG_TRY(S.i32a.reserve(4 * n));
-  RG_TRY(queue_pair(n, m, S.qs0, S.ql0, &A.q[0]));
-  RG_TRY(queue_pair(n, m, S.qs1, S.ql1, &A.q[1]));
+  RG_TRY(radii_args(g, seeds, masks, k, &A));
   const bool order = g->sorted && (h_radii || d_radii_out);
   if (order && !d_radii_out) RG_TRY(S.out.reserve(4 * n));
-  A.out = g->view();
-  A.in = g->in_view();
-  A.chunk_v = g->in_chunks();
-  A.nchunks = (uint32_t)g->nchunks;
-  A.new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
-  A.k = k;
-  for (int i = 0; i < k; i++) {
-    A.seed[i] = seeds[i];
-    A.mask[i] = masks[i];
-  }
-  A.threshold = dense_threshold(g);
-  A.vis = S.u64a.as<unsigned long long>();
-  A.nvis = S.u64b.as<unsigned long long>();
-  A.radii = S.i32a.as<int32_t>();
   A.radii_out = order ? (d_radii_out ? d_radii_out : S.out.as<int32_t>()) : nullptr;
-  A.bits = S.bits0.as<uint32_t>();
-  A.ctl = S.ctl.as<Ctl>();
-  A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = cx.ws.h_info;
-  info[3] = 0;
   CallTimer timer(g);
-  RG_TRY(launch_fused(radii_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
+  RG_TRY(launch_fused(radii_fused<false>, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
   RG_TRY(timer.mark());
   RG_TRY(deliver<int32_t>(g, A.radii, A.radii_out, h_radii, d_radii_out, st));
   RG_CUDA(cudaStreamSynchronize(st));
@@ -1479,6 +1654,27 @@ rg_status radii_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned lon
   g_timing.edges_traversed = (int64_t)info[1];
   g_timing.algorithmic_bytes = 4 * g_timing.edges_traversed + 16 * n + 4 * n;
   if (rounds_out) *rounds_out = (int64_t)info[0];
+  return RG_OK;
+}
+
+rg_status ms_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int u, int k, int32_t* out,
+                       int64_t* rounds_out, bool* done) {
+  Ctx& cx = ctx();
+  cudaStream_t st = cx.stream;
+  const int64_t n = g->n, m = g->m;
+  RadiiArgs A;
+  RG_TRY(radii_args(g, seeds, masks, u, &A));
+  RG_TRY(S.planes.reserve(8 * (size_t)n * kPlanes));
+  A.planes = S.planes.as<unsigned long long>();
+  A.depths = out;
+  A.sources = k;
+  volatile uint64_t* info = cx.ws.h_info;
+  RG_TRY(launch_fused(radii_fused<true>, A, fused_grid(m + n + n * (int64_t)k / 8, kFusedEdgesPerCta), 0, 0, st));
+  RG_CUDA(cudaStreamSynchronize(st));
+  *done = info[3] == 1;
+  if (!*done) return RG_OK;
+  g_timing.edges_traversed += (int64_t)info[1];
+  *rounds_out = (int64_t)info[0];
   return RG_OK;
 }
 

@@ -28,8 +28,11 @@ constexpr int64_t kFusedPrRows = 12000;
 //   BC        2^10 54 / 250, 2^18 204 / 527 (302 / 496), 2^20 576 / 720
 //             (934 / 855), 2^22 1928 / 1569: the line lies between 8e6 and 3.3e7
 //             edges, where the larger grids of the sweeps win
-//   Radii     2^10 71 / 309, 2^18 303 / 584 (340 / 517), 2^20 790 / 792
-//             (1015 / 953): the same line
+//   Radii     2^10 71 / 309, 2^18 270 / 583 (324 / 515), 2^20 619 / 779
+//             (912 / 948), 2^21 801 / 954 (1435 / 1245), 2^22 2044 / 1892: 4e7 edges
+//   multi-source BFS  64 sources: 2^10 74 / 295, 2^18 249 / 615 (363 / 628), 2^21
+//             1244 / 1773 (1825 / 2625); 2 sources: 2^20 417 / 579 (702 / 749), 2^21
+//             609 / 712 (1080 / 990): 6.7e7 edges
 //   PageRank  20 iterations: 2^10 97 / 217, 2^16 304 / 481 (183 / 220), 2^17
 //             546 / 648 (298 / 342), 2^18 1337 / 1033 (573 / 532): 4e6 edges
 //   PageRankDelta  whole, against dense rounds swept and the rest handed over:
@@ -37,9 +40,15 @@ constexpr int64_t kFusedPrRows = 12000;
 //             774 / 815 (605 / 598), 2^20 1441 / 1164 (1146 / 872): 1.7e7 edges
 constexpr int64_t kFusedBfsEdges = INT64_MAX;
 constexpr int64_t kFusedBcEdges = 3 << 23;
-constexpr int64_t kFusedRadiiEdges = 3 << 23;
+constexpr int64_t kFusedRadiiEdges = 5 << 23;
 constexpr int64_t kFusedPagerankEdges = 5 << 20;
 constexpr int64_t kFusedPrdEdges = 1 << 24;
+//   multi-source BC  16 sources: 2^14 190 / 991 (265 / 850), 2^16 487 / 1237
+//             (846 / 1157), 2^17 972 / 1363 (1625 / 1490); 64 sources: 2^14
+//             567 / 1240 (877 / 941), 2^16 1921 / 1491; 5 sources: 2^17 360 / 1013
+//             (569 / 800), 2^18 614 / 1247 (1033 / 963): 4.8e7 edges times sources
+constexpr int64_t kFusedBcRowsEdges = 48 << 20;  // times sources
+constexpr int64_t kFusedMsEdges = 1 << 26;
 
 // Whether a call on g may take the one-launch path: small enough, and no
 // per-level records (rg_set_trace) are asked for.
@@ -51,11 +60,20 @@ rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t
                         int64_t* rounds_out, int64_t* reached_out, int32_t* d_depth_out, bool* done);
 rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* h_deps, int64_t* levels_out,
                        double* d_deps_out, bool* done);
+// k <= 64 independent sources; out: k rows of n (device, original ids); *levels_out:
+// the most levels of any source.  Synchronises.
+rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double* out, int64_t* levels_out,
+                            bool* done);
 // seeds: original ids, each once, with its mask
 rg_status radii_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int k,
                           int32_t* h_radii, int64_t* rounds_out, int32_t* d_radii_out, bool* done);
 rg_status pagerank_fused_run(rg_graph* g, int64_t max_iters, double* h_ranks, int64_t* iters_out, double* l1_out,
                              bool* done);
+// BFS depths from k <= 64 sources; seeds: the distinct ones (original ids) with
+// the mask of the sources at each.  out: k rows of n (device, original ids).
+// Synchronises.
+rg_status ms_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int u, int k, int32_t* out,
+                       int64_t* rounds_out, bool* done);
 
 // PageRankDelta from round `start` on (0: a whole run, which initialises p, ngh
 // and c itself; else p, c and the frontier's bits as the filter of round `start`

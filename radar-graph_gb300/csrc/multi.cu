@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "app_common.cuh"
+#include "fused.cuh"
 #include "pr_exact.cuh"
 
 namespace rg {
@@ -99,6 +100,34 @@ rg_status bfs_multi_run(rg_graph* g, const uint32_t* src_orig, int k, int32_t* h
   RG_TRY(get_ctx(&cx));
   cudaStream_t st = cx->stream;
   const int64_t n = g->n;
+  if (fused_fits(g, kFusedMsEdges)) {
+    uint32_t v[64];
+    unsigned long long mk[64];
+    int u = 0;
+    for (int q = 0; q < k; q++) {
+      const int j = (int)(std::find(v, v + u, src_orig[q]) - v);
+      if (j == u) {
+        v[u] = src_orig[q];
+        mk[u++] = 0ull;
+      }
+      mk[j] |= 1ull << q;
+    }
+    DevBuf rows(true, st);
+    if (!d_depths_out) RG_TRY(rows.reserve(4 * (size_t)n * k));
+    int32_t* out = d_depths_out ? d_depths_out : rows.as<int32_t>();
+    CallTimer timer(g);
+    bool done = false;
+    int64_t rounds = 0;
+    RG_TRY(ms_fused_run(g, v, mk, u, k, out, &rounds, &done));
+    if (done) {
+      RG_TRY(timer.stop());
+      if (h_depths) RG_CUDA(cudaMemcpyAsync(h_depths, out, 4 * (size_t)n * k, cudaMemcpyDeviceToHost, st));
+      RG_CUDA(cudaStreamSynchronize(st));
+      g_timing.algorithmic_bytes = 4 * g_timing.edges_traversed + 4 * (n + 1) + 24 * n + 4 * n * k;
+      if (rounds_out) *rounds_out = rounds;
+      return RG_OK;
+    }
+  }
   static thread_local MsState S;
   RG_TRY(S.F.reserve(8 * n));
   RG_TRY(S.N.reserve(8 * n));

@@ -86,3 +86,53 @@ def test_one_launch_equals_levels(name, directed):
         many = g.pagerank("push-pull", 25)
         rg.set_trace(False)
         assert np.array_equal(one[0], many[0]) and one[1:] == many[1:]
+
+
+@pytest.mark.parametrize("directed", [False, True], ids=["sym", "dir"])
+@pytest.mark.parametrize("k", [1, 2, 31, 33, 64])
+@pytest.mark.parametrize("name", ["one", "path300", "star129", "star5000", "ragged", "hub", "dense"])
+def test_batched_one_launch(name, k, directed):
+    """Sources on one vertex, more sources than groups, rows deeper than the depth
+    planes (63), source counts around a word."""
+    n, s, d = GRAPHS[name]
+    g0 = rg.Graph.from_edges(n, s.astype(np.uint32), d.astype(np.uint32), directed=directed)
+    src = np.random.default_rng(k).integers(0, n, k).astype(np.uint32)
+    src[-1] = src[0]
+    for g in (g0, g0.degree_sort()):
+        one = g.bfs_multi(src), g.bc_multi(src)
+        rg.set_trace(True)
+        many = g.bfs_multi(src), g.bc_multi(src)
+        rg.set_trace(False)
+        assert np.array_equal(one[0][0], many[0][0]) and one[0][1] == many[0][1]
+        assert_close(one[1][0], many[1][0], what="bc rows")
+        assert one[1][1] == many[1][1]
+
+
+@pytest.mark.parametrize("directed", [False, True], ids=["sym", "dir"])
+@pytest.mark.parametrize("name", ["one", "path300", "star129", "star5000", "ragged", "sparse", "hub", "dense"])
+def test_pagerank_delta_one_launch(name, directed):
+    n, s, d = GRAPHS[name]
+    g0 = rg.Graph.from_edges(n, s.astype(np.uint32), d.astype(np.uint32), directed=directed)
+    for g in (g0, g0.degree_sort()):
+        for iters in (0, 1, 2, 100):
+            one = g.pagerank_delta("push-pull", iters)
+            rg.set_trace(True)
+            many = g.pagerank_delta("push-pull", iters)
+            rg.set_trace(False)
+            assert_close(one[0], many[0], what="ranks")
+            assert one[1] == many[1]
+            assert_close([one[2]], [many[2]], what="l1")
+
+
+def test_pagerank_delta_handed_over():
+    """Above the one-launch size: dense rounds swept, the sparse ones handed over."""
+    off, adj = rg.rmat_csr(20, 16, seed=5)
+    with rg.Graph.from_csr(off, adj) as g:
+        one = g.pagerank_delta("push-pull", 100)
+        rg.set_trace(True)
+        many = g.pagerank_delta("push-pull", 100)
+        rg.set_trace(False)
+        want, rounds, _ = orc.pagerank_delta(off, adj, "push", 100, 0)
+    assert one[1] == many[1] == rounds
+    assert_close(one[0], many[0], what="levels")
+    assert_close(one[0], want, what="oracle")
