@@ -387,7 +387,7 @@ rg_status bc_multi_run(rg_graph* g, const uint32_t* src_orig, int k, double* h_o
   RG_TRY(get_ctx(&cx));
   cudaStream_t st = cx->stream;
   const int64_t n = g->n;
-  if (fused_fits(g, kFusedBcRowsEdges / k)) {
+  if (fused_fits(g, std::min(kFusedBcRowsEdges, kFusedBcRowsWork / k))) {
     DevBuf rows(true, st);
     if (!d_out) RG_TRY(rows.reserve(8 * (size_t)n * k));
     double* out = d_out ? d_out : rows.as<double>();

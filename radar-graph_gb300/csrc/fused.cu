@@ -43,9 +43,10 @@ constexpr unsigned kAll = 0xffffffffu;
 constexpr unsigned kSpinLimit = 1u << 21;  // polls of the grid barrier: a second or two
 
 // One level's frontier: queue lengths, members and their degree sum
-// (PageRankDelta: and the round's L1).
+// (PageRankDelta: and the round's L1; BC: the pieces of long lists that a pull
+// puts off).
 struct Slot {
-  unsigned int ns, nl, count, pad;
+  unsigned int ns, nl, count, heavy;
   unsigned long long degsum;
   double l1;
 };
@@ -75,6 +76,19 @@ struct Ctl {
   unsigned int pad[14];
   Slot lv[4];
 };
+
+// The warp's sums of four values: of acc[p] in lanes 8p .. 8p + 7.  Six FP64 adds
+// in place of twenty (GB300 issues one FP64 warp instruction per 16 clocks).
+__device__ __forceinline__ double warp_sum4(const double (&acc)[4]) {
+  const bool hi = threadIdx.x & 16, odd = threadIdx.x & 8;
+  const double x0 = __shfl_xor_sync(kAll, hi ? acc[0] : acc[2], 16);
+  const double x1 = __shfl_xor_sync(kAll, hi ? acc[1] : acc[3], 16);
+  const double y0 = (hi ? acc[2] : acc[0]) + x0, y1 = (hi ? acc[3] : acc[1]) + x1;
+  double z = (odd ? y1 : y0) + __shfl_xor_sync(kAll, odd ? y0 : y1, 8);
+  z += __shfl_xor_sync(kAll, z, 4);
+  z += __shfl_xor_sync(kAll, z, 2);
+  return z + __shfl_xor_sync(kAll, z, 1);
+}
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   unsigned v;
@@ -113,10 +127,11 @@ struct Grid {
   unsigned target;
 
   // All CTAs meet; this CTA's totals go into `slot` first (null: dropped) and the
-  // completed slot comes back in sh->slot (and the completed sum `l1` in sh->l1).  What
+  // completed slot comes back in sh->slot (and the completed sum `l1` in sh->l1).
+  // keep: the totals stay for the next barrier.  What
   // any thread wrote before is visible to every thread after.  False: the wait
   // ran out.
-  __device__ __forceinline__ bool sync(Slot* slot = nullptr, const L1Sum* l1 = nullptr) {
+  __device__ __forceinline__ bool sync(Slot* slot = nullptr, const L1Sum* l1 = nullptr, bool keep = false) {
     __syncthreads();
     target += gridDim.x;
     if (threadIdx.x == 0) {
@@ -124,8 +139,10 @@ struct Grid {
         atomicAdd(&slot->count, sh->count);
         atomicAdd(&slot->degsum, sh->degsum);
       }
-      sh->count = 0;
-      sh->degsum = 0;
+      if (!keep) {
+        sh->count = 0;
+        sh->degsum = 0;
+      }
       int ok = 1;
       if (gridDim.x > 1) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->bar) : "memory");
@@ -486,27 +503,139 @@ __global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
 // BC, one source (BC-manyiter-v2.C:205-367)
 // ---------------------------------------------------------------------------
 struct BcArgs {
-  DevGraph g;  // the lists the forward phase pushes along (the backward phase reads them the other way)
+  DevGraph g;   // the lists the forward phase pushes along (the backward phase reads them the other way)
+  DevGraph gt;  // the same edges by target
+  bool same;    // g and gt are the same lists (a symmetric graph)
+  bool long_lists;  // gt may hold lists above kLongList
   const uint32_t* new_ids;
   uint32_t source[64];  // original ids
   int k;
   bool rows;  // k independent sources, source s to row s of deps_out; else one source, whose dependencies add to deps
   int32_t* lvl;
+  uint32_t* vis;  // the vertices reached, as bits: what a large push tests
   double *sigma, *deps;
   double* deps_out;  // original-id order; null: deps keeps the result
   Queues q;          // every level's frontier, one after another
   uint32_t *first_small, *first_large;  // per level, levels + 1 entries
-  size_t n_small, n_large;              // a group's share of the queues
+  unsigned long long* level_deg;        // per level: its degree sum
+  uint4* heavy;                         // a pulled level's pieces of long lists
+  size_t n_small, n_large, n_heavy;     // a group's share of the queues
   bool first_source;
   Ctl* ctl;
   volatile uint64_t* info;  // mapped, four words per source (or summed over the calls): levels, edges, -, done
 };
 
+constexpr uint32_t kLaneList = 16;    // a pull reads lists up to this with one lane,
+constexpr uint32_t kLongList = 1024;  // up to this with the warp, and longer ones in pieces
+constexpr uint32_t kLongPiece = 512;  // of this many edges
+
+// Sum of sigma over the members of level r among edges [b, e) of a list, read by
+// the whole warp; the same in every lane.
+__device__ __forceinline__ double bc_level_sum(const BcArgs& A, const DevGraph& g, const double* val, uint32_t b,
+                                               uint32_t e, int32_t r) {
+  const int lane = threadIdx.x & 31;
+  double acc = 0.0;
+  for (uint32_t e0 = b; e0 < e; e0 += 128) {
+    uint32_t d[4];
+    int32_t l[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) d[k] = e0 + 32 * k + lane < e ? g.adj[e0 + 32 * k + lane] : kNone;
+#pragma unroll
+    for (int k = 0; k < 4; k++) l[k] = d[k] != kNone ? A.lvl[d[k]] : -2;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (l[k] == r) acc += val[d[k]];
+    }
+  }
+  return warp_sum(acc);
+}
+
+// A forward level as a pull: every vertex not reached yet sums the path counts of
+// its predecessors in level r = level - 1.  False: a wait ran out.
+__device__ bool bc_pull_level(const BcArgs& A, int32_t level, Slot* ns, uint32_t sn, uint32_t ln, Grid& grid,
+                              Appender<true>& ap) {
+  const uint32_t n = A.g.n, nwords = (n + 31) / 32;
+  const int lane = threadIdx.x & 31;
+  const uint32_t gwarp = (uint32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x), nwarps = gridDim.x * kFWarps;
+  for (uint32_t w = gwarp; w < nwords; w += nwarps) {
+    const uint32_t v = w * 32 + lane;
+    uint32_t b = 0, e = 0;
+    if (v < n && !((A.vis[w] >> lane) & 1u)) {
+      b = A.gt.off[v];
+      e = A.gt.off[v + 1];
+    }
+    if (!__any_sync(kAll, b < e)) continue;
+    double sum = 0.0;
+    if (e - b <= kLaneList) {
+      for (uint32_t x = b; x < e; x += 4) {
+        uint32_t u[4];
+        int32_t l[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) u[k] = x + k < e ? A.gt.adj[x + k] : kNone;
+#pragma unroll
+        for (int k = 0; k < 4; k++) l[k] = u[k] != kNone ? A.lvl[u[k]] : -2;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          if (l[k] == level - 1) sum += A.sigma[u[k]];
+        }
+      }
+    }
+    for (unsigned rest = __ballot_sync(kAll, e - b > kLaneList); rest; rest &= rest - 1) {
+      const int j = __ffs(rest) - 1;
+      const uint32_t jb = __shfl_sync(kAll, b, j), je = __shfl_sync(kAll, e, j);
+      if (je - jb <= kLongList) {
+        const double t = bc_level_sum(A, A.gt, A.sigma, jb, je, level - 1);
+        if (lane == j) sum = t;
+      } else {
+        const uint32_t pieces = (je - jb + kLongPiece - 1) / kLongPiece;
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&ns->heavy, pieces);
+        at = __shfl_sync(kAll, at, 0);
+        for (uint32_t p = lane; p < pieces; p += 32) {
+          const uint32_t y = jb + p * kLongPiece;
+          A.heavy[at + p] = make_uint4(w * 32 + j, y, min(y + kLongPiece, je), 0u);
+        }
+      }
+    }
+    const bool won = sum != 0.0;
+    const unsigned now = __ballot_sync(kAll, won);
+    if (lane == 0 && now) A.vis[w] |= now;
+    uint32_t ob = 0, oe = 0;
+    if (won) {
+      A.lvl[v] = level;
+      A.sigma[v] = sum;
+      ob = A.g.off[v];
+      oe = A.g.off[v + 1];
+    }
+    ap.add(won, v, ob, oe, A.q, ns, sn, ln);
+  }
+  if (!A.long_lists) return true;
+  ap.finish(A.q, ns, sn, ln);
+  // (its totals are not published yet: they stay in the CTA until the level ends)
+  if (!grid.sync(nullptr, nullptr, true)) return false;
+  const uint32_t heavy = __ldcg(&ns->heavy);
+  for (uint32_t i = gwarp; i < heavy; i += nwarps) {
+    const uint4 it = A.heavy[i];
+    const double t = bc_level_sum(A, A.gt, A.sigma, it.y, it.z, level - 1);
+    bool won = false;
+    if (lane == 0 && t != 0.0) {
+      atomicAdd(A.sigma + it.x, t);
+      won = atomicCAS(A.lvl + it.x, -1, level) == -1;
+      if (won) atomicOr(A.vis + (it.x >> 5), 1u << (it.x & 31));
+    }
+    ap.add(won, it.x, A.g.off[it.x], A.g.off[it.x + 1], A.q, ns, sn, ln);
+  }
+  return true;
+}
+
 // Forward: sigma is pushed along the frontier's edges to vertices of the next
-// level.  Backward: every vertex sums the dependencies of its successors, so
-// only the pieces of large vertices need an atomic add.  The CTAs of one
-// blockIdx.y are a group with arrays and a barrier of its own; independent
-// sources are dealt out to the groups, whose waits and loads overlap.
+// level or, where far fewer edges lead to vertices not reached yet, pulled by
+// those.  Backward: a level's vertices sum the dependencies of their successors
+// or, where the successors' level has far fewer edges, take them pushed (each
+// direction examines an edge of the level it starts from; on R-MAT s22 the four
+// large steps of pushes examine 2.5e8 edges, the cheaper directions 1.2e8).  The
+// CTAs of one blockIdx.y are a group with arrays and a barrier of its own;
+// independent sources are dealt out to the groups, whose waits and loads overlap.
 __device__ bool bc_source(const BcArgs& A, int s, Grid& grid, Appender<true>& ap, Shared& sh) {
   const uint32_t n = A.g.n;
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
@@ -517,6 +646,7 @@ __device__ bool bc_source(const BcArgs& A, int s, Grid& grid, Appender<true>& ap
     A.sigma[i] = i == src ? 1.0 : 0.0;
     if (A.first_source) A.deps[i] = 0.0;
   }
+  for (uint32_t w = tid; w < (n + 31) / 32; w += nthreads) A.vis[w] = w == src >> 5 ? 1u << (src & 31) : 0u;
   if ((tid >> 5) == 0) {
     if (lane < 3) A.ctl->lv[lane] = Slot{};
     __syncwarp();
@@ -526,48 +656,87 @@ __device__ bool bc_source(const BcArgs& A, int s, Grid& grid, Appender<true>& ap
   if (!grid.sync(&A.ctl->lv[0])) return false;
   uint32_t sbase = 0, lbase = 0;
   int32_t level = 0;
-  unsigned long long edges = 0;
+  unsigned long long edges = 0, seen = 0;  // examined; of vertices reached
   for (;;) {
     Slot* ns = &A.ctl->lv[(level + 1) % 3];
     const Slot c = sh.slot;
     if (tid == 0) {
       A.first_small[level] = sbase;
       A.first_large[level] = lbase;
+      A.level_deg[level] = c.degsum;
     }
     if (c.count == 0) break;
-    edges += c.degsum;
     if (tid == 0) A.ctl->lv[(level + 2) % 3] = Slot{};
     level++;
+    seen += c.degsum;
     const uint32_t sn = sbase + c.ns, ln = lbase + c.nl;  // where the next level's entries begin
-    expand(A.g, A.q, sbase, c.ns, lbase, c.nl, [&](const bool (&in)[4], uint32_t s, const uint32_t (&d)[4]) {
-      int32_t l[4];
+    const unsigned long long rest = A.g.m - seen;  // edges of the vertices not reached yet
+    if (A.same && c.degsum > 2 * rest + n / 8) {
+      edges += rest;
+      if (!bc_pull_level(A, level, ns, sn, ln, grid, ap)) return false;
+    } else if (c.degsum >= n / 4) {
+      // a large level: counts are added without claiming their targets (a claim
+      // is an atomic that returns, and L1 lags behind the claims of other SMs, so
+      // nearly every edge would make one), then one pass over the vertices finds
+      // the ones that now have paths
+      edges += c.degsum;
+      expand(A.g, A.q, sbase, c.ns, lbase, c.nl, [&](const bool (&in)[4], uint32_t u, const uint32_t (&d)[4]) {
+        bool open[4];
 #pragma unroll
-      for (int k = 0; k < 4; k++) l[k] = in[k] ? A.lvl[d[k]] : -2;
-      const double x = A.sigma[s];
-      uint32_t b[4] = {}, e[4] = {};
+        for (int k = 0; k < 4; k++) open[k] = in[k] && !bit_test(A.vis, d[k]);
+        const double x = A.sigma[u];
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        if (l[k] == -1) {
-          b[k] = A.g.off[d[k]];
-          e[k] = A.g.off[d[k] + 1];
-          l[k] = atomicCAS(A.lvl + d[k], -1, level);
-        } else if (l[k] != level) {
-          l[k] = -2;
+        for (int k = 0; k < 4; k++) {
+          if (open[k]) atomicAdd(A.sigma + d[k], x);
         }
+      });
+      if (!grid.sync()) return false;
+      for (uint32_t w0 = (tid & ~31u); w0 < n; w0 += nthreads) {
+        const uint32_t v = min(w0 + lane, n - 1), old = A.vis[w0 >> 5];
+        const bool won = w0 + lane < n && !((old >> lane) & 1u) && A.sigma[v] != 0.0;
+        const unsigned now = __ballot_sync(kAll, won);
+        if (lane == 0 && now) A.vis[w0 >> 5] = old | now;
+        uint32_t b = 0, e = 0;
+        if (won) {
+          A.lvl[v] = level;
+          b = A.g.off[v];
+          e = A.g.off[v + 1];
+        }
+        ap.add(won, v, b, e, A.q, ns, sn, ln);
       }
+    } else {
+      edges += c.degsum;
+      expand(A.g, A.q, sbase, c.ns, lbase, c.nl, [&](const bool (&in)[4], uint32_t u, const uint32_t (&d)[4]) {
+        int32_t l[4];
 #pragma unroll
-      for (int k = 0; k < 4; k++) {  // l: -1 reached here first, level reached by another edge, else not next
-        if (l[k] >= -1) atomicAdd(A.sigma + d[k], x);
-        ap.add(l[k] == -1, d[k], b[k], e[k], A.q, ns, sn, ln);
-      }
-    });
+        for (int k = 0; k < 4; k++) l[k] = in[k] ? A.lvl[d[k]] : -2;
+        const double x = A.sigma[u];
+        uint32_t b[4] = {}, e[4] = {};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          if (l[k] == -1) {
+            b[k] = A.g.off[d[k]];
+            e[k] = A.g.off[d[k] + 1];
+            l[k] = atomicCAS(A.lvl + d[k], -1, level);
+          } else if (l[k] != level) {
+            l[k] = -2;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {  // l: -1 reached here first, level reached by another edge, else not next
+          if (l[k] >= -1) atomicAdd(A.sigma + d[k], x);
+          if (l[k] == -1) atomicOr(A.vis + (d[k] >> 5), 1u << (d[k] & 31));
+          ap.add(l[k] == -1, d[k], b[k], e[k], A.q, ns, sn, ln);
+        }
+      });
+    }
     ap.finish(A.q, ns, sn, ln);
     sbase = sn;
     lbase = ln;
     if (!grid.sync(ns)) return false;
   }
-  // sbase, lbase: the ends of the last level's entries; first_* are written by
-  // thread 0 above, so every CTA waits once before it reads them
+  // first_* and level_deg are written by thread 0 above: every CTA waits once
+  // before it reads them
   if (!grid.sync()) return false;
   const uint32_t gwarp = (uint32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
   const uint32_t nwarps = gridDim.x * kFWarps;
@@ -575,48 +744,83 @@ __device__ bool bc_source(const BcArgs& A, int s, Grid& grid, Appender<true>& ap
     const uint32_t s0 = A.first_small[r], s1 = A.first_small[r + 1];
     const uint32_t l0 = A.first_large[r], l1 = A.first_large[r + 1];
     const bool deepest = r == level - 1;  // its vertices have no successors: 1/sigma alone
-    for (uint32_t i = l0 + gwarp; i < l1; i += nwarps) {
-      const uint4 it = A.q.large[i];
-      double acc = 0.0;
-      if (!deepest) {
-        uint32_t d[4];
-        int32_t l[4];
+    const unsigned long long own = A.level_deg[r], below = deepest ? 0 : A.level_deg[r + 1];
+    const bool push = A.same && !deepest && 4 * below < own;
+    const bool alone = deepest || push;  // this level's edges are not read
+    if (!deepest) edges += push ? below : own;
+    if (push) {
+      expand(A.g, A.q, s1, A.first_small[r + 2] - s1, l1, A.first_large[r + 2] - l1,
+             [&](const bool (&in)[4], uint32_t u, const uint32_t (&d)[4]) {
+               int32_t l[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) d[k] = it.y + 32 * k + lane < it.z ? A.g.adj[it.y + 32 * k + lane] : kNone;
+               for (int k = 0; k < 4; k++) l[k] = in[k] ? A.lvl[d[k]] : -2;
+               const double x = A.deps[u];
 #pragma unroll
-        for (int k = 0; k < 4; k++) l[k] = d[k] != kNone ? A.lvl[d[k]] : -2;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          if (l[k] == r + 1) acc += A.deps[d[k]];
-        }
-      }
-      acc = warp_sum(acc);
-      if (lane == 0) {
-        if (it.w & 1u) acc += 1.0 / A.sigma[it.x];
-        atomicAdd(A.deps + it.x, acc);
-      }
+               for (int k = 0; k < 4; k++) {
+                 if (l[k] == r) atomicAdd(A.deps + d[k], x);
+               }
+             });
     }
-    const uint32_t groups = (s1 - s0 + 7) / 8;
-    for (uint32_t i = gwarp; i < groups; i += nwarps) {
-      const uint32_t j = s0 + i * 8 + (lane >> 2);
-      const uint4 it = j < s1 ? A.q.small[j] : make_uint4(0, 0, 0, 0);
-      const uint32_t s = it.x, b = it.y, end = it.z;
-      double acc = 0.0;
-      for (uint32_t e0 = b + (lane & 3); !deepest && __any_sync(kAll, e0 < end); e0 += 16) {
-        uint32_t d[4];
-        int32_t l[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) d[k] = e0 + 4 * k < end ? A.g.adj[e0 + 4 * k] : kNone;
-#pragma unroll
-        for (int k = 0; k < 4; k++) l[k] = d[k] != kNone ? A.lvl[d[k]] : -2;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          if (l[k] == r + 1) acc += A.deps[d[k]];
-        }
+    // 1/sigma of the level's vertices, a lane each: GB300 issues one FP64 warp
+    // instruction per 16 clocks, a division is ten of them, and beside the sums
+    // one lane of the warp would do it
+    const uint32_t gtid = gwarp * 32 + lane;
+    for (uint32_t i = l0 + gtid; i < l1; i += nthreads) {
+      const uint4 it = A.q.large[i];
+      if (it.w & 1u) atomicAdd(A.deps + it.x, 1.0 / A.sigma[it.x]);
+    }
+    if (alone) {
+      for (uint32_t i = s0 + gtid; i < s1; i += nthreads) {
+        const uint32_t u = A.q.small[i].x;
+        if (push) atomicAdd(A.deps + u, 1.0 / A.sigma[u]);  // beside the pushes
+        else A.deps[u] += 1.0 / A.sigma[u];
       }
-      acc += __shfl_xor_sync(kAll, acc, 1);
-      acc += __shfl_xor_sync(kAll, acc, 2);
-      if (j < s1 && (lane & 3) == 0) A.deps[s] += 1.0 / A.sigma[s] + acc;
+    } else {
+      // four pieces per warp, their sums reduced together
+      for (uint32_t i0 = l0 + gwarp * 4; i0 < l1; i0 += nwarps * 4) {
+        double acc[4];
+        uint32_t v = 0;  // the vertex of piece lane / 8
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+          const uint4 it = i0 + p < l1 ? A.q.large[i0 + p] : make_uint4(0, 0, 0, 0);
+          if (lane / 8 == p) v = it.x;
+          uint32_t d[4];
+          int32_t l[4];
+#pragma unroll
+          for (int k = 0; k < 4; k++) d[k] = it.y + 32 * k + lane < it.z ? A.g.adj[it.y + 32 * k + lane] : kNone;
+#pragma unroll
+          for (int k = 0; k < 4; k++) l[k] = d[k] != kNone ? A.lvl[d[k]] : -2;
+          acc[p] = 0.0;
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            if (l[k] == r + 1) acc[p] += A.deps[d[k]];
+          }
+        }
+        const double z = warp_sum4(acc);
+        if ((lane & 7) == 0 && z != 0.0) atomicAdd(A.deps + v, z);
+      }
+      const uint32_t groups = (s1 - s0 + 7) / 8;
+      for (uint32_t i = gwarp; i < groups; i += nwarps) {
+        const uint32_t j = s0 + i * 8 + (lane >> 2);
+        const uint4 it = j < s1 ? A.q.small[j] : make_uint4(0, 0, 0, 0);
+        const uint32_t u = it.x, b = it.y, end = it.z;
+        double acc = 0.0;
+        for (uint32_t e0 = b + (lane & 3); __any_sync(kAll, e0 < end); e0 += 16) {
+          uint32_t d[4];
+          int32_t l[4];
+#pragma unroll
+          for (int k = 0; k < 4; k++) d[k] = e0 + 4 * k < end ? A.g.adj[e0 + 4 * k] : kNone;
+#pragma unroll
+          for (int k = 0; k < 4; k++) l[k] = d[k] != kNone ? A.lvl[d[k]] : -2;
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            if (l[k] == r + 1) acc += A.deps[d[k]];
+          }
+        }
+        acc += __shfl_xor_sync(kAll, acc, 1);
+        acc += __shfl_xor_sync(kAll, acc, 2);
+        if (j < s1 && (lane & 3) == 0) A.deps[u] += 1.0 / A.sigma[u] + acc;
+      }
     }
     if (!grid.sync()) return false;
   }
@@ -652,12 +856,15 @@ __global__ void __launch_bounds__(kFT, 1) bc_fused(const __grid_constant__ BcArg
     const size_t n = P.g.n, y = blockIdx.y;
     A = P;
     A.lvl += y * n;
+    A.vis += y * ((n + 31) / 32);
     A.sigma += y * n;
     A.deps += y * n;
     A.q.small += y * P.n_small;
     A.q.large += y * P.n_large;
     A.first_small += y * (n + 2);
     A.first_large += y * (n + 2);
+    A.level_deg += y * (n + 2);
+    A.heavy += y * P.n_heavy;
     A.ctl += y;
   }
   __syncthreads();
@@ -1246,18 +1453,25 @@ __global__ void __launch_bounds__(kFT, 1) prd_fused(const __grid_constant__ PrdA
     const bool whole = A.start == 0 && k == 1;  // the queue does not hold the first frontier of a whole run
     if (whole || (A.start == 0 && A.allow_pull && (int64_t)(c.count + c.degsum) > A.threshold)) {
       const uint32_t gwarp = (uint32_t)(wid * gridDim.x + blockIdx.x);
-      for (uint32_t i = gwarp; i < rl; i += nwarps) {
-        const uint4 it = A.rows.large[i];
-        uint32_t u[4];
-        double x[4];
+      for (uint32_t i0 = gwarp * 4; i0 < rl; i0 += nwarps * 4) {
+        double acc[4];
+        uint4 mine = make_uint4(0, 0, 0, 0);  // piece lane / 8
 #pragma unroll
-        for (int j = 0; j < 4; j++) u[j] = it.y + 32 * j + lane < it.z ? A.in.adj[it.y + 32 * j + lane] : kNone;
+        for (int q = 0; q < 4; q++) {
+          const uint4 it = i0 + q < rl ? A.rows.large[i0 + q] : make_uint4(0, 0, 0, 0);
+          if (lane / 8 == q) mine = it;
+          uint32_t u[4];
+          double x[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) x[j] = u[j] != kNone ? A.c[u[j]] : 0.0;
-        const double s = warp_sum((x[0] + x[1]) + (x[2] + x[3]));
-        if (lane == 0) {
-          if (it.w == 3u) A.ngh[it.x] = s;  // the row's only piece
-          else if (s != 0.0) atomicAdd(A.ngh + it.x, s);
+          for (int j = 0; j < 4; j++) u[j] = it.y + 32 * j + lane < it.z ? A.in.adj[it.y + 32 * j + lane] : kNone;
+#pragma unroll
+          for (int j = 0; j < 4; j++) x[j] = u[j] != kNone ? A.c[u[j]] : 0.0;
+          acc[q] = (x[0] + x[1]) + (x[2] + x[3]);
+        }
+        const double s = warp_sum4(acc);
+        if ((lane & 7) == 0 && i0 + lane / 8 < rl) {
+          if (mine.w == 3u) A.ngh[mine.x] = s;  // the row's only piece
+          else if (s != 0.0) atomicAdd(A.ngh + mine.x, s);
         }
       }
       for (uint32_t i = gwarp; i < (rs + 7) / 8; i += nwarps) {
@@ -1380,7 +1594,7 @@ int64_t max_in_degree(const rg_graph* g, cudaStream_t st) {
 
 struct FusedState {
   DevBuf ctl, bits0, bits1, i32a, i32b, f64a, f64b, f64c, u64a, u64b, row, opens, closes, l1, planes, out;
-  DevBuf qs0, qs1, qs2, ql0, ql1, ql2, first_s, first_l;
+  DevBuf qs0, qs1, qs2, ql0, ql1, ql2, first_s, first_l, level_deg, heavy;
 };
 thread_local FusedState S;
 
@@ -1508,8 +1722,18 @@ rg_status bc_arrays(const rg_graph* g, int groups, BcArgs* A) {
   RG_TRY(queue_pair(n, m, S.qs0, S.ql0, &A->q, groups));
   RG_TRY(S.first_s.reserve(4 * (size_t)(n + 2) * groups));
   RG_TRY(S.first_l.reserve(4 * (size_t)(n + 2) * groups));
+  RG_TRY(S.level_deg.reserve(8 * (size_t)(n + 2) * groups));
+  RG_TRY(S.bits0.reserve(4 * (size_t)((n + 31) / 32) * groups));
+  A->vis = S.bits0.as<uint32_t>();
   A->n_small = small_entries(n);
   A->n_large = large_entries(n, m);
+  A->same = !g->directed;
+  A->long_lists = std::max(max_in_degree(g, ctx().stream), (int64_t)g->max_deg) > kLongList;
+  // pieces of lists above kLongList, two at least: at most 3/2 per kLongPiece edges
+  A->n_heavy = A->long_lists ? (size_t)(m / kLongPiece + m / kLongList + 64) : 0;
+  RG_TRY(S.heavy.reserve(16 * std::max<size_t>(A->n_heavy, 1) * groups));
+  A->level_deg = S.level_deg.as<unsigned long long>();
+  A->heavy = S.heavy.as<uint4>();
   A->new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
   A->lvl = S.i32a.as<int32_t>();
   A->sigma = S.f64a.as<double>();
@@ -1541,6 +1765,7 @@ rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* 
   for (int it = 0; it < nsrc; it++) {
     // the reference transposes a directed graph after every source
     A.g = it % 2 == 1 ? g->in_view() : g->view();
+    A.gt = it % 2 == 1 ? g->view() : g->in_view();
     A.source[0] = src_orig[it];
     A.first_source = it == 0;
     A.deps_out = it == nsrc - 1 ? ordered : nullptr;
@@ -1565,13 +1790,17 @@ rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double
   Ctx& cx = ctx();
   cudaStream_t st = cx.stream;
   const int64_t n = g->n, m = g->m;
-  // every source gets a group while there are SMs for it, and the group the
-  // SMs that are left, up to what one traversal can use
-  const int groups = std::min(k, device_sms());
+  // every source gets a group while there are SMs for it and the groups' arrays
+  // (44 bytes per vertex that a traversal keeps returning to) stay in L2; the SMs
+  // are shared out between the groups, up to what one traversal can use
+  const int64_t in_l2 = std::max<int64_t>(1, kFusedBcRowsL2 / (44 * n));
+  const int most = (int)std::min<int64_t>({(int64_t)k, (int64_t)device_sms(), in_l2});
+  const int groups = (k + (k + most - 1) / most - 1) / ((k + most - 1) / most);  // as many rounds, evenly filled
   const int width = std::min(fused_grid(m + n, kFusedEdgesPerCta), std::max(1, device_sms() / groups));
   BcArgs A;
   RG_TRY(bc_arrays(g, groups, &A));
   A.g = g->view();
+  A.gt = g->in_view();
   for (int q = 0; q < k; q++) A.source[q] = src_orig[q];
   A.k = k;
   A.rows = true;

@@ -25,9 +25,8 @@ constexpr int64_t kFusedPrRows = 12000;
 // sorted (in brackets: uniform, unsorted), us:
 //   BFS       2^10 vertices 31 / 182, 2^16 46 / 298, 2^20 95 / 415 (167 / 402),
 //             2^24 560 / 973 (1823 / 2972): every size
-//   BC        2^10 54 / 250, 2^18 204 / 527 (302 / 496), 2^20 576 / 720
-//             (934 / 855), 2^22 1928 / 1569: the line lies between 8e6 and 3.3e7
-//             edges, where the larger grids of the sweeps win
+//   BC        2^10 58 / 246 (75 / 240), 2^18 130 / 506 (153 / 496), 2^22
+//             601 / 1573 (1007 / 1975), 2^24 3519 / 5520 (8066 / 9983): every size
 //   Radii     2^10 71 / 309, 2^18 270 / 583 (324 / 515), 2^20 619 / 779
 //             (912 / 948), 2^21 801 / 954 (1435 / 1245), 2^22 2044 / 1892: 4e7 edges
 //   multi-source BFS  64 sources: 2^10 74 / 295, 2^18 249 / 615 (363 / 628), 2^21
@@ -39,15 +38,21 @@ constexpr int64_t kFusedPrRows = 12000;
 //             2^10 139 / 398 (85 / 238), 2^18 494 / 688 (332 / 440), 2^19
 //             774 / 815 (605 / 598), 2^20 1441 / 1164 (1146 / 872): 1.7e7 edges
 constexpr int64_t kFusedBfsEdges = INT64_MAX;
-constexpr int64_t kFusedBcEdges = 3 << 23;
+constexpr int64_t kFusedBcEdges = INT64_MAX;
 constexpr int64_t kFusedRadiiEdges = 5 << 23;
 constexpr int64_t kFusedPagerankEdges = 5 << 20;
-constexpr int64_t kFusedPrdEdges = 1 << 24;
-//   multi-source BC  16 sources: 2^14 190 / 991 (265 / 850), 2^16 487 / 1237
-//             (846 / 1157), 2^17 972 / 1363 (1625 / 1490); 64 sources: 2^14
-//             567 / 1240 (877 / 941), 2^16 1921 / 1491; 5 sources: 2^17 360 / 1013
-//             (569 / 800), 2^18 614 / 1247 (1033 / 963): 4.8e7 edges times sources
-constexpr int64_t kFusedBcRowsEdges = 48 << 20;  // times sources
+constexpr int64_t kFusedPrdEdges = 1 << 25;
+//   multi-source BC  16 sources: 2^14 116 / 1023 (147 / 864), 2^18 850 / 2055
+//             (900 / 2193), 2^19 1800 / 3010 (3000 / 4154), 2^20 4564 / 5299 (8250 /
+//             6911); 64 sources: 2^16 921 / 1498 (1426 / 1464), 2^17 1764 / 1961
+//             (2016 / 1933), 2^18 3280 / 2978; 5 sources: 2^19 650 / 1613 (770 /
+//             1400), 2^20 1444 / 2468 (2637 / 2436): 2.7e8 edges times sources and
+//             2.5e7 edges
+constexpr int64_t kFusedBcRowsEdges = 24 << 20;
+constexpr int64_t kFusedBcRowsWork = 256 << 20;  // edges times sources
+// Groups' arrays at once: 64 sources on 2^17 vertices 2079 us with all of them
+// (370 MB), 2016 in 80 MB; 16 sources on 2^18 808 us with all (184 MB), 1008 in 80 MB.
+constexpr int64_t kFusedBcRowsL2 = 192 << 20;
 constexpr int64_t kFusedMsEdges = 1 << 26;
 
 // Whether a call on g may take the one-launch path: small enough, and no
