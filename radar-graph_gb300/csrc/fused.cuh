@@ -32,15 +32,18 @@ constexpr int64_t kFusedPrRows = 12000;
 //   multi-source BFS  64 sources: 2^10 74 / 295, 2^18 249 / 615 (363 / 628), 2^21
 //             1244 / 1773 (1825 / 2625); 2 sources: 2^20 417 / 579 (702 / 749), 2^21
 //             609 / 712 (1080 / 990): 6.7e7 edges
-//   PageRank  20 iterations: 2^10 97 / 217, 2^16 304 / 481 (183 / 220), 2^17
-//             546 / 648 (298 / 342), 2^18 1337 / 1033 (573 / 532): 4e6 edges
+//   PageRank  20 iterations, against pulls: 2^10 97 / 217, 2^14 154 / 247 (93 /
+//             160), 2^16 308 / 308 (183 / 245), 2^17 565 / 473 (297 / 365): 3e6
+//             edges; against pushes: 2^16 309 / 730, 2^18 1331 / 1559, 2^19 2737 /
+//             2332: 8e6 edges
 //   PageRankDelta  whole, against dense rounds swept and the rest handed over:
 //             2^10 139 / 398 (85 / 238), 2^18 494 / 688 (332 / 440), 2^19
 //             774 / 815 (605 / 598), 2^20 1441 / 1164 (1146 / 872): 1.7e7 edges
 constexpr int64_t kFusedBfsEdges = INT64_MAX;
 constexpr int64_t kFusedBcEdges = INT64_MAX;
 constexpr int64_t kFusedRadiiEdges = 5 << 23;
-constexpr int64_t kFusedPagerankEdges = 5 << 20;
+constexpr int64_t kFusedPagerankEdges = 3 << 20;
+constexpr int64_t kFusedPagerankPushEdges = 8 << 20;
 constexpr int64_t kFusedPrdEdges = 1 << 25;
 //   multi-source BC  16 sources: 2^14 116 / 1023 (147 / 864), 2^18 850 / 2055
 //             (900 / 2193), 2^19 1800 / 3010 (3000 / 4154), 2^20 4564 / 5299 (8250 /

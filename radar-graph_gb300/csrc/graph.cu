@@ -652,8 +652,6 @@ static rg_status new_graph(rg_graph** out) {
   RG_TRY(get_ctx(&c));
   rg_graph* g = new (std::nothrow) rg_graph();
   if (!g) return fail(RG_ENOMEM, "host allocation failed");
-  static std::atomic<uint64_t> next_uid{1};
-  g->uid = next_uid++;
   g->device = c->device;
   *out = g;
   return RG_OK;

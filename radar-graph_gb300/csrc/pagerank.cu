@@ -41,10 +41,34 @@ namespace {
 constexpr int kSweepThreads = 1024;  // push sweep CTA (one per SM with hub copies)
 constexpr int kPullThreads = 256;
 constexpr uint32_t kNoRow = 0xFFFFFFFFu;
+constexpr int64_t kCacheVertices = 6 << 20;  // contributions above 48 MB
 
 // L1 of the previous iteration (exact) below 1e-7: this iteration is skipped.
 __device__ __forceinline__ bool converged(const U128* l1_prev) {
   return l1_prev != nullptr && less128(*l1_prev, pr_eps_fx());
+}
+
+// A kernel of an iteration is launched while the one before it drains
+// (launch_following): it lets its own follower in and waits for its predecessor
+// to complete before it reads anything.  A plain launch passes straight through.
+__device__ __forceinline__ void follow() {
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+}
+
+template <class... P, class... A>
+cudaError_t launch_following(void (*kern)(P...), int grid, int threads, size_t dyn, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = dyn;
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
 
 // p = 1/n, contrib = p/deg (PageRank.C:126-138), rmag = the integer
@@ -72,6 +96,7 @@ template <int kHub>
 __global__ void __launch_bounds__(kSweepThreads) pr_push_sweep(DevGraph g, const uint32_t* __restrict__ chunk_v,
                                                                uint32_t nchunks, const double* __restrict__ contrib,
                                                                double* acc, HubInfo hub, const U128* l1_prev) {
+  follow();
   if (converged(l1_prev)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   U128* hs = reinterpret_cast<U128*>(smem_raw);
@@ -145,6 +170,7 @@ __global__ void __launch_bounds__(kCache ? 1024 : kPullThreads)
     pr_pull_sweep(DevGraph g, const uint32_t* __restrict__ chunk_v, uint32_t nchunks,
                   const double* __restrict__ contrib, U128* acc, uint32_t H, const U128* l1_prev) {
   static_assert(kItems == 4 || kItems == 8 || kItems == 16, "4, 8 or 16 edges per lane");
+  follow();
   if (converged(l1_prev)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* hc = reinterpret_cast<double*>(smem_raw);
@@ -325,10 +351,16 @@ __global__ void __launch_bounds__(256) pr_finalize(uint32_t n, const uint32_t* _
                                                    double* p, double* contrib,
                                                    const unsigned long long* __restrict__ rmag, double added,
                                                    U128* l1_out, const U128* l1_prev) {
+  follow();
   if (converged(l1_prev)) return;
+  const bool later = l1_prev != nullptr;
   U128 local{0ull, 0ull};
   double* accd = reinterpret_cast<double*>(acc);
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+    // a vertex without in-edges has the rank `added` and the same contribution
+    // from the first iteration on
+    const uint32_t b = pull_off[v], e = pull_off[v + 1];
+    if (later && b == e) continue;
     // the tests of zero and equality are integer compares (the FP64 pipe is
     // the scarce one): every value here is a nonnegative double, not NaN
     double sum;
@@ -337,7 +369,6 @@ __global__ void __launch_bounds__(256) pr_finalize(uint32_t n, const uint32_t* _
       const U128 a = acc[v];
       has = (a.lo | a.hi) != 0ull;
       sum = has ? fx_to_double(a) : 0.0;
-      const uint32_t b = pull_off[v], e = pull_off[v + 1];
       if (e > b && b / step != (e - 1) / step) acc[v] = U128{0ull, 0ull};
     } else {
       sum = accd[v];
@@ -403,7 +434,10 @@ rg_status pagerank_run(rg_graph* g, int variant, int64_t max_iters, double* h_ra
   OptScope opt_scope(g, kAppPagerank);
   Ctx* cx = nullptr;
   RG_TRY(get_ctx(&cx));
-  if (max_iters > 0 && fused_fits(g, kFusedPagerankEdges)) {
+  // pull: the push-pull variant (threshold 0, PageRank.C:122 in src/push-pull)
+  // or the auto direction
+  const bool pull = variant == RG_PUSH_PULL || g_opts.direction == 1;
+  if (max_iters > 0 && fused_fits(g, pull ? kFusedPagerankEdges : kFusedPagerankPushEdges)) {
     bool done = false;
     RG_TRY(pagerank_fused_run(g, max_iters, h_ranks, iters_out, l1_out, &done));
     if (done) return RG_OK;
@@ -428,11 +462,13 @@ rg_status pagerank_run(rg_graph* g, int variant, int64_t max_iters, double* h_ra
   uint32_t pr_budget = (uint32_t)std::min<int64_t>((max_dyn_smem() - 1024) / (int)sizeof(U128), n);
   if (g_opts.hub_slots > 0) pr_budget = (uint32_t)std::min<int64_t>(pr_budget, g_opts.hub_slots);
   if (hub_h) pr_budget = std::min(pr_budget, hub_h);
-  // pull: the push-pull variant (threshold 0, PageRank.C:122 in src/push-pull)
-  // or the auto direction; RADAR's pull keeps the hubs' contributions in
-  // shared memory, the others gather from global memory
-  const bool pull = variant == RG_PUSH_PULL || g_opts.direction == 1;
-  const bool cache = pull && variant == RG_RADAR && g->sorted && g_opts.hub_smem_kb > 0;
+  // RADAR's pull keeps the hubs' contributions in shared memory, the others
+  // gather from global memory
+  // ... and only where the contributions spill from L2 (129 MB, shared with the
+  // edge stream): below that the copies cost more than the gathers they save
+  // (20 iterations, R-MAT edge factor 16, with and without 48 KiB: 2^18 vertices
+  // 1009 and 617 us, 2^20 2417 and 2036, 2^22 8696 and 8404, 2^23 17356 and 18415)
+  const bool cache = pull && variant == RG_RADAR && g->sorted && g_opts.hub_smem_kb > 0 && n > kCacheVertices;
   HubInfo hub;
   size_t dyn = 0;
   if (!pull && hm != kHubNone) {
@@ -487,108 +523,42 @@ rg_status pagerank_run(rg_graph* g, int variant, int64_t max_iters, double* h_ra
   unsigned long long* R = S.rmag.as<unsigned long long>();
   U128* L1 = S.l1.as<U128>();
   // The whole run (init + every iteration) is enqueued without host round
-  // trips; it is captured once as a CUDA graph and replayed on later calls
-  // with the same graph, buffers and schedule (not while per-kernel timing
-  // is on, which needs the launches one by one).
+  // trips; each kernel's launch overlaps the one before it (not while per-kernel
+  // times are taken).  Launching them one by one costs the host 2 us a kernel,
+  // hidden behind kernels that take longer (shorter ones are runs of one launch);
+  // a captured graph would have to be made again for every other graph.
   int64_t launches = 0, edge_launches = 0;
-  auto enqueue = [&]() -> cudaError_t {
-    cudaError_t e = cudaMemsetAsync(L1, 0, sizeof(U128) * (max_iters + 1), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(A, 0, sizeof(U128) * n, st);
-    if (e != cudaSuccess) return e;
-    pr_init<<<vblocks, 256, 0, st>>>((uint32_t)n, g->off.as<uint32_t>(), P, C, R, p0);
+  RG_CUDA(cudaMemsetAsync(L1, 0, sizeof(U128) * (max_iters + 1), st));
+  RG_CUDA(cudaMemsetAsync(A, 0, sizeof(U128) * n, st));
+  pr_init<<<vblocks, 256, 0, st>>>((uint32_t)n, g->off.as<uint32_t>(), P, C, R, p0);
+  RG_CUDA(cudaGetLastError());
+  launches++;
+  auto follow_launch = [&](auto kern, int grid, int threads, size_t smem, auto... args) -> cudaError_t {
     launches++;
-    // iteration i's kernels return at once when iteration i-1 already
-    // reached L1 < 1e-7
-    for (int64_t it = 0; it < max_iters; it++) {
-      const U128* prev = it ? L1 + it - 1 : nullptr;
-      if (g->m > 0) {
-        kt_begin(st);
-        if (pull) {
-          pull_fn<<<sweep_grid, pull_threads, pull_dyn, st>>>(g->in_view(), g->in_chunks(), (uint32_t)g->nchunks, C,
-                                                              A, cacheH, prev);
-        } else {
-          sweep_fn<<<sweep_grid, kSweepThreads, dyn, st>>>(g->view(), g->chunk_v.as<uint32_t>(),
-                                                           (uint32_t)g->nchunks, C, reinterpret_cast<double*>(A), hub,
-                                                           prev);
-        }
-        kt_end(st);
-        launches++;
-        edge_launches++;
-      }
-      if (pull) {
-        pr_finalize<true><<<vblocks, 256, 0, st>>>((uint32_t)n, g->off.as<uint32_t>(), g->in_view().off, pull_step,
-                                                   A, P, C, R, added, L1 + it, prev);
-      } else {
-        pr_finalize<false><<<vblocks, 256, 0, st>>>((uint32_t)n, g->off.as<uint32_t>(), g->off.as<uint32_t>(), 1u,
-                                                    A, P, C, R, added, L1 + it, prev);
-      }
-      launches++;
-    }
+    if (!g_kernel_timing) return launch_following(kern, grid, threads, smem, st, args...);
+    kern<<<(unsigned)grid, (unsigned)threads, smem, st>>>(args...);
     return cudaGetLastError();
   };
-  // the captured launches bake in every pointer below; the graph's uid keeps
-  // a new graph whose buffers reuse a freed graph's addresses from matching
-  struct GraphKey {
-    uint64_t uid;
-    const void *off, *adj, *chunk_v, *hub_bits, *hub_slot, *hub_vertex, *a, *p, *c, *r, *l1;
-    int64_t n, m, iters;
-    int variant, grid, pull, cacheH, hubH, hubmode, shape;
-    bool operator==(const GraphKey& o) const { return memcmp(this, &o, sizeof *this) == 0; }
-  };
-  static thread_local GraphKey cached_key;
-  static thread_local cudaGraphExec_t cached_exec = nullptr;
-  static thread_local int64_t cached_launches = 0, cached_edge_launches = 0;
-  GraphKey key;
-  memset(&key, 0, sizeof key);  // memcmp compares the padding too: set fields one by one
-  key.uid = g->uid;
-  key.off = g->off.p;
-  key.adj = g->adj.p;
-  key.chunk_v = g->chunk_v.p;
-  key.hub_bits = hub.bits;
-  key.hub_slot = hub.slot;
-  key.hub_vertex = hub.vertex;
-  key.a = A;
-  key.p = P;
-  key.c = C;
-  key.r = R;
-  key.l1 = L1;
-  key.n = n;
-  key.m = g->m;
-  key.iters = max_iters;
-  key.variant = variant;
-  key.grid = sweep_grid;
-  key.pull = pull ? 1 : 0;
-  key.cacheH = (int)cacheH;
-  key.hubH = (int)hub.H;
-  key.hubmode = push_hm;
-  key.shape = (int)g_opts.sweep_shape;
-  if (g_kernel_timing || max_iters == 0) {
-    RG_CUDA(enqueue());
-  } else {
-    if (!cached_exec || !(key == cached_key)) {
-      if (cached_exec) cudaGraphExecDestroy(cached_exec);
-      cached_exec = nullptr;
-      cudaGraph_t graph = nullptr;
-      RG_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      const cudaError_t e = enqueue();
-      const cudaError_t e2 = cudaStreamEndCapture(st, &graph);
-      if (e != cudaSuccess || e2 != cudaSuccess) {
-        if (graph) cudaGraphDestroy(graph);
-        return cuda_fail(e != cudaSuccess ? e : e2, "PageRank graph capture", __FILE__, __LINE__);
+  const uint32_t *off = g->off.as<uint32_t>(), *in_off = g->in_view().off;
+  const uint32_t nchunks = (uint32_t)g->nchunks;
+  // iteration i's kernels return at once when iteration i-1 already reached
+  // L1 < 1e-7
+  for (int64_t it = 0; it < max_iters; it++) {
+    const U128* prev = it ? L1 + it - 1 : nullptr;
+    if (g->m > 0) {
+      kt_begin(st);
+      if (pull) {
+        RG_CUDA(follow_launch(pull_fn, sweep_grid, pull_threads, pull_dyn, g->in_view(), g->in_chunks(), nchunks,
+                              (const double*)C, A, cacheH, prev));
+      } else {
+        RG_CUDA(follow_launch(sweep_fn, sweep_grid, kSweepThreads, dyn, g->view(), (const uint32_t*)g->chunk_v.as<uint32_t>(),
+                              nchunks, (const double*)C, reinterpret_cast<double*>(A), hub, prev));
       }
-      const cudaError_t e3 = cudaGraphInstantiate(&cached_exec, graph, 0);
-      cudaGraphDestroy(graph);
-      if (e3 != cudaSuccess) {
-        cached_exec = nullptr;
-        return cuda_fail(e3, "cudaGraphInstantiate", __FILE__, __LINE__);
-      }
-      cached_key = key;
-      cached_launches = launches;
-      cached_edge_launches = edge_launches;
+      kt_end(st);
+      edge_launches++;
     }
-    RG_CUDA(cudaGraphLaunch(cached_exec, st));
-    launches = cached_launches;
-    edge_launches = cached_edge_launches;
+    RG_CUDA(follow_launch(pull ? pr_finalize<true> : pr_finalize<false>, vblocks, 256, 0, (uint32_t)n, off, in_off,
+                          pull ? pull_step : 1u, A, P, C, (const unsigned long long*)R, added, L1 + it, prev));
   }
   g_timing.kernel_launches += launches;
   g_timing.edge_launches += edge_launches;

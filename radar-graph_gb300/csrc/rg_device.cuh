@@ -148,7 +148,6 @@ Ctx& ctx();  // only after a successful get_ctx on this thread
 
 struct rg_graph {
   int device = 0;
-  uint64_t uid = 0;  // unique per graph in the process (device addresses can repeat)
   int64_t n = 0, m = 0;
   rg::DevBuf off{true}, adj{true};  // CSR on the device (out-lists)
   rg::DevBuf chunk_v{true};         // sweep partition: first vertex of every kSweepChunk edges
