@@ -394,8 +394,11 @@ __global__ void pr_gather(const double* __restrict__ p, const uint32_t* __restri
   }
 }
 
+constexpr size_t kPage = 2 << 20;
+
 struct PrState {
-  DevBuf acc, p, contrib, rmag, l1, out;
+  DevBuf arrays;  // contrib, acc (two rows), p, rmag
+  DevBuf l1, out;
 };
 
 }  // namespace
@@ -445,10 +448,10 @@ rg_status pagerank_run(rg_graph* g, int variant, int64_t max_iters, double* h_ra
   cudaStream_t st = cx->stream;
   const int64_t n = g->n;
   static thread_local PrState S;
-  RG_TRY(S.acc.reserve(sizeof(U128) * n));
-  RG_TRY(S.p.reserve(8 * n));
-  RG_TRY(S.contrib.reserve(8 * n));
-  RG_TRY(S.rmag.reserve(8 * n));
+  // the per-vertex arrays in one allocation, whole 2 MiB pages each: apart, their
+  // placement after other allocations moved the sweep between 1.67 and 1.83 ms (2^24)
+  const size_t row = ((size_t)n * 8 + kPage - 1) / kPage * kPage;
+  RG_TRY(S.arrays.reserve(5 * row));
   RG_TRY(S.l1.reserve(sizeof(U128) * (max_iters + 1)));
   RG_TRY(S.out.reserve(8 * n));
   // the reference's constants (PageRank.C:126-138)
@@ -517,10 +520,11 @@ rg_status pagerank_run(rg_graph* g, int variant, int64_t max_iters, double* h_ra
   const int vblocks = (int)std::min<int64_t>((n + 255) / 256, (int64_t)sms * 16);
 
   CallTimer timer(g);
-  U128* A = S.acc.as<U128>();
-  double* P = S.p.as<double>();
-  double* C = S.contrib.as<double>();
-  unsigned long long* R = S.rmag.as<unsigned long long>();
+  char* arrays = S.arrays.as<char>();
+  double* C = reinterpret_cast<double*>(arrays);
+  U128* A = reinterpret_cast<U128*>(arrays + row);
+  double* P = reinterpret_cast<double*>(arrays + 3 * row);
+  unsigned long long* R = reinterpret_cast<unsigned long long*>(arrays + 4 * row);
   U128* L1 = S.l1.as<U128>();
   // The whole run (init + every iteration) is enqueued without host round
   // trips; each kernel's launch overlaps the one before it (not while per-kernel
