@@ -25,6 +25,8 @@
 
 #include <algorithm>
 #include <atomic>
+#include <utility>
+#include <vector>
 
 #include "fused.cuh"
 #include "pr_exact.cuh"
@@ -1592,11 +1594,32 @@ int64_t max_in_degree(const rg_graph* g, cudaStream_t st) {
   return h;
 }
 
-struct FusedState {
-  DevBuf ctl, bits0, bits1, i32a, i32b, f64a, f64b, f64c, u64a, u64b, row, opens, closes, l1, planes, out;
-  DevBuf qs0, qs1, qs2, ql0, ql1, ql2, first_s, first_l, level_deg, heavy;
+// The arrays of one launch, in the thread's one allocation: large ones on whole
+// pages.  (Allocated one by one, their placement after earlier allocations of the
+// process moved BFS on 2^24 vertices between 1.02 and 1.13 ms.)
+thread_local DevBuf g_arena;
+
+class Arrays {
+ public:
+  template <class T>
+  void add(T** p, size_t count) {
+    const size_t bytes = std::max<size_t>(count * sizeof(T), 16);
+    const size_t align = bytes >= kPage ? kPage : 256;
+    total_ = (total_ + align - 1) / align * align;
+    at_.push_back({reinterpret_cast<void**>(p), total_});
+    total_ += bytes;
+  }
+  rg_status place() {
+    RG_TRY(g_arena.reserve(total_));
+    for (const auto& a : at_) *a.first = g_arena.as<char>() + a.second;
+    return RG_OK;
+  }
+
+ private:
+  static constexpr size_t kPage = 2 << 20;
+  std::vector<std::pair<void**, size_t>> at_;
+  size_t total_ = 0;
 };
-thread_local FusedState S;
 
 int fused_grid(int64_t work, int64_t per_cta) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(device_sms(), work / per_cta));
@@ -1630,11 +1653,9 @@ size_t small_entries(int64_t n) { return (size_t)(n + 32); }
 size_t large_entries(int64_t n, int64_t m) {
   return (size_t)(std::min<int64_t>(n, m / (kSmallDeg + 1)) + m / kPiece + 64);
 }
-rg_status queue_pair(int64_t n, int64_t m, DevBuf& s, DevBuf& l, Queues* q, int groups = 1) {
-  RG_TRY(s.reserve(16 * small_entries(n) * groups));
-  RG_TRY(l.reserve(16 * large_entries(n, m) * groups));
-  *q = Queues{s.as<uint4>(), l.as<uint4>()};
-  return RG_OK;
+void add_queues(Arrays& X, Queues* q, int64_t n, int64_t m, int groups = 1) {
+  X.add(&q->small, small_entries(n) * groups);
+  X.add(&q->large, large_entries(n, m) * groups);
 }
 
 int64_t dense_threshold(const rg_graph* g) { return g->m / std::max<int64_t>(g_opts.dense_div, 1); }
@@ -1669,26 +1690,25 @@ rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t
   cudaStream_t st = cx.stream;
   const int64_t n = g->n, m = g->m, nwords = (n + 31) / 32;
   BfsArgs A;
-  RG_TRY(S.ctl.reserve(sizeof(Ctl)));
-  RG_TRY(S.bits0.reserve(4 * nwords));
-  RG_TRY(S.bits1.reserve(4 * nwords));
-  RG_TRY(S.i32a.reserve(4 * n));
-  if (h_parents) RG_TRY(S.i32b.reserve(4 * n));
-  RG_TRY(queue_pair(n, m, S.qs0, S.ql0, &A.q[0]));
-  RG_TRY(queue_pair(n, m, S.qs1, S.ql1, &A.q[1]));
+  A.parents = nullptr;
+  A.depth_out = nullptr;
   const bool order = g->sorted && (h_depth || d_depth_out);
-  if (order && !d_depth_out) RG_TRY(S.out.reserve(4 * n));
+  Arrays X;
+  X.add(&A.ctl, 1);
+  X.add(&A.vis[0], nwords);
+  X.add(&A.vis[1], nwords);
+  X.add(&A.depth, n);
+  if (h_parents) X.add(&A.parents, n);
+  add_queues(X, &A.q[0], n, m);
+  add_queues(X, &A.q[1], n, m);
+  if (order && !d_depth_out) X.add(&A.depth_out, n);
+  RG_TRY(X.place());
+  if (order && d_depth_out) A.depth_out = d_depth_out;
   A.out = g->view();
   A.in = g->in_view();
   A.new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
   A.root = root;
   A.threshold = dense_threshold(g);
-  A.vis[0] = S.bits0.as<uint32_t>();
-  A.vis[1] = S.bits1.as<uint32_t>();
-  A.depth = S.i32a.as<int32_t>();
-  A.parents = h_parents ? S.i32b.as<uint32_t>() : nullptr;
-  A.depth_out = order ? (d_depth_out ? d_depth_out : S.out.as<int32_t>()) : nullptr;
-  A.ctl = S.ctl.as<Ctl>();
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = cx.ws.h_info;
   info[3] = 0;
@@ -1713,35 +1733,29 @@ rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t
 namespace {
 
 // The arrays of `groups` groups of bc_fused.
-rg_status bc_arrays(const rg_graph* g, int groups, BcArgs* A) {
-  const int64_t n = g->n, m = g->m;
-  RG_TRY(S.ctl.reserve(sizeof(Ctl) * groups));
-  RG_TRY(S.i32a.reserve(4 * (size_t)n * groups));
-  RG_TRY(S.f64a.reserve(8 * (size_t)n * groups));
-  RG_TRY(S.f64b.reserve(8 * (size_t)n * groups));
-  RG_TRY(queue_pair(n, m, S.qs0, S.ql0, &A->q, groups));
-  RG_TRY(S.first_s.reserve(4 * (size_t)(n + 2) * groups));
-  RG_TRY(S.first_l.reserve(4 * (size_t)(n + 2) * groups));
-  RG_TRY(S.level_deg.reserve(8 * (size_t)(n + 2) * groups));
-  RG_TRY(S.bits0.reserve(4 * (size_t)((n + 31) / 32) * groups));
-  A->vis = S.bits0.as<uint32_t>();
-  A->n_small = small_entries(n);
-  A->n_large = large_entries(n, m);
+// *ordered (unless null): n results by original id.
+rg_status bc_arrays(const rg_graph* g, int groups, BcArgs* A, double** ordered) {
+  const size_t n = (size_t)g->n, m = (size_t)g->m;
+  A->n_small = small_entries(g->n);
+  A->n_large = large_entries(g->n, g->m);
   A->same = !g->directed;
   A->long_lists = std::max(max_in_degree(g, ctx().stream), (int64_t)g->max_deg) > kLongList;
   // pieces of lists above kLongList, two at least: at most 3/2 per kLongPiece edges
-  A->n_heavy = A->long_lists ? (size_t)(m / kLongPiece + m / kLongList + 64) : 0;
-  RG_TRY(S.heavy.reserve(16 * std::max<size_t>(A->n_heavy, 1) * groups));
-  A->level_deg = S.level_deg.as<unsigned long long>();
-  A->heavy = S.heavy.as<uint4>();
+  A->n_heavy = A->long_lists ? m / kLongPiece + m / kLongList + 64 : 0;
   A->new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
-  A->lvl = S.i32a.as<int32_t>();
-  A->sigma = S.f64a.as<double>();
-  A->deps = S.f64b.as<double>();
-  A->first_small = S.first_s.as<uint32_t>();
-  A->first_large = S.first_l.as<uint32_t>();
-  A->ctl = S.ctl.as<Ctl>();
-  return RG_OK;
+  Arrays X;
+  X.add(&A->ctl, groups);
+  X.add(&A->vis, (n + 31) / 32 * groups);
+  X.add(&A->lvl, n * groups);
+  X.add(&A->sigma, n * groups);
+  X.add(&A->deps, n * groups);
+  add_queues(X, &A->q, g->n, g->m, groups);
+  X.add(&A->first_small, (n + 2) * groups);
+  X.add(&A->first_large, (n + 2) * groups);
+  X.add(&A->level_deg, (n + 2) * groups);
+  X.add(&A->heavy, A->n_heavy * groups);
+  if (ordered) X.add(ordered, n);
+  return X.place();
 }
 
 }  // namespace
@@ -1752,14 +1766,13 @@ rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* 
   cudaStream_t st = cx.stream;
   const int64_t n = g->n, m = g->m;
   BcArgs A;
-  RG_TRY(bc_arrays(g, 1, &A));
   const bool order = g->sorted && (h_deps || d_deps_out);
-  if (order && !d_deps_out) RG_TRY(S.f64c.reserve(8 * n));
+  double* ordered = order ? d_deps_out : nullptr;
+  RG_TRY(bc_arrays(g, 1, &A, order && !d_deps_out ? &ordered : nullptr));
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = cx.ws.h_info;
   info[0] = info[1] = info[3] = 0;
   CallTimer timer(g);
-  double* ordered = order ? (d_deps_out ? d_deps_out : S.f64c.as<double>()) : nullptr;
   A.k = 1;
   A.rows = false;
   for (int it = 0; it < nsrc; it++) {
@@ -1798,7 +1811,7 @@ rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double
   const int groups = (k + (k + most - 1) / most - 1) / ((k + most - 1) / most);  // as many rounds, evenly filled
   const int width = std::min(fused_grid(m + n, kFusedEdgesPerCta), std::max(1, device_sms() / groups));
   BcArgs A;
-  RG_TRY(bc_arrays(g, groups, &A));
+  RG_TRY(bc_arrays(g, groups, &A, nullptr));
   A.g = g->view();
   A.gt = g->in_view();
   for (int q = 0; q < k; q++) A.source[q] = src_orig[q];
@@ -1825,15 +1838,23 @@ rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double
 namespace {
 
 // What Radii and multi-source BFS share; seeds: original ids, each once.
-rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int k, RadiiArgs* A) {
+// ordered: n radii by original id too; planes: the depth planes.
+rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int k, bool ordered,
+                     bool planes, RadiiArgs* A) {
   const int64_t n = g->n, m = g->m;
-  RG_TRY(S.ctl.reserve(sizeof(Ctl)));
-  RG_TRY(S.bits0.reserve(4 * ((n + 31) / 32)));
-  RG_TRY(S.u64a.reserve(8 * n));
-  RG_TRY(S.u64b.reserve(8 * n));
-  RG_TRY(S.i32a.reserve(4 * n));
-  RG_TRY(queue_pair(n, m, S.qs0, S.ql0, &A->q[0]));
-  RG_TRY(queue_pair(n, m, S.qs1, S.ql1, &A->q[1]));
+  A->radii_out = nullptr;
+  A->planes = nullptr;
+  Arrays X;
+  X.add(&A->ctl, 1);
+  X.add(&A->bits, (n + 31) / 32);
+  X.add(&A->vis, n);
+  X.add(&A->nvis, n);
+  X.add(&A->radii, n);
+  add_queues(X, &A->q[0], n, m);
+  add_queues(X, &A->q[1], n, m);
+  if (ordered) X.add(&A->radii_out, n);
+  if (planes) X.add(&A->planes, (size_t)n * kPlanes);
+  RG_TRY(X.place());
   A->out = g->view();
   A->in = g->in_view();
   A->chunk_v = g->in_chunks();
@@ -1845,15 +1866,8 @@ rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned lo
     A->mask[i] = masks[i];
   }
   A->threshold = dense_threshold(g);
-  A->vis = S.u64a.as<unsigned long long>();
-  A->nvis = S.u64b.as<unsigned long long>();
-  A->radii = S.i32a.as<int32_t>();
-  A->radii_out = nullptr;
-  A->bits = S.bits0.as<uint32_t>();
-  A->planes = nullptr;
   A->depths = nullptr;
   A->sources = 0;
-  A->ctl = S.ctl.as<Ctl>();
   A->info = ctx().ws.h_info_dev;
   ctx().ws.h_info[3] = 0;
   return RG_OK;
@@ -1867,10 +1881,9 @@ rg_status radii_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned lon
   cudaStream_t st = cx.stream;
   const int64_t n = g->n, m = g->m;
   RadiiArgs A;
-  RG_TRY(radii_args(g, seeds, masks, k, &A));
   const bool order = g->sorted && (h_radii || d_radii_out);
-  if (order && !d_radii_out) RG_TRY(S.out.reserve(4 * n));
-  A.radii_out = order ? (d_radii_out ? d_radii_out : S.out.as<int32_t>()) : nullptr;
+  RG_TRY(radii_args(g, seeds, masks, k, order && !d_radii_out, false, &A));
+  if (order && d_radii_out) A.radii_out = d_radii_out;
   volatile uint64_t* info = cx.ws.h_info;
   CallTimer timer(g);
   RG_TRY(launch_fused(radii_fused<false>, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
@@ -1892,9 +1905,7 @@ rg_status ms_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long l
   cudaStream_t st = cx.stream;
   const int64_t n = g->n, m = g->m;
   RadiiArgs A;
-  RG_TRY(radii_args(g, seeds, masks, u, &A));
-  RG_TRY(S.planes.reserve(8 * (size_t)n * kPlanes));
-  A.planes = S.planes.as<unsigned long long>();
+  RG_TRY(radii_args(g, seeds, masks, u, false, true, &A));
   A.depths = out;
   A.sources = k;
   volatile uint64_t* info = cx.ws.h_info;
@@ -1926,34 +1937,28 @@ rg_status pagerank_fused_run(rg_graph* g, int64_t max_iters, double* h_ranks, in
   // a row is not shared between CTAs: one with far more edges than a CTA's
   // share would hold the others up
   if (rows > kFusedPrRows || max_in_degree(g, st) > 2 * share) return RG_OK;
-  RG_TRY(S.ctl.reserve(sizeof(Ctl)));
-  RG_TRY(S.row.reserve(4 * (size_t)(m / 4 + 32 * (grid + 2) + 64)));
-  RG_TRY(S.opens.reserve(sizeof(U128) * (size_t)(m / kPrStep + 2 * grid + 4)));
-  RG_TRY(S.closes.reserve(sizeof(U128) * (size_t)(m / kPrStep + 2 * grid + 4)));
-  RG_TRY(S.f64a.reserve(8 * n));
-  RG_TRY(S.f64b.reserve(8 * n));
-  RG_TRY(S.u64b.reserve(8 * n));
-  RG_TRY(S.u64a.reserve(8 * n));
-  RG_TRY(S.l1.reserve(sizeof(L1Sum) * std::max<int64_t>(max_iters, 1)));
   const bool order = g->sorted && h_ranks;
-  if (order) RG_TRY(S.f64c.reserve(8 * n));
+  const size_t steps = (size_t)(m / kPrStep + 2 * grid + 4);
+  A.ranks_out = nullptr;
+  Arrays X;
+  X.add(&A.ctl, 1);
+  X.add(&A.lane_row, (size_t)(m / 4 + 32 * (grid + 2) + 64));
+  X.add(&A.opens, steps);
+  X.add(&A.closes, steps);
+  X.add(&A.p, n);
+  X.add(&A.contrib[0], n);
+  X.add(&A.contrib[1], n);
+  X.add(&A.rmag, n);
+  X.add(&A.l1, std::max<int64_t>(max_iters, 1));
+  if (order) X.add(&A.ranks_out, n);
+  RG_TRY(X.place());
   A.in = g->in_view();
   A.out_off = g->off.as<uint32_t>();
   A.chunk_v = g->in_chunks();
   A.new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
-  A.lane_row = S.row.as<uint32_t>();
-  A.opens = S.opens.as<U128>();
-  A.closes = S.closes.as<U128>();
-  A.p = S.f64a.as<double>();
-  A.contrib[0] = S.f64b.as<double>();
-  A.contrib[1] = S.u64b.as<double>();
-  A.rmag = S.u64a.as<unsigned long long>();
-  A.ranks_out = order ? S.f64c.as<double>() : nullptr;
-  A.l1 = S.l1.as<L1Sum>();
   A.max_iters = max_iters;
   A.p0 = 1 / (double)n;
   A.added = (1 - kPrDamp) * (1 / (double)n);
-  A.ctl = S.ctl.as<Ctl>();
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = cx.ws.h_info;
   info[3] = 0;
@@ -1981,11 +1986,13 @@ rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max
   cudaStream_t st = cx.stream;
   const int64_t n = g->n, m = g->m;
   PrdArgs A;
-  RG_TRY(S.ctl.reserve(sizeof(Ctl)));
-  RG_TRY(queue_pair(n, m, S.qs0, S.ql0, &A.q[0]));
-  RG_TRY(queue_pair(n, m, S.qs1, S.ql1, &A.q[1]));
-  if (start == 0) RG_TRY(queue_pair(n, m, S.qs2, S.ql2, &A.rows));
-  else A.rows = Queues{};
+  A.rows = Queues{};
+  Arrays X;
+  X.add(&A.ctl, 1);
+  add_queues(X, &A.q[0], n, m);
+  add_queues(X, &A.q[1], n, m);
+  if (start == 0) add_queues(X, &A.rows, n, m);
+  RG_TRY(X.place());
   A.out = g->view();
   A.in = g->in_view();
   A.new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
@@ -2000,7 +2007,6 @@ rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max
   A.one_over_n = 1 / (double)n;
   A.added = (1 - kPrDamp) * A.one_over_n;
   A.ranks_out = ranks_out;
-  A.ctl = S.ctl.as<Ctl>();
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = cx.ws.h_info;
   info[3] = 0;
