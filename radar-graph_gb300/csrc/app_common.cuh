@@ -63,6 +63,29 @@ struct CallTimer {
 int device_sms();     // of the calling thread's current device
 int max_dyn_smem();   // opt-in shared memory per block, same device
 
+// A kernel of a sequence is launched while the one before it drains
+// (launch_following): it lets its own follower in and waits for its predecessor
+// to complete before it reads anything.  A plain launch passes straight through.
+__device__ __forceinline__ void follow() {
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+}
+
+template <class... P, class... A>
+cudaError_t launch_following(void (*kern)(P...), int grid, int threads, size_t dyn, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = dyn;
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 // Runs fn (returning rg_status) once per device, however many threads call:
 // kernel attributes are per device, and a flag without the device id would
 // leave a second device unset.  `done` holds one bit per device id.

@@ -1378,11 +1378,13 @@ struct PrdArgs {
   const uint32_t* new_ids;
   double *p, *ngh, *c;
   uint32_t* bits;  // the frontier, as the last filter left it
+  uint32_t* touched;  // the vertices that a short push reached (0 between rounds)
   Queues rows;     // every row with in-edges (whole runs only)
   Queues q[2];
   int64_t start;   // rounds already run level by level (0: a whole run)
   int64_t max_iters;
   int64_t threshold;
+  int64_t short_push;  // edges up to which a push notes what it reaches
   bool allow_pull;
   double one_over_n, added;
   double* ranks_out;  // original-id order; null: not wanted (or not sorted)
@@ -1395,6 +1397,12 @@ struct PrdArgs {
 // next frontier as prd_filter does, skipping words that nothing reached and that
 // held no member.  A run can be taken over after its dense first rounds, which
 // large graphs sweep with a launch of their own.
+//
+// A round of few edges is a chain of latencies: two grid barriers, the push and the
+// filter.  Its push notes the vertices that it reaches, so that the filter looks at
+// up to 1024 vertices at a time and loads only what has changed: reading every sum
+// instead, a word after the other, was most of such a round (2^21 vertices, 14
+// rounds: 270 us).
 __global__ void __launch_bounds__(kFT, 1) prd_fused(const __grid_constant__ PrdArgs A) {
   __shared__ Shared sh;
   __shared__ Member buf[kFWarps][kBuf];
@@ -1417,7 +1425,7 @@ __global__ void __launch_bounds__(kFT, 1) prd_fused(const __grid_constant__ PrdA
         const uint32_t d = A.out.off[v + 1] - A.out.off[v];
         A.c[v] = d ? A.one_over_n / d : 0.0;
       }
-      if (lane == 0) A.bits[w] = 0u;
+      if (lane == 0) A.bits[w] = A.touched[w] = 0u;
       const uint32_t b = A.in.off[v], e = A.in.off[v + 1];
       ap.add(in && e > b, v, b, e, A.rows, &A.ctl->lv[3], 0, 0);
     }
@@ -1435,6 +1443,7 @@ __global__ void __launch_bounds__(kFT, 1) prd_fused(const __grid_constant__ PrdA
   } else {
     for (uint32_t w = warp; w < nwords; w += nwarps) {
       const uint32_t x = A.bits[w];
+      if (lane == 0) A.touched[w] = 0u;
       if (!x) continue;
       const uint32_t v = min(w * 32 + lane, n - 1);
       ap.add((x >> lane) & 1u, v, A.out.off[v], A.out.off[v + 1], A.q[0], &A.ctl->lv[0], 0, 0);
@@ -1453,7 +1462,9 @@ __global__ void __launch_bounds__(kFT, 1) prd_fused(const __grid_constant__ PrdA
     k++;
     edges += c.degsum;
     const bool whole = A.start == 0 && k == 1;  // the queue does not hold the first frontier of a whole run
-    if (whole || (A.start == 0 && A.allow_pull && (int64_t)(c.count + c.degsum) > A.threshold)) {
+    const bool pull = whole || (A.start == 0 && A.allow_pull && (int64_t)(c.count + c.degsum) > A.threshold);
+    const bool noted = !pull && (int64_t)c.degsum <= A.short_push;
+    if (pull) {
       const uint32_t gwarp = (uint32_t)(wid * gridDim.x + blockIdx.x);
       for (uint32_t i0 = gwarp * 4; i0 < rl; i0 += nwarps * 4) {
         double acc[4];
@@ -1498,20 +1509,22 @@ __global__ void __launch_bounds__(kFT, 1) prd_fused(const __grid_constant__ PrdA
         const double x = A.c[s];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-          if (in[j]) atomicAdd(A.ngh + d[j], x);
+          if (in[j]) {
+            atomicAdd(A.ngh + d[j], x);
+            if (noted) atomicOr(A.touched + (d[j] >> 5), 1u << (d[j] & 31));
+          }
         }
       });
     }
     if (!grid.sync()) return;
     const Queues nq = A.q[cq ^ 1];
     double local = 0.0;
-    for (uint32_t w = warp; w < nwords; w += nwarps) {
+    auto filter = [&](uint32_t w) {
       const bool in = w * 32 + lane < n;
       const uint32_t v = in ? w * 32 + lane : n - 1;
       const double g = in ? A.ngh[v] : 0.0;
-      const uint32_t old = A.bits[w];
       // nothing arrived and nobody was active: delta is 0, the vertex stays as it is
-      if (round > 1 && !old && !__any_sync(kAll, g != 0.0)) continue;
+      if (!noted && round > 1 && !A.bits[w] && !__any_sync(kAll, g != 0.0)) return;
       bool act = false;
       uint32_t b = 0, e = 0;
       if (in) {
@@ -1536,6 +1549,19 @@ __global__ void __launch_bounds__(kFT, 1) prd_fused(const __grid_constant__ PrdA
       const unsigned now = __ballot_sync(kAll, act);
       if (lane == 0) A.bits[w] = now;
       ap.add(act, v, b, e, nq, ns, 0, 0);
+    };
+    if (noted) {
+      const uint32_t take = min((nwords + nwarps - 1) / nwarps, 32u);  // words a warp looks at together
+      for (uint32_t w0 = warp * take; w0 < nwords; w0 += nwarps * take) {
+        const uint32_t w = w0 + lane;
+        const bool mine = lane < (int)take && w < nwords;
+        const uint32_t t = mine ? A.touched[w] : 0u;
+        unsigned todo = __ballot_sync(kAll, t || (mine && A.bits[w]));
+        if (t) A.touched[w] = 0u;
+        for (; todo; todo &= todo - 1) filter(w0 + __ffs(todo) - 1);
+      }
+    } else {
+      for (uint32_t w = warp; w < nwords; w += nwarps) filter(w);
     }
     ap.finish(nq, ns, 0, 0);
     local = warp_sum(local);
@@ -1992,6 +2018,7 @@ rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max
   add_queues(X, &A.q[0], n, m);
   add_queues(X, &A.q[1], n, m);
   if (start == 0) add_queues(X, &A.rows, n, m);
+  X.add(&A.touched, (n + 31) / 32);
   RG_TRY(X.place());
   A.out = g->view();
   A.in = g->in_view();
@@ -2003,6 +2030,7 @@ rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max
   A.start = start;
   A.max_iters = max_iters;
   A.threshold = dense_threshold(g);
+  A.short_push = n / 64;
   A.allow_pull = allow_pull;
   A.one_over_n = 1 / (double)n;
   A.added = (1 - kPrDamp) * A.one_over_n;

@@ -96,8 +96,26 @@ constexpr double kPrdEps = 0.0000001, kPrdEps2 = 0.01;  // PageRankDelta.C:103-1
 // The exact pull of pagerank.cu over signed contributions (PageRankDelta's):
 // acc[v] = sum of c over v's in-neighbours as a 128-bit two's complement fixed
 // point number.  acc must be 0 in the rows that cross a step of kExactStep edges.
+// The sweep does nothing if the gate is closed; it follows the kernel before it
+// (launch_following).
 constexpr uint32_t kExactStep = 512;
-rg_status exact_pull_signed(rg_graph* g, const double* c, U128* acc, cudaStream_t st);
+
+// What a PageRankDelta filter found, and the gate it is to the next round: that
+// pulls if the frontier is dense and the run goes on (a round that did nothing
+// leaves zeros, which close the gates after it).
+struct PrdTotals {
+  unsigned long long count, degsum;
+  double l1;
+  unsigned long long unused;
+};
+struct PrdGate {
+  const PrdTotals* prev;  // null: open
+  int64_t threshold;
+  __device__ __forceinline__ bool open() const {
+    return !prev || ((int64_t)(prev->count + prev->degsum) > threshold && !(prev->l1 < kPrdEps));
+  }
+};
+rg_status exact_pull_signed(rg_graph* g, const double* c, U128* acc, const PrdGate& gate, cudaStream_t st);
 
 // acc[v] += x for a 128-bit sum shared with other warps: the low word's
 // atomic returns the old value, so the carry out of it is known and goes into

@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -43,33 +44,15 @@ constexpr int kPullThreads = 256;
 constexpr uint32_t kNoRow = 0xFFFFFFFFu;
 constexpr int64_t kCacheVertices = 6 << 20;  // contributions above 48 MB
 
-// L1 of the previous iteration (exact) below 1e-7: this iteration is skipped.
+// Whether a sweep is skipped.  PageRank: the L1 of the previous iteration (exact)
+// is below 1e-7; PageRankDelta: the round's gate is closed.
 __device__ __forceinline__ bool converged(const U128* l1_prev) {
   return l1_prev != nullptr && less128(*l1_prev, pr_eps_fx());
 }
+__device__ __forceinline__ bool converged(const PrdGate& gate) { return !gate.open(); }
 
-// A kernel of an iteration is launched while the one before it drains
-// (launch_following): it lets its own follower in and waits for its predecessor
-// to complete before it reads anything.  A plain launch passes straight through.
-__device__ __forceinline__ void follow() {
-  cudaTriggerProgrammaticLaunchCompletion();
-  cudaGridDependencySynchronize();
-}
-
-template <class... P, class... A>
-cudaError_t launch_following(void (*kern)(P...), int grid, int threads, size_t dyn, cudaStream_t st, A&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = dyn;
-  cfg.stream = st;
-  cudaLaunchAttribute at = {};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
-}
+template <bool kSigned>
+using SkipArg = std::conditional_t<kSigned, PrdGate, const U128*>;
 
 // p = 1/n, contrib = p/deg (PageRank.C:126-138), rmag = the integer
 // reciprocal of each degree that is neither 0, 1 nor a power of two (for the
@@ -168,10 +151,10 @@ __global__ void __launch_bounds__(kSweepThreads) pr_push_sweep(DevGraph g, const
 template <bool kCache, int kItems, int kMode, bool kSigned = false>
 __global__ void __launch_bounds__(kCache ? 1024 : kPullThreads)
     pr_pull_sweep(DevGraph g, const uint32_t* __restrict__ chunk_v, uint32_t nchunks,
-                  const double* __restrict__ contrib, U128* acc, uint32_t H, const U128* l1_prev) {
+                  const double* __restrict__ contrib, U128* acc, uint32_t H, SkipArg<kSigned> skip) {
   static_assert(kItems == 4 || kItems == 8 || kItems == 16, "4, 8 or 16 edges per lane");
   follow();
-  if (converged(l1_prev)) return;
+  if (converged(skip)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* hc = reinterpret_cast<double*>(smem_raw);
   if (kCache) {
@@ -403,7 +386,7 @@ struct PrState {
 
 }  // namespace
 
-rg_status exact_pull_signed(rg_graph* g, const double* c, U128* acc, cudaStream_t st) {
+rg_status exact_pull_signed(rg_graph* g, const double* c, U128* acc, const PrdGate& gate, cudaStream_t st) {
   auto kern = pr_pull_sweep<false, 16, 1, true>;
   static std::atomic<uint64_t> carveout_set{0};
   RG_TRY(once_per_device(carveout_set, [&]() -> rg_status {
@@ -421,11 +404,10 @@ rg_status exact_pull_signed(rg_graph* g, const double* c, U128* acc, cudaStream_
                                          std::max<int64_t>((g->nchunks * 32 + kPullThreads - 1) / kPullThreads, 1));
   static_assert(kExactStep == 32 * 16, "a warp step of 16 edges per lane");
   kt_begin(st);
-  kern<<<(unsigned)grid, kPullThreads, 0, st>>>(g->in_view(), g->in_chunks(), (uint32_t)g->nchunks, c, acc, 0u, nullptr);
+  RG_CUDA(launch_following(kern, (int)grid, kPullThreads, 0, st, g->in_view(), g->in_chunks(), (uint32_t)g->nchunks, c,
+                           acc, 0u, gate));
   kt_end(st);
-  RG_CUDA(cudaGetLastError());
   g_timing.kernel_launches++;
-  g_timing.edge_launches++;
   return RG_OK;
 }
 

@@ -145,14 +145,41 @@ __host__ __device__ __forceinline__ unsigned long long mulhi64(unsigned long lon
 #endif
 }
 
+// a / d and its remainder for a < d * 2^32, with inv = 1.0f / d: an estimate of
+// 22 bits, one more for what it left (below 2^11 d), then at most one step either
+// way.  The compiler's 64-bit division costs several times as much.
+__host__ __device__ __forceinline__ uint32_t div_step(unsigned long long a, uint32_t d, float inv,
+                                                      unsigned long long* rem) {
+#ifdef __CUDA_ARCH__
+  uint32_t q = __float2uint_rz(__ull2float_rn(a) * inv);  // saturates
+#else
+  const float f = (float)a * inv;
+  uint32_t q = f >= 4294967296.0f ? 0xFFFFFFFFu : (uint32_t)f;
+#endif
+  long long r = (long long)(a - (unsigned long long)q * d);
+  const int t = (int)floorf((float)r * inv);
+  q += (uint32_t)t;
+  r -= (long long)t * d;
+  if (r < 0) {
+    q--;
+    r += d;
+  } else if (r >= (long long)d) {
+    q++;
+    r -= d;
+  }
+  *rem = (unsigned long long)r;
+  return q;
+}
+
 // The integer reciprocal of a degree d >= 3 that is not a power of two:
 // R = floor(2^(63+l) / d) with 2^(l-1) < d < 2^l, so R lies in [2^63, 2^64).
 // Long division in two 64-by-32-bit steps.
 __host__ __device__ __forceinline__ unsigned long long recip_magic(uint32_t d) {
   const int l = 32 - clz32(d);
-  const unsigned long long hi = 1ull << (31 + l);  // 2^(63+l) = hi * 2^32
-  const unsigned long long q1 = hi / d, r1 = hi % d;
-  return (q1 << 32) | ((r1 << 32) / d);
+  const float inv = 1.0f / (float)d;
+  unsigned long long r;
+  const unsigned long long q1 = div_step(1ull << (31 + l), d, inv, &r);  // 2^(63+l) = 2^(31+l) * 2^32
+  return (q1 << 32) | div_step(r << 32, d, inv, &r);
 }
 
 // a / d rounded to nearest, ties to even (the IEEE quotient), on the integer
@@ -202,6 +229,14 @@ __host__ __device__ __forceinline__ double deg_quotient(double a, uint32_t d, un
   if (d == 0) return 0.0;
   if ((d & (d - 1)) == 0) return double_of(bits_of(a) - ((unsigned long long)(31 - clz32(d)) << 52));
   return div_by_magic(a, d, R);
+}
+
+// The same quotient for a of either sign; values so small that it would be
+// subnormal (which no PageRankDelta run reaches) divide in FP64.
+__device__ __forceinline__ double deg_quotient_signed(double a, uint32_t d, unsigned long long R) {
+  const unsigned long long s = bits_of(a) & (1ull << 63), b = bits_of(a) ^ s;
+  if (b < (123ull << 52)) return d ? __ddiv_rn(a, (double)d) : 0.0;  // below 2^-900
+  return double_of(bits_of(deg_quotient(double_of(b), d, R)) | s);
 }
 
 // The L1 threshold of PageRank.C:172 (epsilon = 1e-7, the double) scaled
