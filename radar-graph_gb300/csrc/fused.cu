@@ -329,8 +329,11 @@ __device__ __forceinline__ void begin(Grid& grid, Shared* sh, Ctl* ctl) {
 // ---------------------------------------------------------------------------
 // BFS (BFS.C:122-188)
 // ---------------------------------------------------------------------------
+constexpr uint32_t kPullWords = 8;  // words of the visited bitmap that a warp takes together, at most
+
 struct BfsArgs {
   DevGraph out, in;  // push and pull lists
+  bool same;         // the same lists (a symmetric graph)
   const uint32_t* new_ids;  // null: not sorted
   uint32_t root;            // original id
   int64_t threshold;
@@ -345,7 +348,9 @@ struct BfsArgs {
 
 // A push level claims vertices with an atomicOr on the visited bitmap; a pull
 // level reads one bitmap and writes the other (a visited in-neighbour of an
-// unvisited vertex is in the frontier, so visited is all a pull has to test).
+// unvisited vertex is in the frontier, so visited is all a pull has to test) and, on
+// a symmetric graph, marks vertices without edges visited, so that later pulls pass
+// them by.
 __global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
   __shared__ Shared sh;
   __shared__ Member buf[kFWarps][kBuf];
@@ -356,6 +361,7 @@ __global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
   const int lane = threadIdx.x & 31;
   const uint32_t warp = tid >> 5, nwarps = nthreads >> 5;
+  const uint32_t take = min((nwords + nwarps - 1) / nwarps, kPullWords);
   const uint32_t root = A.new_ids ? A.new_ids[A.root] : A.root;
   for (uint32_t i = tid; i < n; i += nthreads) {
     A.depth[i] = i == root ? 0 : -1;
@@ -380,61 +386,96 @@ __global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
     reached += c.count;
     edges += c.degsum;
     if (tid == 0) A.ctl->lv[(level + 2) % 3] = Slot{};
-    const bool pull = (int64_t)(c.count + c.degsum) > A.threshold && c.degsum > 0;
+    // a symmetric graph's unvisited vertices hold the edges that no frontier had:
+    // where those are fewer, looking at them is cheaper than the frontier's pushes
+    const bool few = A.same && c.degsum > 2 * (A.out.m - edges) + n / 8;
+    const bool pull = ((int64_t)(c.count + c.degsum) > A.threshold || few) && c.degsum > 0;
     level++;
     uint32_t* vis = A.vis[cv];
     if (pull) {
       uint32_t* nvis = A.vis[cv ^ 1];
       unsigned count = 0;
       unsigned long long degsum = 0;
-      for (uint32_t w = warp; w < nwords; w += nwarps) {
-        const uint32_t seen = vis[w];
-        const uint32_t v = w * 32 + lane;
-        const bool want = v < n && !((seen >> lane) & 1u);
-        uint32_t b = 0, e = 0, from = kNone;
-        if (want) {
-          b = A.in.off[v];
-          e = A.in.off[v + 1];
-        }
-        // each lane tries its first 16 neighbours, four at a time; the lists
-        // that are longer are then read by the whole warp, one at a time
-        const uint32_t stop = min(e, b + 16);
-        for (; b < stop && from == kNone; b += 4) {
-          uint32_t u[4];
-          bool hit[4];
+      for (uint32_t w0 = warp; w0 < nwords; w0 += nwarps * take) {
+        const uint32_t mw = w0 + lane * nwarps;
+        const bool mine = lane < (int)take && mw < nwords;
+        uint32_t word = mine ? vis[mw] : kNone;
+        unsigned todo = __ballot_sync(kAll, (word | (mw == n >> 5 ? ~0u << (n & 31) : 0u)) != kNone);
+        uint32_t next = word;
+        while (todo) {
+          // two words at a time: the chain offset - neighbour - its bit is all latency
+          int j[2];
+          j[0] = __ffs(todo) - 1;
+          todo &= todo - 1;
+          j[1] = todo ? __ffs(todo) - 1 : j[0];
+          const bool two = todo != 0;
+          todo &= todo - 1;
+          uint32_t v[2], b[2], e[2], from[2];
 #pragma unroll
-          for (int k = 0; k < 4; k++) u[k] = b + k < e ? A.in.adj[b + k] : kNone;
-#pragma unroll
-          for (int k = 0; k < 4; k++) hit[k] = u[k] != kNone && bit_test(vis, u[k]);
-#pragma unroll
-          for (int k = 3; k >= 0; k--) {
-            if (hit[k]) from = u[k];
+          for (int i = 0; i < 2; i++) {
+            const uint32_t seen = __shfl_sync(kAll, word, j[i]);
+            v[i] = (w0 + j[i] * nwarps) * 32 + lane;
+            const bool want = (i == 0 || two) && v[i] < n && !((seen >> lane) & 1u);
+            b[i] = want ? A.in.off[v[i]] : 0u;
+            e[i] = want ? A.in.off[v[i] + 1] : 0u;
+            from[i] = kNone;
+            const unsigned alone = __ballot_sync(kAll, want && b[i] == e[i]);
+            if (A.same && lane == j[i]) next |= alone;
           }
-        }
-        unsigned rest = __ballot_sync(kAll, from == kNone && b < e);
-        while (rest) {
-          const int j = __ffs(rest) - 1;
-          rest &= rest - 1;
-          const uint32_t jb = __shfl_sync(kAll, b, j), je = __shfl_sync(kAll, e, j);
-          for (uint32_t x = jb; x < je; x += 32) {
-            const uint32_t u = x + lane < je ? A.in.adj[x + lane] : kNone;
-            const unsigned hits = __ballot_sync(kAll, u != kNone && bit_test(vis, u));
-            if (hits) {
-              const uint32_t f = __shfl_sync(kAll, u, __ffs(hits) - 1);
-              if (lane == j) from = f;
-              break;
+          // each lane tries its first 16 neighbours, four at a time; the lists
+          // that are longer are then read by the whole warp, one at a time
+          for (int t = 0; t < 4; t++) {
+            uint32_t u[2][4];
+            bool more = false;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+              const bool go = from[i] == kNone && b[i] < e[i];
+              more |= go;
+#pragma unroll
+              for (int k = 0; k < 4; k++) u[i][k] = go && b[i] + k < e[i] ? A.in.adj[b[i] + k] : kNone;
+            }
+            if (!__any_sync(kAll, more)) break;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+              bool hit[4];
+#pragma unroll
+              for (int k = 0; k < 4; k++) hit[k] = u[i][k] != kNone && bit_test(vis, u[i][k]);
+#pragma unroll
+              for (int k = 3; k >= 0; k--) {
+                if (hit[k]) from[i] = u[i][k];
+              }
+              b[i] = min(b[i] + 4, e[i]);
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            unsigned rest = __ballot_sync(kAll, from[i] == kNone && b[i] < e[i]);
+            while (rest) {
+              const int l = __ffs(rest) - 1;
+              rest &= rest - 1;
+              const uint32_t jb = __shfl_sync(kAll, b[i], l), je = __shfl_sync(kAll, e[i], l);
+              for (uint32_t x = jb; x < je; x += 32) {
+                const uint32_t u = x + lane < je ? A.in.adj[x + lane] : kNone;
+                const unsigned hits = __ballot_sync(kAll, u != kNone && bit_test(vis, u));
+                if (hits) {
+                  const uint32_t f = __shfl_sync(kAll, u, __ffs(hits) - 1);
+                  if (lane == l) from[i] = f;
+                  break;
+                }
+              }
+            }
+            const bool won = from[i] != kNone;
+            const unsigned now = __ballot_sync(kAll, won);
+            if (lane == j[i]) next |= now;
+            if (won) {
+              A.depth[v[i]] = level;
+              if (A.parents) A.parents[v[i]] = from[i];
+              count++;
+              degsum += A.out.off[v[i] + 1] - A.out.off[v[i]];
             }
           }
         }
-        const bool won = from != kNone;
-        const unsigned now = __ballot_sync(kAll, won);
-        if (lane == 0) nvis[w] = seen | now;
-        if (won) {
-          A.depth[v] = level;
-          if (A.parents) A.parents[v] = from;
-          count++;
-          degsum += A.out.off[v + 1] - A.out.off[v];
-        }
+        if (mine) nvis[mw] = next;
       }
       count = __reduce_add_sync(kAll, count);
       if (count) {
@@ -449,11 +490,15 @@ __global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
     } else {
       if (!queued) {  // after a pull: the frontier is what it added to the bitmap
         const uint32_t* old = A.vis[cv ^ 1];
-        for (uint32_t w = warp; w < nwords; w += nwarps) {
-          const uint32_t x = vis[w] & ~old[w];
-          if (!x) continue;
-          const uint32_t v = min(w * 32 + lane, n - 1);
-          ap.add((x >> lane) & 1u, v, A.out.off[v], A.out.off[v + 1], A.q[cq], cs, 0, 0);
+        for (uint32_t w0 = warp; w0 < nwords; w0 += nwarps * take) {
+          const uint32_t mw = w0 + lane * nwarps;
+          const uint32_t word = lane < (int)take && mw < nwords ? vis[mw] & ~old[mw] : 0u;
+          for (unsigned todo = __ballot_sync(kAll, word != 0u); todo; todo &= todo - 1) {
+            const int j = __ffs(todo) - 1;
+            const uint32_t x = __shfl_sync(kAll, word, j);
+            const uint32_t v = min((w0 + j * nwarps) * 32 + lane, n - 1);
+            ap.add((x >> lane) & 1u, v, A.out.off[v], A.out.off[v + 1], A.q[cq], cs, 0, 0);
+          }
         }
         ap.finish(A.q[cq], cs, 0, 0);
         if (!grid.sync()) return;  // (its members were counted by the pull)
