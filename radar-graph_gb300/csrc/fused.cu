@@ -1791,6 +1791,7 @@ rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t
   RG_TRY(download_orig<uint32_t>(g, A.parents, h_parents, tmp, st));
   RG_CUDA(cudaStreamSynchronize(st));
   RG_TRY(timer.finish());
+  A.same = !g->directed;
   *done = info[3] == 1;
   if (!*done) return RG_OK;
   g_timing.edges_traversed = (int64_t)info[2];
