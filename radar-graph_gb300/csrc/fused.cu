@@ -1731,6 +1731,18 @@ void add_queues(Arrays& X, Queues* q, int64_t n, int64_t m, int groups = 1) {
 
 int64_t dense_threshold(const rg_graph* g) { return g->m / std::max<int64_t>(g_opts.dense_div, 1); }
 
+// Where a launch may write its results by original id itself: page-locked memory of
+// the caller (null: none, they are delivered afterwards).  The host link takes a
+// kernel's stores at the rate of a copy (183 of 186 GB/s), so the reordering, a
+// random read per vertex, and the result's way through memory hide behind it: BFS
+// of 2^24 vertices 805 us, 927 with a copy.  (Rows of several sources are
+// copied: stores to 64 rows at once took 2.7 ms in place of 2.0.)
+template <class T>
+T* direct_results(const rg_graph* g, const T* host_out, const T* dev_out) {
+  if (!g->sorted || !host_out || dev_out || g_opts.async_results) return nullptr;
+  return static_cast<T*>(device_alias(host_out, sizeof(T) * g->n, sizeof(T)));
+}
+
 // The results of a finished launch on their way to the caller: `dev_out`
 // (device, original ids) and `host_out`.  `internal` holds them by internal
 // id, `ordered` (when the launch wrote it) by original id.
@@ -1772,11 +1784,14 @@ rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t
   if (h_parents) X.add(&A.parents, n);
   add_queues(X, &A.q[0], n, m);
   add_queues(X, &A.q[1], n, m);
-  if (order && !d_depth_out) X.add(&A.depth_out, n);
+  int32_t* direct = direct_results(g, h_depth, d_depth_out);
+  if (order && !d_depth_out && !direct) X.add(&A.depth_out, n);
   RG_TRY(X.place());
+  if (direct) A.depth_out = direct;
   if (order && d_depth_out) A.depth_out = d_depth_out;
   A.out = g->view();
   A.in = g->in_view();
+  A.same = !g->directed;
   A.new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
   A.root = root;
   A.threshold = dense_threshold(g);
@@ -1786,12 +1801,11 @@ rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t
   CallTimer timer(g);
   RG_TRY(launch_fused(bfs_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
   RG_TRY(timer.mark());
-  RG_TRY(deliver<int32_t>(g, A.depth, A.depth_out, h_depth, d_depth_out, st));
+  if (!direct) RG_TRY(deliver<int32_t>(g, A.depth, A.depth_out, h_depth, d_depth_out, st));
   DevBuf tmp(true, st);  // parents by original id
   RG_TRY(download_orig<uint32_t>(g, A.parents, h_parents, tmp, st));
   RG_CUDA(cudaStreamSynchronize(st));
   RG_TRY(timer.finish());
-  A.same = !g->directed;
   *done = info[3] == 1;
   if (!*done) return RG_OK;
   g_timing.edges_traversed = (int64_t)info[2];
@@ -1839,8 +1853,9 @@ rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* 
   const int64_t n = g->n, m = g->m;
   BcArgs A;
   const bool order = g->sorted && (h_deps || d_deps_out);
-  double* ordered = order ? d_deps_out : nullptr;
-  RG_TRY(bc_arrays(g, 1, &A, order && !d_deps_out ? &ordered : nullptr));
+  double* direct = direct_results(g, h_deps, d_deps_out);
+  double* ordered = !order ? nullptr : direct ? direct : d_deps_out;
+  RG_TRY(bc_arrays(g, 1, &A, order && !ordered ? &ordered : nullptr));
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = cx.ws.h_info;
   info[0] = info[1] = info[3] = 0;
@@ -1857,7 +1872,7 @@ rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* 
     RG_TRY(launch_fused(bc_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
   }
   RG_TRY(timer.mark());
-  RG_TRY(deliver<double>(g, A.deps, ordered, h_deps, d_deps_out, st));
+  if (!direct) RG_TRY(deliver<double>(g, A.deps, ordered, h_deps, d_deps_out, st));
   RG_CUDA(cudaStreamSynchronize(st));
   RG_TRY(timer.finish());
   *done = info[3] == (uint64_t)nsrc;
@@ -1954,13 +1969,15 @@ rg_status radii_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned lon
   const int64_t n = g->n, m = g->m;
   RadiiArgs A;
   const bool order = g->sorted && (h_radii || d_radii_out);
-  RG_TRY(radii_args(g, seeds, masks, k, order && !d_radii_out, false, &A));
+  int32_t* direct = direct_results(g, h_radii, d_radii_out);
+  RG_TRY(radii_args(g, seeds, masks, k, order && !d_radii_out && !direct, false, &A));
+  if (direct) A.radii_out = direct;
   if (order && d_radii_out) A.radii_out = d_radii_out;
   volatile uint64_t* info = cx.ws.h_info;
   CallTimer timer(g);
   RG_TRY(launch_fused(radii_fused<false>, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
   RG_TRY(timer.mark());
-  RG_TRY(deliver<int32_t>(g, A.radii, A.radii_out, h_radii, d_radii_out, st));
+  if (!direct) RG_TRY(deliver<int32_t>(g, A.radii, A.radii_out, h_radii, d_radii_out, st));
   RG_CUDA(cudaStreamSynchronize(st));
   RG_TRY(timer.finish());
   *done = info[3] == 1;

@@ -9,6 +9,7 @@
 // relabelled in place order (IO.h:877-895 keeps the order, it does not
 // re-sort).
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdarg.h>
 #include <stdio.h>
@@ -89,6 +90,32 @@ rg_status read_small(const void* d_src, void* h_dst, size_t bytes, cudaStream_t 
   RG_CUDA(cudaStreamSynchronize(st));
   memcpy(h_dst, ws.h_small, bytes);
   return RG_OK;
+}
+
+void* device_alias(const void* p, size_t bytes, size_t align) {
+  typedef CUresult (*GetAttributes)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+  static const GetAttributes get = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      f = nullptr;
+    }
+    return reinterpret_cast<GetAttributes>(f);
+  }();
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+  if (!p || !get || at % align) return nullptr;
+  unsigned int type = 0, managed = 0;
+  CUdeviceptr dev = 0, start = 0;
+  size_t size = 0;
+  CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void* into[] = {&type, &managed, &dev, &start, &size};
+  if (get(5, what, into, (CUdeviceptr)at) != CUDA_SUCCESS) return nullptr;
+  if (type != CU_MEMORYTYPE_HOST || managed || !dev || !start || dev < start || dev - start > size) return nullptr;
+  return size - (dev - start) >= bytes ? reinterpret_cast<void*>(dev) : nullptr;
 }
 
 static thread_local Ctx* t_ctx = nullptr;
@@ -1164,15 +1191,6 @@ namespace rg {
 rg_status build_in_lists(rg_graph* g, cudaStream_t st);
 }
 
-// The device's address of page-locked host memory (false: pageable).
-static bool host_on_device(const uint32_t* h, const uint32_t** d) {
-  cudaPointerAttributes pa;
-  const bool ok = cudaPointerGetAttributes(&pa, h) == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer;
-  cudaGetLastError();  // an unregistered pointer is not an error here
-  if (ok) *d = static_cast<const uint32_t*>(pa.devicePointer);
-  return ok;
-}
-
 // Shared by the symmetric and directed builders.  Symmetric: entries
 // (a, b) = [src, dst] x [dst, src]; directed: (src, dst) only, and the
 // in-lists are built afterwards.
@@ -1216,7 +1234,11 @@ static rg_status create_from_edges(const char* who, int64_t n, int64_t num_edges
       RG_TRY(k1.reserve(8 * (size_t)k + 16));
       RG_TRY(sort_begin(sort, k, passes, st));
       const uint32_t *d_src = src, *d_dst = dst;
-      if (!on_device && !(host_on_device(src, &d_src) && host_on_device(dst, &d_dst))) {
+      if (!on_device) {
+        d_src = static_cast<const uint32_t*>(device_alias(src, 4 * num_edges, 4));
+        d_dst = static_cast<const uint32_t*>(device_alias(dst, 4 * num_edges, 4));
+      }
+      if (!d_src || !d_dst) {
         // pageable: copied (into the sort's second buffer, free until its first pass)
         uint32_t* c2 = k1.as<uint32_t>();
         RG_CUDA(cudaMemcpyAsync(c2, src, 4 * num_edges, cudaMemcpyHostToDevice, st));

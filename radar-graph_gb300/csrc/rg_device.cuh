@@ -195,6 +195,10 @@ namespace rg {
 // copy): small reads on a level's critical path then never wait behind a
 // large copy another stream has on a copy engine.  Syncs `st`.
 constexpr size_t kSmallRead = 65536;
+// The device's address of `bytes` of page-locked host memory at p, aligned to
+// `align`, for kernels that write results there themselves; null for any other
+// memory and for a range that the allocation does not hold.
+void* device_alias(const void* p, size_t bytes, size_t align);
 rg_status read_small(const void* d_src, void* h_dst, size_t bytes, cudaStream_t st);
 
 // Exclusive scan of `n` uint32 values into out[0..n] (out[n] = total).
