@@ -75,7 +75,10 @@ struct L1Sum {
 // Zeroed before every launch.
 struct Ctl {
   unsigned int bar, fail;
-  unsigned int pad[14];
+  unsigned int bar_all;  // of all groups (BC)
+  int levels;            // of the group's source (BC)
+  unsigned long long edges;
+  unsigned int pad[10];
   Slot lv[4];
 };
 
@@ -103,9 +106,16 @@ struct Member {
   uint32_t v, b, e;
 };
 
+// The CTAs that meet at a barrier.
+struct Team {
+  unsigned *bar, *fail;
+  unsigned target, ctas;
+};
+
 // What a CTA shares: its members' totals, what the last barrier completed and
 // the barrier's verdict.
 struct Shared {
+  Team team[2];  // the group's CTAs, and all of them (BC)
   unsigned int count;
   unsigned long long degsum;
   Slot slot;  // the frontier that the last barrier completed
@@ -124,9 +134,8 @@ __device__ __forceinline__ Slot read_slot(const Slot* s) {
 }
 
 struct Grid {
-  Ctl* ctl;
   Shared* sh;
-  unsigned target;
+  int which;
 
   // All CTAs meet; this CTA's totals go into `slot` first (null: dropped) and the
   // completed slot comes back in sh->slot (and the completed sum `l1` in sh->l1).
@@ -135,8 +144,9 @@ struct Grid {
   // ran out.
   __device__ __forceinline__ bool sync(Slot* slot = nullptr, const L1Sum* l1 = nullptr, bool keep = false) {
     __syncthreads();
-    target += gridDim.x;
     if (threadIdx.x == 0) {
+      Team& t = sh->team[which];
+      t.target += t.ctas;
       if (slot && sh->count) {
         atomicAdd(&slot->count, sh->count);
         atomicAdd(&slot->degsum, sh->degsum);
@@ -146,12 +156,12 @@ struct Grid {
         sh->degsum = 0;
       }
       int ok = 1;
-      if (gridDim.x > 1) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->bar) : "memory");
+      if (t.ctas > 1) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.bar) : "memory");
         unsigned spins = 0;
-        while ((int)(ld_acquire(&ctl->bar) - target) < 0) {
+        while ((int)(ld_acquire(t.bar) - t.target) < 0) {
           if (++spins > kSpinLimit) {
-            atomicExch(&ctl->fail, 1u);
+            atomicExch(t.fail, 1u);
             ok = 0;
             break;
           }
@@ -276,13 +286,14 @@ struct Appender {
 };
 
 // fn(lane has an edge, source, neighbour) over every edge of a frontier, all
-// lanes of a warp together, four edges per lane in flight.
+// lanes of a warp together, four edges per lane in flight.  The caller is CTA
+// `cta` of the `ctas` that share the frontier.
 template <class Fn>
 __device__ __forceinline__ void expand(const DevGraph& g, const Queues& q, uint32_t sbase, uint32_t ns, uint32_t lbase,
-                                       uint32_t nl, Fn&& fn) {
+                                       uint32_t nl, uint32_t cta, uint32_t ctas, Fn&& fn) {
   const int lane = threadIdx.x & 31;
-  const uint32_t warp = (uint32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);  // neighbours on other SMs
-  const uint32_t nwarps = gridDim.x * kFWarps;
+  const uint32_t warp = (threadIdx.x >> 5) * ctas + cta;  // neighbours on other SMs
+  const uint32_t nwarps = ctas * kFWarps;
   for (uint32_t i = warp; i < nl; i += nwarps) {
     const uint4 it = q.large[lbase + i];
     uint32_t d[4];
@@ -315,10 +326,10 @@ __device__ __forceinline__ void expand(const DevGraph& g, const Queues& q, uint3
 }
 
 __device__ __forceinline__ void begin(Grid& grid, Shared* sh, Ctl* ctl) {
-  grid.ctl = ctl;
   grid.sh = sh;
-  grid.target = 0;
+  grid.which = 0;
   if (threadIdx.x == 0) {
+    sh->team[0] = Team{&ctl->bar, &ctl->fail, 0, gridDim.x};
     sh->count = 0;
     sh->degsum = 0;
     sh->ok = 1;
@@ -506,7 +517,7 @@ __global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
         queued = true;
       }
       const Queues nq = A.q[cq ^ 1];
-      expand(A.out, A.q[cq], 0, c.ns, 0, c.nl, [&](const bool (&in)[4], uint32_t s, const uint32_t (&d)[4]) {
+      expand(A.out, A.q[cq], 0, c.ns, 0, c.nl, blockIdx.x, gridDim.x, [&](const bool (&in)[4], uint32_t s, const uint32_t (&d)[4]) {
         bool won[4];
         uint32_t b[4] = {}, e[4] = {};
 #pragma unroll
@@ -683,7 +694,7 @@ __device__ bool bc_pull_level(const BcArgs& A, int32_t level, Slot* ns, uint32_t
 // large steps of pushes examine 2.5e8 edges, the cheaper directions 1.2e8).  The
 // CTAs of one blockIdx.y are a group with arrays and a barrier of its own;
 // independent sources are dealt out to the groups, whose waits and loads overlap.
-__device__ bool bc_source(const BcArgs& A, int s, Grid& grid, Appender<true>& ap, Shared& sh) {
+__device__ bool bc_forward(const BcArgs& A, int s, Grid& grid, Appender<true>& ap, Shared& sh) {
   const uint32_t n = A.g.n;
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
   const int lane = threadIdx.x & 31;
@@ -691,7 +702,7 @@ __device__ bool bc_source(const BcArgs& A, int s, Grid& grid, Appender<true>& ap
   for (uint32_t i = tid; i < n; i += nthreads) {
     A.lvl[i] = i == src ? 0 : -1;
     A.sigma[i] = i == src ? 1.0 : 0.0;
-    if (A.first_source) A.deps[i] = 0.0;
+    if (A.first_source && (A.rows || s == 0)) A.deps[i] = 0.0;
   }
   for (uint32_t w = tid; w < (n + 31) / 32; w += nthreads) A.vis[w] = w == src >> 5 ? 1u << (src & 31) : 0u;
   if ((tid >> 5) == 0) {
@@ -727,7 +738,7 @@ __device__ bool bc_source(const BcArgs& A, int s, Grid& grid, Appender<true>& ap
       // nearly every edge would make one), then one pass over the vertices finds
       // the ones that now have paths
       edges += c.degsum;
-      expand(A.g, A.q, sbase, c.ns, lbase, c.nl, [&](const bool (&in)[4], uint32_t u, const uint32_t (&d)[4]) {
+      expand(A.g, A.q, sbase, c.ns, lbase, c.nl, blockIdx.x, gridDim.x, [&](const bool (&in)[4], uint32_t u, const uint32_t (&d)[4]) {
         bool open[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) open[k] = in[k] && !bit_test(A.vis, d[k]);
@@ -753,7 +764,7 @@ __device__ bool bc_source(const BcArgs& A, int s, Grid& grid, Appender<true>& ap
       }
     } else {
       edges += c.degsum;
-      expand(A.g, A.q, sbase, c.ns, lbase, c.nl, [&](const bool (&in)[4], uint32_t u, const uint32_t (&d)[4]) {
+      expand(A.g, A.q, sbase, c.ns, lbase, c.nl, blockIdx.x, gridDim.x, [&](const bool (&in)[4], uint32_t u, const uint32_t (&d)[4]) {
         int32_t l[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) l[k] = in[k] ? A.lvl[d[k]] : -2;
@@ -782,11 +793,21 @@ __device__ bool bc_source(const BcArgs& A, int s, Grid& grid, Appender<true>& ap
     lbase = ln;
     if (!grid.sync(ns)) return false;
   }
-  // first_* and level_deg are written by thread 0 above: every CTA waits once
-  // before it reads them
-  if (!grid.sync()) return false;
-  const uint32_t gwarp = (uint32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
-  const uint32_t nwarps = gridDim.x * kFWarps;
+  if (tid == 0) {  // (first_* and level_deg too: a barrier follows before anyone reads them)
+    A.ctl->levels = level;
+    A.ctl->edges = edges;
+  }
+  return true;
+}
+
+// The backward phase of source s, whose levels the group `A` holds, by `ctas` CTAs.
+__device__ bool bc_backward(const BcArgs& A, int s, bool last, Grid& grid, uint32_t cta, uint32_t ctas) {
+  const uint32_t n = A.g.n;
+  const int lane = threadIdx.x & 31;
+  const uint32_t tid = cta * kFT + threadIdx.x, nthreads = ctas * kFT;
+  const uint32_t gwarp = (threadIdx.x >> 5) * ctas + cta, nwarps = ctas * kFWarps;
+  const int32_t level = __ldcg(&A.ctl->levels);
+  unsigned long long edges = __ldcg(&A.ctl->edges);
   for (int32_t r = level - 1; r >= 0; r--) {
     const uint32_t s0 = A.first_small[r], s1 = A.first_small[r + 1];
     const uint32_t l0 = A.first_large[r], l1 = A.first_large[r + 1];
@@ -796,7 +817,7 @@ __device__ bool bc_source(const BcArgs& A, int s, Grid& grid, Appender<true>& ap
     const bool alone = deepest || push;  // this level's edges are not read
     if (!deepest) edges += push ? below : own;
     if (push) {
-      expand(A.g, A.q, s1, A.first_small[r + 2] - s1, l1, A.first_large[r + 2] - l1,
+      expand(A.g, A.q, s1, A.first_small[r + 2] - s1, l1, A.first_large[r + 2] - l1, cta, ctas,
              [&](const bool (&in)[4], uint32_t u, const uint32_t (&d)[4]) {
                int32_t l[4];
 #pragma unroll
@@ -872,7 +893,7 @@ __device__ bool bc_source(const BcArgs& A, int s, Grid& grid, Appender<true>& ap
     if (!grid.sync()) return false;
   }
   // D = (D - 1/sigma) / (1/sigma), as bc_final forms it (unreached: NaN)
-  if (A.deps_out) {
+  if (A.deps_out && last) {
     double* out = A.deps_out + (A.rows ? (size_t)s * n : 0);
     for (uint32_t i = tid; i < n; i += nthreads) {
       const uint32_t v = A.new_ids ? A.new_ids[i] : i;
@@ -895,32 +916,64 @@ __device__ bool bc_source(const BcArgs& A, int s, Grid& grid, Appender<true>& ap
   return true;
 }
 
+// The arrays of group y.  s: its source; a chain's odd sources run on the transposed
+// graph (the reference transposes a directed graph after every source).
+__device__ void bc_group(const BcArgs& P, size_t y, int s, BcArgs* A) {
+  const size_t n = P.g.n;
+  *A = P;
+  if (!P.rows && s % 2 == 1) {
+    A->g = P.gt;
+    A->gt = P.g;
+  }
+  A->lvl += y * n;
+  A->vis += y * ((n + 31) / 32);
+  A->sigma += y * n;
+  if (P.rows) A->deps += y * n;
+  A->q.small += y * P.n_small;
+  A->q.large += y * P.n_large;
+  A->first_small += y * (n + 2);
+  A->first_large += y * (n + 2);
+  A->level_deg += y * (n + 2);
+  A->heavy += y * P.n_heavy;
+  A->ctl += y;
+}
+
+// Group y of CTAs (blockIdx.y) takes every gridDim.y-th source, on its own arrays.
+// Independent sources (rows) never meet.  The sources of a chain add to the
+// dependencies that the ones before left, so only their forward phases run side by
+// side; then all CTAs take the backward phases one after another.
 __global__ void __launch_bounds__(kFT, 1) bc_fused(const __grid_constant__ BcArgs P) {
   __shared__ Shared sh;
   __shared__ Member buf[kFWarps][kBuf];
   __shared__ BcArgs A;  // with the group's own arrays
-  if (threadIdx.x == 0) {
-    const size_t n = P.g.n, y = blockIdx.y;
-    A = P;
-    A.lvl += y * n;
-    A.vis += y * ((n + 31) / 32);
-    A.sigma += y * n;
-    A.deps += y * n;
-    A.q.small += y * P.n_small;
-    A.q.large += y * P.n_large;
-    A.first_small += y * (n + 2);
-    A.first_large += y * (n + 2);
-    A.level_deg += y * (n + 2);
-    A.heavy += y * P.n_heavy;
-    A.ctl += y;
-  }
-  __syncthreads();
   Grid grid;
   Appender<true> ap{buf[threadIdx.x >> 5], &sh, 0};
-  begin(grid, &sh, A.ctl);
-  for (int s = blockIdx.y; s < P.k; s += gridDim.y) {
-    if (!bc_source(A, s, grid, ap, sh)) return;
-    if (s + (int)gridDim.y < P.k && !grid.sync()) return;  // the arrays are free for the next source
+  begin(grid, &sh, P.ctl + blockIdx.y);
+  if (threadIdx.x == 0) sh.team[1] = Team{&P.ctl->bar_all, &P.ctl->fail, 0, gridDim.x * gridDim.y};
+  const int groups = gridDim.y;
+  for (int s0 = 0; s0 < P.k; s0 += groups) {
+    const int s = s0 + (int)blockIdx.y;
+    if (P.rows && s >= P.k) return;
+    if (s < P.k) {
+      __syncthreads();
+      if (threadIdx.x == 0) bc_group(P, blockIdx.y, s, &A);
+      __syncthreads();
+      if (!bc_forward(A, s, grid, ap, sh)) return;
+    }
+    Grid team = grid;
+    team.which = P.rows ? 0 : 1;
+    if (!team.sync()) return;
+    const int first = P.rows ? s : s0, end = P.rows ? s + 1 : min(s0 + groups, P.k);
+    for (int t = first; t < end; t++) {
+      if (!P.rows && groups > 1) {
+        __syncthreads();
+        if (threadIdx.x == 0) bc_group(P, t - s0, t, &A);
+        __syncthreads();
+      }
+      const uint32_t cta = P.rows ? blockIdx.x : blockIdx.y * gridDim.x + blockIdx.x;
+      if (!bc_backward(A, t, P.rows || t == P.k - 1, team, cta, sh.team[team.which].ctas)) return;
+      if (t + (P.rows ? groups : 1) < P.k && !team.sync()) return;  // the arrays are free for the next source
+    }
   }
 }
 
@@ -1135,7 +1188,7 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
       ap.finish(nq, ns, 0, 0);
       if (!grid.sync(ns)) return;
     } else {
-      expand(A.out, A.q[cq], 0, c.ns, 0, c.nl, [&](const bool (&in)[4], uint32_t s, const uint32_t (&d)[4]) {
+      expand(A.out, A.q[cq], 0, c.ns, 0, c.nl, blockIdx.x, gridDim.x, [&](const bool (&in)[4], uint32_t s, const uint32_t (&d)[4]) {
         unsigned long long vd[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) vd[k] = in[k] ? A.vis[d[k]] : ~0ull;
@@ -1550,7 +1603,7 @@ __global__ void __launch_bounds__(kFT, 1) prd_fused(const __grid_constant__ PrdA
         if (j < rs && (lane & 3) == 0) A.ngh[it.x] = s;
       }
     } else {
-      expand(A.out, A.q[cq], 0, c.ns, 0, c.nl, [&](const bool (&in)[4], uint32_t s, const uint32_t (&d)[4]) {
+      expand(A.out, A.q[cq], 0, c.ns, 0, c.nl, blockIdx.x, gridDim.x, [&](const bool (&in)[4], uint32_t s, const uint32_t (&d)[4]) {
         const double x = A.c[s];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -1844,6 +1897,17 @@ rg_status bc_arrays(const rg_graph* g, int groups, BcArgs* A, double** ordered) 
   return X.place();
 }
 
+// Groups for k sources and the CTAs of each.  Every source gets a group while there
+// are SMs for it and the groups' arrays (44 bytes per vertex that a traversal keeps
+// returning to) stay in L2; the SMs are shared out between the groups, up to what
+// one traversal can use.
+void bc_split(const rg_graph* g, int k, int* groups, int* width) {
+  const int64_t in_l2 = std::max<int64_t>(1, kFusedBcRowsL2 / (44 * g->n));
+  const int most = (int)std::min<int64_t>({(int64_t)k, (int64_t)device_sms(), in_l2});
+  *groups = (k + (k + most - 1) / most - 1) / ((k + most - 1) / most);  // as many rounds, evenly filled
+  *width = std::min(fused_grid(g->m + g->n, kFusedEdgesPerCta), std::max(1, device_sms() / *groups));
+}
+
 }  // namespace
 
 rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* h_deps, int64_t* levels_out,
@@ -1855,21 +1919,22 @@ rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* 
   const bool order = g->sorted && (h_deps || d_deps_out);
   double* direct = direct_results(g, h_deps, d_deps_out);
   double* ordered = !order ? nullptr : direct ? direct : d_deps_out;
-  RG_TRY(bc_arrays(g, 1, &A, order && !ordered ? &ordered : nullptr));
+  int groups = 1, width = fused_grid(m + n, kFusedEdgesPerCta);
+  if (m <= std::min(kFusedBcRowsEdges, kFusedBcRowsWork / std::max(nsrc, 1))) bc_split(g, std::min(nsrc, 64), &groups, &width);
+  RG_TRY(bc_arrays(g, groups, &A, order && !ordered ? &ordered : nullptr));
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = cx.ws.h_info;
   info[0] = info[1] = info[3] = 0;
   CallTimer timer(g);
-  A.k = 1;
   A.rows = false;
-  for (int it = 0; it < nsrc; it++) {
-    // the reference transposes a directed graph after every source
-    A.g = it % 2 == 1 ? g->in_view() : g->view();
-    A.gt = it % 2 == 1 ? g->view() : g->in_view();
-    A.source[0] = src_orig[it];
+  A.g = g->view();
+  A.gt = g->in_view();
+  for (int it = 0; it < nsrc; it += 64) {
+    A.k = std::min(nsrc - it, 64);
+    for (int q = 0; q < A.k; q++) A.source[q] = src_orig[it + q];
     A.first_source = it == 0;
-    A.deps_out = it == nsrc - 1 ? ordered : nullptr;
-    RG_TRY(launch_fused(bc_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
+    A.deps_out = it + A.k == nsrc ? ordered : nullptr;
+    RG_TRY(launch_fused(bc_fused, A, dim3(width, groups), 0, 0, st));
   }
   RG_TRY(timer.mark());
   if (!direct) RG_TRY(deliver<double>(g, A.deps, ordered, h_deps, d_deps_out, st));
@@ -1890,13 +1955,8 @@ rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double
   Ctx& cx = ctx();
   cudaStream_t st = cx.stream;
   const int64_t n = g->n, m = g->m;
-  // every source gets a group while there are SMs for it and the groups' arrays
-  // (44 bytes per vertex that a traversal keeps returning to) stay in L2; the SMs
-  // are shared out between the groups, up to what one traversal can use
-  const int64_t in_l2 = std::max<int64_t>(1, kFusedBcRowsL2 / (44 * n));
-  const int most = (int)std::min<int64_t>({(int64_t)k, (int64_t)device_sms(), in_l2});
-  const int groups = (k + (k + most - 1) / most - 1) / ((k + most - 1) / most);  // as many rounds, evenly filled
-  const int width = std::min(fused_grid(m + n, kFusedEdgesPerCta), std::max(1, device_sms() / groups));
+  int groups, width;
+  bc_split(g, k, &groups, &width);
   BcArgs A;
   RG_TRY(bc_arrays(g, groups, &A, nullptr));
   A.g = g->view();
