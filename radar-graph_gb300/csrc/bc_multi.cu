@@ -389,15 +389,16 @@ rg_status bc_multi_run(rg_graph* g, const uint32_t* src_orig, int k, double* h_o
   const int64_t n = g->n;
   if (fused_fits(g, std::min(kFusedBcRowsEdges, kFusedBcRowsWork / k))) {
     DevBuf rows(true, st);
-    if (!d_out) RG_TRY(rows.reserve(8 * (size_t)n * k));
-    double* out = d_out ? d_out : rows.as<double>();
+    double* direct = d_out ? nullptr : static_cast<double*>(device_alias(h_out, 8 * (size_t)n * k, 8));
+    if (!d_out && !direct) RG_TRY(rows.reserve(8 * (size_t)n * k));
+    double* out = d_out ? d_out : direct ? direct : rows.as<double>();
     CallTimer timer(g);
     bool done = false;
     int64_t levels = 0;
     RG_TRY(bc_rows_fused_run(g, src_orig, k, out, &levels, &done));
     if (done) {
       RG_TRY(timer.stop());
-      if (h_out) RG_CUDA(cudaMemcpyAsync(h_out, out, 8 * (size_t)n * k, cudaMemcpyDeviceToHost, st));
+      if (h_out && !direct) RG_CUDA(cudaMemcpyAsync(h_out, out, 8 * (size_t)n * k, cudaMemcpyDeviceToHost, st));
       RG_CUDA(cudaStreamSynchronize(st));
       g_timing.algorithmic_bytes = 4 * g_timing.edges_traversed + (int64_t)k * 16 * n + 24 * n;
       if (levels_out) *levels_out = levels - 1;
