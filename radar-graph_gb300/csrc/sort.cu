@@ -84,8 +84,8 @@ struct Tile {
   uint32_t tile;
 };
 
-// kFull: the tile has kTile keys.
-template <bool kFull>
+// kFull: the tile has kTile keys.  kBits: the most that a digit has.
+template <int kBits, bool kFull>
 __device__ __forceinline__ void sort_tile(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, int64_t k,
                                           int here, int shift, uint32_t digits, uint32_t pass,
                                           const uint32_t* __restrict__ base, uint64_t* status, uint32_t* head, Tile& T,
@@ -103,10 +103,10 @@ __device__ __forceinline__ void sort_tile(const uint64_t* __restrict__ in, uint6
     const uint32_t d = kFull || j0 + i * 32 < here ? digit_of(key[i], shift, digits) : 256u;
     unsigned peers;
     if (kFull && (i % kMatchOf)) {
-      // equal digits by eight votes ...
+      // equal digits by a vote per bit ...
       peers = kAll;
 #pragma unroll
-      for (int b = 0; b < 8; b++) {
+      for (int b = 0; b < kBits; b++) {
         const int bit = ((int)(d << (31 - b))) >> 31;
         peers &= ~(__ballot_sync(kAll, bit) ^ (unsigned)bit);
       }
@@ -201,6 +201,7 @@ __device__ __forceinline__ void sort_tile(const uint64_t* __restrict__ in, uint6
   }
 }
 
+template <int kBits>
 __global__ void __launch_bounds__(kThreads, 3) sort_sweep(const uint64_t* __restrict__ in, uint64_t* __restrict__ out,
                                                           int64_t k, int shift, uint32_t digits, uint32_t pass,
                                                           const uint32_t* __restrict__ base, uint64_t* status,
@@ -213,8 +214,8 @@ __global__ void __launch_bounds__(kThreads, 3) sort_sweep(const uint64_t* __rest
   __syncthreads();
   const int64_t t0 = (int64_t)T.tile * kTile;
   const int here = (int)min((int64_t)kTile, k - t0);
-  if (here == kTile) sort_tile<true>(in + t0, out, k, here, shift, digits, pass, base, status, head, T, keys);
-  else sort_tile<false>(in + t0, out, k, here, shift, digits, pass, base, status, head, T, keys);
+  if (here == kTile) sort_tile<kBits, true>(in + t0, out, k, here, shift, digits, pass, base, status, head, T, keys);
+  else sort_tile<kBits, false>(in + t0, out, k, here, shift, digits, pass, base, status, head, T, keys);
 }
 
 }  // namespace
@@ -235,23 +236,36 @@ rg_status sort_count(SortScratch& s, const uint64_t* keys, int64_t k, int lo, in
   return RG_OK;
 }
 
-rg_status sort_run(SortScratch& s, uint64_t** keys, uint64_t** other, int64_t k, int lo, int hi, cudaStream_t st) {
+namespace {
+
+template <int kBits>
+rg_status sort_passes_of(SortScratch& s, uint64_t** keys, uint64_t** other, int64_t k, int lo, int hi,
+                         cudaStream_t st) {
   static std::atomic<uint64_t> limit_set{0};
-  RG_TRY(allow_max_dyn_smem(limit_set, sort_sweep));
-  const int passes = sort_passes(lo, hi);
+  RG_TRY(allow_max_dyn_smem(limit_set, sort_sweep<kBits>));
+  const int passes = sort_passes(lo, hi), width = sort_width(lo, hi);
   const int64_t tiles = (k + kTile - 1) / kTile;
-  if (tiles == 0) return RG_OK;
-  sort_bases<<<passes, 256, 0, st>>>(sort_counts(s));
   for (int p = 0; p < passes; p++) {
-    const int shift = lo + 8 * p;
-    const uint32_t digits = (1u << std::min(8, hi - shift)) - 1u;
-    sort_sweep<<<(unsigned)tiles, kThreads, kTile * sizeof(uint64_t), st>>>(
+    const int shift = lo + width * p;
+    const uint32_t digits = (1u << std::min(width, hi - shift)) - 1u;
+    sort_sweep<kBits><<<(unsigned)tiles, kThreads, kTile * sizeof(uint64_t), st>>>(
         *keys, *other, k, shift, digits, (uint32_t)p, sort_counts(s) + 256 * p, s.status.as<uint64_t>(),
         s.hist.as<uint32_t>());
     std::swap(*keys, *other);
   }
   RG_CUDA(cudaGetLastError());
   return RG_OK;
+}
+
+}  // namespace
+
+rg_status sort_run(SortScratch& s, uint64_t** keys, uint64_t** other, int64_t k, int lo, int hi, cudaStream_t st) {
+  if (k == 0) return RG_OK;
+  sort_bases<<<sort_passes(lo, hi), 256, 0, st>>>(sort_counts(s));
+  const int width = sort_width(lo, hi);
+  auto run = width > 7 ? sort_passes_of<8> : width > 6 ? sort_passes_of<7> : width > 5 ? sort_passes_of<6>
+                                                                                        : sort_passes_of<5>;
+  return run(s, keys, other, k, lo, hi, st);
 }
 
 uint32_t* sort_counts(SortScratch& s) { return s.hist.as<uint32_t>() + kHead; }

@@ -9,8 +9,14 @@ namespace rg {
 
 constexpr int kMaxSortPasses = 8;
 
-// The passes a sort on bits [lo, hi) takes, 8 bits each.
-inline int sort_passes(int lo, int hi) { return (hi - lo + 7) / 8; }
+// The passes a sort on bits [lo, hi) takes, of up to 8 bits each, and the bits of
+// each: evenly many, as a pass ranks its keys bit by bit (42 bits as 8 8 8 8 8 2 took
+// 2.17 ms for 67e6 keys, as six times 7 2.07).
+__host__ __device__ inline int sort_passes(int lo, int hi) { return (hi - lo + 7) / 8; }
+__host__ __device__ inline int sort_width(int lo, int hi) {
+  const int passes = sort_passes(lo, hi);
+  return passes > 0 ? (hi - lo + passes - 1) / passes : 0;
+}
 
 // Scratch of one sort, kept by the caller until its stream has passed the sort.
 struct SortScratch {
@@ -44,7 +50,9 @@ __device__ __forceinline__ void sort_zero(uint32_t* sh, int passes) {
 }
 __device__ __forceinline__ void sort_count_key(uint32_t* sh, uint64_t key, int lo, int hi, int passes) {
   const uint64_t x = hi >= 64 ? key : key & ((1ull << hi) - 1);
-  for (int p = 0; p < passes; p++) atomicAdd(sh + p * 256 + ((x >> (lo + 8 * p)) & 255u), 1u);
+  const int width = sort_width(lo, hi);
+  const uint32_t digits = (1u << width) - 1u;
+  for (int p = 0; p < passes; p++) atomicAdd(sh + p * 256 + ((uint32_t)(x >> (lo + width * p)) & digits), 1u);
 }
 __device__ __forceinline__ void sort_flush(const uint32_t* sh, uint32_t* hist, int passes) {
   __syncthreads();
