@@ -49,6 +49,20 @@ def test_builders(n, edges, pinned):
         assert np.array_equal(o, np.searchsorted(key // n, np.arange(n + 1))) and np.array_equal(a, key % n)
 
 
+@pytest.mark.parametrize("n,edges", [(1, 12 << 20), (300, 12 << 20), (1 << 16, (12 << 20) + 1), ((1 << 20) + 1, 13000000)])
+def test_builder_halves(n, edges):
+    """Enough edges to be sorted once each: none kept, nearly all dropped, ragged."""
+    r = np.random.default_rng(n)
+    src = r.integers(0, n, edges).astype(np.uint32)
+    dst = np.minimum(r.integers(0, n, edges), r.integers(0, n, edges)).astype(np.uint32)
+    lo, hi = np.minimum(src, dst).astype(np.int64), np.maximum(src, dst).astype(np.int64)
+    half = np.unique((lo * n + hi)[lo != hi])
+    key = np.sort(np.concatenate([half, half % n * n + half // n]))
+    with rg.Graph.from_edges(n, src, dst) as g:
+        o, a, _ = g.download()
+    assert np.array_equal(o, np.searchsorted(key // n, np.arange(n + 1))) and np.array_equal(a, key % n)
+
+
 def test_endpoint_out_of_range():
     for bad in ([0, 5], [5, 0]):
         with pytest.raises(rg.RgError, match="edge endpoint 5 >= n"):
