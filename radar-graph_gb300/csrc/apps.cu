@@ -580,7 +580,7 @@ rg_status radii_run(rg_graph* g, int variant, const uint32_t* seeds_orig, int k,
   OptScope opt_scope(g, kAppRadii);
   Ctx* cx = nullptr;
   RG_TRY(get_ctx(&cx));
-  if (fused_fits(g, kFusedRadiiEdges)) {
+  if (fused_fits(g, g->sorted ? kFusedRadiiSortedEdges : kFusedRadiiEdges)) {
     // each seed once, the largest bit on a repeat (as the seeding loop below)
     uint32_t v[64];
     unsigned long long mk[64];

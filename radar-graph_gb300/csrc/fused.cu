@@ -992,7 +992,7 @@ struct RadiiArgs {
   unsigned long long *vis, *nvis;
   int32_t* radii;
   int32_t* radii_out;  // original-id order; null: not wanted (or not sorted)
-  uint32_t* bits;
+  uint32_t* bits[2];  // what a pull reached
   Queues q[2];
   // multi-source BFS: bit q of plane p of v is bit p of v's depth from source q
   unsigned long long* planes;
@@ -1008,10 +1008,10 @@ constexpr int kPlanes = 6;  // depths up to 63; deeper searches run level by lev
 
 // The vertex's new mask becomes current.
 template <bool kDepths>
-__device__ __forceinline__ void radii_advance(const RadiiArgs& A, uint32_t v, int32_t round) {
-  const unsigned long long now = A.nvis[v];
+__device__ __forceinline__ void radii_advance(const RadiiArgs& A, uint32_t v, int32_t round, unsigned long long now,
+                                              unsigned long long old) {
   if (kDepths) {
-    const unsigned long long w = now & ~A.vis[v];
+    const unsigned long long w = now & ~old;
 #pragma unroll
     for (int p = 0; p < kPlanes; p++) {
       if ((round >> p) & 1) A.planes[(size_t)p * A.out.n + v] |= w;
@@ -1050,18 +1050,18 @@ __device__ __forceinline__ void write_depths(const RadiiArgs& A) {
   }
 }
 
-__device__ __forceinline__ void radii_flush(const RadiiArgs& A, uint32_t row, unsigned long long part) {
+__device__ __forceinline__ void radii_flush(const RadiiArgs& A, uint32_t* bits, uint32_t row, unsigned long long part) {
   const unsigned long long w = part & ~A.vis[row];
   if (!w) return;
   atomicOr(A.nvis + row, w);
-  bit_set(A.bits, row);
+  bit_set(bits, row);
 }
 
 // Rounds push over the queue or, dense ones, pull every row's neighbour masks
 // (4 edges per lane, one segmented OR scan per 128 edges, as mask_pull_sweep
 // with shorter steps: a small graph has more warps than 512-edge chunks).  A
-// vertex pass after either makes the new masks current and queues the vertices
-// that grew.  kDepths: the same propagation, one bit per source, is a
+// vertex pass after either makes the new masks current.  What a pull reached is
+// queued only before a push.  kDepths: the same propagation, one bit per source, is a
 // multi-source BFS (BFS.C); the bits that arrive in a round have that depth.
 template <bool kDepths>
 __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ RadiiArgs A) {
@@ -1074,12 +1074,13 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
   const int lane = threadIdx.x & 31;
   const uint32_t warp = tid >> 5, nwarps = nthreads >> 5;
+  const uint32_t take = min((nwords + nwarps - 1) / nwarps, kPullWords);
   for (uint32_t i = tid; i < n; i += nthreads) {
     A.vis[i] = 0ull;
     A.nvis[i] = 0ull;
     A.radii[i] = -1;
   }
-  for (uint32_t w = tid; w < nwords; w += nthreads) A.bits[w] = 0u;
+  for (uint32_t w = tid; w < nwords; w += nthreads) A.bits[0][w] = A.bits[1][w] = 0u;
   unsigned long long full = 0ull;  // the bits that can spread: seeds with out-edges
   for (int j = lane; j < A.k; j += 32) {
     const uint32_t v = A.new_ids ? A.new_ids[A.seed[j]] : A.seed[j];
@@ -1102,12 +1103,15 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
     ap.finish(A.q[0], &A.ctl->lv[0], 0, 0);
   }
   if (!grid.sync(&A.ctl->lv[0])) return;
-  int cq = 0;
+  int cq = 0;  // the queue pair that holds the frontier
+  int cb = 0;  // the bitmap that holds it after a pull; a bitmap that does not is clear
+  bool queued = true;
   int32_t round = 0;
   unsigned long long edges = 0;
   for (;;) {
+    Slot* cs = &A.ctl->lv[round % 3];
     Slot* ns = &A.ctl->lv[(round + 1) % 3];
-    const Slot c = sh.slot;
+    Slot c = sh.slot;
     if (c.count == 0) break;
     edges += c.degsum;
     if (tid == 0) A.ctl->lv[(round + 2) % 3] = Slot{};
@@ -1121,12 +1125,13 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
     }
     const Queues nq = A.q[cq ^ 1];
     if ((int64_t)(c.count + c.degsum) > A.threshold && A.in.m > 0) {
+      uint32_t *bits = A.bits[cb ^ 1], *old_bits = A.bits[cb];
       const uint32_t steps = (A.in.m + 127) / 128;
       const uint32_t gwarp = (uint32_t)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
       const bool wide = A.nchunks >= kWideChunks * nwarps;
       if (wide) {
         for (uint32_t c = gwarp; c < A.nchunks; c += nwarps) {
-          mask_pull_chunk<16, false>(A.in, c, A.chunk_v[c], A.chunk_v[c + 1], A.vis, A.nvis, A.bits, full);
+          mask_pull_chunk<16, false>(A.in, c, A.chunk_v[c], A.chunk_v[c + 1], A.vis, A.nvis, bits, full);
         }
       }
       for (uint32_t t = gwarp; t < steps && !wide; t += nwarps) {
@@ -1156,7 +1161,7 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
 #pragma unroll
           for (int k = 0; k < 4; k++) {
             if (rows[k] != row) {
-              radii_flush(A, row, part);
+              radii_flush(A, bits, row, part);
               part = 0ull;
               row = rows[k];
             }
@@ -1170,24 +1175,78 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
           if (lane >= o && tr == row) part |= p;
         }
         const uint32_t next_row = __shfl_down_sync(kAll, row, 1);
-        if (row != kNone && (lane == 31 || next_row != row)) radii_flush(A, row, part);
+        if (row != kNone && (lane == 31 || next_row != row)) radii_flush(A, bits, row, part);
       }
       if (!grid.sync()) return;
-      for (uint32_t w = warp; w < nwords; w += nwarps) {
-        const uint32_t x = A.bits[w];
-        if (!x) continue;
-        const uint32_t v = min(w * 32 + lane, n - 1);
-        const bool in = (x >> lane) & 1u;
-        if (in) {
-          A.radii[v] = round;
-          radii_advance<kDepths>(A, v, round);
+      // the members' masks become current, two words of them at a time (a chain of
+      // latencies); they are queued only if the next round pushes
+      unsigned count = 0;
+      unsigned long long degsum = 0;
+      for (uint32_t w0 = warp; w0 < nwords; w0 += nwarps * take) {
+        const uint32_t mw = w0 + lane * nwarps;
+        const bool mine = lane < (int)take && mw < nwords;
+        const uint32_t word = mine ? bits[mw] : 0u;
+        if (mine && !queued) old_bits[mw] = 0u;
+        unsigned todo = __ballot_sync(kAll, word != 0u);
+        while (todo) {
+          int j[2];
+          j[0] = __ffs(todo) - 1;
+          todo &= todo - 1;
+          j[1] = todo ? __ffs(todo) - 1 : j[0];
+          const bool two = todo != 0;
+          todo &= todo - 1;
+          uint32_t v[2];
+          bool in[2];
+          unsigned long long now[2], old[2];
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            const uint32_t x = __shfl_sync(kAll, word, j[i]);
+            v[i] = (w0 + j[i] * nwarps) * 32 + lane;
+            in[i] = (i == 0 || two) && ((x >> lane) & 1u);
+            now[i] = in[i] ? A.nvis[v[i]] : 0ull;
+            old[i] = kDepths && in[i] ? A.vis[v[i]] : 0ull;
+            if (in[i]) degsum += A.out.off[v[i] + 1] - A.out.off[v[i]];
+            count += in[i];
+          }
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            if (!in[i]) continue;
+            A.radii[v[i]] = round;
+            radii_advance<kDepths>(A, v[i], round, now[i], old[i]);
+          }
         }
-        if (lane == 0) A.bits[w] = 0u;
-        ap.add(in, v, A.out.off[v], A.out.off[v + 1], nq, ns, 0, 0);
       }
-      ap.finish(nq, ns, 0, 0);
+      count = __reduce_add_sync(kAll, count);
+      if (count) {
+        degsum = warp_sum(degsum);
+        if (lane == 0) {
+          atomicAdd(&sh.count, count);
+          atomicAdd(&sh.degsum, degsum);
+        }
+      }
+      cb ^= 1;
+      queued = false;
       if (!grid.sync(ns)) return;
     } else {
+      if (!queued) {  // after a pull
+        uint32_t* bits = A.bits[cb];
+        for (uint32_t w0 = warp; w0 < nwords; w0 += nwarps * take) {
+          const uint32_t mw = w0 + lane * nwarps;
+          const bool mine = lane < (int)take && mw < nwords;
+          const uint32_t word = mine ? bits[mw] : 0u;
+          if (word) bits[mw] = 0u;
+          for (unsigned todo = __ballot_sync(kAll, word != 0u); todo; todo &= todo - 1) {
+            const int j = __ffs(todo) - 1;
+            const uint32_t x = __shfl_sync(kAll, word, j);
+            const uint32_t v = min((w0 + j * nwarps) * 32 + lane, n - 1);
+            ap.add((x >> lane) & 1u, v, A.out.off[v], A.out.off[v + 1], A.q[cq], cs, 0, 0);
+          }
+        }
+        ap.finish(A.q[cq], cs, 0, 0);
+        if (!grid.sync()) return;  // (its members were counted by the pull)
+        c = read_slot(cs);
+        queued = true;
+      }
       expand(A.out, A.q[cq], 0, c.ns, 0, c.nl, blockIdx.x, gridDim.x, [&](const bool (&in)[4], uint32_t s, const uint32_t (&d)[4]) {
         unsigned long long vd[4];
 #pragma unroll
@@ -1219,11 +1278,12 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
       if (!grid.sync(ns)) return;
       const Slot nx = sh.slot;
       for (uint32_t i = tid; i < nx.ns; i += nthreads) {
-        radii_advance<kDepths>(A, nq.small[i].x, round);
+        const uint32_t v = nq.small[i].x;
+        radii_advance<kDepths>(A, v, round, A.nvis[v], A.vis[v]);
       }
       for (uint32_t i = tid; i < nx.nl; i += nthreads) {
         const uint4 it = nq.large[i];
-        if (it.w & 1u) radii_advance<kDepths>(A, it.x, round);
+        if (it.w & 1u) radii_advance<kDepths>(A, it.x, round, A.nvis[it.x], A.vis[it.x]);
       }
       if (!grid.sync()) return;
     }
@@ -1993,7 +2053,8 @@ rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned lo
   A->planes = nullptr;
   Arrays X;
   X.add(&A->ctl, 1);
-  X.add(&A->bits, (n + 31) / 32);
+  X.add(&A->bits[0], (n + 31) / 32);
+  X.add(&A->bits[1], (n + 31) / 32);
   X.add(&A->vis, n);
   X.add(&A->nvis, n);
   X.add(&A->radii, n);
@@ -2012,7 +2073,10 @@ rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned lo
     A->seed[i] = seeds[i];
     A->mask[i] = masks[i];
   }
-  A->threshold = dense_threshold(g);
+  // a push reads the frontier's edges alone, a pull all of them: where a level is
+  // more than latencies, up to twice the share of edges is still pushed (64 sources,
+  // R-MAT 2^20 561 -> 486 us, uniform 816 -> 761; uniform 2^10 would lose 8 of 52)
+  A->threshold = dense_threshold(g) * (g->m >= 1 << 22 ? 2 : 1);
   A->depths = nullptr;
   A->sources = 0;
   A->info = ctx().ws.h_info_dev;

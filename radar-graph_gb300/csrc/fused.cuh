@@ -27,11 +27,15 @@ constexpr int64_t kFusedPrRows = 12000;
 //             2^24 560 / 973 (1823 / 2972): every size
 //   BC        2^10 58 / 246 (75 / 240), 2^18 130 / 506 (153 / 496), 2^22
 //             601 / 1573 (1007 / 1975), 2^24 3519 / 5520 (8066 / 9983): every size
-//   Radii     2^10 71 / 309, 2^18 270 / 583 (324 / 515), 2^20 619 / 779
-//             (912 / 948), 2^21 801 / 954 (1435 / 1245), 2^22 2044 / 1892: 4e7 edges
-//   multi-source BFS  64 sources: 2^10 74 / 295, 2^18 249 / 615 (363 / 628), 2^21
-//             1244 / 1773 (1825 / 2625); 2 sources: 2^20 417 / 579 (702 / 749), 2^21
-//             609 / 712 (1080 / 990): 6.7e7 edges
+//   Radii     2^10 73 / 309, 2^18 246 / 583 (300 / 515), 2^20 491 / 789 (765 /
+//             963), 2^20.5 631 / 913 (997 / 1012), 2^21 749 / 988 (1293 / 1249), 2^22
+//             1658 / 1866 (2623 / 2355), 2^22.5 2609 / 2739, 2^23 2970 / 2758: sorted
+//             1.7e8 edges, others 5e7 (their pulls want more warps than one CTA per
+//             SM holds)
+//   multi-source BFS  64 sources: 2^10 74 / 295, 2^18 226 / 615 (330 / 628), 2^21
+//             943 / 1760 (1535 / 2633), 2^22 1800 / 2992 (3076 / 4666); 2 sources:
+//             2^20 331 / 584 (539 / 746), 2^21 481 / 726 (918 / 988), 2^22 1050 / 1364
+//             (1768 / 1736): 1.3e8 edges
 //   PageRank  20 iterations, against pulls: 2^10 97 / 217, 2^14 154 / 247 (93 /
 //             160), 2^16 308 / 308 (183 / 245), 2^17 565 / 473 (297 / 365): 3e6
 //             edges; against pushes: 2^16 309 / 730, 2^18 1331 / 1559, 2^19 2737 /
@@ -41,7 +45,7 @@ constexpr int64_t kFusedPrRows = 12000;
 //             774 / 815 (605 / 598), 2^20 1441 / 1164 (1146 / 872): 1.7e7 edges
 constexpr int64_t kFusedBfsEdges = INT64_MAX;
 constexpr int64_t kFusedBcEdges = INT64_MAX;
-constexpr int64_t kFusedRadiiEdges = 5 << 23;
+constexpr int64_t kFusedRadiiEdges = 6 << 23, kFusedRadiiSortedEdges = 5 << 25;
 constexpr int64_t kFusedPagerankEdges = 3 << 20;
 constexpr int64_t kFusedPagerankPushEdges = 8 << 20;
 constexpr int64_t kFusedPrdEdges = 1 << 25;
@@ -56,7 +60,7 @@ constexpr int64_t kFusedBcRowsWork = 256 << 20;  // edges times sources
 // Groups' arrays at once: 64 sources on 2^17 vertices 2079 us with all of them
 // (370 MB), 2016 in 80 MB; 16 sources on 2^18 808 us with all (184 MB), 1008 in 80 MB.
 constexpr int64_t kFusedBcRowsL2 = 192 << 20;
-constexpr int64_t kFusedMsEdges = 1 << 26;
+constexpr int64_t kFusedMsEdges = 1 << 27;
 
 // Whether a call on g may take the one-launch path: small enough, and no
 // per-level records (rg_set_trace) are asked for.
