@@ -233,9 +233,9 @@ __host__ __device__ __forceinline__ double deg_quotient(double a, uint32_t d, un
 
 // The same quotient for a of either sign; values so small that it would be
 // subnormal (which no PageRankDelta run reaches) divide in FP64.
-__device__ __forceinline__ double deg_quotient_signed(double a, uint32_t d, unsigned long long R) {
+__host__ __device__ __forceinline__ double deg_quotient_signed(double a, uint32_t d, unsigned long long R) {
   const unsigned long long s = bits_of(a) & (1ull << 63), b = bits_of(a) ^ s;
-  if (b < (123ull << 52)) return d ? __ddiv_rn(a, (double)d) : 0.0;  // below 2^-900
+  if (b < (123ull << 52)) return d ? a / (double)d : 0.0;  // below 2^-900
   return double_of(bits_of(deg_quotient(double_of(b), d, R)) | s);
 }
 

@@ -196,7 +196,9 @@ size_t working_bytes(const rg_graph* g, int kind, int k) {
   }
   // one BFS: two queues of vertices and of 128-edge pieces (16 bytes each) beside the depths
   if (k == 1) return 88 * n + (size_t)g->m / 4;
-  return (size_t)(8 * k + 40) * n;  // masks, depth rows and their original-order copy, two frontiers
+  // masks, depth rows and their original-order copy, two frontiers; or, in one launch,
+  // masks, depth planes, two queues and the rows
+  return std::max((size_t)(8 * k + 40) * n, (size_t)(4 * k + 140) * n + (size_t)g->m / 4);
 }
 
 void worker_main(rg_server* S) {
