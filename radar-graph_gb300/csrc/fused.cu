@@ -21,6 +21,7 @@
 // the host sees that the run did not finish and answers level by level.
 
 #include <cuda_runtime.h>
+#include <math_constants.h>
 #include <string.h>
 
 #include <algorithm>
@@ -571,7 +572,9 @@ struct BcArgs {
   bool rows;  // k independent sources, source s to row s of deps_out; else one source, whose dependencies add to deps
   int32_t* lvl;
   uint32_t* vis;  // the vertices reached, as bits: what a large push tests
-  double *sigma, *deps;
+  double *sigma, *even, *odd;  // path counts; dependencies of even and of odd levels
+  double* inv;                 // 1/sigma of the vertices reached
+  double* deps;                // a chain's dependencies so far
   double* deps_out;  // original-id order; null: deps keeps the result
   Queues q;          // every level's frontier, one after another
   uint32_t *first_small, *first_large;  // per level, levels + 1 entries
@@ -702,7 +705,7 @@ __device__ bool bc_forward(const BcArgs& A, int s, Grid& grid, Appender<true>& a
   for (uint32_t i = tid; i < n; i += nthreads) {
     A.lvl[i] = i == src ? 0 : -1;
     A.sigma[i] = i == src ? 1.0 : 0.0;
-    if (A.first_source && (A.rows || s == 0)) A.deps[i] = 0.0;
+    A.even[i] = A.odd[i] = 0.0;
   }
   for (uint32_t w = tid; w < (n + 31) / 32; w += nthreads) A.vis[w] = w == src >> 5 ? 1u << (src & 31) : 0u;
   if ((tid >> 5) == 0) {
@@ -801,6 +804,10 @@ __device__ bool bc_forward(const BcArgs& A, int s, Grid& grid, Appender<true>& a
 }
 
 // The backward phase of source s, whose levels the group `A` holds, by `ctas` CTAs.
+// The dependencies of even and of odd levels are kept apart: a vertex of level r finds
+// its successors' among all its neighbours' in the other array (level r - 1 is still
+// zero there), one gather per edge in place of a level and a value (8e6 vertices,
+// 2^27 edges: 1460 -> 1380 us a call).
 __device__ bool bc_backward(const BcArgs& A, int s, bool last, Grid& grid, uint32_t cta, uint32_t ctas) {
   const uint32_t n = A.g.n;
   const int lane = threadIdx.x & 31;
@@ -808,9 +815,13 @@ __device__ bool bc_backward(const BcArgs& A, int s, bool last, Grid& grid, uint3
   const uint32_t gwarp = (threadIdx.x >> 5) * ctas + cta, nwarps = ctas * kFWarps;
   const int32_t level = __ldcg(&A.ctl->levels);
   unsigned long long edges = __ldcg(&A.ctl->edges);
+  // what the sources before left: it counts among a vertex's own
+  const double* left = A.rows || (A.first_source && s == 0) ? nullptr : A.deps;
   for (int32_t r = level - 1; r >= 0; r--) {
     const uint32_t s0 = A.first_small[r], s1 = A.first_small[r + 1];
     const uint32_t l0 = A.first_large[r], l1 = A.first_large[r + 1];
+    double* dep = r & 1 ? A.odd : A.even;
+    const double* next = r & 1 ? A.even : A.odd;
     const bool deepest = r == level - 1;  // its vertices have no successors: 1/sigma alone
     const unsigned long long own = A.level_deg[r], below = deepest ? 0 : A.level_deg[r + 1];
     const bool push = A.same && !deepest && 4 * below < own;
@@ -822,10 +833,10 @@ __device__ bool bc_backward(const BcArgs& A, int s, bool last, Grid& grid, uint3
                int32_t l[4];
 #pragma unroll
                for (int k = 0; k < 4; k++) l[k] = in[k] ? A.lvl[d[k]] : -2;
-               const double x = A.deps[u];
+               const double x = next[u];
 #pragma unroll
                for (int k = 0; k < 4; k++) {
-                 if (l[k] == r) atomicAdd(A.deps + d[k], x);
+                 if (l[k] == r) atomicAdd(dep + d[k], x);
                }
              });
     }
@@ -835,15 +846,28 @@ __device__ bool bc_backward(const BcArgs& A, int s, bool last, Grid& grid, uint3
     const uint32_t gtid = gwarp * 32 + lane;
     for (uint32_t i = l0 + gtid; i < l1; i += nthreads) {
       const uint4 it = A.q.large[i];
-      if (it.w & 1u) atomicAdd(A.deps + it.x, 1.0 / A.sigma[it.x]);
+      if (it.w & 1u) {
+        const double x = 1.0 / A.sigma[it.x];
+        A.inv[it.x] = x;
+        atomicAdd(dep + it.x, left ? left[it.x] + x : x);
+      }
     }
     if (alone) {
       for (uint32_t i = s0 + gtid; i < s1; i += nthreads) {
         const uint32_t u = A.q.small[i].x;
-        if (push) atomicAdd(A.deps + u, 1.0 / A.sigma[u]);  // beside the pushes
-        else A.deps[u] += 1.0 / A.sigma[u];
+        const double x = 1.0 / A.sigma[u];
+        A.inv[u] = x;
+        const double own = left ? left[u] + x : x;
+        if (push) atomicAdd(dep + u, own);  // beside the pushes
+        else dep[u] = own;
       }
     } else {
+      auto successors = [&](const uint32_t (&d)[4]) {  // the sum over those of d in the next level
+        double x[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) x[k] = d[k] != kNone ? next[d[k]] : 0.0;
+        return (x[0] + x[1]) + (x[2] + x[3]);
+      };
       // four pieces per warp, their sums reduced together
       for (uint32_t i0 = l0 + gwarp * 4; i0 < l1; i0 += nwarps * 4) {
         double acc[4];
@@ -853,58 +877,52 @@ __device__ bool bc_backward(const BcArgs& A, int s, bool last, Grid& grid, uint3
           const uint4 it = i0 + p < l1 ? A.q.large[i0 + p] : make_uint4(0, 0, 0, 0);
           if (lane / 8 == p) v = it.x;
           uint32_t d[4];
-          int32_t l[4];
 #pragma unroll
           for (int k = 0; k < 4; k++) d[k] = it.y + 32 * k + lane < it.z ? A.g.adj[it.y + 32 * k + lane] : kNone;
-#pragma unroll
-          for (int k = 0; k < 4; k++) l[k] = d[k] != kNone ? A.lvl[d[k]] : -2;
-          acc[p] = 0.0;
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            if (l[k] == r + 1) acc[p] += A.deps[d[k]];
-          }
+          acc[p] = successors(d);
         }
         const double z = warp_sum4(acc);
-        if ((lane & 7) == 0 && z != 0.0) atomicAdd(A.deps + v, z);
+        if ((lane & 7) == 0 && z != 0.0) atomicAdd(dep + v, z);
       }
-      const uint32_t groups = (s1 - s0 + 7) / 8;
-      for (uint32_t i = gwarp; i < groups; i += nwarps) {
-        const uint32_t j = s0 + i * 8 + (lane >> 2);
-        const uint4 it = j < s1 ? A.q.small[j] : make_uint4(0, 0, 0, 0);
-        const uint32_t u = it.x, b = it.y, end = it.z;
-        double acc = 0.0;
-        for (uint32_t e0 = b + (lane & 3); __any_sync(kAll, e0 < end); e0 += 16) {
-          uint32_t d[4];
-          int32_t l[4];
+      // 8 vertices at a time, of 32 where the level has enough for every warp: one
+      // division serves them
+      const uint32_t per = s1 - s0 >= nwarps * 32 ? 4 : 1;
+      for (uint32_t i = gwarp * per; i < (s1 - s0 + 7) / 8; i += nwarps * per) {
+        const uint32_t own = s0 + i * 8 + lane;
+        const bool mine = own < s1 && lane < (int)per * 8;
+        const uint32_t w = mine ? A.q.small[own].x : 0u;
+        double x = mine ? A.sigma[w] : 1.0;
+        if (per > 1) x = 1.0 / x;
+        for (uint32_t t = 0; t < per; t++) {
+          const uint32_t j = s0 + (i + t) * 8 + (lane >> 2);
+          const uint4 it = j < s1 ? A.q.small[j] : make_uint4(0, 0, 0, 0);
+          const uint32_t u = it.x, b = it.y, end = it.z;
+          double acc = 0.0;
+          for (uint32_t e0 = b + (lane & 3); __any_sync(kAll, e0 < end); e0 += 16) {
+            uint32_t d[4];
 #pragma unroll
-          for (int k = 0; k < 4; k++) d[k] = e0 + 4 * k < end ? A.g.adj[e0 + 4 * k] : kNone;
-#pragma unroll
-          for (int k = 0; k < 4; k++) l[k] = d[k] != kNone ? A.lvl[d[k]] : -2;
-#pragma unroll
-          for (int k = 0; k < 4; k++) {
-            if (l[k] == r + 1) acc += A.deps[d[k]];
+            for (int k = 0; k < 4; k++) d[k] = e0 + 4 * k < end ? A.g.adj[e0 + 4 * k] : kNone;
+            acc += successors(d);
           }
+          acc += __shfl_xor_sync(kAll, acc, 1);
+          acc += __shfl_xor_sync(kAll, acc, 2);
+          if (per == 1) x = 1.0 / x;  // (a short chain: the division waits for nothing)
+          const double y = __shfl_sync(kAll, x, t * 8 + (lane >> 2));
+          if (j < s1 && (lane & 3) == 0) dep[u] = left ? left[u] + (y + acc) : y + acc;
         }
-        acc += __shfl_xor_sync(kAll, acc, 1);
-        acc += __shfl_xor_sync(kAll, acc, 2);
-        if (j < s1 && (lane & 3) == 0) A.deps[u] += 1.0 / A.sigma[u] + acc;
+        if (mine) A.inv[w] = x;
       }
     }
     if (!grid.sync()) return false;
   }
-  // D = (D - 1/sigma) / (1/sigma), as bc_final forms it (unreached: NaN)
-  if (A.deps_out && last) {
-    double* out = A.deps_out + (A.rows ? (size_t)s * n : 0);
-    for (uint32_t i = tid; i < n; i += nthreads) {
-      const uint32_t v = A.new_ids ? A.new_ids[i] : i;
-      const double x = A.sigma[v];
-      out[i] = (A.deps[v] - 1 / x) * x;
-    }
-  } else {
-    for (uint32_t i = tid; i < n; i += nthreads) {
-      const double x = A.sigma[i];
-      A.deps[i] = (A.deps[i] - 1 / x) * x;
-    }
+  // D = (D - 1/sigma) / (1/sigma), as bc_final forms it (unreached: NaN); by original
+  // id for the caller (page-locked results: behind the host link)
+  double* out = A.deps_out && last ? A.deps_out + (A.rows ? (size_t)s * n : 0) : nullptr;
+  double* to = out ? out : A.deps;
+  for (uint32_t i = tid; i < n; i += nthreads) {
+    const uint32_t v = out && A.new_ids ? A.new_ids[i] : i;
+    const double d = A.even[v] + A.odd[v];  // one of them is 0; both: not reached
+    to[i] = d != 0.0 ? (d - A.inv[v]) * A.sigma[v] : CUDART_NAN;
   }
   if (tid == 0) {
     volatile uint64_t* f = A.info + (A.rows ? 4 * s : 0);
@@ -928,7 +946,9 @@ __device__ void bc_group(const BcArgs& P, size_t y, int s, BcArgs* A) {
   A->lvl += y * n;
   A->vis += y * ((n + 31) / 32);
   A->sigma += y * n;
-  if (P.rows) A->deps += y * n;
+  A->even += y * n;
+  A->odd += y * n;
+  A->inv += y * n;
   A->q.small += y * P.n_small;
   A->q.large += y * P.n_large;
   A->first_small += y * (n + 2);
@@ -1933,7 +1953,7 @@ namespace {
 
 // The arrays of `groups` groups of bc_fused.
 // *ordered (unless null): n results by original id.
-rg_status bc_arrays(const rg_graph* g, int groups, BcArgs* A, double** ordered) {
+rg_status bc_arrays(const rg_graph* g, int groups, bool chain, BcArgs* A, double** ordered) {
   const size_t n = (size_t)g->n, m = (size_t)g->m;
   A->n_small = small_entries(g->n);
   A->n_large = large_entries(g->n, g->m);
@@ -1947,12 +1967,15 @@ rg_status bc_arrays(const rg_graph* g, int groups, BcArgs* A, double** ordered) 
   X.add(&A->vis, (n + 31) / 32 * groups);
   X.add(&A->lvl, n * groups);
   X.add(&A->sigma, n * groups);
-  X.add(&A->deps, n * groups);
+  X.add(&A->even, n * groups);
+  X.add(&A->odd, n * groups);
+  X.add(&A->inv, n * groups);
   add_queues(X, &A->q, g->n, g->m, groups);
   X.add(&A->first_small, (n + 2) * groups);
   X.add(&A->first_large, (n + 2) * groups);
   X.add(&A->level_deg, (n + 2) * groups);
   X.add(&A->heavy, A->n_heavy * groups);
+  if (chain) X.add(&A->deps, n);
   if (ordered) X.add(ordered, n);
   return X.place();
 }
@@ -1981,7 +2004,7 @@ rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* 
   double* ordered = !order ? nullptr : direct ? direct : d_deps_out;
   int groups = 1, width = fused_grid(m + n, kFusedEdgesPerCta);
   if (m <= std::min(kFusedBcRowsEdges, kFusedBcRowsWork / std::max(nsrc, 1))) bc_split(g, std::min(nsrc, 64), &groups, &width);
-  RG_TRY(bc_arrays(g, groups, &A, order && !ordered ? &ordered : nullptr));
+  RG_TRY(bc_arrays(g, groups, true, &A, order && !ordered ? &ordered : nullptr));
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = cx.ws.h_info;
   info[0] = info[1] = info[3] = 0;
@@ -2018,7 +2041,7 @@ rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double
   int groups, width;
   bc_split(g, k, &groups, &width);
   BcArgs A;
-  RG_TRY(bc_arrays(g, groups, &A, nullptr));
+  RG_TRY(bc_arrays(g, groups, false, &A, nullptr));
   A.g = g->view();
   A.gt = g->in_view();
   for (int q = 0; q < k; q++) A.source[q] = src_orig[q];
