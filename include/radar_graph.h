@@ -449,10 +449,10 @@ typedef enum rg_option {
    * variants push in dense iterations (dense_forward), push-pull pulls.
    * 1: dense iterations pull in every variant (no atomics; BFS exits at the
    * first frontier neighbour; Radii and multi-source BFS OR every neighbour's
-   * mask).  Results are identical either way.  rg_bfs, and the other apps on
-   * graphs of up to a few million edges, run their levels in one launch that
-   * pulls dense iterations in every variant, whatever this option says; while
-   * rg_set_trace is on they run level by level. */
+   * mask).  Results are identical either way.  BFS and BC, and the other apps
+   * on small and mid-sized graphs, run in one launch that chooses each level's
+   * direction itself, whatever this option says; while rg_set_trace is on they
+   * run level by level. */
   RG_OPT_DIRECTION = 0,
   /* hub copies per CTA for HUBDUP/RADAR; 0 = as many as the budget allows */
   RG_OPT_HUB_SLOTS = 1,
@@ -460,7 +460,8 @@ typedef enum rg_option {
    * (default 48; PageRank's full sweeps use one CTA per SM and all of it);
    * 0 = no hub copies (HUBDUP/RADAR then update hubs with global atomics) */
   RG_OPT_HUB_SMEM_KB = 2,
-  /* dense iteration when |F| + outdeg(F) > m / value (default 20, ligra.h:283) */
+  /* dense iteration when |F| + outdeg(F) > m / value (default 20, ligra.h:283;
+   * Radii and multi-source BFS in one launch: 2 m / value from 2^22 edges on) */
   RG_OPT_DENSE_DIV = 3,
   /* shape of the full-graph PageRank pull sweep: 10 * (edges per lane, 4, 8
    * or 16) + cache mode (0 plain loads; 1 streamed edge array; 2 streamed
@@ -505,7 +506,8 @@ rg_status rg_graph_clear_tuning(rg_graph* g);
  * Timing of the last app call (CUDA events on the launching stream).
  * ------------------------------------------------------------------------ */
 typedef struct rg_timing {
-  double total_ms;          /* whole app call on the device */
+  double total_ms;          /* whole app call on the device (with the results' way to the host
+                               where a kernel writes page-locked results itself) */
   double edge_ms;           /* time inside edge kernels */
   int64_t edges_traversed;  /* GTEPS numerator: edges examined by the edge maps */
   int64_t algorithmic_bytes;/* compulsory bytes of the app's byte model */

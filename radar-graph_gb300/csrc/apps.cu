@@ -1,10 +1,11 @@
 // App drivers (Compute of PageRank.C, BFS.C, BC-manyiter-v2.C, Radii.C) on
 // the device engine, and the engine-level C ABI (rg_edgemap/rg_vertexmap).
 //
-// Every app keeps its arrays resident in HBM for the whole call, reads back
-// only the per-level frontier size (one 16-byte copy per level, the same
-// information the reference's edgeMapData gathers to choose a mode), and
-// copies the result to the host once at the end.
+// BFS, BC and Radii run in one launch (fused.cu) where that is the faster way.
+// Here they run level by level: every app keeps its arrays resident in HBM for the
+// whole call, reads back only the per-level frontier size (the same information the
+// reference's edgeMapData gathers to choose a mode), and copies the result to the
+// host once at the end.
 
 #include <cuda_runtime.h>
 #include <math.h>

@@ -31,6 +31,8 @@ constexpr unsigned kAll = 0xffffffffu;
 // The pairs (u, v), u > v, of a symmetric graph, ordered by v: counted per
 // kSweepChunk edges (a warp each; rows from the chunk starts), then written as
 // u << bits | v at the chunk's place with the digit counts of the sort by u.
+// Bound by the row searches' latency: four edges per lane share one (7.3e6 entries:
+// 42 and 47 us with a search each, 19 and 30 now).
 template <bool kEmit>
 __global__ void __launch_bounds__(256) upper_pairs(DevGraph g, const uint32_t* __restrict__ chunk_v, uint32_t nchunks,
                                                    uint32_t* __restrict__ count, const uint32_t* __restrict__ place,
@@ -43,19 +45,46 @@ __global__ void __launch_bounds__(256) upper_pairs(DevGraph g, const uint32_t* _
   for (uint32_t c = warp; c < nchunks; c += nwarps) {
     const uint32_t vlo = chunk_v[c], vhi = chunk_v[c + 1];
     uint32_t n = 0, at = kEmit ? place[c] : 0;
-    for (int r = 0; r < kSweepChunk / 32; r++) {
-      const uint32_t e = c * kSweepChunk + r * 32 + lane;
-      const uint32_t v = e < g.m ? upper_index(g.off, vlo, vhi, e) : 0, u = e < g.m ? g.adj[e] : 0;
-      const unsigned keep = __ballot_sync(kAll, u > v);
-      if (kEmit && u > v) {
-        const uint64_t k = ((uint64_t)u << bits) | v;
-        key[at + __popc(keep & ((1u << lane) - 1u))] = k;
-        sort_count_key(sh, k, bits, 2 * bits, passes);
+    // four edges per lane: one row search for them
+    for (int r = 0; r < kSweepChunk / 128; r++) {
+      const uint32_t e = c * kSweepChunk + r * 128 + lane * 4;
+      uint32_t u[4] = {}, v[4] = {}, own = 0;
+      if (e < g.m) {
+        const uint4 x = __ldg(reinterpret_cast<const uint4*>(g.adj + e));  // adj is padded past m
+        u[0] = x.x, u[1] = x.y, u[2] = x.z, u[3] = x.w;
+        uint32_t row = upper_index(g.off, vlo, vhi, e), next = g.off[row + 1];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          while (e + k < g.m && e + k >= next) next = g.off[++row + 1];
+          v[k] = row;
+          if (e + k >= g.m) u[k] = 0;
+          own += u[k] > v[k];
+        }
       }
-      at += __popc(keep);
-      n += __popc(keep);
+      if (!kEmit) {
+        n += own;
+        continue;
+      }
+      uint32_t inc = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(kAll, inc, o);
+        if (lane >= o) inc += t;
+      }
+      uint32_t to = at + inc - own;
+      at += __shfl_sync(kAll, inc, 31);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        if (u[k] <= v[k]) continue;
+        const uint64_t x = ((uint64_t)u[k] << bits) | v[k];
+        key[to++] = x;
+        sort_count_key(sh, x, bits, 2 * bits, passes);
+      }
     }
-    if (!kEmit && lane == 0) count[c] = n;
+    if (!kEmit) {
+      n = __reduce_add_sync(kAll, n);
+      if (lane == 0) count[c] = n;
+    }
   }
   if (kEmit) sort_flush(sh, hist, passes);
 }

@@ -3,7 +3,9 @@
 // copies on/off and their shared-memory budget, PageRank's sweep shape) and
 // keeps the fastest per app
 // in the graph.  Later app calls on that graph use the choice.  No schedule
-// changes any result, so tuning is safe to run on live graphs.
+// changes any result, so tuning is safe to run on live graphs.  (Calls that are
+// answered by one launch choose a direction per level themselves: of the options
+// only the dense threshold reaches them.)
 
 #include <cuda_runtime.h>
 
