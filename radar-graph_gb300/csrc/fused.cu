@@ -877,13 +877,14 @@ __device__ bool bc_backward(const BcArgs& A, int s, bool last, Grid& grid, uint3
         for (int k = 0; k < 4; k++) x[k] = d[k] != kNone ? next[d[k]] : 0.0;
         return (x[0] + x[1]) + (x[2] + x[3]);
       };
-      // four pieces per warp, their sums reduced together
-      for (uint32_t i0 = l0 + gwarp * 4; i0 < l1; i0 += nwarps * 4) {
+      // four pieces per warp, their sums reduced together (one where there are few)
+      const uint32_t each = l1 - l0 > nwarps ? 4 : 1;
+      for (uint32_t i0 = l0 + gwarp * each; i0 < l1; i0 += nwarps * each) {
         double acc[4];
         uint32_t v = 0;  // the vertex of piece lane / 8
 #pragma unroll
         for (int p = 0; p < 4; p++) {
-          const uint4 it = i0 + p < l1 ? A.q.large[i0 + p] : make_uint4(0, 0, 0, 0);
+          const uint4 it = p < (int)each && i0 + p < l1 ? A.q.large[i0 + p] : make_uint4(0, 0, 0, 0);
           if (lane / 8 == p) v = it.x;
           uint32_t d[4];
 #pragma unroll
@@ -896,7 +897,18 @@ __device__ bool bc_backward(const BcArgs& A, int s, bool last, Grid& grid, uint3
       // 8 vertices at a time, of 32 where the level has enough for every warp: one
       // division serves them
       const uint32_t per = s1 - s0 >= nwarps * 32 ? 4 : 1;
-      for (uint32_t i = gwarp * per; i < (s1 - s0 + 7) / 8; i += nwarps * per) {
+      const bool few = s1 - s0 <= nwarps;  // a vertex per warp, an edge per lane
+      for (uint32_t i = s0 + gwarp; few && i < s1; i += nwarps) {
+        const uint4 it = A.q.small[i];
+        const double x = 1.0 / A.sigma[it.x];
+        const uint32_t d = it.y + lane < it.z ? A.g.adj[it.y + lane] : kNone;
+        const double acc = warp_sum(d != kNone ? next[d] : 0.0);
+        if (lane == 0) {
+          A.inv[it.x] = x;
+          dep[it.x] = left ? left[it.x] + (x + acc) : x + acc;
+        }
+      }
+      for (uint32_t i = gwarp * per; !few && i < (s1 - s0 + 7) / 8; i += nwarps * per) {
         const uint32_t own = s0 + i * 8 + lane;
         const bool mine = own < s1 && lane < (int)per * 8;
         const uint32_t w = mine ? A.q.small[own].x : 0u;
