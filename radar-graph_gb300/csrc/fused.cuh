@@ -23,11 +23,11 @@ constexpr int64_t kFusedPrRows = 12000;
 // Largest graphs (edges, and vertices) that take the one-launch path, by app.
 // Device time against the level-by-level run, R-MAT edge factor 16, degree
 // sorted (in brackets: uniform, unsorted), us:
-//   BFS       2^10 vertices 31 / 182, 2^16 46 / 298, 2^20 95 / 415 (167 / 402),
-//             2^24 560 / 973 (1823 / 2972): every size
-//   BC        2^10 58 / 246 (75 / 240), 2^18 130 / 506 (153 / 496), 2^22
-//             601 / 1573 (1007 / 1975), 2^24 3519 / 5520 (8066 / 9983): every size
-//   Radii     2^10 73 / 309, 2^18 246 / 583 (300 / 515), 2^20 491 / 789 (765 /
+//   BFS       2^10 vertices 27 / 182, 2^16 43 / 298, 2^20 87 / 415 (104 / 402),
+//             2^24 450 / 973 (1680 / 2972): every size
+//   BC        2^10 51 / 246 (72 / 240), 2^18 125 / 506 (125 / 496), 2^22
+//             703 / 1573 (970 / 1975), 2^24 3150 / 5520 (5560 / 9983): every size
+//   Radii     2^10 63 / 309, 2^18 231 / 583 (257 / 515), 2^20 462 / 789 (718 /
 //             963), 2^20.5 631 / 913 (997 / 1012), 2^21 749 / 988 (1293 / 1249), 2^22
 //             1658 / 1866 (2623 / 2355), 2^22.5 2609 / 2739, 2^23 2970 / 2758: sorted
 //             1.7e8 edges, others 5e7 (their pulls want more warps than one CTA per
@@ -41,14 +41,16 @@ constexpr int64_t kFusedPrRows = 12000;
 //             edges; against pushes: 2^16 309 / 730, 2^18 1331 / 1559, 2^19 2737 /
 //             2332: 8e6 edges
 //   PageRankDelta  whole, against dense rounds swept and the rest handed over:
-//             2^10 139 / 398 (85 / 238), 2^18 494 / 688 (332 / 440), 2^19
-//             774 / 815 (605 / 598), 2^20 1441 / 1164 (1146 / 872): 1.7e7 edges
+//             2^14 167 / 173 (85 / 102), 2^17 374 / 369 (164 / 175), 2^18 411 / 343
+//             (258 / 239), 2^19 619 / 495 (462 / 381), 2^20 1086 / 829 (842 / 646):
+//             6e6 edges; where dense rounds would push level by level, 3.3e7
 constexpr int64_t kFusedBfsEdges = INT64_MAX;
 constexpr int64_t kFusedBcEdges = INT64_MAX;
 constexpr int64_t kFusedRadiiEdges = 6 << 23, kFusedRadiiSortedEdges = 5 << 25;
 constexpr int64_t kFusedPagerankEdges = 3 << 20;
 constexpr int64_t kFusedPagerankPushEdges = 8 << 20;
-constexpr int64_t kFusedPrdEdges = 1 << 25;
+constexpr int64_t kFusedPrdEdges = 6 << 20;
+constexpr int64_t kFusedPrdPushEdges = 1 << 25;
 //   multi-source BC  16 sources: 2^14 116 / 1023 (147 / 864), 2^18 850 / 2055
 //             (900 / 2193), 2^19 1800 / 3010 (3000 / 4154), 2^20 4564 / 5299 (8250 /
 //             6911); 64 sources: 2^16 921 / 1498 (1426 / 1464), 2^17 1764 / 1961

@@ -170,7 +170,7 @@ rg_status pagerank_delta_run(rg_graph* g, int variant, int64_t max_iters, double
   const int64_t n = g->n;
   static thread_local PrdState S;
   const bool pulls = variant == RG_PUSH_PULL || g_opts.direction == 1;
-  const bool small = fused_fits(g, kFusedPrdEdges);
+  const bool small = fused_fits(g, pulls ? kFusedPrdEdges : kFusedPrdPushEdges);
   // the per-vertex arrays in one allocation, whole 2 MiB pages each (apart, their
   // placement moves the gathers' speed)
   const size_t page = 2u << 20, row = ((size_t)n * 8 + page - 1) / page * page;
