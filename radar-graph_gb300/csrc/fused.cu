@@ -73,7 +73,8 @@ struct L1Sum {
   }
 };
 
-// Zeroed before every launch.
+// Zero when a launch begins.  Two sets take turns: a launch clears the one that the
+// launch before it used (a memset of its own cost a call 3 us: BFS 2^10 40 -> 37).
 struct Ctl {
   unsigned int bar, fail;
   unsigned int bar_all;  // of all groups (BC)
@@ -334,7 +335,11 @@ __device__ __forceinline__ void expand(const DevGraph& g, const Queues& q, uint3
   }
 }
 
-__device__ __forceinline__ void begin(Grid& grid, Shared* sh, Ctl* ctl) {
+__device__ __forceinline__ void begin(Grid& grid, Shared* sh, Ctl* ctl, Ctl* stale, int nstale) {
+  if (blockIdx.x == 0 && blockIdx.y == 0) {  // what the launch before used, for the one after
+    unsigned* w = reinterpret_cast<unsigned*>(stale);
+    for (int i = threadIdx.x; i < nstale * (int)(sizeof(Ctl) / 4); i += kFT) w[i] = 0u;
+  }
   grid.sh = sh;
   grid.which = 0;
   if (threadIdx.x == 0) {
@@ -363,7 +368,8 @@ struct BfsArgs {
   uint32_t* parents;  // null: not wanted
   int32_t* depth_out;  // original-id order; null: not wanted (or not sorted)
   Queues q[2];
-  Ctl* ctl;
+  Ctl *ctl, *stale;
+  int nstale;
   volatile uint64_t* info;  // mapped: rounds, reached, edges, done
 };
 
@@ -377,7 +383,7 @@ __global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
   __shared__ Member buf[kFWarps][kBuf];
   Grid grid;
   Appender<false> ap{buf[threadIdx.x >> 5], &sh, 0};
-  begin(grid, &sh, A.ctl);
+  begin(grid, &sh, A.ctl, A.stale, A.nstale);
   const uint32_t n = A.out.n, nwords = (n + 31) / 32;
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
   const int lane = threadIdx.x & 31;
@@ -591,7 +597,8 @@ struct BcArgs {
   uint4* heavy;                         // a pulled level's pieces of long lists
   size_t n_small, n_large, n_heavy;     // a group's share of the queues
   bool first_source;
-  Ctl* ctl;
+  Ctl *ctl, *stale;
+  int nstale;
   volatile uint64_t* info;  // mapped, four words per source (or summed over the calls): levels, edges, -, done
 };
 
@@ -989,7 +996,7 @@ __global__ void __launch_bounds__(kFT, 1) bc_fused(const __grid_constant__ BcArg
   __shared__ BcArgs A;  // with the group's own arrays
   Grid grid;
   Appender<true> ap{buf[threadIdx.x >> 5], &sh, 0};
-  begin(grid, &sh, P.ctl + blockIdx.y);
+  begin(grid, &sh, P.ctl + blockIdx.y, P.stale, P.nstale);
   if (threadIdx.x == 0) sh.team[1] = Team{&P.ctl->bar_all, &P.ctl->fail, 0, gridDim.x * gridDim.y};
   const int groups = gridDim.y;
   for (int s0 = 0; s0 < P.k; s0 += groups) {
@@ -1039,7 +1046,8 @@ struct RadiiArgs {
   unsigned long long* planes;
   int32_t* depths;  // sources rows of n, original-id order
   int sources;
-  Ctl* ctl;
+  Ctl *ctl, *stale;
+  int nstale;
   volatile uint64_t* info;  // mapped: rounds, edges, -, done
 };
 // Chunks of kSweepChunk edges per warp from which a dense round takes them whole
@@ -1110,7 +1118,7 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
   __shared__ Member buf[kFWarps][kBuf];
   Grid grid;
   Appender<true> ap{buf[threadIdx.x >> 5], &sh, 0};
-  begin(grid, &sh, A.ctl);
+  begin(grid, &sh, A.ctl, A.stale, A.nstale);
   const uint32_t n = A.out.n, nwords = (n + 31) / 32;
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
   const int lane = threadIdx.x & 31;
@@ -1374,7 +1382,8 @@ struct PrArgs {
   uint32_t row_weight;  // a row counts as this many edges when rows are shared out
   int64_t max_iters;
   double p0, added;
-  Ctl* ctl;
+  Ctl *ctl, *stale;
+  int nstale;
   volatile uint64_t* info;  // mapped: iterations run, last L1 (2 words), done, broke
 };
 
@@ -1471,7 +1480,7 @@ __global__ void __launch_bounds__(kFT, 1) pagerank_fused(const __grid_constant__
   extern __shared__ __align__(16) unsigned char smem_raw[];
   U128* acc = reinterpret_cast<U128*>(smem_raw);
   Grid grid;
-  begin(grid, &sh, A.ctl);
+  begin(grid, &sh, A.ctl, A.stale, A.nstale);
   const uint32_t n = A.in.n, m = A.in.m;
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1592,7 +1601,8 @@ struct PrdArgs {
   bool allow_pull;
   double one_over_n, added;
   double* ranks_out;  // original-id order; null: not wanted (or not sorted)
-  Ctl* ctl;
+  Ctl *ctl, *stale;
+  int nstale;
   volatile uint64_t* info;  // mapped: rounds, L1 (bits), edges, done
 };
 
@@ -1613,7 +1623,7 @@ __global__ void __launch_bounds__(kFT, 1) prd_fused(const __grid_constant__ PrdA
   __shared__ double s_l1[kFWarps];
   Grid grid;
   Appender<false> ap{buf[threadIdx.x >> 5], &sh, 0};
-  begin(grid, &sh, A.ctl);
+  begin(grid, &sh, A.ctl, A.stale, A.nstale);
   const uint32_t n = A.out.n, nwords = (n + 31) / 32;
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1855,8 +1865,10 @@ int fused_grid(int64_t work, int64_t per_cta) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(device_sms(), work / per_cta));
 }
 
+constexpr unsigned kMostGroups = 64;
+
 template <class K, class Args>
-rg_status launch_fused(K kern, const Args& args, dim3 grid, size_t dyn, size_t most_dyn, cudaStream_t st) {
+rg_status launch_fused(K kern, Args& args, dim3 grid, size_t dyn, size_t most_dyn, cudaStream_t st) {
   static std::atomic<uint64_t> checked{0};
   RG_TRY(once_per_device(checked, [&]() -> rg_status {
     // one CTA per SM must fit, with all the dynamic shared memory it may ask for
@@ -1868,11 +1880,27 @@ rg_status launch_fused(K kern, const Args& args, dim3 grid, size_t dyn, size_t m
     RG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFT, most_dyn));
     return per_sm > 0 ? RG_OK : fail(RG_ECUDA, "one-launch traversal does not fit an SM");
   }));
-  RG_CUDA(cudaMemsetAsync(args.ctl, 0, sizeof(Ctl) * grid.y, st));
-  void* p[] = {const_cast<Args*>(&args)};
+  Workspace& ws = ctx().ws;
+  if (grid.y > kMostGroups) return fail(RG_EINVAL, "more groups than control blocks");
+  if (!ws.one_launch.p) {
+    RG_TRY(ws.one_launch.reserve(2 * kMostGroups * sizeof(Ctl)));
+    ws.one_launch_used = 0;
+    const cudaError_t e = cudaMemsetAsync(ws.one_launch.p, 0, 2 * kMostGroups * sizeof(Ctl), st);
+    if (e != cudaSuccess) ws.one_launch.release();
+    RG_CUDA(e);
+  }
+  Ctl* sets = ws.one_launch.as<Ctl>();
+  args.ctl = sets + ws.one_launch_set * kMostGroups;
+  args.stale = sets + (ws.one_launch_set ^ 1) * kMostGroups;
+  args.nstale = ws.one_launch_used;
+  void* p[] = {&args};
   kt_begin(st);
-  RG_CUDA(cudaLaunchCooperativeKernel((const void*)kern, grid, dim3(kFT), p, dyn, st));
+  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)kern, grid, dim3(kFT), p, dyn, st);
+  if (e != cudaSuccess) ws.one_launch.release();  // cleared anew by the next launch
+  RG_CUDA(e);
   kt_end(st);
+  ws.one_launch_used = (int)grid.y;
+  ws.one_launch_set ^= 1;
   g_timing.kernel_launches++;
   g_timing.edge_launches++;
   return RG_OK;
@@ -1936,7 +1964,6 @@ rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t
   A.depth_out = nullptr;
   const bool order = g->sorted && (h_depth || d_depth_out);
   Arrays X;
-  X.add(&A.ctl, 1);
   X.add(&A.vis[0], nwords);
   X.add(&A.vis[1], nwords);
   X.add(&A.depth, n);
@@ -1989,7 +2016,6 @@ rg_status bc_arrays(const rg_graph* g, int groups, bool chain, BcArgs* A, double
   A->n_heavy = A->long_lists ? m / kLongPiece + m / kLongList + 64 : 0;
   A->new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
   Arrays X;
-  X.add(&A->ctl, groups);
   X.add(&A->vis, (n + 31) / 32 * groups);
   X.add(&A->lvl, n * groups);
   X.add(&A->sigma, n * groups);
@@ -2012,7 +2038,7 @@ rg_status bc_arrays(const rg_graph* g, int groups, bool chain, BcArgs* A, double
 // one traversal can use.
 void bc_split(const rg_graph* g, int k, int* groups, int* width) {
   const int64_t in_l2 = std::max<int64_t>(1, kFusedBcRowsL2 / (44 * g->n));
-  const int most = (int)std::min<int64_t>({(int64_t)k, (int64_t)device_sms(), in_l2});
+  const int most = (int)std::min<int64_t>({(int64_t)k, (int64_t)device_sms(), in_l2, (int64_t)kMostGroups});
   *groups = (k + (k + most - 1) / most - 1) / ((k + most - 1) / most);  // as many rounds, evenly filled
   *width = std::min(fused_grid(g->m + g->n, kFusedEdgesPerCta), std::max(1, device_sms() / *groups));
 }
@@ -2101,7 +2127,6 @@ rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned lo
   A->radii_out = nullptr;
   A->planes = nullptr;
   Arrays X;
-  X.add(&A->ctl, 1);
   X.add(&A->bits[0], (n + 31) / 32);
   X.add(&A->bits[1], (n + 31) / 32);
   X.add(&A->vis, n);
@@ -2203,7 +2228,6 @@ rg_status pagerank_fused_run(rg_graph* g, int64_t max_iters, double* h_ranks, in
   const size_t steps = (size_t)(m / kPrStep + 2 * grid + 4);
   A.ranks_out = nullptr;
   Arrays X;
-  X.add(&A.ctl, 1);
   X.add(&A.lane_row, (size_t)(m / 4 + 32 * (grid + 2) + 64));
   X.add(&A.opens, steps);
   X.add(&A.closes, steps);
@@ -2250,7 +2274,6 @@ rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max
   PrdArgs A;
   A.rows = Queues{};
   Arrays X;
-  X.add(&A.ctl, 1);
   add_queues(X, &A.q[0], n, m);
   add_queues(X, &A.q[1], n, m);
   if (start == 0) add_queues(X, &A.rows, n, m);

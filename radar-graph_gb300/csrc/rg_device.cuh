@@ -108,6 +108,8 @@ struct Workspace {
   DevBuf tiles;          // push tile -> first frontier entry
   DevBuf counters;       // small device scalars
   DevBuf lookup;         // lookup_ids staging
+  DevBuf one_launch;     // fused.cu: the launches' control blocks, two sets
+  int one_launch_set = 0, one_launch_used = 0;  // the next launch's set; blocks of the last one's
   uint64_t* h_info = nullptr;      // pinned, mapped host mirror of level info (count, degsum, ...)
   uint64_t* h_info_dev = nullptr;  // the device's address of h_info (kernels write it directly)
   unsigned char* h_small = nullptr;      // pinned, mapped scratch for small reads (read_small)
