@@ -536,6 +536,14 @@ typedef struct rg_level_trace {
 rg_status rg_set_trace(int on);
 rg_status rg_trace_take(rg_level_trace* h_out, int64_t cap, int64_t* count);
 
+/* Waits of the calling thread's launches (CTAs of one launch wait for each other)
+ * give up after this many polls: a traversal is then answered level by level, a
+ * graph build or sort returns RG_ECUDA.  Negative (the default): each kind of wait
+ * has a limit of its own, about a second.  The first `from` barriers of a traversal's
+ * launch keep that limit.  For tests of what follows a wait that ran out.  Per
+ * thread; never changes a result. */
+rg_status rg_set_wait_polls(int64_t polls, int from);
+
 #ifdef __cplusplus
 }
 #endif

@@ -21,6 +21,8 @@ extern thread_local rg_timing g_timing;
 extern bool g_kernel_timing;
 // rg_set_trace: the calling thread's per-level edgeMap records
 extern thread_local bool g_trace_on;
+extern thread_local int64_t g_wait_polls;  // rg_set_wait_polls; negative: each wait's own limit
+extern thread_local uint32_t g_wait_from;
 extern thread_local std::vector<rg_level_trace> g_trace;
 
 // NVTX range for the lifetime of the object (no cost without a profiler)

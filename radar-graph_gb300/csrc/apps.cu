@@ -30,6 +30,8 @@ namespace rg {
 thread_local rg_timing g_timing;
 bool g_kernel_timing = false;
 thread_local bool g_trace_on = false;
+thread_local int64_t g_wait_polls = -1;
+thread_local uint32_t g_wait_from = 0;
 thread_local std::vector<rg_level_trace> g_trace;
 thread_local std::vector<std::pair<cudaEvent_t, cudaEvent_t>> g_kt_events;
 thread_local size_t g_kt_used = 0;
@@ -734,6 +736,13 @@ rg_status rg_trace_take(rg_level_trace* h_out, int64_t cap, int64_t* count) {
   std::copy(g_trace.begin(), g_trace.begin() + k, h_out);
   *count = k;
   g_trace.clear();
+  return RG_OK;
+}
+
+rg_status rg_set_wait_polls(int64_t polls, int from) {
+  if (polls > 1 << 30 || from < 0) return fail(RG_EINVAL, "rg_set_wait_polls: at most 2^30 polls, from >= 0");
+  g_wait_polls = polls;
+  g_wait_from = (uint32_t)from;
   return RG_OK;
 }
 

@@ -17,8 +17,8 @@
 // each, so a hub and a leaf cost the same per edge.  Winners are collected in a
 // per-warp shared-memory buffer and appended with one counter update per flush.
 //
-// Every wait is bounded: a CTA that waits too long raises `fail` and returns,
-// the host sees that the run did not finish and answers level by level.
+// Every wait is bounded: a CTA that waits too long says so to the host and returns,
+// and the host, whatever the other CTAs made of it, answers level by level.
 
 #include <cuda_runtime.h>
 #include <math_constants.h>
@@ -43,7 +43,7 @@ constexpr uint32_t kPiece = 128;      // edges per piece of a larger vertex
 constexpr int kFlushAt = 64;          // winners a warp collects before it appends them
 constexpr int kBuf = kFlushAt + 32;
 constexpr unsigned kAll = 0xffffffffu;
-constexpr unsigned kSpinLimit = 1u << 21;  // polls of the grid barrier: a second or two
+constexpr unsigned kPolls = 1u << 21;  // of the grid barrier: a second or two
 
 // One level's frontier: queue lengths, members and their degree sum
 // (PageRankDelta: and the round's L1; BC: the pieces of long lists that a pull
@@ -76,12 +76,22 @@ struct L1Sum {
 // Zero when a launch begins.  Two sets take turns: a launch clears the one that the
 // launch before it used (a memset of its own cost a call 3 us: BFS 2^10 40 -> 37).
 struct Ctl {
-  unsigned int bar, fail;
+  unsigned int bar;
   unsigned int bar_all;  // of all groups (BC)
   int levels;            // of the group's source (BC)
+  unsigned int pad0;
   unsigned long long edges;
   unsigned int pad[10];
   Slot lv[4];
+};
+
+// What every launch gets besides its own arguments (launch_fused fills it in).
+struct Launch {
+  Ctl *ctl, *stale;
+  int nstale;
+  unsigned polls, from;        // polls of a grid barrier, from the launch's `from`-th on, before it gives up
+  volatile uint64_t* gave_up;  // mapped: set by a CTA that did.  (The last barrier's others pass and say that
+                               // the run is done, without that CTA's share of the results.)
 };
 
 // The warp's sums of four values: of acc[p] in lanes 8p .. 8p + 7.  Six FP64 adds
@@ -110,7 +120,7 @@ struct Member {
 
 // The CTAs that meet at a barrier.
 struct Team {
-  unsigned *bar, *fail;
+  unsigned* bar;
   unsigned target, ctas;
 };
 
@@ -118,6 +128,8 @@ struct Team {
 // the barrier's verdict.
 struct Shared {
   Team team[2];  // the group's CTAs, and all of them (BC)
+  unsigned polls, from, met;   // (met: barriers so far)
+  volatile uint64_t* gave_up;
   unsigned int count;
   unsigned long long degsum;
   Slot slot;  // the frontier that the last barrier completed
@@ -161,10 +173,11 @@ struct Grid {
       int ok = 1;
       if (t.ctas > 1) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.bar) : "memory");
+        const unsigned polls = sh->met++ < sh->from ? kPolls : sh->polls;
         unsigned spins = 0;
         while ((int)(ld_acquire(t.bar) - t.target) < 0) {
-          if (++spins > kSpinLimit) {
-            atomicExch(t.fail, 1u);
+          if (++spins > polls) {
+            *sh->gave_up = 1;
             ok = 0;
             break;
           }
@@ -335,15 +348,19 @@ __device__ __forceinline__ void expand(const DevGraph& g, const Queues& q, uint3
   }
 }
 
-__device__ __forceinline__ void begin(Grid& grid, Shared* sh, Ctl* ctl, Ctl* stale, int nstale) {
+__device__ __forceinline__ void begin(Grid& grid, Shared* sh, const Launch& L, Ctl* ctl) {
   if (blockIdx.x == 0 && blockIdx.y == 0) {  // what the launch before used, for the one after
-    unsigned* w = reinterpret_cast<unsigned*>(stale);
-    for (int i = threadIdx.x; i < nstale * (int)(sizeof(Ctl) / 4); i += kFT) w[i] = 0u;
+    unsigned* w = reinterpret_cast<unsigned*>(L.stale);
+    for (int i = threadIdx.x; i < L.nstale * (int)(sizeof(Ctl) / 4); i += kFT) w[i] = 0u;
   }
   grid.sh = sh;
   grid.which = 0;
   if (threadIdx.x == 0) {
-    sh->team[0] = Team{&ctl->bar, &ctl->fail, 0, gridDim.x};
+    sh->team[0] = Team{&ctl->bar, 0, gridDim.x};
+    sh->polls = L.polls;
+    sh->from = L.from;
+    sh->met = 0;
+    sh->gave_up = L.gave_up;
     sh->count = 0;
     sh->degsum = 0;
     sh->taken = 0;
@@ -357,7 +374,7 @@ __device__ __forceinline__ void begin(Grid& grid, Shared* sh, Ctl* ctl, Ctl* sta
 // ---------------------------------------------------------------------------
 constexpr uint32_t kPullWords = 8;  // words of the visited bitmap that a warp takes together, at most
 
-struct BfsArgs {
+struct BfsArgs : Launch {
   DevGraph out, in;  // push and pull lists
   bool same;         // the same lists (a symmetric graph)
   const uint32_t* new_ids;  // null: not sorted
@@ -368,8 +385,6 @@ struct BfsArgs {
   uint32_t* parents;  // null: not wanted
   int32_t* depth_out;  // original-id order; null: not wanted (or not sorted)
   Queues q[2];
-  Ctl *ctl, *stale;
-  int nstale;
   volatile uint64_t* info;  // mapped: rounds, reached, edges, done
 };
 
@@ -383,7 +398,7 @@ __global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
   __shared__ Member buf[kFWarps][kBuf];
   Grid grid;
   Appender<false> ap{buf[threadIdx.x >> 5], &sh, 0};
-  begin(grid, &sh, A.ctl, A.stale, A.nstale);
+  begin(grid, &sh, A, A.ctl);
   const uint32_t n = A.out.n, nwords = (n + 31) / 32;
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
   const int lane = threadIdx.x & 31;
@@ -576,7 +591,7 @@ __global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
 // ---------------------------------------------------------------------------
 // BC, one source (BC-manyiter-v2.C:205-367)
 // ---------------------------------------------------------------------------
-struct BcArgs {
+struct BcArgs : Launch {
   DevGraph g;   // the lists the forward phase pushes along (the backward phase reads them the other way)
   DevGraph gt;  // the same edges by target
   bool same;    // g and gt are the same lists (a symmetric graph)
@@ -597,8 +612,6 @@ struct BcArgs {
   uint4* heavy;                         // a pulled level's pieces of long lists
   size_t n_small, n_large, n_heavy;     // a group's share of the queues
   bool first_source;
-  Ctl *ctl, *stale;
-  int nstale;
   volatile uint64_t* info;  // mapped, four words per source (or summed over the calls): levels, edges, -, done
 };
 
@@ -996,8 +1009,8 @@ __global__ void __launch_bounds__(kFT, 1) bc_fused(const __grid_constant__ BcArg
   __shared__ BcArgs A;  // with the group's own arrays
   Grid grid;
   Appender<true> ap{buf[threadIdx.x >> 5], &sh, 0};
-  begin(grid, &sh, P.ctl + blockIdx.y, P.stale, P.nstale);
-  if (threadIdx.x == 0) sh.team[1] = Team{&P.ctl->bar_all, &P.ctl->fail, 0, gridDim.x * gridDim.y};
+  begin(grid, &sh, P, P.ctl + blockIdx.y);
+  if (threadIdx.x == 0) sh.team[1] = Team{&P.ctl->bar_all, 0, gridDim.x * gridDim.y};
   const int groups = gridDim.y;
   for (int s0 = 0; s0 < P.k; s0 += groups) {
     const int s = s0 + (int)blockIdx.y;
@@ -1028,7 +1041,7 @@ __global__ void __launch_bounds__(kFT, 1) bc_fused(const __grid_constant__ BcArg
 // ---------------------------------------------------------------------------
 // Radii (Radii.C:140-218)
 // ---------------------------------------------------------------------------
-struct RadiiArgs {
+struct RadiiArgs : Launch {
   DevGraph out, in;
   const uint32_t* chunk_v;  // the pull lists' partition
   uint32_t nchunks;
@@ -1046,8 +1059,6 @@ struct RadiiArgs {
   unsigned long long* planes;
   int32_t* depths;  // sources rows of n, original-id order
   int sources;
-  Ctl *ctl, *stale;
-  int nstale;
   volatile uint64_t* info;  // mapped: rounds, edges, -, done
 };
 // Chunks of kSweepChunk edges per warp from which a dense round takes them whole
@@ -1118,7 +1129,7 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
   __shared__ Member buf[kFWarps][kBuf];
   Grid grid;
   Appender<true> ap{buf[threadIdx.x >> 5], &sh, 0};
-  begin(grid, &sh, A.ctl, A.stale, A.nstale);
+  begin(grid, &sh, A, A.ctl);
   const uint32_t n = A.out.n, nwords = (n + 31) / 32;
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
   const int lane = threadIdx.x & 31;
@@ -1367,7 +1378,7 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
 // ---------------------------------------------------------------------------
 // PageRank (PageRank.C:120-189), the exact-sum pull of pagerank.cu
 // ---------------------------------------------------------------------------
-struct PrArgs {
+struct PrArgs : Launch {
   DevGraph in;
   const uint32_t* out_off;
   const uint32_t* chunk_v;
@@ -1382,8 +1393,6 @@ struct PrArgs {
   uint32_t row_weight;  // a row counts as this many edges when rows are shared out
   int64_t max_iters;
   double p0, added;
-  Ctl *ctl, *stale;
-  int nstale;
   volatile uint64_t* info;  // mapped: iterations run, last L1 (2 words), done, broke
 };
 
@@ -1480,7 +1489,7 @@ __global__ void __launch_bounds__(kFT, 1) pagerank_fused(const __grid_constant__
   extern __shared__ __align__(16) unsigned char smem_raw[];
   U128* acc = reinterpret_cast<U128*>(smem_raw);
   Grid grid;
-  begin(grid, &sh, A.ctl, A.stale, A.nstale);
+  begin(grid, &sh, A, A.ctl);
   const uint32_t n = A.in.n, m = A.in.m;
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1586,7 +1595,7 @@ __global__ void __launch_bounds__(kFT, 1) pagerank_fused(const __grid_constant__
 // ---------------------------------------------------------------------------
 // PageRankDelta (PageRankDelta.C:98-155)
 // ---------------------------------------------------------------------------
-struct PrdArgs {
+struct PrdArgs : Launch {
   DevGraph out, in;
   const uint32_t* new_ids;
   double *p, *ngh, *c;
@@ -1601,8 +1610,6 @@ struct PrdArgs {
   bool allow_pull;
   double one_over_n, added;
   double* ranks_out;  // original-id order; null: not wanted (or not sorted)
-  Ctl *ctl, *stale;
-  int nstale;
   volatile uint64_t* info;  // mapped: rounds, L1 (bits), edges, done
 };
 
@@ -1623,7 +1630,7 @@ __global__ void __launch_bounds__(kFT, 1) prd_fused(const __grid_constant__ PrdA
   __shared__ double s_l1[kFWarps];
   Grid grid;
   Appender<false> ap{buf[threadIdx.x >> 5], &sh, 0};
-  begin(grid, &sh, A.ctl, A.stale, A.nstale);
+  begin(grid, &sh, A, A.ctl);
   const uint32_t n = A.out.n, nwords = (n + 31) / 32;
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1867,6 +1874,19 @@ int fused_grid(int64_t work, int64_t per_cta) {
 
 constexpr unsigned kMostGroups = 64;
 
+// Words of the host's info block: what the launches write for their callers, 3 (or
+// 3 of every source's four) once thread 0 is done, and kGaveUp.
+constexpr int kDone = 3, kGaveUp = 7;
+
+// Before a call's first launch.
+volatile uint64_t* info_begin() {
+  volatile uint64_t* info = ctx().ws.h_info;
+  info[0] = info[1] = info[kDone] = info[kGaveUp] = 0;
+  return info;
+}
+// Once the stream has passed the call's launches: whether every CTA of them ran to its end.
+bool all_ran() { return ctx().ws.h_info[kGaveUp] == 0; }
+
 template <class K, class Args>
 rg_status launch_fused(K kern, Args& args, dim3 grid, size_t dyn, size_t most_dyn, cudaStream_t st) {
   static std::atomic<uint64_t> checked{0};
@@ -1893,6 +1913,9 @@ rg_status launch_fused(K kern, Args& args, dim3 grid, size_t dyn, size_t most_dy
   args.ctl = sets + ws.one_launch_set * kMostGroups;
   args.stale = sets + (ws.one_launch_set ^ 1) * kMostGroups;
   args.nstale = ws.one_launch_used;
+  args.polls = g_wait_polls >= 0 ? (unsigned)g_wait_polls : kPolls;
+  args.from = g_wait_from;
+  args.gave_up = ws.h_info_dev + kGaveUp;
   void* p[] = {&args};
   kt_begin(st);
   const cudaError_t e = cudaLaunchCooperativeKernel((const void*)kern, grid, dim3(kFT), p, dyn, st);
@@ -1982,8 +2005,7 @@ rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t
   A.root = root;
   A.threshold = dense_threshold(g);
   A.info = cx.ws.h_info_dev;
-  volatile uint64_t* info = cx.ws.h_info;
-  info[3] = 0;
+  volatile uint64_t* info = info_begin();
   CallTimer timer(g);
   RG_TRY(launch_fused(bfs_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
   RG_TRY(timer.mark());
@@ -1992,7 +2014,7 @@ rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t
   RG_TRY(download_orig<uint32_t>(g, A.parents, h_parents, tmp, st));
   RG_CUDA(cudaStreamSynchronize(st));
   RG_TRY(timer.finish());
-  *done = info[3] == 1;
+  *done = info[kDone] == 1 && all_ran();
   if (!*done) return RG_OK;
   g_timing.edges_traversed = (int64_t)info[2];
   g_timing.algorithmic_bytes =
@@ -2058,8 +2080,7 @@ rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* 
   if (m <= std::min(kFusedBcRowsEdges, kFusedBcRowsWork / std::max(nsrc, 1))) bc_split(g, std::min(nsrc, 64), &groups, &width);
   RG_TRY(bc_arrays(g, groups, true, &A, order && !ordered ? &ordered : nullptr));
   A.info = cx.ws.h_info_dev;
-  volatile uint64_t* info = cx.ws.h_info;
-  info[0] = info[1] = info[3] = 0;
+  volatile uint64_t* info = info_begin();
   CallTimer timer(g);
   A.rows = false;
   A.g = g->view();
@@ -2075,7 +2096,7 @@ rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* 
   if (!direct) RG_TRY(deliver<double>(g, A.deps, ordered, h_deps, d_deps_out, st));
   RG_CUDA(cudaStreamSynchronize(st));
   RG_TRY(timer.finish());
-  *done = info[3] == (uint64_t)nsrc;
+  *done = info[kDone] == (uint64_t)nsrc && all_ran();
   if (!*done) return RG_OK;
   g_timing.edges_traversed = (int64_t)info[1];
   g_timing.algorithmic_bytes =
@@ -2089,7 +2110,6 @@ rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double
                             bool* done) {
   Ctx& cx = ctx();
   cudaStream_t st = cx.stream;
-  const int64_t n = g->n, m = g->m;
   int groups, width;
   bc_split(g, k, &groups, &width);
   BcArgs A;
@@ -2104,11 +2124,13 @@ rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double
   A.info = reinterpret_cast<volatile uint64_t*>(cx.ws.h_small_dev);
   volatile uint64_t* info = reinterpret_cast<volatile uint64_t*>(cx.ws.h_small);
   for (int i = 0; i < 4 * k; i++) info[i] = 0;
+  info_begin();
   RG_TRY(launch_fused(bc_fused, A, dim3(width, groups), 0, 0, st));
   RG_CUDA(cudaStreamSynchronize(st));
+  if (!all_ran()) return RG_OK;
   int64_t levels = 0;
   for (int q = 0; q < k; q++) {
-    if (info[4 * q + 3] != 1) return RG_OK;
+    if (info[4 * q + kDone] != 1) return RG_OK;
     levels = std::max(levels, (int64_t)info[4 * q]);
     g_timing.edges_traversed += (int64_t)info[4 * q + 1];
   }
@@ -2154,7 +2176,7 @@ rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned lo
   A->depths = nullptr;
   A->sources = 0;
   A->info = ctx().ws.h_info_dev;
-  ctx().ws.h_info[3] = 0;
+  info_begin();
   return RG_OK;
 }
 
@@ -2178,7 +2200,7 @@ rg_status radii_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned lon
   if (!direct) RG_TRY(deliver<int32_t>(g, A.radii, A.radii_out, h_radii, d_radii_out, st));
   RG_CUDA(cudaStreamSynchronize(st));
   RG_TRY(timer.finish());
-  *done = info[3] == 1;
+  *done = info[kDone] == 1 && all_ran();
   if (!*done) return RG_OK;
   g_timing.edges_traversed = (int64_t)info[1];
   g_timing.algorithmic_bytes = 4 * g_timing.edges_traversed + 16 * n + 4 * n;
@@ -2198,7 +2220,7 @@ rg_status ms_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long l
   volatile uint64_t* info = cx.ws.h_info;
   RG_TRY(launch_fused(radii_fused<true>, A, fused_grid(m + n + n * (int64_t)k / 8, kFusedEdgesPerCta), 0, 0, st));
   RG_CUDA(cudaStreamSynchronize(st));
-  *done = info[3] == 1;
+  *done = info[kDone] == 1 && all_ran();
   if (!*done) return RG_OK;
   g_timing.edges_traversed += (int64_t)info[1];
   *rounds_out = (int64_t)info[0];
@@ -2246,15 +2268,14 @@ rg_status pagerank_fused_run(rg_graph* g, int64_t max_iters, double* h_ranks, in
   A.p0 = 1 / (double)n;
   A.added = (1 - kPrDamp) * (1 / (double)n);
   A.info = cx.ws.h_info_dev;
-  volatile uint64_t* info = cx.ws.h_info;
-  info[3] = 0;
+  volatile uint64_t* info = info_begin();
   CallTimer timer(g);
   RG_TRY(launch_fused(pagerank_fused, A, grid, sizeof(U128) * (size_t)rows, sizeof(U128) * kFusedPrRows, st));
   RG_TRY(timer.mark());
   RG_TRY(deliver<double>(g, A.p, A.ranks_out, h_ranks, nullptr, st));
   RG_CUDA(cudaStreamSynchronize(st));
   RG_TRY(timer.finish());
-  *done = info[3] == 1;
+  *done = info[kDone] == 1 && all_ran();
   if (!*done) return RG_OK;
   const int64_t run = (int64_t)info[0];
   const bool broke = info[4] != 0;
@@ -2295,11 +2316,10 @@ rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max
   A.added = (1 - kPrDamp) * A.one_over_n;
   A.ranks_out = ranks_out;
   A.info = cx.ws.h_info_dev;
-  volatile uint64_t* info = cx.ws.h_info;
-  info[3] = 0;
+  volatile uint64_t* info = info_begin();
   RG_TRY(launch_fused(prd_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
   RG_CUDA(cudaStreamSynchronize(st));
-  *done = info[3] == 1;
+  *done = info[kDone] == 1 && all_ran();
   if (!*done) return RG_OK;
   *rounds = (int64_t)info[0];
   *l1 = double_of(info[1]);

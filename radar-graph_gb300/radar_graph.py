@@ -103,6 +103,7 @@ _SIGS = {
     "rg_last_timing": [_P(Timing)],
     "rg_set_kernel_timing": [C.c_int],
     "rg_set_trace": [C.c_int],
+    "rg_set_wait_polls": [C.c_int64, C.c_int],
     "rg_trace_take": [_P(LevelTrace), C.c_int64, _i64p],
     "rg_device_info": [C.c_char_p, C.c_int, _i32p, _f64p],
     "rg_bfs_depth_noalloc": [C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_uint32, C.c_void_p, C.c_void_p,
@@ -252,6 +253,12 @@ TRACE_MODES = {0: "sparse-push", 1: "dense-push", 2: "pull"}
 def set_trace(on):
     """Record one entry per edgeMap of this thread (rg_set_trace)."""
     _check(lib().rg_set_trace(1 if on else 0))
+
+
+def set_wait_polls(polls, first=0):
+    """Polls after which a wait inside a launch gives up, from its barrier number `first` on
+    (rg_set_wait_polls); negative: the default."""
+    _check(lib().rg_set_wait_polls(int(polls), int(first)))
 
 
 def take_trace(cap=4096):
