@@ -811,8 +811,11 @@ __global__ void sort_init(const uint32_t* __restrict__ off, uint32_t n, uint64_t
   }
 }
 
+// failed: nonzero when the sort gave up, whose output then has holes (nothing is done)
 __global__ void rank_to_ids(const uint64_t* __restrict__ sorted, const uint32_t* __restrict__ off, uint32_t n,
-                            uint32_t* __restrict__ new_ids, uint32_t* __restrict__ new_deg) {
+                            uint32_t* __restrict__ new_ids, uint32_t* __restrict__ new_deg,
+                            const unsigned int* failed) {
+  if (*failed) return;
   int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r < n) {
     const uint32_t v = (uint32_t)sorted[r];
@@ -826,11 +829,14 @@ __global__ void rank_to_ids(const uint64_t* __restrict__ sorted, const uint32_t*
 // partition, and writes new_ids[neighbour] at the source's new position.
 // The neighbour array may be pinned host memory read over the host link
 // (rg_graph_create_sorted); it then has no padding, so the last partial
-// group of four is read entry by entry.
+// group of four is read entry by entry.  failed: as for rank_to_ids (there are no
+// new ids then).
 __global__ void __launch_bounds__(256) relabel_sweep(DevGraph g, const uint32_t* __restrict__ chunk_v,
                                                      uint32_t nchunks, const uint32_t* __restrict__ new_ids,
                                                      const uint32_t* __restrict__ new_off,
-                                                     uint32_t* __restrict__ new_adj, unsigned int* bad_id) {
+                                                     uint32_t* __restrict__ new_adj, unsigned int* bad_id,
+                                                     const unsigned int* failed) {
+  if (*failed) return;
   const int lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -877,7 +883,8 @@ __global__ void __launch_bounds__(256) relabel_sweep(DevGraph g, const uint32_t*
 
 // in-degree of each rank's vertex (a directed graph's new in-lists)
 __global__ void rank_in_deg(const uint64_t* __restrict__ sorted, const uint32_t* __restrict__ in_off, uint32_t n,
-                            uint32_t* __restrict__ new_in_deg) {
+                            uint32_t* __restrict__ new_in_deg, const unsigned int* failed) {
+  if (*failed) return;
   int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r < n) {
     const uint32_t v = (uint32_t)sorted[r];
@@ -900,6 +907,7 @@ static rg_status degree_sort_impl(const rg_graph* g, bool by_out, rg_graph** out
   DevBuf k0{true, st}, k1{true, st}, new_deg{true, st}, bad{true, st};
   RG_TRY(bad.reserve(16));
   RG_CUDA(cudaMemsetAsync(bad.p, 0, 8, st));
+  unsigned int* failed = bad.as<unsigned int>() + 1;
   RG_TRY(k0.reserve(8 * n));
   RG_TRY(k1.reserve(8 * n));
   sort_init<<<(unsigned)((n + 255) / 256), 256, 0, st>>>((by_in ? g->in_off : g->off).as<uint32_t>(), (uint32_t)n,
@@ -915,7 +923,7 @@ static rg_status degree_sort_impl(const rg_graph* g, bool by_out, rg_graph** out
     RG_TRY(sort_begin(sort, n, sort_passes(32, 32 + bits), st));
     RG_TRY(sort_count(sort, order, n, 32, 32 + bits, st));
     RG_TRY(sort_run(sort, &order, &other, n, 32, 32 + bits, st));
-    RG_CUDA(cudaMemcpyAsync(bad.as<unsigned int>() + 1, sort_failed(sort), 4, cudaMemcpyDeviceToDevice, st));
+    RG_CUDA(cudaMemcpyAsync(failed, sort_failed(sort), 4, cudaMemcpyDeviceToDevice, st));
   }
   RG_CUDA(cudaGetLastError());
   rg_graph* ng = nullptr;
@@ -929,7 +937,7 @@ static rg_status degree_sort_impl(const rg_graph* g, bool by_out, rg_graph** out
     return s;
   }
   rank_to_ids<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(order, g->off.as<uint32_t>(), (uint32_t)n,
-                                                          ng->new_ids.as<uint32_t>(), new_deg.as<uint32_t>());
+                                                          ng->new_ids.as<uint32_t>(), new_deg.as<uint32_t>(), failed);
   if ((s = scan_u32(ws, new_deg.as<uint32_t>(), ng->off.as<uint32_t>(), n, st)) != RG_OK) {
     delete ng;
     return s;
@@ -941,7 +949,7 @@ static rg_status degree_sort_impl(const rg_graph* g, bool by_out, rg_graph** out
       return s;
     }
     rank_in_deg<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(order, g->in_off.as<uint32_t>(), (uint32_t)n,
-                                                            new_deg.as<uint32_t>());
+                                                            new_deg.as<uint32_t>(), failed);
     if ((s = scan_u32(ws, new_deg.as<uint32_t>(), ng->in_off.as<uint32_t>(), n, st)) != RG_OK) {
       delete ng;
       return s;
@@ -953,11 +961,11 @@ static rg_status degree_sort_impl(const rg_graph* g, bool by_out, rg_graph** out
     const int64_t blocks = std::min<int64_t>((g->nchunks * 32 + 255) / 256, (int64_t)std::max(sms, 1) * 8);
     relabel_sweep<<<(unsigned)blocks, 256, 0, st>>>(g->view(), g->chunk_v.as<uint32_t>(), (uint32_t)g->nchunks,
                                                     ng->new_ids.as<uint32_t>(), ng->off.as<uint32_t>(),
-                                                    ng->adj.as<uint32_t>(), bad.as<unsigned int>());
+                                                    ng->adj.as<uint32_t>(), bad.as<unsigned int>(), failed);
     if (g->directed) {
       relabel_sweep<<<(unsigned)blocks, 256, 0, st>>>(g->in_view(), g->in_chunks(), (uint32_t)g->nchunks,
                                                       ng->new_ids.as<uint32_t>(), ng->in_off.as<uint32_t>(),
-                                                      ng->in_adj.as<uint32_t>(), bad.as<unsigned int>());
+                                                      ng->in_adj.as<uint32_t>(), bad.as<unsigned int>(), failed);
     }
   }
   cudaError_t e = cudaMemsetAsync(ng->adj.as<uint32_t>() + m, 0, 32, st);
@@ -1159,15 +1167,17 @@ enum CsrPart { kAlone, kUpper, kLower, kPlace };
 struct CsrOut {
   uint32_t* off;          // kAlone, kUpper, kLower: the rows' offsets, n + 1
   uint32_t* adj;          // not kUpper
-  uint32_t m;             // entries of adj
   const uint32_t* other;  // kLower: the offsets of kUpper; kPlace: those of kLower
   uint64_t* back;         // kUpper: value << bits | row
+  const uint32_t* failed;  // kLower, kPlace: the second sort's flag, which the host has not seen yet (its output,
+                           // and the offsets made of it, are no indices then)
 };
 
 template <bool kClean, CsrPart kPart>
 __global__ void __launch_bounds__(kCsrThreads) csr_emit(const uint64_t* __restrict__ key, int64_t k, int bits,
                                                         const uint32_t* __restrict__ tile_first, uint32_t n,
                                                         CsrOut out) {
+  if ((kPart == kLower || kPart == kPlace) && *out.failed) return;
   // a warp's sub-tile of kCsrItems x 32 entries, 32 at a time: writes stay coalesced
   __shared__ uint32_t wsum[kCsrThreads / 32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1217,11 +1227,7 @@ __global__ void __launch_bounds__(kCsrThreads) csr_emit(const uint64_t* __restri
       const uint32_t row = (uint32_t)(x[s] >> bits), value = (uint32_t)(x[s] & mask);
       if (keep) {
         if (kPart == kAlone) out.adj[pos] = value;
-        if (kPart == kLower || kPart == kPlace) {
-          // (out of range only when a wait of the second sort gave up)
-          const uint32_t to = row < n ? pos + out.other[row + (kPart == kPlace)] : out.m;
-          if (to < out.m) out.adj[to] = value;
-        }
+        if (kPart == kLower || kPart == kPlace) out.adj[pos + out.other[row + (kPart == kPlace)]] = value;
         if (kPart == kUpper) out.back[pos] = ((uint64_t)value << bits) | row;
       }
       if (kPart == kPlace) continue;
@@ -1305,7 +1311,7 @@ static rg_status csr_from_sorted(Workspace& ws, const uint64_t* key, int64_t k, 
   RG_TRY(csr_kept<kClean>(ws, key, k, bits, n, first, m_out, nullptr, failed, max_id, who, st));
   RG_TRY(off.reserve(4 * (size_t)(n + 1)));
   RG_TRY(adj.reserve(4 * (size_t)(*m_out + 8)));
-  const CsrOut out{off.as<uint32_t>(), adj.as<uint32_t>(), (uint32_t)*m_out, nullptr, nullptr};
+  const CsrOut out{off.as<uint32_t>(), adj.as<uint32_t>(), nullptr, nullptr, nullptr};
   RG_TRY((csr_emit_run<kClean, kAlone>(key, k, bits, first.as<uint32_t>(), n, out, st)));
   RG_CUDA(cudaMemsetAsync(adj.as<uint32_t>() + *m_out, 0, 32, st));
   return RG_OK;
@@ -1336,16 +1342,15 @@ static rg_status csr_from_edges_sorted(Workspace& ws, const uint64_t* key, uint6
   RG_TRY(upper.reserve(4 * (size_t)(n + 1)));
   RG_TRY(lower.reserve(4 * (size_t)(n + 1)));
   RG_TRY(back.reserve(8 * (size_t)std::max<int64_t>(kept, 1)));
-  const uint32_t m = (uint32_t)*m_out;
-  CsrOut out{upper.as<uint32_t>(), nullptr, m, nullptr, back.as<uint64_t>()};
+  CsrOut out{upper.as<uint32_t>(), nullptr, nullptr, back.as<uint64_t>(), nullptr};
   RG_TRY((csr_emit_run<true, kUpper>(key, k, bits, first.as<uint32_t>(), n, out, st)));
   uint32_t gave_up = 0;
   if (kept > 0) {
     uint64_t *a = back.as<uint64_t>(), *b = other;
     RG_TRY(sort_run(sort, &a, &b, kept, bits, 2 * bits, st));
-    out = CsrOut{lower.as<uint32_t>(), adj.as<uint32_t>(), m, upper.as<uint32_t>(), nullptr};
+    out = CsrOut{lower.as<uint32_t>(), adj.as<uint32_t>(), upper.as<uint32_t>(), nullptr, sort_failed(sort)};
     RG_TRY((csr_emit_run<false, kLower>(a, kept, bits, nullptr, n, out, st)));
-    out = CsrOut{nullptr, adj.as<uint32_t>(), m, lower.as<uint32_t>(), nullptr};
+    out = CsrOut{nullptr, adj.as<uint32_t>(), lower.as<uint32_t>(), nullptr, sort_failed(sort)};
     RG_TRY((csr_emit_run<true, kPlace>(key, k, bits, first.as<uint32_t>(), n, out, st)));
   } else {
     RG_CUDA(cudaMemsetAsync(lower.p, 0, 4 * (size_t)(n + 1), st));

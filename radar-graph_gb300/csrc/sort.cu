@@ -30,7 +30,7 @@ constexpr int kTile = kThreads * kItems;  // 48 KiB of keys: three CTAs per SM
 constexpr int kMatchOf = 3;  // one item in this many finds its equals by a match, the others by votes
 constexpr unsigned kAll = 0xffffffffu;
 constexpr int kBack = 4;  // earlier tiles looked at together
-constexpr unsigned kSpinLimit = 1u << 20;
+constexpr unsigned kPolls = 1u << 20;  // of the look-back before it gives up
 constexpr size_t kHead = 64;  // words of hist before the counts: tickets (0..7) and the failure flag (8)
 
 // base[p][d] = keys of pass p with a digit below d (in place of the counts)
@@ -89,7 +89,7 @@ template <int kBits, bool kFull>
 __device__ __forceinline__ void sort_tile(const uint64_t* __restrict__ in, uint64_t* __restrict__ out, int64_t k,
                                           int here, int shift, uint32_t digits, uint32_t pass,
                                           const uint32_t* __restrict__ base, uint64_t* status, uint32_t* head, Tile& T,
-                                          uint64_t* keys) {
+                                          uint64_t* keys, unsigned polls) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int j0 = w * 32 * kItems + lane;
   const unsigned lt = (1u << lane) - 1u;
@@ -178,7 +178,7 @@ __device__ __forceinline__ void sort_tile(const uint64_t* __restrict__ in, uint6
           t--;
         }
       }
-      if (!whole && ++spins > kSpinLimit) {
+      if (!whole && ++spins > polls) {
         atomicExch(head + 8, 1u);
         break;
       }
@@ -205,7 +205,7 @@ template <int kBits>
 __global__ void __launch_bounds__(kThreads, 3) sort_sweep(const uint64_t* __restrict__ in, uint64_t* __restrict__ out,
                                                           int64_t k, int shift, uint32_t digits, uint32_t pass,
                                                           const uint32_t* __restrict__ base, uint64_t* status,
-                                                          uint32_t* head) {
+                                                          uint32_t* head, unsigned polls) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint64_t* keys = reinterpret_cast<uint64_t*>(smem_raw);
   __shared__ Tile T;
@@ -214,8 +214,8 @@ __global__ void __launch_bounds__(kThreads, 3) sort_sweep(const uint64_t* __rest
   __syncthreads();
   const int64_t t0 = (int64_t)T.tile * kTile;
   const int here = (int)min((int64_t)kTile, k - t0);
-  if (here == kTile) sort_tile<kBits, true>(in + t0, out, k, here, shift, digits, pass, base, status, head, T, keys);
-  else sort_tile<kBits, false>(in + t0, out, k, here, shift, digits, pass, base, status, head, T, keys);
+  if (here == kTile) sort_tile<kBits, true>(in + t0, out, k, here, shift, digits, pass, base, status, head, T, keys, polls);
+  else sort_tile<kBits, false>(in + t0, out, k, here, shift, digits, pass, base, status, head, T, keys, polls);
 }
 
 }  // namespace
@@ -250,7 +250,7 @@ rg_status sort_passes_of(SortScratch& s, uint64_t** keys, uint64_t** other, int6
     const uint32_t digits = (1u << std::min(width, hi - shift)) - 1u;
     sort_sweep<kBits><<<(unsigned)tiles, kThreads, kTile * sizeof(uint64_t), st>>>(
         *keys, *other, k, shift, digits, (uint32_t)p, sort_counts(s) + 256 * p, s.status.as<uint64_t>(),
-        s.hist.as<uint32_t>());
+        s.hist.as<uint32_t>(), g_wait_polls >= 0 ? (unsigned)g_wait_polls : kPolls);
     std::swap(*keys, *other);
   }
   RG_CUDA(cudaGetLastError());

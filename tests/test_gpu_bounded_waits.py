@@ -1,7 +1,7 @@
 """Waits inside a launch that run out (rg_set_wait_polls makes them short): whatever
 barrier the CTAs give up at, the last one included, the call's results are those of
 an undisturbed one, and so are the next call's.  Integers and exact sums are equal,
-BC and PageRankDelta 1e-9 relative."""
+BC and PageRankDelta 1e-9 relative.  A sort that gives up is an error of its call."""
 
 import numpy as np
 import pytest
@@ -80,3 +80,41 @@ def test_a_launch_that_gives_up(graphs, polls, kind, app):
     polls(-1)
     check(app, call(), want)
     assert rg.last_timing()["kernel_launches"] <= 3
+
+
+def built_lists(g):
+    return [x for x in g.download() if x is not None]
+
+
+@pytest.mark.parametrize("build", ["edges", "edges-halves", "edges-directed", "sort", "sort-directed", "triangles"])
+def test_a_sort_that_gives_up(polls, build):
+    """The call fails, or is right where no wait was needed; nothing is indexed with
+    what the sort left behind, and the next call is right."""
+    r = np.random.default_rng(4)
+    n, ne = (300000, 13 << 20) if build == "edges-halves" else (90001, 400000)
+    s, d = (r.integers(0, n, ne).astype(np.uint32) for _ in range(2))
+    directed = build.endswith("directed")
+    if build.startswith("edges"):
+        call, lists = lambda: rg.Graph.from_edges(n, s, d, directed=directed), built_lists
+    else:
+        g = rg.Graph.from_edges(n, s, d, directed=directed)
+        if build == "triangles":
+            g = g.degree_sort()
+            call, lists = g.triangles, lambda x: [x[0]]
+        else:
+            call, lists = g.degree_sort, built_lists
+    want = lists(call())
+    failed = 0
+    for limit in [0, 0, 1, 2, 4, 8, 16]:
+        polls(limit)
+        try:
+            got = call()
+        except rg.RgError as e:
+            failed += 1
+            assert "did not finish" in str(e)
+            got = None
+        polls(-1)
+        if got is not None:
+            assert all(np.array_equal(a, b) for a, b in zip(lists(got), want))
+    assert failed
+    assert all(np.array_equal(a, b) for a, b in zip(lists(call()), want))
