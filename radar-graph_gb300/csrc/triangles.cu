@@ -13,7 +13,8 @@
 //
 // The lower lists come from one stable sort: walking the rows v in order and
 // keeping the neighbours u > v yields the pairs (u, v) ordered by v, so sorting
-// them by u alone leaves every list ascending.
+// them by u alone leaves every list ascending.  That holds for a cleaned symmetric
+// graph; one with repeats, or with edges in one direction alone, is cleaned first.
 
 #include <cuda_runtime.h>
 
@@ -28,20 +29,32 @@ namespace {
 
 constexpr unsigned kAll = 0xffffffffu;
 
+// An edge's share of a sum that is 0 over both directions of every edge (and, but for
+// chance in 2^64, over nothing else that is not balanced): negative from the lower id.
+__device__ __forceinline__ unsigned long long edge_share(uint32_t u, uint32_t v) {
+  unsigned long long x = ((unsigned long long)max(u, v) << 32 | min(u, v)) * 0x9E3779B97F4A7C15ull;
+  x = (x ^ (x >> 29)) * 0xD6E8FEB86659FD93ull;
+  x ^= x >> 32;
+  return u > v ? x : u < v ? 0ull - x : 0ull;
+}
+
 // The pairs (u, v), u > v, of a symmetric graph, ordered by v: counted per
-// kSweepChunk edges (a warp each; rows from the chunk starts), then written as
-// u << bits | v at the chunk's place with the digit counts of the sort by u.
+// kSweepChunk edges (a warp each; rows from the chunk starts) with the sum of the
+// edges' shares (balance), then written as u << bits | v at the chunk's place with the
+// digit counts of the sort by u.
 // Bound by the row searches' latency: four edges per lane share one (7.3e6 entries:
 // 42 and 47 us with a search each, 19 and 30 now).
 template <bool kEmit>
 __global__ void __launch_bounds__(256) upper_pairs(DevGraph g, const uint32_t* __restrict__ chunk_v, uint32_t nchunks,
                                                    uint32_t* __restrict__ count, const uint32_t* __restrict__ place,
-                                                   int bits, uint64_t* __restrict__ key, int passes, uint32_t* hist) {
+                                                   int bits, uint64_t* __restrict__ key, int passes, uint32_t* hist,
+                                                   unsigned long long* balance) {
   __shared__ uint32_t sh[kEmit ? kMaxSortPasses * 256 : 1];
   if (kEmit) sort_zero(sh, passes);
   const int lane = threadIdx.x & 31;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+  unsigned long long sum = 0;
   for (uint32_t c = warp; c < nchunks; c += nwarps) {
     const uint32_t vlo = chunk_v[c], vhi = chunk_v[c + 1];
     uint32_t n = 0, at = kEmit ? place[c] : 0;
@@ -57,8 +70,9 @@ __global__ void __launch_bounds__(256) upper_pairs(DevGraph g, const uint32_t* _
         for (int k = 0; k < 4; k++) {
           while (e + k < g.m && e + k >= next) next = g.off[++row + 1];
           v[k] = row;
-          if (e + k >= g.m) u[k] = 0;
+          if (e + k >= g.m) u[k] = v[k];
           own += u[k] > v[k];
+          if (!kEmit) sum += edge_share(u[k], v[k]);
         }
       }
       if (!kEmit) {
@@ -86,7 +100,12 @@ __global__ void __launch_bounds__(256) upper_pairs(DevGraph g, const uint32_t* _
       if (lane == 0) count[c] = n;
     }
   }
-  if (kEmit) sort_flush(sh, hist, passes);
+  if (kEmit) {
+    sort_flush(sh, hist, passes);
+  } else {
+    sum = warp_sum(sum);
+    if (lane == 0 && sum) atomicAdd(balance, sum);
+  }
 }
 
 constexpr int kTcThreads = 512;
@@ -257,8 +276,30 @@ struct TcState {
   DevBuf tri, total, out;
 };
 
-// Lower lists of the degree-ordered graph rs, and their members' count.
-rg_status lower_lists(rg_graph* rs, DevBuf& off, DevBuf& adj, int64_t* entries, cudaStream_t st) {
+// The entries of a graph, one by one.
+__global__ void __launch_bounds__(256) entry_ends(DevGraph g, const uint32_t* __restrict__ chunk_v, uint32_t* src,
+                                                  uint32_t* dst) {
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < g.m; e += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t c = (uint32_t)(e / kSweepChunk);
+    src[e] = upper_index(g.off, chunk_v[c], chunk_v[c + 1], (uint32_t)e);
+    dst[e] = g.adj[e];
+  }
+}
+
+// The graph with both directions of every edge of g, each once.
+rg_status cleaned(rg_graph* g, rg_graph** out, cudaStream_t st) {
+  DevBuf ends(true, st);
+  RG_TRY(ends.reserve(8 * (size_t)g->m));
+  uint32_t *src = ends.as<uint32_t>(), *dst = src + g->m;
+  entry_ends<<<(unsigned)(device_sms() * 16), 256, 0, st>>>(g->view(), g->chunk_v.as<uint32_t>(), src, dst);
+  RG_CUDA(cudaGetLastError());
+  return rg_graph_create_from_edges(g->n, g->m, src, dst, 1, out);
+}
+
+// Lower lists of the degree-ordered graph rs, and their members' count.  *clean:
+// whether every edge of rs is there once in either direction (else the lists are not
+// rs's).
+rg_status lower_lists(rg_graph* rs, DevBuf& off, DevBuf& adj, int64_t* entries, bool* clean, cudaStream_t st) {
   const int64_t n = rs->n;
   const uint32_t nchunks = (uint32_t)rs->nchunks;
   int bits = 1;
@@ -266,29 +307,35 @@ rg_status lower_lists(rg_graph* rs, DevBuf& off, DevBuf& adj, int64_t* entries, 
   const int passes = sort_passes(bits, 2 * bits);
   DevBuf place(true, st), k0(true, st), k1(true, st);
   SortScratch sort(st);
-  RG_TRY(place.reserve(4 * ((size_t)nchunks + 1)));
+  const uint32_t sum_at = (nchunks + 2) & ~1u;  // the balance, behind the scan's total
+  RG_TRY(place.reserve(4 * ((size_t)sum_at + 2)));
   uint32_t* pl = place.as<uint32_t>();
+  RG_CUDA(cudaMemsetAsync(pl + sum_at, 0, 8, st));
   const unsigned blocks =
       (unsigned)std::max<int64_t>(1, std::min<int64_t>((rs->nchunks * 32 + 255) / 256, (int64_t)device_sms() * 8));
   upper_pairs<false><<<blocks, 256, 0, st>>>(rs->view(), rs->chunk_v.as<uint32_t>(), nchunks, pl, nullptr, bits,
-                                             nullptr, passes, nullptr);
+                                             nullptr, passes, nullptr,
+                                             reinterpret_cast<unsigned long long*>(pl + sum_at));
   RG_CUDA(cudaGetLastError());
   RG_TRY(scan_u32(ctx().ws, pl, pl, nchunks, st));
-  uint32_t k = 0;
-  RG_TRY(read_small(pl + nchunks, &k, 4, st));
+  uint32_t read[4];  // the total, the balance in the last two
+  RG_TRY(read_small(pl + nchunks, read, 4 * (sum_at + 2 - nchunks), st));
+  const uint32_t k = read[0];
   *entries = k;
-  if (k == 0) return RG_OK;
+  *clean = (read[sum_at - nchunks] | read[sum_at + 1 - nchunks]) == 0;
+  if (k == 0 || !*clean) return RG_OK;
   RG_TRY(k0.reserve(8 * (size_t)k));
   RG_TRY(k1.reserve(8 * (size_t)k));
   RG_TRY(sort_begin(sort, k, passes, st));
   upper_pairs<true><<<blocks, 256, 0, st>>>(rs->view(), rs->chunk_v.as<uint32_t>(), nchunks, nullptr, pl, bits,
-                                            k0.as<uint64_t>(), passes, sort_counts(sort));
+                                            k0.as<uint64_t>(), passes, sort_counts(sort), nullptr);
   RG_CUDA(cudaGetLastError());
   uint64_t *key = k0.as<uint64_t>(), *other = k1.as<uint64_t>();
   RG_TRY(sort_run(sort, &key, &other, k, bits, 2 * bits, st));
   g_timing.kernel_launches += 3 + passes;
-  // (repeats are dropped, as the loaders drop them)
-  return csr_from_sorted_rows(ctx().ws, key, k, bits, n, true, off, adj, entries, sort, "lower lists", st);
+  RG_TRY(csr_from_sorted_rows(ctx().ws, key, k, bits, n, true, off, adj, entries, sort, "lower lists", st));
+  *clean = *entries == k;
+  return RG_OK;
 }
 
 }  // namespace
@@ -315,19 +362,26 @@ rg_status triangle_run(rg_graph* g, uint64_t* h_counts, uint64_t* total_out) {
     rs = tmp;
   }
   uint64_t t = 0;
+  rg_graph* gt = nullptr;  // rs cleaned, where it needs that
   auto count = [&]() -> rg_status {
     RG_CUDA(cudaMemsetAsync(tri, 0, 8 * n, st));
     RG_CUDA(cudaMemsetAsync(total, 0, 16, st));
     DevBuf off(true, st), adj(true, st);
     int64_t k = 0;
-    if (m > 0) RG_TRY(lower_lists(rs, off, adj, &k, st));
+    bool clean = true;
+    if (m > 0) RG_TRY(lower_lists(rs, off, adj, &k, &clean, st));
+    if (!clean) {
+      RG_TRY(cleaned(rs, &gt, st));
+      RG_TRY(lower_lists(gt, off, adj, &k, &clean, st));
+    }
+    rg_graph* const lists = gt ? gt : rs;
     if (k > 0) {
       static std::atomic<uint64_t> limit_set{0};
       RG_TRY(allow_max_dyn_smem(limit_set, count_triangles));
-      const int64_t grid = std::min<int64_t>((m + 32 * kTcWarps - 1) / (32 * kTcWarps), (int64_t)device_sms() * 4);
+      const int64_t grid = std::min<int64_t>((lists->m + 32 * kTcWarps - 1) / (32 * kTcWarps), (int64_t)device_sms() * 4);
       kt_begin(st);
       count_triangles<<<(unsigned)grid, kTcThreads, sizeof(TcShared), st>>>(
-          rs->view(), rs->chunk_v.as<uint32_t>(), off.as<uint32_t>(), adj.as<uint32_t>(),
+          lists->view(), lists->chunk_v.as<uint32_t>(), off.as<uint32_t>(), adj.as<uint32_t>(),
           (unsigned int*)(total + 1), tri, total);
       kt_end(st);
       RG_CUDA(cudaGetLastError());
@@ -344,6 +398,7 @@ rg_status triangle_run(rg_graph* g, uint64_t* h_counts, uint64_t* total_out) {
     return read_small(total, &t, 8, st);
   };
   const rg_status s = count();
+  if (gt) rg_graph_free(gt);
   if (tmp) rg_graph_free(tmp);
   RG_TRY(s);
   RG_TRY(timer.stop());

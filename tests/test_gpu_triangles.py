@@ -93,3 +93,33 @@ def test_cli_reads_gap_edge_lists(tmp_path, fmt):
     r = subprocess.run([exe, "-s", "-rounds", "0", path], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
     assert f"{want} triangles" in r.stdout
+
+
+@pytest.mark.parametrize("sorted_handle", [False, True])
+@pytest.mark.parametrize("kind", ["repeats", "repeats one way", "one way", "loops", "shuffled"])
+def test_graphs_that_need_cleaning(kind, sorted_handle):
+    """rg_graph_create takes any CSR: repeated entries, edges listed in one direction
+    alone, self loops and unsorted rows count as in the cleaned graph."""
+    off, adj = rg.rmat_csr(11, 12, seed=6)
+    want, wt = orc.triangles(off, adj, 0)
+    n = len(off) - 1
+    src, dst = np.repeat(np.arange(n, dtype=np.uint32), np.diff(off.astype(np.int64))), adj
+    r = np.random.default_rng(2)
+    pick = r.random(len(src)) < 0.2
+    if kind == "repeats":
+        src, dst = np.concatenate([src, src[pick], dst[pick]]), np.concatenate([dst, dst[pick], src[pick]])
+    elif kind == "repeats one way":
+        src, dst = np.concatenate([src, src[pick]]), np.concatenate([dst, dst[pick]])
+    elif kind == "one way":
+        keep = ~(pick & (src < dst))
+        src, dst = src[keep], dst[keep]
+    elif kind == "loops":
+        loops = np.arange(0, n, 3, dtype=np.uint32)
+        src, dst = np.concatenate([src, loops]), np.concatenate([dst, loops])
+    order = np.lexsort((r.random(len(src)) if kind == "shuffled" else dst, src))
+    src, dst = src[order], dst[order]
+    off = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.uint32)
+    with rg.Graph.from_csr(off, dst) as g, g.degree_sort() as s:
+        counts, total = (s if sorted_handle else g).triangles()
+    assert total == wt
+    assert np.array_equal(counts, want)
