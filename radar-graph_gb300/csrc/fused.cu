@@ -1974,7 +1974,7 @@ rg_status deliver(rg_graph* g, const T* internal, const T* ordered, T* host_out,
 }  // namespace
 
 bool fused_fits(const rg_graph* g, int64_t max_edges) {
-  return g->m <= max_edges && g->n <= max_edges && !g_trace_on;
+  return g->m <= max_edges && g->n <= max_edges && strides_fit(g->n, g->m) && !g_trace_on;
 }
 
 rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t* h_depth,

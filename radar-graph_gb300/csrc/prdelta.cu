@@ -225,7 +225,7 @@ rg_status pagerank_delta_run(rg_graph* g, int variant, int64_t max_iters, double
       return launch_following(filter, vblocks, 256, 0, st, (uint32_t)n, g->off.as<uint32_t>(), g->in_view().off, p, ngh,
                               acc, c, rmag, one_over_n, added, cur.bits, nxt.bits, gate, t);
     };
-    bool hand_over = !g_trace_on;  // sparse rounds go to one launch (once)
+    bool hand_over = !g_trace_on && strides_fit(n, g->m);  // sparse rounds go to one launch (once)
     while (round++ < max_iters) {
       const bool dense = cur.count + cur.degsum > threshold;
       if (!dense && round > 1 && hand_over) {

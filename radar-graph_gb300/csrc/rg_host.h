@@ -23,6 +23,12 @@ rg_status read_edges(const char* path, int64_t* n_out, int64_t* ne_out, uint32_t
 rg_status read_graph(const char* path, int symmetric, int binary, int64_t* n_out, int64_t* m_out,
                      uint32_t** off_out, uint32_t** adj_out);
 
+// Ids and edge places are 32-bit words, and a loop over them steps by up to all the
+// threads of a launch (fewer than 2^20): above this, a step past the end would wrap
+// around to the beginning.
+constexpr int64_t kMostStrided = 0xFFFFFFFFll - (1 << 20);
+inline bool strides_fit(int64_t n, int64_t m) { return n <= kMostStrided && m <= kMostStrided; }
+
 // Ligra's 64-bit hashInt (utils.h:350-358), a published integer mix whose
 // constants decide which vertices Radii samples, so they must be the same.
 inline uint64_t hash_u64(uint64_t a) {
