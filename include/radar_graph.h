@@ -250,10 +250,11 @@ rg_status rg_bfs_multi(rg_graph* g, const uint32_t* h_sources, int k, int32_t* h
  * h_deps: k*n doubles, row q equal to rg_bc_sources(g, variant, &sources[q], 1,
  * row) for every variant (the single-source pass of
  * BC-manyiter-v2.C:180-232) up to summation order; NaN where sources[q] does not
- * reach the vertex.  Small and mid-sized graphs run the sources side by side, each
- * with the arithmetic of rg_bc_sources (double path counts, exact below 2^53);
- * larger ones share a traversal: the sources' levels from one 64-wide bitmask BFS,
- * then path counts (exact 64-bit integers) and dependencies for all sources per
+ * reach the vertex.  Path counts below 2^64 are exact.  Small and mid-sized graphs
+ * run the sources side by side, each with the arithmetic of rg_bc_sources (double
+ * path counts, exact below 2^53); larger ones, and those whose counts lie between
+ * 2^53 and 2^64, share a traversal: the sources' levels from one 64-wide bitmask
+ * BFS, then path counts (64-bit integers) and dependencies for all sources per
  * level, one row of k values per vertex, and one single-source pass per source
  * where path counts pass 2^64. */
 rg_status rg_bc_multi(rg_graph* g, const uint32_t* h_sources, int k, double* h_deps,

@@ -612,8 +612,12 @@ struct BcArgs : Launch {
   uint4* heavy;                         // a pulled level's pieces of long lists
   size_t n_small, n_large, n_heavy;     // a group's share of the queues
   bool first_source;
-  volatile uint64_t* info;  // mapped, four words per source (or summed over the calls): levels, edges, -, done
+  volatile uint64_t* info;  // mapped, four words per source (or summed over the calls): levels, edges, counts (rows), done
 };
+
+// Path counts are integers: doubles hold them below the first of these, 64-bit
+// integers below the second.
+constexpr double kExactCounts = 0x1p53, kIntegerCounts = 0x1p64;
 
 constexpr uint32_t kLaneList = 16;    // a pull reads lists up to this with one lane,
 constexpr uint32_t kLongList = 1024;  // up to this with the warp, and longer ones in pieces
@@ -960,10 +964,16 @@ __device__ bool bc_backward(const BcArgs& A, int s, bool last, Grid& grid, uint3
   // id for the caller (page-locked results: behind the host link)
   double* out = A.deps_out && last ? A.deps_out + (A.rows ? (size_t)s * n : 0) : nullptr;
   double* to = out ? out : A.deps;
+  unsigned long long most = 0;  // the largest path count's bits
   for (uint32_t i = tid; i < n; i += nthreads) {
     const uint32_t v = out && A.new_ids ? A.new_ids[i] : i;
     const double d = A.even[v] + A.odd[v];  // one of them is 0; both: not reached
-    to[i] = d != 0.0 ? (d - A.inv[v]) * A.sigma[v] : CUDART_NAN;
+    const double count = A.sigma[v];
+    to[i] = d != 0.0 ? (d - A.inv[v]) * count : CUDART_NAN;
+    most = max(most, bits_of(count));
+  }
+  if (A.rows && most >= bits_of(kExactCounts)) {
+    reinterpret_cast<volatile unsigned char*>(A.info + 4 * s + 2)[most >= bits_of(kIntegerCounts)] = 1;
   }
   if (tid == 0) {
     volatile uint64_t* f = A.info + (A.rows ? 4 * s : 0);
@@ -2129,11 +2139,19 @@ rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double
   RG_CUDA(cudaStreamSynchronize(st));
   if (!all_ran()) return RG_OK;
   int64_t levels = 0;
+  bool rounded = false, past_integers = false;
   for (int q = 0; q < k; q++) {
     if (info[4 * q + kDone] != 1) return RG_OK;
+    const uint64_t counts = info[4 * q + 2];
+    const unsigned char* c = reinterpret_cast<const unsigned char*>(&counts);
+    rounded |= c[0] != 0;
+    past_integers |= c[1] != 0;
     levels = std::max(levels, (int64_t)info[4 * q]);
     g_timing.edges_traversed += (int64_t)info[4 * q + 1];
   }
+  // Counts that doubles round and 64-bit integers would not: the shared traversal
+  // sums those.  (Past its integers it would answer with doubles itself.)
+  if (rounded && !past_integers) return RG_OK;
   *done = true;
   *levels_out = levels;
   return RG_OK;

@@ -4,6 +4,8 @@ BC-manyiter-v2 output), within 1e-9 relative and with identical NaN
 positions, on symmetric and directed, unsorted and degree-sorted graphs, for
 1..64 sources including repeats and isolated vertices."""
 
+from fractions import Fraction
+
 import numpy as np
 import pytest
 
@@ -147,3 +149,39 @@ def test_no_edges(n):
             want = np.full(n, np.nan)
             want[s] = 0.0
             assert_close(rows[q], want, what=f"isolated source {s}")
+
+
+def _fibonacci(layers):
+    """Two vertices a layer; the first of the next has both as predecessors, the
+    second the first alone: path counts are the Fibonacci numbers."""
+    i = np.arange(layers - 1, dtype=np.uint32)
+    a, b = 1 + 2 * i, 2 + 2 * i
+    src, dst = np.concatenate([[0, 0], a, b, a]), np.concatenate([[1, 2], a + 2, a + 2, b + 2])
+    return rg.csr_from_edges(2 * layers + 1, src.astype(np.uint32), dst.astype(np.uint32))
+
+
+@pytest.mark.parametrize("layers,shared", [(70, False), (77, False), (78, True), (88, True), (93, False), (120, False)])
+def test_counts_that_doubles_would_round(layers, shared):
+    """The largest count lies below 2^53, where doubles are exact, between that and 2^64,
+    where the shared traversal's integers are and the one launch is not taken, or above."""
+    off, adj = _fibonacci(layers)
+    fib = [1, 1]
+    while len(fib) <= layers:
+        fib.append(fib[-1] + fib[-2])
+    assert (2 ** 53 <= fib[layers] < 2 ** 64) == shared
+    with rg.Graph.from_csr(off, adj) as G:
+        rows, _ = G.bc_multi(np.array([0, 1], np.uint32))
+        assert (rg.last_timing()["kernel_launches"] > 1) == shared
+        _check_rows(G, np.array([0, 1], np.uint32), f"fibonacci {layers}")
+    # exact dependencies of the source's pass, in rationals
+    n = len(off) - 1
+    level = np.concatenate([[0], 1 + np.arange(n - 1) // 2])
+    sigma, dep = [0] * n, [Fraction(0)] * n
+    sigma[0] = 1
+    for v in range(1, n):
+        sigma[v] = sum(sigma[u] for u in adj[off[v]:off[v + 1]] if level[u] < level[v])
+    for v in range(n - 1, -1, -1):
+        for u in adj[off[v]:off[v + 1]]:
+            if level[u] < level[v]:
+                dep[u] += Fraction(sigma[u], sigma[v]) * (1 + dep[v])
+    assert_close(rows[0], np.array([float(x) for x in dep]), what="exact")
