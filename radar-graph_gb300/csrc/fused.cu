@@ -128,7 +128,7 @@ struct Team {
 // the barrier's verdict.
 struct Shared {
   Team team[2];  // the group's CTAs, and all of them (BC)
-  unsigned polls, from, met;   // (met: barriers so far)
+  unsigned polls, from;
   volatile uint64_t* gave_up;
   unsigned int count;
   unsigned long long degsum;
@@ -148,6 +148,19 @@ __device__ __forceinline__ Slot read_slot(const Slot* s) {
   return r;
 }
 
+// The barrier's wait, after a first look.  0: it ran out.  (Out of line: what it needs
+// of shared memory is read beside the polls, off the path of a wait that ends.)
+__device__ __noinline__ int poll(Shared* sh, const Team& t) {
+  unsigned left = t.target / t.ctas > sh->from ? sh->polls : kPolls;
+  do {
+    if (left-- == 0) {
+      *sh->gave_up = 1;
+      return 0;
+    }
+  } while ((int)(ld_acquire(t.bar) - t.target) < 0);
+  return 1;
+}
+
 struct Grid {
   Shared* sh;
   int which;
@@ -161,31 +174,21 @@ struct Grid {
     __syncthreads();
     if (threadIdx.x == 0) {
       Team& t = sh->team[which];
-      t.target += t.ctas;
       if (slot && sh->count) {
         atomicAdd(&slot->count, sh->count);
         atomicAdd(&slot->degsum, sh->degsum);
       }
+      const bool others = t.ctas > 1;
+      if (others) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.bar) : "memory");
+      else __threadfence();
+      t.target += t.ctas;
       if (!keep) {
         sh->count = 0;
         sh->degsum = 0;
       }
-      int ok = 1;
-      if (t.ctas > 1) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(t.bar) : "memory");
-        const unsigned polls = sh->met++ < sh->from ? kPolls : sh->polls;
-        unsigned spins = 0;
-        while ((int)(ld_acquire(t.bar) - t.target) < 0) {
-          if (++spins > polls) {
-            *sh->gave_up = 1;
-            ok = 0;
-            break;
-          }
-        }
-      } else {
-        __threadfence();
-      }
       sh->taken = 0;
+      int ok = 1;
+      if (others && (int)(ld_acquire(t.bar) - t.target) < 0) ok = poll(sh, t);
       if (l1) sh->l1 = l1->read();
       if (slot) sh->slot = read_slot(slot);  // once per CTA: thousands of warps would queue on its line
       sh->ok = ok;
@@ -359,7 +362,6 @@ __device__ __forceinline__ void begin(Grid& grid, Shared* sh, const Launch& L, C
     sh->team[0] = Team{&ctl->bar, 0, gridDim.x};
     sh->polls = L.polls;
     sh->from = L.from;
-    sh->met = 0;
     sh->gave_up = L.gave_up;
     sh->count = 0;
     sh->degsum = 0;
