@@ -46,9 +46,9 @@ constexpr unsigned kAll = 0xffffffffu;
 constexpr unsigned kPolls = 1u << 21;  // of the grid barrier: a second or two
 
 // One level's frontier: queue lengths, members and their degree sum
-// (PageRankDelta: and the round's L1; BC: the pieces of long lists that a pull
-// puts off).
-struct Slot {
+// (PageRankDelta: and the round's L1; BFS and BC: the pieces of long lists that a
+// pull puts off).
+struct alignas(16) Slot {
   unsigned int ns, nl, count, heavy;
   unsigned long long degsum;
   double l1;
@@ -139,13 +139,9 @@ struct Shared {
 };
 
 __device__ __forceinline__ Slot read_slot(const Slot* s) {
-  Slot r;
-  r.ns = __ldcg(&s->ns);
-  r.nl = __ldcg(&s->nl);
-  r.count = __ldcg(&s->count);
-  r.degsum = __ldcg(&s->degsum);
-  r.l1 = __ldcg(&s->l1);
-  return r;
+  const uint4 a = __ldcg(reinterpret_cast<const uint4*>(s));
+  const ulonglong2 b = __ldcg(reinterpret_cast<const ulonglong2*>(&s->degsum));
+  return Slot{a.x, a.y, a.z, a.w, b.x, __longlong_as_double((long long)b.y)};
 }
 
 // The barrier's wait, after a first look.  0: it ran out.  (Out of line: what it needs
@@ -375,6 +371,12 @@ __device__ __forceinline__ void begin(Grid& grid, Shared* sh, const Launch& L, C
 // BFS (BFS.C:122-188)
 // ---------------------------------------------------------------------------
 constexpr uint32_t kPullWords = 8;  // words of the visited bitmap that a warp takes together, at most
+// A pull's warp reads this much of a vertex's list beyond its first 48 edges; the rest
+// of a longer one, as a rule a hub's that the search does not reach at all, is put off
+// and read in pieces by all warps.  (By one warp, 32 edges after 32: 2^20 vertices
+// beside a star of 2e6 that they do not reach 32.8 ms, 0.11 now; beside as many
+// vertices again, degree sorted, 17.3 and 0.43.)
+constexpr uint32_t kRestList = 256, kRestPiece = 512;
 
 struct BfsArgs : Launch {
   DevGraph out, in;  // push and pull lists
@@ -387,8 +389,47 @@ struct BfsArgs : Launch {
   uint32_t* parents;  // null: not wanted
   int32_t* depth_out;  // original-id order; null: not wanted (or not sorted)
   Queues q[2];
+  uint4* rest;  // a pulled level's pieces: vertex, edges [y, z)
   volatile uint64_t* info;  // mapped: rounds, reached, edges, done
 };
+
+// The first edge among [b, e) of a list whose neighbour is visited, as the neighbour;
+// kNone: none.  The whole warp, the same in every lane.
+__device__ __noinline__ uint32_t first_visited(const uint32_t* adj, const uint32_t* vis, uint32_t b, uint32_t e) {
+  const int lane = threadIdx.x & 31;
+  for (uint32_t x = b; x < e; x += 128) {
+    uint32_t u[4];
+    bool hit[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) u[k] = x + 32 * k + lane < e ? adj[x + 32 * k + lane] : kNone;
+#pragma unroll
+    for (int k = 0; k < 4; k++) hit[k] = u[k] != kNone && bit_test(vis, u[k]);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const unsigned hits = __ballot_sync(kAll, hit[k]);
+      if (hits) return __shfl_sync(kAll, u[k], __ffs(hits) - 1);
+    }
+  }
+  return kNone;
+}
+
+// The same for the rest of an unvisited vertex's list, which is put off where it is long.
+__device__ __noinline__ uint32_t read_on(const uint32_t* adj, const uint32_t* vis, uint32_t b, uint32_t e, uint32_t v,
+                                         uint4* rest, unsigned* nrest) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t near = min(b + kRestList, e);
+  const uint32_t f = first_visited(adj, vis, b, near);
+  if (f != kNone || near == e) return f;
+  const uint32_t pieces = (e - near + kRestPiece - 1) / kRestPiece;
+  uint32_t at = 0;
+  if (lane == 0) at = atomicAdd(nrest, pieces);
+  at = __shfl_sync(kAll, at, 0);
+  for (uint32_t p = lane; p < pieces; p += 32) {
+    const uint32_t y = near + p * kRestPiece;
+    rest[at + p] = make_uint4(v, y, min(y + kRestPiece, e), 0u);
+  }
+  return kNone;
+}
 
 // A push level claims vertices with an atomicOr on the visited bitmap; a pull
 // level reads one bitmap and writes the other (a visited in-neighbour of an
@@ -498,15 +539,13 @@ __global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
               const int l = __ffs(rest) - 1;
               rest &= rest - 1;
               const uint32_t jb = __shfl_sync(kAll, b[i], l), je = __shfl_sync(kAll, e[i], l);
-              for (uint32_t x = jb; x < je; x += 32) {
-                const uint32_t u = x + lane < je ? A.in.adj[x + lane] : kNone;
-                const unsigned hits = __ballot_sync(kAll, u != kNone && bit_test(vis, u));
-                if (hits) {
-                  const uint32_t f = __shfl_sync(kAll, u, __ffs(hits) - 1);
-                  if (lane == l) from[i] = f;
-                  break;
-                }
+              const uint32_t u = jb + lane < je ? A.in.adj[jb + lane] : kNone;
+              const unsigned hits = __ballot_sync(kAll, u != kNone && bit_test(vis, u));
+              uint32_t f = hits ? __shfl_sync(kAll, u, __ffs(hits) - 1) : kNone;
+              if (!hits && je - jb > 32) {
+                f = read_on(A.in.adj, vis, jb + 32, je, __shfl_sync(kAll, v[i], l), A.rest, &ns->heavy);
               }
+              if (lane == l) from[i] = f;
             }
             const bool won = from[i] != kNone;
             const unsigned now = __ballot_sync(kAll, won);
@@ -531,6 +570,21 @@ __global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
       }
       cv ^= 1;
       queued = false;
+      if (!grid.sync(ns)) return;
+      const uint32_t put_off = sh.slot.heavy;
+      if (!put_off) continue;
+      for (uint32_t i = warp; i < put_off; i += nwarps) {
+        const uint4 it = A.rest[i];
+        if (__any_sync(kAll, (__ldcg(nvis + (it.x >> 5)) >> (it.x & 31)) & 1u)) continue;  // found by another piece
+        const uint32_t f = first_visited(A.in.adj, vis, it.y, it.z);
+        const uint32_t bit = 1u << (it.x & 31);
+        if (f != kNone && lane == 0 && !(atomicOr(nvis + (it.x >> 5), bit) & bit)) {
+          A.depth[it.x] = level;
+          if (A.parents) A.parents[it.x] = f;
+          atomicAdd(&sh.count, 1u);
+          atomicAdd(&sh.degsum, (unsigned long long)(A.out.off[it.x + 1] - A.out.off[it.x]));
+        }
+      }
     } else {
       if (!queued) {  // after a pull: the frontier is what it added to the bitmap
         const uint32_t* old = A.vis[cv ^ 1];
@@ -2005,6 +2059,7 @@ rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t
   if (h_parents) X.add(&A.parents, n);
   add_queues(X, &A.q[0], n, m);
   add_queues(X, &A.q[1], n, m);
+  X.add(&A.rest, (size_t)(m / kRestPiece + m / (kRestList + 48) + 64));  // the last piece of a list may be short
   int32_t* direct = direct_results(g, h_depth, d_depth_out);
   if (order && !d_depth_out && !direct) X.add(&A.depth_out, n);
   RG_TRY(X.place());

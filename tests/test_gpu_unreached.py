@@ -1,0 +1,99 @@
+"""Pulls beside long lists and empty rows that the search has not reached: hubs whose
+only reached neighbour is the last of their list, at the lengths where a pull's reading
+changes hands, and calls whose time must not follow what they do not reach."""
+
+import numpy as np
+import pytest
+
+import oracle as orc
+import radar_graph as rg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def built():
+    import build as b
+    b.build()
+
+
+def core(n, base):
+    """Every pair of n vertices from id `base` on."""
+    i, j = np.triu_indices(n, 1)
+    return base + i, base + j
+
+
+def graph(n, parts, directed=False):
+    s, d = (np.concatenate([np.asarray(p[k], np.int64) for p in parts]).astype(np.uint32) for k in (0, 1))
+    return rg.Graph.from_edges(n, s, d, directed=directed)
+
+
+# 16 edges by a lane, 32 and 256 by its warp, pieces of 512 after that
+LENGTHS = [16, 17, 48, 49, 304, 305, 304 + 512, 304 + 513, 304 + 2 * 512, 9001]
+
+
+@pytest.mark.parametrize("directed", [False, True], ids=["sym", "dir"])
+@pytest.mark.parametrize("many", [False, True], ids=["last", "every"])
+def test_hubs_found_by_their_last_edges(directed, many):
+    """Hub after hub of the lengths above: ids of its leaves, then of the hubs, then of a
+    dense core (whose frontier is pulled); the core is next to a hub's last entry, or
+    (every) to every 97th as well, so that several pieces find it."""
+    leaves, hubs = sum(LENGTHS), len(LENGTHS)
+    base = leaves + hubs
+    rng = np.random.default_rng(1)
+    parts, at = [core(300, base)], 0
+    for h, length in enumerate(LENGTHS):
+        mine = np.arange(at, at + length - 1)
+        if many:
+            mine[::97] = base + rng.choice(300, len(mine[::97]), replace=False) if len(mine[::97]) < 300 else mine[::97]
+        parts.append((mine, np.full(len(mine), leaves + h)))
+        parts.append(([base + 299], [leaves + h]))
+        at += length
+    with graph(base + 300, parts, directed) as g:
+        off, adj, _ = g.download()
+        for root in (base, base + 299):
+            par, depth, rounds, reached = g.bfs("push", root)
+            assert rg.last_timing()["kernel_launches"] == 1
+            if directed:
+                rg.set_trace(True)
+                _, want, r2, n2 = g.bfs("push", root)
+                rg.set_trace(False)
+                assert (rounds, reached) == (r2, n2)
+            else:
+                want = orc.bfs_depths(off, adj, root)
+            assert np.array_equal(depth, want)
+            assert reached == int((want >= 0).sum())
+            v = np.nonzero(depth > 0)[0]
+            assert np.array_equal(depth[par[v]] + 1, depth[v])
+        with g.degree_sort() as s:
+            assert np.array_equal(s.bfs("push", base)[1], g.bfs("push", base)[1])
+
+
+def device_ms(call, reps=5):
+    call()
+    best = 1e9
+    for _ in range(reps):
+        call()
+        best = min(best, rg.last_timing()["total_ms"])
+    return best
+
+
+def one_launch_against_levels(call):
+    one = device_ms(call)
+    assert rg.last_timing()["kernel_launches"] <= 2
+    rg.set_trace(True)
+    levels = device_ms(call)
+    rg.set_trace(False)
+    return one, levels
+
+
+@pytest.mark.parametrize("directed", [False, True], ids=["sym", "dir"])
+def test_bfs_time_beside_an_unreached_hub(directed):
+    """A star of 2e6 that the root does not reach (read by one warp it took 60 times the
+    level-by-level run; the bound leaves room for a busy machine)."""
+    src, dst = rg.generate_edges(18, 16, seed=2)
+    n = 1 << 18
+    hub = (n + 1 + np.arange(2000000), np.full(2000000, n))
+    with graph(n + 2000001, [(src, dst), hub], directed) as g:
+        one, levels = one_launch_against_levels(lambda: g.bfs("push", int(src[0]), parents=False))
+        assert one < 3 * levels, (one, levels)
