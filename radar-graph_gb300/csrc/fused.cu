@@ -1130,6 +1130,9 @@ struct RadiiArgs : Launch {
 // Chunks of kSweepChunk edges per warp from which a dense round takes them whole
 // (16 edges per lane, a quarter of the scans) instead of in steps of 128.
 constexpr uint32_t kWideChunks = 2;
+// Rows of a chunk up to which a round may be pulled: a lane walks from row to row, and
+// over those without edges too (4e6 of them in one place: 0.8 s).
+constexpr uint32_t kPullRows = 2048;
 constexpr int kPlanes = 6;  // depths up to 63; deeper searches run level by level
 
 // The vertex's new mask becomes current.
@@ -1207,6 +1210,9 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
     A.radii[i] = -1;
   }
   for (uint32_t w = tid; w < nwords; w += nthreads) A.bits[0][w] = A.bits[1][w] = 0u;
+  for (uint32_t c = tid; c < A.nchunks; c += nthreads) {
+    if (A.chunk_v[c + 1] - A.chunk_v[c] > kPullRows) A.ctl->lv[0].heavy = 1;
+  }
   unsigned long long full = 0ull;  // the bits that can spread: seeds with out-edges
   for (int j = lane; j < A.k; j += 32) {
     const uint32_t v = A.new_ids ? A.new_ids[A.seed[j]] : A.seed[j];
@@ -1229,6 +1235,7 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
     ap.finish(A.q[0], &A.ctl->lv[0], 0, 0);
   }
   if (!grid.sync(&A.ctl->lv[0])) return;
+  const int64_t threshold = sh.slot.heavy ? INT64_MAX : A.threshold;
   int cq = 0;  // the queue pair that holds the frontier
   int cb = 0;  // the bitmap that holds it after a pull; a bitmap that does not is clear
   bool queued = true;
@@ -1250,7 +1257,7 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
       }
     }
     const Queues nq = A.q[cq ^ 1];
-    if ((int64_t)(c.count + c.degsum) > A.threshold && A.in.m > 0) {
+    if ((int64_t)(c.count + c.degsum) > threshold && A.in.m > 0) {
       uint32_t *bits = A.bits[cb ^ 1], *old_bits = A.bits[cb];
       const uint32_t steps = (A.in.m + 127) / 128;
       // a CTA's warps take its share as they get done: chunks whose rows are complete

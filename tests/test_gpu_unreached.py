@@ -97,3 +97,40 @@ def test_bfs_time_beside_an_unreached_hub(directed):
     with graph(n + 2000001, [(src, dst), hub], directed) as g:
         one, levels = one_launch_against_levels(lambda: g.bfs("push", int(src[0]), parents=False))
         assert one < 3 * levels, (one, levels)
+
+
+def test_radii_and_batched_bfs_beside_empty_rows():
+    """4e6 ids without edges between two halves of the others (a lane that walked over
+    their rows one by one took 0.8 s): results as level by level, and the time of the
+    graph without the gap but for the passes over its vertices."""
+    src, dst = rg.generate_edges(18, 16, seed=3)
+    n, gap = 1 << 18, 4000000
+
+    def shift(x):
+        return np.where(x >= n // 2, x + gap, x)
+
+    seeds = rg.radii_query_seeds(5, n)
+    times = []
+    for f, size in ((lambda x: x, n), (shift, n + gap)):
+        with graph(size, [(f(src.astype(np.int64)), f(dst.astype(np.int64)))]) as g:
+            s = f(seeds.astype(np.int64)).astype(np.uint32)
+            for variant in ("push", "push-pull"):
+                call = lambda: g.radii_seeds(s, variant)
+                ms = device_ms(call)
+                one = call()
+                assert rg.last_timing()["kernel_launches"] == 1
+                rg.set_trace(True)
+                levels = call()
+                rg.set_trace(False)
+                assert np.array_equal(one[0], levels[0]) and one[1] == levels[1]
+                times.append(ms)
+            ms = device_ms(lambda: g.bfs_multi(s))
+            one = g.bfs_multi(s)
+            assert rg.last_timing()["kernel_launches"] == 1
+            rg.set_trace(True)
+            levels = g.bfs_multi(s)
+            rg.set_trace(False)
+            assert np.array_equal(one[0], levels[0]) and one[1] == levels[1]
+            times.append(ms)
+    for plain, gapped in zip(times[:3], times[3:]):
+        assert gapped < 10 * plain, times
