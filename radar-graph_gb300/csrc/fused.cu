@@ -1130,9 +1130,6 @@ struct RadiiArgs : Launch {
 // Chunks of kSweepChunk edges per warp from which a dense round takes them whole
 // (16 edges per lane, a quarter of the scans) instead of in steps of 128.
 constexpr uint32_t kWideChunks = 2;
-// Rows of a chunk up to which a round may be pulled: a lane walks from row to row, and
-// over those without edges too (4e6 of them in one place: 0.8 s).
-constexpr uint32_t kPullRows = 2048;
 constexpr int kPlanes = 6;  // depths up to 63; deeper searches run level by level
 
 // The vertex's new mask becomes current.
@@ -1895,23 +1892,40 @@ __global__ void find_max_degree(const uint32_t* __restrict__ off, uint32_t n, un
   if ((threadIdx.x & 31) == 0) atomicMax(out, mx);
 }
 
-int64_t max_in_degree(const rg_graph* g, cudaStream_t st) {
-  if (!g->directed) return g->max_deg;
-  int64_t v = g->max_in_deg.load(std::memory_order_relaxed);
+__global__ void find_max_chunk(const uint32_t* __restrict__ chunk_v, uint32_t nchunks, unsigned int* out) {
+  unsigned int mx = 0;
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nchunks; c += gridDim.x * blockDim.x) {
+    mx = max(mx, chunk_v[c + 1] - chunk_v[c]);
+  }
+  mx = __reduce_max_sync(kAll, mx);
+  if ((threadIdx.x & 31) == 0) atomicMax(out, mx);
+}
+
+// A value that `find` leaves in a zeroed word, kept in `known`; `unknown` on an error.
+template <class Find>
+int64_t found_once(std::atomic<int64_t>& known, int64_t unknown, cudaStream_t st, Find find) {
+  int64_t v = known.load(std::memory_order_relaxed);
   if (v >= 0) return v;
   unsigned int* d = reinterpret_cast<unsigned int*>(ctx().ws.counters.as<uint64_t>() + 8);  // a free scratch word
   uint32_t h = 0;
   cudaError_t e = cudaMemsetAsync(d, 0, 4, st);
   if (e == cudaSuccess) {
-    find_max_degree<<<64, 256, 0, st>>>(g->in_view().off, (uint32_t)g->n, d);
+    find(d);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess || read_small(d, &h, 4, st) != RG_OK) {
     cudaGetLastError();
-    return g->n;  // too large a row for the one-launch path
+    return unknown;
   }
-  g->max_in_deg.store(h, std::memory_order_relaxed);
+  known.store(h, std::memory_order_relaxed);
   return h;
+}
+
+int64_t max_in_degree(const rg_graph* g, cudaStream_t st) {
+  if (!g->directed) return g->max_deg;
+  return found_once(g->max_in_deg, g->n, st, [&](unsigned int* d) {  // (n: too large a row for the one-launch path)
+    find_max_degree<<<64, 256, 0, st>>>(g->in_view().off, (uint32_t)g->n, d);
+  });
 }
 
 // The arrays of one launch, in the thread's one allocation: large ones on whole
@@ -2045,6 +2059,12 @@ rg_status deliver(rg_graph* g, const T* internal, const T* ordered, T* host_out,
 }
 
 }  // namespace
+
+bool short_chunks(const rg_graph* g, cudaStream_t st) {
+  return found_once(g->max_chunk_rows, 0, st, [&](unsigned int* d) {
+           find_max_chunk<<<64, 256, 0, st>>>(g->in_chunks(), (uint32_t)g->nchunks, d);
+         }) <= kPullRows;
+}
 
 bool fused_fits(const rg_graph* g, int64_t max_edges) {
   return g->m <= max_edges && g->n <= max_edges && strides_fit(g->n, g->m) && !g_trace_on;

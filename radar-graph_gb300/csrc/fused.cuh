@@ -68,6 +68,12 @@ constexpr int64_t kFusedMsEdges = 1 << 27;
 // per-level records (rg_set_trace) are asked for.
 bool fused_fits(const rg_graph* g, int64_t max_edges);
 
+// Rows of a chunk up to which a sweep pulls: a lane walks from row to row, and over
+// those without edges too (4e6 of them in one place: 0.8 s a sweep).
+constexpr uint32_t kPullRows = 2048;
+// Whether g's pull lists have no chunk of more (found once per graph).
+bool short_chunks(const rg_graph* g, cudaStream_t st);
+
 // Each sets *done when the launch answered the call; otherwise (its bounded
 // waits ran out) the caller answers level by level.
 rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t* h_depth,

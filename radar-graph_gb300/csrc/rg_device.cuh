@@ -172,6 +172,7 @@ struct rg_graph {
   uint32_t max_deg = 0;
   mutable std::atomic<int64_t> pull_split{-1};  // pull_split()'s cached value, -1 = not yet known
   mutable std::atomic<int64_t> max_in_deg{-1};  // directed: largest in-degree, -1 = not yet known
+  mutable std::atomic<int64_t> max_chunk_rows{-1};  // most rows that a chunk of the pull lists spans, -1 = not yet known
   bool tuned[4] = {false, false, false, false};  // per app: PageRank, BFS, BC, Radii
   rg::Options topt[4];                           // the autotuner's choice per app
   rg::DevGraph view() const {

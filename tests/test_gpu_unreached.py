@@ -7,6 +7,7 @@ import pytest
 
 import oracle as orc
 import radar_graph as rg
+from conftest import assert_close
 
 pytestmark = pytest.mark.gpu
 
@@ -134,3 +135,21 @@ def test_radii_and_batched_bfs_beside_empty_rows():
             times.append(ms)
     for plain, gapped in zip(times[:3], times[3:]):
         assert gapped < 10 * plain, times
+
+
+def test_pagerank_delta_beside_empty_rows():
+    """The same for PageRankDelta's swept rounds, on a graph above the one-launch size."""
+    src, dst = rg.generate_edges(18, 24, seed=3)
+    n, gap = 1 << 18, 4000000
+
+    def shift(x):
+        return np.where(x >= n // 2, x + gap, x).astype(np.int64)
+
+    with graph(n + gap, [(shift(src), shift(dst))]) as g:
+        assert g.m > 6 << 20
+        ms = device_ms(lambda: g.pagerank_delta("push-pull", 100), reps=2)
+        pushed = device_ms(lambda: g.pagerank_delta("push", 100), reps=2)
+        assert ms < 5 * pushed, (ms, pushed)
+        one, levels = g.pagerank_delta("push-pull", 100), g.pagerank_delta("push", 100)
+        assert one[1] == levels[1]
+        assert_close(one[0], levels[0], what="ranks")
