@@ -65,13 +65,12 @@ struct CallTimer {
 int device_sms();     // of the calling thread's current device
 int max_dyn_smem();   // opt-in shared memory per block, same device
 
-// A kernel of a sequence is launched while the one before it drains
-// (launch_following): it lets its own follower in and waits for its predecessor
-// to complete before it reads anything.  A plain launch passes straight through.
-__device__ __forceinline__ void follow() {
-  cudaTriggerProgrammaticLaunchCompletion();
-  cudaGridDependencySynchronize();
-}
+// A kernel of a sequence is launched as the one before it ends (launch_following) and
+// waits for it to complete before it reads anything.  A plain launch passes straight
+// through.  (Its follower comes in when it has exited: let in from the start, the
+// follower's waiting CTAs take slots from this one's.  PageRank, 20 iterations, degree
+// sorted: 2^17 vertices 450 us, 375 now; 2^18 659 and 606.)
+__device__ __forceinline__ void follow() { cudaGridDependencySynchronize(); }
 
 template <class... P, class... A>
 cudaError_t launch_following(void (*kern)(P...), int grid, int threads, size_t dyn, cudaStream_t st, A&&... args) {
