@@ -1122,7 +1122,7 @@ struct RadiiArgs : Launch {
   uint32_t* bits[2];  // what a pull reached
   Queues q[2];
   // multi-source BFS: bit q of plane p of v is bit p of v's depth from source q
-  unsigned long long* planes;
+  unsigned long long* planes;  // as many as the bits of the largest depth there can be
   int32_t* depths;  // sources rows of n, original-id order
   int sources;
   volatile uint64_t* info;  // mapped: rounds, edges, -, done
@@ -1130,7 +1130,7 @@ struct RadiiArgs : Launch {
 // Chunks of kSweepChunk edges per warp from which a dense round takes them whole
 // (16 edges per lane, a quarter of the scans) instead of in steps of 128.
 constexpr uint32_t kWideChunks = 2;
-constexpr int kPlanes = 6;  // depths up to 63; deeper searches run level by level
+constexpr int kFewPlanes = 6;  // depths up to 63
 
 // The vertex's new mask becomes current.
 template <bool kDepths>
@@ -1138,10 +1138,7 @@ __device__ __forceinline__ void radii_advance(const RadiiArgs& A, uint32_t v, in
                                               unsigned long long old) {
   if (kDepths) {
     const unsigned long long w = now & ~old;
-#pragma unroll
-    for (int p = 0; p < kPlanes; p++) {
-      if ((round >> p) & 1) A.planes[(size_t)p * A.out.n + v] |= w;
-    }
+    for (unsigned b = (unsigned)round; b; b &= b - 1) A.planes[(size_t)(__ffs(b) - 1) * A.out.n + v] |= w;
   }
   A.vis[v] = now;
 }
@@ -1151,6 +1148,7 @@ __device__ __forceinline__ void radii_advance(const RadiiArgs& A, uint32_t v, in
 // of every row before).
 template <int kUsed>
 __device__ __forceinline__ void write_depths(const RadiiArgs& A) {
+  static_assert(kUsed <= kFewPlanes, "held in registers");
   const uint32_t n = A.out.n;
   const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
   for (uint32_t i = tid; i < n; i += nthreads) {
@@ -1172,6 +1170,22 @@ __device__ __forceinline__ void write_depths(const RadiiArgs& A) {
         for (int p = 0; p < kUsed; p++) d |= ((x[p] >> q) & 1u) << p;
         *row = (s >> q) & 1u ? (int32_t)d : -1;
       }
+    }
+  }
+}
+
+// The same for deep searches, whose rounds cost far more than reading the planes a
+// source at a time.
+__device__ __noinline__ void write_depths_deep(const RadiiArgs& A, int used) {
+  const uint32_t n = A.out.n;
+  const uint32_t tid = blockIdx.x * kFT + threadIdx.x, nthreads = gridDim.x * kFT;
+  for (uint32_t i = tid; i < n; i += nthreads) {
+    const uint32_t v = A.new_ids ? A.new_ids[i] : i;
+    const unsigned long long seen = A.vis[v];
+    for (int q = 0; q < A.sources; q++) {
+      uint32_t d = 0;
+      for (int p = 0; p < used; p++) d |= (uint32_t)((A.planes[(size_t)p * n + v] >> q) & 1u) << p;
+      A.depths[(size_t)q * n + i] = (seen >> q) & 1u ? (int32_t)d : -1;
     }
   }
 }
@@ -1247,7 +1261,6 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
     if (tid == 0) A.ctl->lv[(round + 2) % 3] = Slot{};
     round++;
     if (kDepths) {
-      if (round >> kPlanes) return;  // too deep: answered level by level
       if ((round & (round - 1)) == 0) {  // the first round of a plane (a barrier lies before its first use)
         unsigned long long* pl = A.planes + (size_t)(31 - __clz(round)) * n;
         for (uint32_t i = tid; i < n; i += nthreads) pl[i] = 0ull;
@@ -1431,7 +1444,8 @@ __global__ void __launch_bounds__(kFT, 1) radii_fused(const __grid_constant__ Ra
       case 3: write_depths<3>(A); break;
       case 4: write_depths<4>(A); break;
       case 5: write_depths<5>(A); break;
-      default: write_depths<6>(A); break;
+      case 6: write_depths<6>(A); break;
+      default: write_depths_deep(A, 32 - __clz(round)); break;
     }
   }
   if (A.radii_out) {
@@ -2243,6 +2257,13 @@ rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double
 
 namespace {
 
+// Bits of a depth: at most n - 1, and the round that finds nothing more counts.
+int depth_planes(int64_t n) {
+  int p = 1;
+  while (n >> p) p++;
+  return p;
+}
+
 // What Radii and multi-source BFS share; seeds: original ids, each once.
 // ordered: n radii by original id too; planes: the depth planes.
 rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int k, bool ordered,
@@ -2259,7 +2280,7 @@ rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned lo
   add_queues(X, &A->q[0], n, m);
   add_queues(X, &A->q[1], n, m);
   if (ordered) X.add(&A->radii_out, n);
-  if (planes) X.add(&A->planes, (size_t)n * kPlanes);
+  if (planes) X.add(&A->planes, (size_t)n * depth_planes(n));
   RG_TRY(X.place());
   A->out = g->view();
   A->in = g->in_view();

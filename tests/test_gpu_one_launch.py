@@ -136,3 +136,19 @@ def test_pagerank_delta_handed_over():
     assert one[1] == many[1] == rounds
     assert_close(one[0], many[0], what="levels")
     assert_close(one[0], want, what="oracle")
+
+
+@pytest.mark.parametrize("sorted_handle", [False, True])
+@pytest.mark.parametrize("length", [62, 63, 64, 65, 127, 128, 1025, 5000])
+def test_deep_batched_bfs(length, sorted_handle):
+    """Depths around the planes that the kernel holds in registers (63) and powers of
+    two above, in one launch."""
+    n = length + 1 + 40
+    off, adj = rg.csr_from_edges(n, np.arange(length, dtype=np.uint32), 1 + np.arange(length, dtype=np.uint32))
+    src = np.array([0, length, length // 2, 3, n - 1, 0], np.uint32)  # n - 1: isolated
+    with rg.Graph.from_csr(off, adj) as g, g.degree_sort() as s:
+        rows, rounds = (s if sorted_handle else g).bfs_multi(src)
+        assert rg.last_timing()["kernel_launches"] == 1
+    assert rounds == length + 1
+    for q, root in enumerate(src):
+        assert np.array_equal(rows[q], orc.bfs_depths(off, adj, int(root)))
