@@ -1945,10 +1945,19 @@ int64_t max_in_degree(const rg_graph* g, cudaStream_t st) {
 // The arrays of one launch, in the thread's one allocation: large ones on whole
 // pages.  (Allocated one by one, their placement after earlier allocations of the
 // process moved BFS on 2^24 vertices between 1.02 and 1.13 ms.)
-thread_local DevBuf g_arena;
+// It is kept for the thread's next call.
+struct Arena {
+  DevBuf buf;
+  int device = -1;
+  bool in_use = false;  // a call's launches may be reading and writing it
+};
+thread_local Arena g_arena;
 
 class Arrays {
  public:
+  Arrays() = default;
+  Arrays(const Arrays&) = delete;
+  ~Arrays() { g_arena.in_use = false; }
   template <class T>
   void add(T** p, size_t count) {
     const size_t bytes = std::max<size_t>(count * sizeof(T), 16);
@@ -1957,9 +1966,21 @@ class Arrays {
     at_.push_back({reinterpret_cast<void**>(p), total_});
     total_ += bytes;
   }
-  rg_status place() {
-    RG_TRY(g_arena.reserve(total_));
-    for (const auto& a : at_) *a.first = g_arena.as<char>() + a.second;
+  // *fits: false where the memory is too small for them (the level-by-level runs need
+  // a third of it)
+  rg_status place(bool* fits) {
+    const int device = ctx().device;
+    if (g_arena.device != device) g_arena.buf.release();
+    g_arena.device = device;
+    const rg_status s = g_arena.buf.reserve(total_);
+    *fits = s == RG_OK;
+    if (s == RG_ENOMEM) {
+      clear_error();
+      return RG_OK;
+    }
+    RG_TRY(s);
+    g_arena.in_use = true;
+    for (const auto& a : at_) *a.first = g_arena.buf.as<char>() + a.second;
     return RG_OK;
   }
 
@@ -2080,6 +2101,12 @@ bool short_chunks(const rg_graph* g, cudaStream_t st) {
          }) <= kPullRows;
 }
 
+bool release_idle_arena() {
+  if (g_arena.in_use || !g_arena.buf.p) return false;
+  g_arena.buf.release();
+  return true;
+}
+
 bool fused_fits(const rg_graph* g, int64_t max_edges) {
   return g->m <= max_edges && g->n <= max_edges && strides_fit(g->n, g->m) && !g_trace_on;
 }
@@ -2103,7 +2130,9 @@ rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t
   X.add(&A.rest, (size_t)(m / kRestPiece + m / (kRestList + 48) + 64));  // the last piece of a list may be short
   int32_t* direct = direct_results(g, h_depth, d_depth_out);
   if (order && !d_depth_out && !direct) X.add(&A.depth_out, n);
-  RG_TRY(X.place());
+  bool fits = false;
+  RG_TRY(X.place(&fits));
+  if (!fits) return RG_OK;
   if (direct) A.depth_out = direct;
   if (order && d_depth_out) A.depth_out = d_depth_out;
   A.out = g->view();
@@ -2136,7 +2165,7 @@ namespace {
 
 // The arrays of `groups` groups of bc_fused.
 // *ordered (unless null): n results by original id.
-rg_status bc_arrays(const rg_graph* g, int groups, bool chain, BcArgs* A, double** ordered) {
+rg_status bc_arrays(const rg_graph* g, int groups, bool chain, BcArgs* A, double** ordered, Arrays& X, bool* fits) {
   const size_t n = (size_t)g->n, m = (size_t)g->m;
   A->n_small = small_entries(g->n);
   A->n_large = large_entries(g->n, g->m);
@@ -2145,7 +2174,6 @@ rg_status bc_arrays(const rg_graph* g, int groups, bool chain, BcArgs* A, double
   // pieces of lists above kLongList, two at least: at most 3/2 per kLongPiece edges
   A->n_heavy = A->long_lists ? m / kLongPiece + m / kLongList + 64 : 0;
   A->new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
-  Arrays X;
   X.add(&A->vis, (n + 31) / 32 * groups);
   X.add(&A->lvl, n * groups);
   X.add(&A->sigma, n * groups);
@@ -2159,7 +2187,7 @@ rg_status bc_arrays(const rg_graph* g, int groups, bool chain, BcArgs* A, double
   X.add(&A->heavy, A->n_heavy * groups);
   if (chain) X.add(&A->deps, n);
   if (ordered) X.add(ordered, n);
-  return X.place();
+  return X.place(fits);
 }
 
 // Groups for k sources and the CTAs of each.  Every source gets a group while there
@@ -2186,7 +2214,10 @@ rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* 
   double* ordered = !order ? nullptr : direct ? direct : d_deps_out;
   int groups = 1, width = fused_grid(m + n, kFusedEdgesPerCta);
   if (m <= std::min(kFusedBcRowsEdges, kFusedBcRowsWork / std::max(nsrc, 1))) bc_split(g, std::min(nsrc, 64), &groups, &width);
-  RG_TRY(bc_arrays(g, groups, true, &A, order && !ordered ? &ordered : nullptr));
+  Arrays X;
+  bool fits = false;
+  RG_TRY(bc_arrays(g, groups, true, &A, order && !ordered ? &ordered : nullptr, X, &fits));
+  if (!fits) return RG_OK;
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = info_begin();
   CallTimer timer(g);
@@ -2221,7 +2252,10 @@ rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double
   int groups, width;
   bc_split(g, k, &groups, &width);
   BcArgs A;
-  RG_TRY(bc_arrays(g, groups, false, &A, nullptr));
+  Arrays X;
+  bool fits = false;
+  RG_TRY(bc_arrays(g, groups, false, &A, nullptr, X, &fits));
+  if (!fits) return RG_OK;
   A.g = g->view();
   A.gt = g->in_view();
   for (int q = 0; q < k; q++) A.source[q] = src_orig[q];
@@ -2267,11 +2301,10 @@ int depth_planes(int64_t n) {
 // What Radii and multi-source BFS share; seeds: original ids, each once.
 // ordered: n radii by original id too; planes: the depth planes.
 rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int k, bool ordered,
-                     bool planes, RadiiArgs* A) {
+                     bool planes, RadiiArgs* A, Arrays& X, bool* fits) {
   const int64_t n = g->n, m = g->m;
   A->radii_out = nullptr;
   A->planes = nullptr;
-  Arrays X;
   X.add(&A->bits[0], (n + 31) / 32);
   X.add(&A->bits[1], (n + 31) / 32);
   X.add(&A->vis, n);
@@ -2281,7 +2314,8 @@ rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned lo
   add_queues(X, &A->q[1], n, m);
   if (ordered) X.add(&A->radii_out, n);
   if (planes) X.add(&A->planes, (size_t)n * depth_planes(n));
-  RG_TRY(X.place());
+  RG_TRY(X.place(fits));
+  if (!*fits) return RG_OK;
   A->out = g->view();
   A->in = g->in_view();
   A->chunk_v = g->in_chunks();
@@ -2313,7 +2347,10 @@ rg_status radii_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned lon
   RadiiArgs A;
   const bool order = g->sorted && (h_radii || d_radii_out);
   int32_t* direct = direct_results(g, h_radii, d_radii_out);
-  RG_TRY(radii_args(g, seeds, masks, k, order && !d_radii_out && !direct, false, &A));
+  Arrays X;
+  bool fits = false;
+  RG_TRY(radii_args(g, seeds, masks, k, order && !d_radii_out && !direct, false, &A, X, &fits));
+  if (!fits) return RG_OK;
   if (direct) A.radii_out = direct;
   if (order && d_radii_out) A.radii_out = d_radii_out;
   volatile uint64_t* info = cx.ws.h_info;
@@ -2337,7 +2374,10 @@ rg_status ms_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long l
   cudaStream_t st = cx.stream;
   const int64_t n = g->n, m = g->m;
   RadiiArgs A;
-  RG_TRY(radii_args(g, seeds, masks, u, false, true, &A));
+  Arrays X;
+  bool fits = false;
+  RG_TRY(radii_args(g, seeds, masks, u, false, true, &A, X, &fits));
+  if (!fits) return RG_OK;
   A.depths = out;
   A.sources = k;
   volatile uint64_t* info = cx.ws.h_info;
@@ -2382,7 +2422,9 @@ rg_status pagerank_fused_run(rg_graph* g, int64_t max_iters, double* h_ranks, in
   X.add(&A.rmag, n);
   X.add(&A.l1, std::max<int64_t>(max_iters, 1));
   if (order) X.add(&A.ranks_out, n);
-  RG_TRY(X.place());
+  bool fits = false;
+  RG_TRY(X.place(&fits));
+  if (!fits) return RG_OK;
   A.in = g->in_view();
   A.out_off = g->off.as<uint32_t>();
   A.chunk_v = g->in_chunks();
@@ -2411,7 +2453,8 @@ rg_status pagerank_fused_run(rg_graph* g, int64_t max_iters, double* h_ranks, in
 }
 
 rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max_iters, double* p, double* ngh,
-                        double* c, uint32_t* bits, double* ranks_out, int64_t* rounds, double* l1, bool* done) {
+                        double* c, uint32_t* bits, double* ranks_out, int64_t* rounds, double* l1, bool* launched,
+                        bool* done) {
   Ctx& cx = ctx();
   cudaStream_t st = cx.stream;
   const int64_t n = g->n, m = g->m;
@@ -2422,7 +2465,9 @@ rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max
   add_queues(X, &A.q[1], n, m);
   if (start == 0) add_queues(X, &A.rows, n, m);
   X.add(&A.touched, (n + 31) / 32);
-  RG_TRY(X.place());
+  bool fits = false;
+  RG_TRY(X.place(&fits));
+  if (!fits) return RG_OK;
   A.out = g->view();
   A.in = g->in_view();
   A.new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
@@ -2441,6 +2486,7 @@ rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = info_begin();
   RG_TRY(launch_fused(prd_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
+  *launched = true;
   RG_CUDA(cudaStreamSynchronize(st));
   *done = info[kDone] == 1 && all_ran();
   if (!*done) return RG_OK;

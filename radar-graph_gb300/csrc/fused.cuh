@@ -75,7 +75,8 @@ constexpr uint32_t kPullRows = 2048;
 bool short_chunks(const rg_graph* g, cudaStream_t st);
 
 // Each sets *done when the launch answered the call; otherwise (its bounded
-// waits ran out) the caller answers level by level.
+// waits ran out, or its arrays do not fit the memory) the caller answers level by
+// level.
 rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t* h_depth,
                         int64_t* rounds_out, int64_t* reached_out, int32_t* d_depth_out, bool* done);
 rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* h_deps, int64_t* levels_out,
@@ -97,10 +98,12 @@ rg_status ms_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long l
 
 // PageRankDelta from round `start` on (0: a whole run, which initialises p, ngh
 // and c itself; else p, c and the frontier's bits as the filter of round `start`
-// left them, ngh 0).  Synchronises; *rounds as the reference counts them.
+// left them, ngh 0).  Synchronises; *rounds as the reference counts them.  *launched:
+// p, ngh and c have changed, whether the launch ran to its end or not.
 // ranks_out (device, original ids) may be null.
 rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max_iters, double* p, double* ngh,
-                        double* c, uint32_t* bits, double* ranks_out, int64_t* rounds, double* l1, bool* done);
+                        double* c, uint32_t* bits, double* ranks_out, int64_t* rounds, double* l1, bool* launched,
+                        bool* done);
 
 constexpr double kPrDamp = 0.85;  // PageRank.C:126
 constexpr double kPrdEps = 0.0000001, kPrdEps2 = 0.01;  // PageRankDelta.C:103-104

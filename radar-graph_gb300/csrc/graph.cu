@@ -52,6 +52,13 @@ rg_status cuda_fail(cudaError_t e, const char* what, const char* file, int line)
 rg_status DevBuf::reserve(size_t b) {
   if (b <= bytes && p) return RG_OK;
   release();
+  const rg_status s = allocate(b);
+  if (s != RG_ENOMEM || !release_idle_arena()) return s;
+  clear_error();
+  return allocate(b);
+}
+
+rg_status DevBuf::allocate(size_t b) {
   size_t want = b < 256 ? 256 : b;
   if (pooled && on_stream) {  // used and released in its stream's order
     RG_CUDA(cudaMallocAsync(&p, want, free_stream));

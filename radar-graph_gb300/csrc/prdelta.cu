@@ -180,7 +180,15 @@ rg_status pagerank_delta_run(rg_graph* g, int variant, int64_t max_iters, double
   // placement moves the gathers' speed)
   const size_t page = 2u << 20, row = ((size_t)n * 8 + page - 1) / page * page;
   auto reserve_rows = [&](int rows) { return S.arrays.reserve(rows * row); };
-  RG_TRY(reserve_rows(small ? 3 : pulls ? 6 : 4));
+  auto reserve_levels = [&]() -> rg_status {
+    if (pulls && reserve_rows(6) != RG_OK) {  // pushed, without the exact sums' 16 bytes a vertex
+      clear_error();
+      pulls = false;
+      g_opts.direction = 0;
+    }
+    return reserve_rows(pulls ? 6 : 4);
+  };
+  RG_TRY(small ? reserve_rows(3) : reserve_levels());
   RG_TRY(S.totals.reserve(sizeof(PrdTotals) * (kPulledRounds + 1)));
   RG_TRY(frontier_alloc(g, S.f[0]));
   RG_TRY(frontier_alloc(g, S.f[1]));
@@ -193,13 +201,14 @@ rg_status pagerank_delta_run(rg_graph* g, int variant, int64_t max_iters, double
   int64_t round = 0;
   double l1 = 0.0;
   CallTimer timer(g);
-  bool whole = false;  // answered by one launch
+  bool whole = false, launched = false;  // answered by one launch
   if (small) {
-    RG_TRY(prd_fused_run(g, true, 0, max_iters, p, ngh, c, S.f[0].bits.as<uint32_t>(), nullptr, &round, &l1, &whole));
+    RG_TRY(prd_fused_run(g, true, 0, max_iters, p, ngh, c, S.f[0].bits.as<uint32_t>(), nullptr, &round, &l1, &launched,
+                         &whole));
   }
   if (!whole) {
-    if (small) {  // (the launch gave up)
-      RG_TRY(reserve_rows(pulls ? 6 : 4));
+    if (small) {
+      RG_TRY(reserve_levels());
       p = array(0), ngh = array(1), c = array(2);
     }
     unsigned long long* rmag = reinterpret_cast<unsigned long long*>(array(3));
@@ -235,13 +244,16 @@ rg_status pagerank_delta_run(rg_graph* g, int variant, int64_t max_iters, double
       const bool dense = cur.count + cur.degsum > threshold;
       if (!dense && round > 1 && hand_over) {
         bool done = false;
-        // (a launch that gives up has changed p, ngh and c: the run starts again, level by level)
-        RG_TRY(prd_fused_run(g, false, round - 1, max_iters, p, ngh, c, cur.bits, nullptr, &round, &l1, &done));
+        launched = false;
+        RG_TRY(prd_fused_run(g, false, round - 1, max_iters, p, ngh, c, cur.bits, nullptr, &round, &l1, &launched,
+                             &done));
         if (done) break;
         hand_over = false;
-        RG_TRY(start());
-        round = 0;
-        continue;
+        if (launched) {  // gave up, having changed p, ngh and c: the run starts again, level by level
+          RG_TRY(start());
+          round = 0;
+          continue;
+        }
       }
       if (dense && g->m > 0 && pulls) {
         const int k = (int)std::min<int64_t>(kPulledRounds, max_iters - round + 1);

@@ -85,8 +85,13 @@ struct DevBuf {
   }
   // Grows (never shrinks) to at least `b` bytes; contents are not kept.
   rg_status reserve(size_t b);
+  rg_status allocate(size_t b);
   template <class T> T* as() const { return static_cast<T*>(p); }
 };
+
+// Gives back the arrays that the thread's one-launch calls keep, unless a call is using
+// them (fused.cu); false: there was nothing to give back.
+bool release_idle_arena();
 
 // Device frontier: compacted queue of ids (ascending when produced by the
 // engine), the exclusive scan of their degrees (for edge-balanced push), and

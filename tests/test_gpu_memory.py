@@ -1,0 +1,123 @@
+"""Calls on a nearly full device: the one-launch traversals' arrays, which are larger than
+the level-by-level runs', give way to those instead of failing, and what a thread's
+calls keep is given back to a later allocation that needs it."""
+
+import threading
+import time
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import radar_graph as rg  # noqa: E402
+from conftest import assert_close  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+N = 1 << 24
+
+
+@pytest.fixture(scope="module", autouse=True)
+def built():
+    import build as b
+    b.build()
+
+
+@pytest.fixture(scope="module")
+def g():
+    r = np.random.default_rng(3)
+    with rg.Graph.from_edges(N, *(r.integers(0, N, 1 << 20).astype(np.uint32) for _ in range(2))) as g:
+        yield g
+
+
+def free_bytes():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def in_thread(fn):
+    """fn's result from a thread of its own, whose scratch goes with it."""
+    box = []
+
+    def run():
+        try:
+            box.append((fn(), None))
+        except Exception as e:  # noqa: BLE001
+            box.append((None, e))
+
+    t = threading.Thread(target=run)
+    t.start()
+    t.join()
+    time.sleep(0.3)  # join returns before the thread's destructors have run
+    if box[0][1] is not None:
+        raise box[0][1]
+    return box[0][0]
+
+
+def measured(call, trace):
+    """(result, device bytes that a first call in a thread takes and keeps, launches)."""
+    in_thread(call)  # (code is loaded on first use)
+
+    def fn():
+        rg.set_trace(trace)
+        before = free_bytes()
+        out = call()
+        return out, before - free_bytes(), rg.last_timing()["kernel_launches"]
+    return in_thread(fn)
+
+
+class Filled:
+    """The device's free memory down to `leave` bytes."""
+
+    def __init__(self, leave):
+        self.leave = leave
+
+    def __enter__(self):
+        torch.cuda.empty_cache()
+        self.block = torch.empty(free_bytes() - self.leave, dtype=torch.uint8, device="cuda")
+
+    def __exit__(self, *_):
+        del self.block
+        torch.cuda.empty_cache()
+
+
+CALLS = {
+    "bfs": lambda g: g.bfs("push", 5, parents=False)[1:],
+    "bc": lambda g: g.bc_sources(np.array([5], np.uint32), "push"),
+    "radii": lambda g: g.radii_seeds(rg.radii_query_seeds(1, N), "push"),
+    "delta": lambda g: g.pagerank_delta("push-pull", 100)[:2],  # (its sparse rounds are handed over)
+}
+
+
+@pytest.mark.parametrize("app", CALLS)
+def test_the_level_by_level_run_answers_where_one_launch_does_not_fit(g, app):
+    call = lambda: CALLS[app](g)  # noqa: E731
+    want, one, launches = measured(call, False)
+    assert app == "delta" or launches <= 2
+    _, levels, _ = measured(call, True)
+    assert one > levels + (64 << 20), (one, levels)
+    with Filled((one + levels) // 2):
+        got, launches = in_thread(lambda: (call(), rg.last_timing()["kernel_launches"]))
+    assert launches > 2
+    if app in ("bc", "delta"):
+        assert_close(got[0], want[0], what=app)
+    else:
+        assert np.array_equal(got[0], want[0])
+    assert got[1:] == want[1:]
+
+
+def test_kept_arrays_are_given_back(g):
+    """After a BFS in one launch, a BC level by level that only fits without the arrays
+    that the BFS has left with the thread."""
+    want, _, _ = measured(lambda: CALLS["bc"](g), True)
+    _, one, _ = measured(lambda: CALLS["bfs"](g), False)
+    _, levels, _ = measured(lambda: CALLS["bc"](g), True)
+
+    def both():
+        CALLS["bfs"](g)
+        rg.set_trace(True)
+        with Filled(levels - one // 2):
+            return CALLS["bc"](g)
+
+    assert_close(in_thread(both)[0], want[0], what="bc")
