@@ -1966,6 +1966,7 @@ class Arrays {
     at_.push_back({reinterpret_cast<void**>(p), total_});
     total_ += bytes;
   }
+  size_t total() const { return total_; }
   // *fits: false where the memory is too small for them (the level-by-level runs need
   // a third of it)
   rg_status place(bool* fits) {
@@ -2111,25 +2112,34 @@ bool fused_fits(const rg_graph* g, int64_t max_edges) {
   return g->m <= max_edges && g->n <= max_edges && strides_fit(g->n, g->m) && !g_trace_on;
 }
 
+namespace {
+
+void bfs_arrays(const rg_graph* g, bool parents, bool ordered, BfsArgs* A, Arrays& X) {
+  const int64_t n = g->n, m = g->m, nwords = (n + 31) / 32;
+  A->parents = nullptr;
+  A->depth_out = nullptr;
+  X.add(&A->vis[0], nwords);
+  X.add(&A->vis[1], nwords);
+  X.add(&A->depth, n);
+  if (parents) X.add(&A->parents, n);
+  add_queues(X, &A->q[0], n, m);
+  add_queues(X, &A->q[1], n, m);
+  X.add(&A->rest, (size_t)(m / kRestPiece + m / (kRestList + 48) + 64));  // the last piece of a list may be short
+  if (ordered) X.add(&A->depth_out, n);
+}
+
+}  // namespace
+
 rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t* h_depth,
                         int64_t* rounds_out, int64_t* reached_out, int32_t* d_depth_out, bool* done) {
   Ctx& cx = ctx();
   cudaStream_t st = cx.stream;
-  const int64_t n = g->n, m = g->m, nwords = (n + 31) / 32;
+  const int64_t n = g->n, m = g->m;
   BfsArgs A;
-  A.parents = nullptr;
-  A.depth_out = nullptr;
   const bool order = g->sorted && (h_depth || d_depth_out);
-  Arrays X;
-  X.add(&A.vis[0], nwords);
-  X.add(&A.vis[1], nwords);
-  X.add(&A.depth, n);
-  if (h_parents) X.add(&A.parents, n);
-  add_queues(X, &A.q[0], n, m);
-  add_queues(X, &A.q[1], n, m);
-  X.add(&A.rest, (size_t)(m / kRestPiece + m / (kRestList + 48) + 64));  // the last piece of a list may be short
   int32_t* direct = direct_results(g, h_depth, d_depth_out);
-  if (order && !d_depth_out && !direct) X.add(&A.depth_out, n);
+  Arrays X;
+  bfs_arrays(g, h_parents != nullptr, order && !d_depth_out && !direct, &A, X);
   bool fits = false;
   RG_TRY(X.place(&fits));
   if (!fits) return RG_OK;
@@ -2165,12 +2175,12 @@ namespace {
 
 // The arrays of `groups` groups of bc_fused.
 // *ordered (unless null): n results by original id.
-rg_status bc_arrays(const rg_graph* g, int groups, bool chain, BcArgs* A, double** ordered, Arrays& X, bool* fits) {
+void bc_arrays(const rg_graph* g, int groups, bool chain, bool long_lists, BcArgs* A, double** ordered, Arrays& X) {
   const size_t n = (size_t)g->n, m = (size_t)g->m;
   A->n_small = small_entries(g->n);
   A->n_large = large_entries(g->n, g->m);
   A->same = !g->directed;
-  A->long_lists = std::max(max_in_degree(g, ctx().stream), (int64_t)g->max_deg) > kLongList;
+  A->long_lists = long_lists;
   // pieces of lists above kLongList, two at least: at most 3/2 per kLongPiece edges
   A->n_heavy = A->long_lists ? m / kLongPiece + m / kLongList + 64 : 0;
   A->new_ids = g->sorted ? g->new_ids.as<uint32_t>() : nullptr;
@@ -2187,7 +2197,10 @@ rg_status bc_arrays(const rg_graph* g, int groups, bool chain, BcArgs* A, double
   X.add(&A->heavy, A->n_heavy * groups);
   if (chain) X.add(&A->deps, n);
   if (ordered) X.add(ordered, n);
-  return X.place(fits);
+}
+
+bool has_long_lists(const rg_graph* g, cudaStream_t st) {
+  return std::max(max_in_degree(g, st), (int64_t)g->max_deg) > kLongList;
 }
 
 // Groups for k sources and the CTAs of each.  Every source gets a group while there
@@ -2216,7 +2229,8 @@ rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* 
   if (m <= std::min(kFusedBcRowsEdges, kFusedBcRowsWork / std::max(nsrc, 1))) bc_split(g, std::min(nsrc, 64), &groups, &width);
   Arrays X;
   bool fits = false;
-  RG_TRY(bc_arrays(g, groups, true, &A, order && !ordered ? &ordered : nullptr, X, &fits));
+  bc_arrays(g, groups, true, has_long_lists(g, st), &A, order && !ordered ? &ordered : nullptr, X);
+  RG_TRY(X.place(&fits));
   if (!fits) return RG_OK;
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = info_begin();
@@ -2254,7 +2268,8 @@ rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double
   BcArgs A;
   Arrays X;
   bool fits = false;
-  RG_TRY(bc_arrays(g, groups, false, &A, nullptr, X, &fits));
+  bc_arrays(g, groups, false, has_long_lists(g, st), &A, nullptr, X);
+  RG_TRY(X.place(&fits));
   if (!fits) return RG_OK;
   A.g = g->view();
   A.gt = g->in_view();
@@ -2298,10 +2313,9 @@ int depth_planes(int64_t n) {
   return p;
 }
 
-// What Radii and multi-source BFS share; seeds: original ids, each once.
+// What Radii and multi-source BFS share.
 // ordered: n radii by original id too; planes: the depth planes.
-rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int k, bool ordered,
-                     bool planes, RadiiArgs* A, Arrays& X, bool* fits) {
+void radii_arrays(const rg_graph* g, bool ordered, bool planes, RadiiArgs* A, Arrays& X) {
   const int64_t n = g->n, m = g->m;
   A->radii_out = nullptr;
   A->planes = nullptr;
@@ -2314,8 +2328,10 @@ rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned lo
   add_queues(X, &A->q[1], n, m);
   if (ordered) X.add(&A->radii_out, n);
   if (planes) X.add(&A->planes, (size_t)n * depth_planes(n));
-  RG_TRY(X.place(fits));
-  if (!*fits) return RG_OK;
+}
+
+// The rest of their arguments; seeds: original ids, each once.
+void radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int k, RadiiArgs* A) {
   A->out = g->view();
   A->in = g->in_view();
   A->chunk_v = g->in_chunks();
@@ -2334,7 +2350,6 @@ rg_status radii_args(const rg_graph* g, const uint32_t* seeds, const unsigned lo
   A->sources = 0;
   A->info = ctx().ws.h_info_dev;
   info_begin();
-  return RG_OK;
 }
 
 }  // namespace
@@ -2349,8 +2364,10 @@ rg_status radii_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned lon
   int32_t* direct = direct_results(g, h_radii, d_radii_out);
   Arrays X;
   bool fits = false;
-  RG_TRY(radii_args(g, seeds, masks, k, order && !d_radii_out && !direct, false, &A, X, &fits));
+  radii_arrays(g, order && !d_radii_out && !direct, false, &A, X);
+  RG_TRY(X.place(&fits));
   if (!fits) return RG_OK;
+  radii_args(g, seeds, masks, k, &A);
   if (direct) A.radii_out = direct;
   if (order && d_radii_out) A.radii_out = d_radii_out;
   volatile uint64_t* info = cx.ws.h_info;
@@ -2376,8 +2393,10 @@ rg_status ms_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long l
   RadiiArgs A;
   Arrays X;
   bool fits = false;
-  RG_TRY(radii_args(g, seeds, masks, u, false, true, &A, X, &fits));
+  radii_arrays(g, false, true, &A, X);
+  RG_TRY(X.place(&fits));
   if (!fits) return RG_OK;
+  radii_args(g, seeds, masks, u, &A);
   A.depths = out;
   A.sources = k;
   volatile uint64_t* info = cx.ws.h_info;
@@ -2388,6 +2407,26 @@ rg_status ms_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long l
   g_timing.edges_traversed += (int64_t)info[1];
   *rounds_out = (int64_t)info[0];
   return RG_OK;
+}
+
+size_t one_launch_bytes(const rg_graph* g, int kind, int k) {
+  Arrays X;
+  if (kind == RG_QUERY_BC) {
+    if (!fused_fits(g, k > 1 ? std::min(kFusedBcRowsEdges, kFusedBcRowsWork / k) : kFusedBcEdges)) return 0;
+    int groups = 1, width = 0;
+    if (k > 1) bc_split(g, k, &groups, &width);
+    BcArgs A;
+    bc_arrays(g, groups, k == 1, true, &A, nullptr, X);
+  } else if (kind == RG_QUERY_BFS && k == 1) {
+    if (!fused_fits(g, kFusedBfsEdges)) return 0;
+    BfsArgs A;
+    bfs_arrays(g, false, false, &A, X);
+  } else if (kind == RG_QUERY_BFS ? fused_fits(g, kFusedMsEdges)
+                                  : k == 1 && fused_fits(g, g->sorted ? kFusedRadiiSortedEdges : kFusedRadiiEdges)) {
+    RadiiArgs A;
+    radii_arrays(g, false, kind == RG_QUERY_BFS, &A, X);
+  }
+  return X.total();
 }
 
 rg_status pagerank_fused_run(rg_graph* g, int64_t max_iters, double* h_ranks, int64_t* iters_out, double* l1_out,

@@ -105,6 +105,10 @@ rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max
                         double* c, uint32_t* bits, double* ranks_out, int64_t* rounds, double* l1, bool* launched,
                         bool* done);
 
+// Device memory of the arrays that a served query (RG_QUERY_*) of k sources takes in one
+// launch, its result beside them; 0 where it does not.
+size_t one_launch_bytes(const rg_graph* g, int kind, int k);
+
 constexpr double kPrDamp = 0.85;  // PageRank.C:126
 constexpr double kPrdEps = 0.0000001, kPrdEps2 = 0.01;  // PageRankDelta.C:103-104
 

@@ -45,6 +45,7 @@
 #include <vector>
 
 #include "app_common.cuh"
+#include "fused.cuh"
 
 namespace {
 
@@ -187,18 +188,18 @@ rg_status calibrate_bc(rg_graph* g, int* breakeven) {
 
 size_t working_bytes(const rg_graph* g, int kind, int k) {
   const size_t n = (size_t)g->n;
-  // multi-source BC: two rows of ceil4(k) columns, the level store, masks and frontiers
-  if (kind == RG_QUERY_BC) return k > 1 ? (size_t)(16 * ((k + 3) & ~3) + 112) * n : 80 * n + (size_t)g->m / 4;
-  if (kind == RG_QUERY_RADII) {  // two mask rows of W words, radii rows and their copy, two frontiers
+  size_t levels;  // of the level-by-level run
+  if (kind == RG_QUERY_BC) {  // several: two rows of ceil4(k) columns, the level store, masks and frontiers
+    levels = k > 1 ? (size_t)(16 * ((k + 3) & ~3) + 112) * n : 72 * n;
+  } else if (kind == RG_QUERY_RADII) {  // two mask rows of W words, radii rows and their copy, two frontiers
     int W = 1;
     while (W < k) W *= 2;
-    return (size_t)(16 * W + 8 * k + 40) * n + (k == 1 ? 64 * n + (size_t)g->m / 4 : 0);
+    levels = (size_t)(16 * W + 8 * k + 40) * n;
+  } else {  // masks, depth rows and their original-order copy, two frontiers
+    levels = (size_t)(8 * k + 40) * n;
   }
-  // one BFS: two queues of vertices and of 128-edge pieces (16 bytes each) beside the depths
-  if (k == 1) return 88 * n + (size_t)g->m / 4;
-  // masks, depth rows and their original-order copy, two frontiers; or, in one launch,
-  // masks, depth planes, two queues and the rows
-  return std::max((size_t)(8 * k + 40) * n, (size_t)(4 * k + 140) * n + (size_t)g->m / 4);
+  // (a batch below the break-even size runs query by query)
+  return std::max({levels, rg::one_launch_bytes(g, kind, k), rg::one_launch_bytes(g, kind, 1)});
 }
 
 void worker_main(rg_server* S) {

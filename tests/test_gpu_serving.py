@@ -173,3 +173,36 @@ def test_wait_times_out_and_cancel_drops_the_query(graphs):
         assert e.value.status == 9
         with pytest.raises(rg.RgError):
             S.cancel(12345)  # unknown ticket
+
+
+@pytest.mark.parametrize("queries", [16, 1])
+def test_bc_batches_are_admitted_by_what_they_allocate(queries):
+    """Two BC batches on two graphs side by side, within a budget that holds what two
+    level-by-level runs take but not two one-launch runs: the second batch waits."""
+    torch = pytest.importorskip("torch")
+    off, adj = rg.rmat_csr(19, 14, seed=3)
+    n, m = len(off) - 1, len(adj)
+    # every vertex: a level, five doubles, a queue entry, a level's three words; and its pieces
+    one = (4 + 40 + 16 + 16) * n + 16 * (min(n, m // 33) + m // 128)
+    if queries == 16:
+        levels = (16 * 16 + 112) * n
+        group, groups = one - 8 * n, 8  # of sources, while 44 bytes a vertex stay within 192 MB
+        assert group * groups > 1.5 * levels
+        one = group * groups
+    else:
+        levels = 80 * n + m // 4
+        assert one > 1.05 * levels
+    result = 8 * n * queries
+    budget = levels + one + 2 * result
+    with rg.Graph.from_csr(off, adj) as a, rg.Graph.from_csr(off, adj) as b:
+        src = a.bc_pick_sources(queries)
+        waits = 0
+        for _ in range(5):
+            with rg.Server([a, b], workers=2, hbm_fraction=budget / torch.cuda.mem_get_info()[0]) as S:
+                S.pause(True)
+                tickets = [(gi, S.submit(gi, "bc", int(s))) for gi in (0, 1) for s in src]
+                S.pause(False)
+                for gi, t in tickets:
+                    S.wait(t, gi, "bc")
+                waits += S.stats()["admission_waits"]
+        assert waits > 0
