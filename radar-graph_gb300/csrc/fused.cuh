@@ -43,7 +43,11 @@ constexpr int64_t kFusedPrRows = 12000;
 //   PageRankDelta  whole, against dense rounds swept and the rest handed over:
 //             2^14 167 / 173 (85 / 102), 2^17 374 / 369 (164 / 175), 2^18 411 / 343
 //             (258 / 239), 2^19 619 / 495 (462 / 381), 2^20 1086 / 829 (842 / 646):
-//             6e6 edges; where dense rounds would push level by level, 3.3e7
+//             6e6 edges; where dense rounds would push level by level, 3.3e7.  Its
+//             vertices cost a warp of few per SM more than its edges do: uniform, 2
+//             edges a vertex, 2^19 772 / 680, 2^20 1961 / 1370, 2^21 3637 / 2224, a star
+//             of 3e6 11718 / 3858 (pushed level by level: 781 / 1290, 1954 / 2477, 3637 /
+//             3149, 11714 / 152065): 2^18 vertices; against pushes 2^21, pulled above
 constexpr int64_t kFusedBfsEdges = INT64_MAX;
 constexpr int64_t kFusedBcEdges = INT64_MAX;
 constexpr int64_t kFusedRadiiEdges = 6 << 23, kFusedRadiiSortedEdges = 5 << 25;
@@ -51,6 +55,7 @@ constexpr int64_t kFusedPagerankEdges = 3 << 20;
 constexpr int64_t kFusedPagerankPushEdges = 8 << 20;
 constexpr int64_t kFusedPrdEdges = 6 << 20;
 constexpr int64_t kFusedPrdPushEdges = 1 << 25;
+constexpr int64_t kFusedPrdVertices = 1 << 18, kFusedPrdPushVertices = 1 << 21;
 //   multi-source BC  16 sources: 2^14 116 / 1023 (147 / 864), 2^18 850 / 2055
 //             (900 / 2193), 2^19 1800 / 3010 (3000 / 4154), 2^20 4564 / 5299 (8250 /
 //             6911); 64 sources: 2^16 921 / 1498 (1426 / 1464), 2^17 1764 / 1961

@@ -170,7 +170,11 @@ rg_status pagerank_delta_run(rg_graph* g, int variant, int64_t max_iters, double
   const int64_t n = g->n;
   static thread_local PrdState S;
   bool pulls = variant == RG_PUSH_PULL || g_opts.direction == 1;
-  const bool small = fused_fits(g, pulls ? kFusedPrdEdges : kFusedPrdPushEdges);
+  // a whole run in one launch; push variants on graphs with more vertices than that is
+  // good for are pulled, as they would be there
+  const bool fits = fused_fits(g, pulls ? kFusedPrdEdges : kFusedPrdPushEdges);
+  const bool small = fits && n <= (pulls ? kFusedPrdVertices : kFusedPrdPushVertices);
+  if (fits && !small) pulls = true;
   // (2^20 vertices with 4e6 empty rows among them: 1120 ms pulled, 2.7 pushed)
   if (pulls && !small && !short_chunks(g, st)) {
     pulls = false;

@@ -153,3 +153,16 @@ def test_pagerank_delta_beside_empty_rows():
         one, levels = g.pagerank_delta("push-pull", 100), g.pagerank_delta("push", 100)
         assert one[1] == levels[1]
         assert_close(one[0], levels[0], what="ranks")
+
+
+@pytest.mark.parametrize("variant", ["push", "push-pull"])
+def test_pagerank_delta_time_of_a_star(variant):
+    """Few edges a vertex: no slower than the swept rounds that rg_set_trace asks for (in
+    one launch 2.9 times as slow)."""
+    n = 2500001
+    with graph(n, [(np.zeros(n - 1), 1 + np.arange(n - 1))]) as g:
+        ms = device_ms(lambda: g.pagerank_delta(variant, 100), reps=3)
+        rg.set_trace(True)
+        swept = device_ms(lambda: g.pagerank_delta("push-pull", 100), reps=3)
+        rg.set_trace(False)
+    assert ms < 1.6 * swept, (ms, swept)
