@@ -387,9 +387,9 @@ rg_status bc_multi_run(rg_graph* g, const uint32_t* src_orig, int k, double* h_o
   RG_TRY(get_ctx(&cx));
   cudaStream_t st = cx->stream;
   const int64_t n = g->n;
-  if (fused_fits(g, std::min(kFusedBcRowsEdges, kFusedBcRowsWork / k))) {
+  double* direct = d_out ? nullptr : static_cast<double*>(device_alias(h_out, 8 * (size_t)n * k, 8));
+  if (bc_rows_fit(g, k, direct != nullptr)) {
     DevBuf rows(true, st);
-    double* direct = d_out ? nullptr : static_cast<double*>(device_alias(h_out, 8 * (size_t)n * k, 8));
     if (!d_out && !direct) RG_TRY(rows.reserve(8 * (size_t)n * k));
     double* out = d_out ? d_out : direct ? direct : rows.as<double>();
     CallTimer timer(g);

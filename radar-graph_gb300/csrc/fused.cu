@@ -2112,6 +2112,15 @@ bool fused_fits(const rg_graph* g, int64_t max_edges) {
   return g->m <= max_edges && g->n <= max_edges && strides_fit(g->n, g->m) && !g_trace_on;
 }
 
+bool bc_rows_fit(const rg_graph* g, int k, bool direct) {
+  return fused_fits(g, std::min(kFusedBcRowsEdges, kFusedBcRowsWork / k)) &&
+         (direct || g->m >= g->n || k <= kFusedBcRowsFew || g->n * k <= kFusedBcRowsCells);
+}
+
+bool ms_fits(const rg_graph* g) {
+  return fused_fits(g, kFusedMsEdges) && (2 * g->m >= g->n || g->n <= kFusedMsVertices);
+}
+
 namespace {
 
 void bfs_arrays(const rg_graph* g, bool parents, bool ordered, BfsArgs* A, Arrays& X) {
@@ -2412,7 +2421,7 @@ rg_status ms_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long l
 size_t one_launch_bytes(const rg_graph* g, int kind, int k) {
   Arrays X;
   if (kind == RG_QUERY_BC) {
-    if (!fused_fits(g, k > 1 ? std::min(kFusedBcRowsEdges, kFusedBcRowsWork / k) : kFusedBcEdges)) return 0;
+    if (!(k > 1 ? bc_rows_fit(g, k, false) : fused_fits(g, kFusedBcEdges))) return 0;
     int groups = 1, width = 0;
     if (k > 1) bc_split(g, k, &groups, &width);
     BcArgs A;
@@ -2421,7 +2430,7 @@ size_t one_launch_bytes(const rg_graph* g, int kind, int k) {
     if (!fused_fits(g, kFusedBfsEdges)) return 0;
     BfsArgs A;
     bfs_arrays(g, false, false, &A, X);
-  } else if (kind == RG_QUERY_BFS ? fused_fits(g, kFusedMsEdges)
+  } else if (kind == RG_QUERY_BFS ? ms_fits(g)
                                   : k == 1 && fused_fits(g, g->sorted ? kFusedRadiiSortedEdges : kFusedRadiiEdges)) {
     RadiiArgs A;
     radii_arrays(g, false, kind == RG_QUERY_BFS, &A, X);

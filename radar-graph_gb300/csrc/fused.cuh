@@ -68,6 +68,17 @@ constexpr int64_t kFusedBcRowsWork = 256 << 20;  // edges times sources
 // (370 MB), 2016 in 80 MB; 16 sources on 2^18 808 us with all (184 MB), 1008 in 80 MB.
 constexpr int64_t kFusedBcRowsL2 = 192 << 20;
 constexpr int64_t kFusedMsEdges = 1 << 27;
+// Graphs of fewer edges than vertices, where a source costs passes over the vertices
+// alone (device us, one launch / shared): 2^20 vertices, 1000 edges, 2 sources 51 / 127,
+// 16 269 / 196, 64 1022 / 449; 2^24 vertices 2 sources 463 / 707, 10 2147 / 1361; 2^16
+// vertices, 64 sources 97 / 2239.  (Page-locked rows are written by the launch: 2992 /
+// 3312 a whole call for 64 sources on 2^20.)
+constexpr int64_t kFusedBcRowsFew = 3, kFusedBcRowsCells = 8 << 20;  // sources; vertices times sources
+// Multi-source BFS, half as many edges as vertices: 2^24 vertices, 2 sources 194 / 157,
+// 10 284 / 246; 2^20 vertices 31 / 75 and 44 / 89.
+constexpr int64_t kFusedMsVertices = 6 << 20;
+bool bc_rows_fit(const rg_graph* g, int k, bool direct);
+bool ms_fits(const rg_graph* g);
 
 // Whether a call on g may take the one-launch path: small enough, and no
 // per-level records (rg_set_trace) are asked for.

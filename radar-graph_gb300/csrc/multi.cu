@@ -100,7 +100,7 @@ rg_status bfs_multi_run(rg_graph* g, const uint32_t* src_orig, int k, int32_t* h
   RG_TRY(get_ctx(&cx));
   cudaStream_t st = cx->stream;
   const int64_t n = g->n;
-  if (fused_fits(g, kFusedMsEdges)) {
+  if (ms_fits(g)) {
     uint32_t v[64];
     unsigned long long mk[64];
     int u = 0;

@@ -2,6 +2,8 @@
 only reached neighbour is the last of their list, at the lengths where a pull's reading
 changes hands, and calls whose time must not follow what they do not reach."""
 
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -166,3 +168,39 @@ def test_pagerank_delta_time_of_a_star(variant):
         swept = device_ms(lambda: g.pagerank_delta("push-pull", 100), reps=3)
         rg.set_trace(False)
     assert ms < 1.6 * swept, (ms, swept)
+
+
+@pytest.mark.parametrize("k,pinned,one", [(3, False, True), (16, False, False), (16, True, True)])
+def test_batched_calls_on_many_vertices_without_edges(k, pinned, one):
+    """Fewer edges than vertices: which calls are one launch, and their results."""
+    n, rng = 1 << 20, np.random.default_rng(8)
+    src = rng.integers(0, n, k).astype(np.uint32)
+    ends = rng.integers(0, n, (2, 1000))
+    ends[0, 0] = src[0]
+    with graph(n, [tuple(ends)]) as g:
+        rg.set_trace(True)
+        want, levels = g.bc_multi(src)
+        rg.set_trace(False)
+        if pinned:
+            got = rg.pinned_empty((k, n), np.float64)
+            count = C.c_int64()
+            rg._check(rg.lib().rg_bc_multi(g.handle, src.ctypes.data_as(C.POINTER(C.c_uint32)), k,
+                                           got.ctypes.data_as(C.POINTER(C.c_double)), C.byref(count)))
+            assert count.value == levels
+        else:
+            got, count = g.bc_multi(src)
+            assert count == levels
+        assert (rg.last_timing()["kernel_launches"] == 1) == one
+        assert_close(got, want, what="bc rows")
+
+
+@pytest.mark.parametrize("n,one", [(6 << 20, True), (7 << 20, False)])
+def test_batched_bfs_on_many_vertices_without_edges(n, one):
+    src = np.array([5, 9], np.uint32)
+    with graph(n, [(np.arange(5, 50), np.arange(6, 51))]) as g:
+        rows, rounds = g.bfs_multi(src)
+        assert (rg.last_timing()["kernel_launches"] == 1) == one
+        assert rounds == 46
+        for row, s in zip(rows, src):
+            assert np.array_equal(row[5:51], np.abs(np.arange(5, 51) - int(s)))
+            assert (row[:5] == -1).all() and (row[51:] == -1).all()
