@@ -1028,8 +1028,11 @@ __device__ bool bc_backward(const BcArgs& A, int s, bool last, Grid& grid, uint3
     to[i] = d != 0.0 ? (d - A.inv[v]) * count : CUDART_NAN;
     most = max(most, bits_of(count));
   }
-  if (A.rows && most >= bits_of(kExactCounts)) {
-    reinterpret_cast<volatile unsigned char*>(A.info + 4 * s + 2)[most >= bits_of(kIntegerCounts)] = 1;
+  if (A.rows) {
+    volatile unsigned char* counts = reinterpret_cast<volatile unsigned char*>(A.info + 4 * s + 2);
+    const bool rounded = __any_sync(kAll, most >= bits_of(kExactCounts));
+    const bool past_integers = __any_sync(kAll, most >= bits_of(kIntegerCounts));
+    if (rounded && lane == 0) counts[past_integers] = 1;
   }
   if (tid == 0) {
     volatile uint64_t* f = A.info + (A.rows ? 4 * s : 0);
@@ -2010,9 +2013,9 @@ volatile uint64_t* info_begin() {
 // Once the stream has passed the call's launches: whether every CTA of them ran to its end.
 bool all_ran() { return ctx().ws.h_info[kGaveUp] == 0; }
 
-template <class K, class Args>
-rg_status launch_fused(K kern, Args& args, dim3 grid, size_t dyn, size_t most_dyn, cudaStream_t st) {
-  static std::atomic<uint64_t> checked{0};
+template <auto kern, class Args>
+rg_status launch_fused(Args& args, dim3 grid, size_t dyn, size_t most_dyn, cudaStream_t st) {
+  static std::atomic<uint64_t> checked{0};  // of this kernel (two of one type are two)
   RG_TRY(once_per_device(checked, [&]() -> rg_status {
     // one CTA per SM must fit, with all the dynamic shared memory it may ask for
     if (most_dyn) {
@@ -2163,7 +2166,7 @@ rg_status bfs_fused_run(rg_graph* g, uint32_t root, uint32_t* h_parents, int32_t
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = info_begin();
   CallTimer timer(g);
-  RG_TRY(launch_fused(bfs_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
+  RG_TRY(launch_fused<bfs_fused>(A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
   RG_TRY(timer.mark());
   if (!direct) RG_TRY(deliver<int32_t>(g, A.depth, A.depth_out, h_depth, d_depth_out, st));
   DevBuf tmp(true, st);  // parents by original id
@@ -2252,7 +2255,7 @@ rg_status bc_fused_run(rg_graph* g, const uint32_t* src_orig, int nsrc, double* 
     for (int q = 0; q < A.k; q++) A.source[q] = src_orig[it + q];
     A.first_source = it == 0;
     A.deps_out = it + A.k == nsrc ? ordered : nullptr;
-    RG_TRY(launch_fused(bc_fused, A, dim3(width, groups), 0, 0, st));
+    RG_TRY(launch_fused<bc_fused>(A, dim3(width, groups), 0, 0, st));
   }
   RG_TRY(timer.mark());
   if (!direct) RG_TRY(deliver<double>(g, A.deps, ordered, h_deps, d_deps_out, st));
@@ -2291,7 +2294,7 @@ rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double
   volatile uint64_t* info = reinterpret_cast<volatile uint64_t*>(cx.ws.h_small);
   for (int i = 0; i < 4 * k; i++) info[i] = 0;
   info_begin();
-  RG_TRY(launch_fused(bc_fused, A, dim3(width, groups), 0, 0, st));
+  RG_TRY(launch_fused<bc_fused>(A, dim3(width, groups), 0, 0, st));
   RG_CUDA(cudaStreamSynchronize(st));
   if (!all_ran()) return RG_OK;
   int64_t levels = 0;
@@ -2381,7 +2384,7 @@ rg_status radii_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned lon
   if (order && d_radii_out) A.radii_out = d_radii_out;
   volatile uint64_t* info = cx.ws.h_info;
   CallTimer timer(g);
-  RG_TRY(launch_fused(radii_fused<false>, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
+  RG_TRY(launch_fused<radii_fused<false>>(A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
   RG_TRY(timer.mark());
   if (!direct) RG_TRY(deliver<int32_t>(g, A.radii, A.radii_out, h_radii, d_radii_out, st));
   RG_CUDA(cudaStreamSynchronize(st));
@@ -2409,7 +2412,7 @@ rg_status ms_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long l
   A.depths = out;
   A.sources = k;
   volatile uint64_t* info = cx.ws.h_info;
-  RG_TRY(launch_fused(radii_fused<true>, A, fused_grid(m + n + n * (int64_t)k / 8, kFusedEdgesPerCta), 0, 0, st));
+  RG_TRY(launch_fused<radii_fused<true>>(A, fused_grid(m + n + n * (int64_t)k / 8, kFusedEdgesPerCta), 0, 0, st));
   RG_CUDA(cudaStreamSynchronize(st));
   *done = info[kDone] == 1 && all_ran();
   if (!*done) return RG_OK;
@@ -2483,7 +2486,7 @@ rg_status pagerank_fused_run(rg_graph* g, int64_t max_iters, double* h_ranks, in
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = info_begin();
   CallTimer timer(g);
-  RG_TRY(launch_fused(pagerank_fused, A, grid, sizeof(U128) * (size_t)rows, sizeof(U128) * kFusedPrRows, st));
+  RG_TRY(launch_fused<pagerank_fused>(A, grid, sizeof(U128) * (size_t)rows, sizeof(U128) * kFusedPrRows, st));
   RG_TRY(timer.mark());
   RG_TRY(deliver<double>(g, A.p, A.ranks_out, h_ranks, nullptr, st));
   RG_CUDA(cudaStreamSynchronize(st));
@@ -2533,7 +2536,7 @@ rg_status prd_fused_run(rg_graph* g, bool allow_pull, int64_t start, int64_t max
   A.ranks_out = ranks_out;
   A.info = cx.ws.h_info_dev;
   volatile uint64_t* info = info_begin();
-  RG_TRY(launch_fused(prd_fused, A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
+  RG_TRY(launch_fused<prd_fused>(A, fused_grid(m + n, kFusedEdgesPerCta), 0, 0, st));
   *launched = true;
   RG_CUDA(cudaStreamSynchronize(st));
   *done = info[kDone] == 1 && all_ran();

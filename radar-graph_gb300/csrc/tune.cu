@@ -54,8 +54,8 @@ std::vector<Options> candidates(int app, bool hubs, const Options& base) {
         for (int64_t div : {20, 80}) add(0, div, kb);
       for (int64_t div : {2, 5, 20}) add(1, div, 0);
       break;
-    default:  // BC pushes (its pull scans every unvisited vertex: measured slower),
-              // with hub copies in both phases or in the backward phase only
+    default:  // BC level by level pushes (its pull scans every unvisited vertex: measured
+              // slower), with hub copies in both phases or in the backward phase only
       for (int64_t kb : kbs)
         for (int64_t div : {20, 80}) {
           add(0, div, kb);
