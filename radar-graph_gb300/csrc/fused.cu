@@ -985,7 +985,7 @@ __device__ bool bc_backward(const BcArgs& A, int s, bool last, Grid& grid, uint3
         const double acc = warp_sum(d != kNone ? next[d] : 0.0);
         if (lane == 0) {
           A.inv[it.x] = x;
-          dep[it.x] = left ? left[it.x] + (x + acc) : x + acc;
+          dep[it.x] = (left ? left[it.x] + x : x) + acc;
         }
       }
       for (uint32_t i = gwarp * per; !few && i < (s1 - s0 + 7) / 8; i += nwarps * per) {
@@ -1009,7 +1009,7 @@ __device__ bool bc_backward(const BcArgs& A, int s, bool last, Grid& grid, uint3
           acc += __shfl_xor_sync(kAll, acc, 2);
           if (per == 1) x = 1.0 / x;  // (a short chain: the division waits for nothing)
           const double y = __shfl_sync(kAll, x, t * 8 + (lane >> 2));
-          if (j < s1 && (lane & 3) == 0) dep[u] = left ? left[u] + (y + acc) : y + acc;
+          if (j < s1 && (lane & 3) == 0) dep[u] = (left ? left[u] + y : y) + acc;
         }
         if (mine) A.inv[w] = x;
       }
