@@ -18,7 +18,7 @@
 //  * BC queries waiting for the same graph are coalesced the same way into one
 //    multi-source BC (rg_bc_multi: levels from one bitmask BFS, path counts
 //    and dependencies for every source per level); below the graph's BC
-//    break-even size (measured at start-up from two batch sizes against one
+//    break-even size (measured at start-up from three batch sizes against one
 //    single-source BC) each runs BC-manyiter-v2's single-source pass.
 // Results stay in device memory (stream-ordered allocations) until the client
 // fetches them with rg_server_wait, which copies one query's array straight
@@ -132,6 +132,19 @@ size_t result_bytes(const rg_graph* g, int kind, int k) {
   return kind == RG_QUERY_BC ? 8 * n * k : 4 * n * k;
 }
 
+// The smallest k, up to 64, for which a batch takes less than k calls of one (ks[0] =
+// 1), by the times t of batches of ks[1] < ks[2] ... and straight lines between and past
+// them; 65: none does.
+int break_even(const int* ks, const double* t, int points) {
+  for (int k = 2; k <= 64; k++) {
+    int i = 2;
+    while (i + 1 < points && ks[i] < k) i++;
+    const double per = std::max(0.0, (t[i] - t[i - 1]) / (ks[i] - ks[i - 1]));
+    if (t[i - 1] + per * (k - ks[i - 1]) < k * t[0]) return k;
+  }
+  return 65;
+}
+
 // Break-even batch size for one graph: time one single-source BFS and one
 // 64-source traversal (each after a warm-up run) on the calling thread.
 rg_status calibrate_bfs(rg_graph* g, int* breakeven) {
@@ -157,32 +170,42 @@ rg_status calibrate_bfs(rg_graph* g, int* breakeven) {
   return RG_OK;
 }
 
-// BC break-even: one single-source pass against multi-source passes of 2 and
-// 16 sources (cost ~ a + b k); the smallest k with a + b k < k * single.
-rg_status calibrate_bc(rg_graph* g, int* breakeven) {
+// BC break-even: one single-source pass against multi-source passes of 2, 16 and
+// (where the memory holds them) max_batch sources, straight lines between them; the
+// smallest k that takes less than k single ones.  (A source costs less the more there
+// are: 2^22 vertices 0.64 ms alone, 2.41, 0.97 and 0.48 among 2, 16 and 64, so a line
+// through the first two never crosses.)
+rg_status calibrate_bc(rg_graph* g, int max_batch, int* breakeven) {
   using namespace rg;
   const int64_t n = g->n;
-  std::vector<uint32_t> src(16);
-  RG_TRY(bc_pick(g, 16, src.data()));
-  DevBuf out;
-  RG_TRY(out.reserve(8 * (size_t)n * 16));
   const int variant = g->sorted ? RG_DEGSORT : RG_PUSH;
-  double t1 = 0, t2 = 0, t16 = 0;
-  for (int rep = 0; rep < 2; rep++) {
-    auto a = Clock::now();
-    RG_TRY(bc_run(g, variant, src.data(), 1, nullptr, nullptr, 0, out.as<double>()));
-    RG_CUDA(cudaStreamSynchronize(ctx().stream));
-    auto b = Clock::now();
-    RG_TRY(bc_multi_run(g, src.data(), 2, nullptr, out.as<double>(), nullptr));
-    auto c = Clock::now();
-    RG_TRY(bc_multi_run(g, src.data(), 16, nullptr, out.as<double>(), nullptr));
-    auto d = Clock::now();
-    t1 = std::chrono::duration<double>(b - a).count();
-    t2 = std::chrono::duration<double>(c - b).count();
-    t16 = std::chrono::duration<double>(d - c).count();
+  int ks[] = {1, 2, 16, std::max(max_batch, 17)};
+  double t[4] = {0, 0, 0, 0};
+  int points = 4;
+  std::vector<uint32_t> src(ks[3]);
+  RG_TRY(bc_pick(g, ks[3], src.data()));
+  DevBuf out;
+  if (out.reserve(8 * (size_t)n * ks[3]) != RG_OK) {
+    clear_error();
+    points = 3;
+    RG_TRY(out.reserve(8 * (size_t)n * 16));
   }
-  const double per = std::max(0.0, (t16 - t2) / 14.0), fixed = std::max(0.0, t2 - 2 * per);
-  *breakeven = t1 > per ? (int)std::min(65.0, std::max(2.0, std::floor(fixed / (t1 - per)) + 1)) : 65;
+  for (int rep = 0; rep < 2; rep++) {
+    for (int i = 0; i < points; i++) {
+      const auto a = Clock::now();
+      const rg_status s = i ? bc_multi_run(g, src.data(), ks[i], nullptr, out.as<double>(), nullptr)
+                            : bc_run(g, variant, src.data(), 1, nullptr, nullptr, 0, out.as<double>());
+      if (s == RG_ENOMEM && i == 3) {
+        clear_error();
+        points = 3;
+        break;
+      }
+      RG_TRY(s);
+      RG_CUDA(cudaStreamSynchronize(ctx().stream));
+      t[i] = std::chrono::duration<double>(Clock::now() - a).count();
+    }
+  }
+  *breakeven = break_even(ks, t, points);
   return RG_OK;
 }
 
@@ -386,7 +409,7 @@ rg_status rg_server_create(rg_graph* const* graphs, int ngraphs, int nworkers, i
   S->bc_breakeven.assign(ngraphs, 2);
   for (int i = 0; i < ngraphs; i++) {
     rg_status cs = calibrate_bfs(S->graphs[i], &S->bfs_breakeven[i]);
-    if (cs == RG_OK && S->graphs[i]->m > 0) cs = calibrate_bc(S->graphs[i], &S->bc_breakeven[i]);
+    if (cs == RG_OK && S->graphs[i]->m > 0) cs = calibrate_bc(S->graphs[i], max_batch, &S->bc_breakeven[i]);
     if (cs != RG_OK) {
       delete S;
       return cs;

@@ -206,3 +206,26 @@ def test_bc_batches_are_admitted_by_what_they_allocate(queries):
                     S.wait(t, gi, "bc")
                 waits += S.stats()["admission_waits"]
         assert waits > 0
+
+
+def test_bc_queries_are_coalesced_where_only_large_batches_pay():
+    """2^21 vertices: 2 or 16 sources together take longer than one by one, 64 do not."""
+    src, dst = rg.generate_edges(21, 16, seed=1)
+    with rg.Graph.from_edges(1 << 21, src, dst) as plain, plain.degree_sort() as g:
+        roots = g.bc_pick_sources(64)
+
+        def ms(call):
+            call()
+            call()
+            return rg.last_timing()["total_ms"]
+
+        one, many = ms(lambda: g.bc_sources(roots[:1], "radar")), ms(lambda: g.bc_multi(roots))
+        assert many < 0.8 * 64 * one, (one, many)
+        with rg.Server([g], workers=1) as S:
+            S.pause(True)
+            tickets = [S.submit(0, "bc", int(s)) for s in roots]
+            S.pause(False)
+            for t in tickets:
+                S.wait(t, 0, "bc")
+            st = S.stats()
+    assert st["launches"] == 1 and st["batched"] == 64
