@@ -39,7 +39,8 @@ constexpr int64_t kFusedPrRows = 12000;
 //   PageRank  20 iterations, against pulls: 2^10 97 / 217, 2^14 154 / 247 (93 /
 //             160), 2^16 308 / 308 (183 / 245), 2^17 565 / 473 (297 / 365): 3e6
 //             edges; against pushes: 2^16 309 / 730, 2^18 1331 / 1559, 2^19 2737 /
-//             2332: 8e6 edges
+//             2332: 8e6 edges.  Few edges a vertex: 2^20 vertices, one each 735 / 794
+//             (skewed 809 / 811), 1.36e6 1069 / 834: 2^20 vertices against pulls
 //   PageRankDelta  whole, against dense rounds swept and the rest handed over:
 //             2^14 167 / 173 (85 / 102), 2^17 374 / 369 (164 / 175), 2^18 411 / 343
 //             (258 / 239), 2^19 619 / 495 (462 / 381), 2^20 1086 / 829 (842 / 646):
@@ -53,6 +54,7 @@ constexpr int64_t kFusedBcEdges = INT64_MAX;
 constexpr int64_t kFusedRadiiEdges = 6 << 23, kFusedRadiiSortedEdges = 5 << 25;
 constexpr int64_t kFusedPagerankEdges = 3 << 20;
 constexpr int64_t kFusedPagerankPushEdges = 8 << 20;
+constexpr int64_t kFusedPagerankVertices = 1 << 20;
 constexpr int64_t kFusedPrdEdges = 6 << 20;
 constexpr int64_t kFusedPrdPushEdges = 1 << 25;
 constexpr int64_t kFusedPrdVertices = 1 << 18, kFusedPrdPushVertices = 1 << 21;

@@ -204,3 +204,18 @@ def test_batched_bfs_on_many_vertices_without_edges(n, one):
         for row, s in zip(rows, src):
             assert np.array_equal(row[5:51], np.abs(np.arange(5, 51) - int(s)))
             assert (row[:5] == -1).all() and (row[51:] == -1).all()
+
+
+def test_pagerank_time_of_many_vertices():
+    """1.4e6 vertices, one edge each: pulled, no slower than the swept iterations that
+    rg_set_trace asks for (in one launch 1.3 times as slow); ranks bit-equal."""
+    n, rng = 1400000, np.random.default_rng(2)
+    with graph(n, [tuple((n * rng.random((2, n)) ** 6).astype(np.int64))]) as g:
+        ms = device_ms(lambda: g.pagerank("push-pull", 20))
+        got = g.pagerank("push-pull", 20)
+        rg.set_trace(True)
+        swept = device_ms(lambda: g.pagerank("push-pull", 20))
+        want = g.pagerank("push-pull", 20)
+        rg.set_trace(False)
+    assert ms < 1.12 * swept, (ms, swept)
+    assert np.array_equal(got[0], want[0]) and got[1:] == want[1:]
