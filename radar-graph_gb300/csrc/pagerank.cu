@@ -340,21 +340,22 @@ __global__ void __launch_bounds__(256) pr_finalize(uint32_t n, const uint32_t* _
   U128 local{0ull, 0ull};
   double* accd = reinterpret_cast<double*>(acc);
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-    // a vertex without in-edges has the rank `added` and the same contribution
-    // from the first iteration on
-    const uint32_t b = pull_off[v], e = pull_off[v + 1];
-    if (later && b == e) continue;
-    // the tests of zero and equality are integer compares (the FP64 pipe is
-    // the scarce one): every value here is a nonnegative double, not NaN
+    // a vertex without in-edges, to which nothing is pushed, has the rank `added` and
+    // the same contribution from the first iteration on.  The tests of zero and
+    // equality are integer compares (the FP64 pipe is the scarce one): every value
+    // here is a nonnegative double, not NaN
     double sum;
     bool has;
     if (kExact) {
+      const uint32_t b = pull_off[v], e = pull_off[v + 1];
+      if (later && b == e) continue;
       const U128 a = acc[v];
       has = (a.lo | a.hi) != 0ull;
       sum = has ? fx_to_double(a) : 0.0;
       if (e > b && b / step != (e - 1) / step) acc[v] = U128{0ull, 0ull};
     } else {
       sum = accd[v];
+      if (later && bits_of(sum) == 0ull) continue;
       has = (bits_of(sum) << 1) != 0ull;
       accd[v] = 0.0;
     }
