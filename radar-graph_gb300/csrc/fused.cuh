@@ -40,7 +40,7 @@ constexpr int64_t kFusedPrRows = 12000;
 //             160), 2^16 308 / 308 (183 / 245), 2^17 565 / 473 (297 / 365): 3e6
 //             edges; against pushes: 2^16 309 / 730, 2^18 1331 / 1559, 2^19 2737 /
 //             2332: 8e6 edges.  Few edges a vertex: 2^20 vertices, one each 735 / 794
-//             (skewed 809 / 811), 1.36e6 1069 / 834: 2^20 vertices against pulls
+//             (skewed 809 / 811), 1.36e6 1069 / 834: 2^20 vertices
 //   PageRankDelta  whole, against dense rounds swept and the rest handed over:
 //             2^14 167 / 173 (85 / 102), 2^17 374 / 369 (164 / 175), 2^18 411 / 343
 //             (258 / 239), 2^19 619 / 495 (462 / 381), 2^20 1086 / 829 (842 / 646):
@@ -106,7 +106,8 @@ rg_status bc_rows_fused_run(rg_graph* g, const uint32_t* src_orig, int k, double
 // seeds: original ids, each once, with its mask
 rg_status radii_fused_run(rg_graph* g, const uint32_t* seeds, const unsigned long long* masks, int k,
                           int32_t* h_radii, int64_t* rounds_out, int32_t* d_radii_out, bool* done);
-rg_status pagerank_fused_run(rg_graph* g, int64_t max_iters, double* h_ranks, int64_t* iters_out, double* l1_out,
+// pull: the call would be answered by pulls otherwise.
+rg_status pagerank_fused_run(rg_graph* g, bool pull, int64_t max_iters, double* h_ranks, int64_t* iters_out, double* l1_out,
                              bool* done);
 // BFS depths from k <= 64 sources; seeds: the distinct ones (original ids) with
 // the mask of the sources at each.  out: k rows of n (device, original ids).

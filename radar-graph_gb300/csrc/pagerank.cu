@@ -423,10 +423,10 @@ rg_status pagerank_run(rg_graph* g, int variant, int64_t max_iters, double* h_ra
   // pull: the push-pull variant (threshold 0, PageRank.C:122 in src/push-pull)
   // or the auto direction
   const bool pull = variant == RG_PUSH_PULL || g_opts.direction == 1;
-  if (max_iters > 0 && fused_fits(g, pull ? kFusedPagerankEdges : kFusedPagerankPushEdges) &&
-      !(pull && g->n > kFusedPagerankVertices)) {
+  if (max_iters > 0 && g->n <= kFusedPagerankVertices &&
+      fused_fits(g, pull ? kFusedPagerankEdges : kFusedPagerankPushEdges)) {
     bool done = false;
-    RG_TRY(pagerank_fused_run(g, max_iters, h_ranks, iters_out, l1_out, &done));
+    RG_TRY(pagerank_fused_run(g, pull, max_iters, h_ranks, iters_out, l1_out, &done));
     if (done) return RG_OK;
   }
   cudaStream_t st = cx->stream;

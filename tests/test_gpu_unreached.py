@@ -219,3 +219,22 @@ def test_pagerank_time_of_many_vertices():
         rg.set_trace(False)
     assert ms < 1.12 * swept, (ms, swept)
     assert np.array_equal(got[0], want[0]) and got[1:] == want[1:]
+
+
+@pytest.mark.parametrize("n,m", [(1700000, 4200000), (1000000, 3500000)])
+def test_pagerank_time_of_skewed_rows(n, m):
+    """Rows that a CTA of the one launch can hold only by counting for hundreds of edges
+    each (12 times as slow as the pushes that rg_set_trace asks for)."""
+    rng = np.random.default_rng(2)
+    ends = (n * rng.random((2, m)) ** [[4], [3]]).astype(np.int64)
+    with graph(n, [tuple(ends)]) as g, g.degree_sort() as s:
+        for G, variant in ((g, "push"), (s, "radar")):
+            ms = device_ms(lambda: G.pagerank(variant, 20))
+            got = G.pagerank(variant, 20)
+            rg.set_trace(True)
+            levels = device_ms(lambda: G.pagerank(variant, 20))
+            want = G.pagerank(variant, 20)
+            rg.set_trace(False)
+            assert ms < 1.5 * levels, (variant, ms, levels)
+            assert_close(got[0], want[0], what=variant)
+            assert got[1] == want[1]
