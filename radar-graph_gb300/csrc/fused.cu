@@ -2462,8 +2462,9 @@ rg_status pagerank_fused_run(rg_graph* g, bool pull, int64_t max_iters, double* 
   const int64_t rows = std::min<int64_t>(n, share / weight + 2);
   A.row_weight = (uint32_t)weight;
   // a row is not shared between CTAs: one with far more edges than a CTA's
-  // share would hold the others up
-  if (rows > kFusedPrRows || max_in_degree(g, st) > 2 * share) return RG_OK;
+  // share would hold the others up (one launch / swept, us: 4.7e5 vertices, 2.9e6 edges,
+  // a row of 2.4 shares 1095 / 620; 8e4, 2.2e6, 1.75 445 / 337; 2.6e5, 6e5, 1.5 316 / 332)
+  if (rows > kFusedPrRows || max_in_degree(g, st) > (pull && m > 1 << 20 ? 1 : 2) * share) return RG_OK;
   const bool order = g->sorted && h_ranks;
   const size_t steps = (size_t)(m / kPrStep + 2 * grid + 4);
   A.ranks_out = nullptr;
