@@ -8,8 +8,8 @@
 // graphs, which get one CTA) and take every decision from counters that all of
 // them read after the barrier.  What bounds a small graph now is the chain of
 // dependent loads of a level, about 5 us with its barrier (BFS, R-MAT edge
-// factor 16: 2^10 vertices 182 -> 31 us, 2^16 298 -> 46 us); a large one is bound
-// by its pulls' gathers, as level by level (2^24: 973 -> 560 us; the compactions
+// factor 16: 2^10 vertices 182 -> 27 us, 2^16 298 -> 43 us); a large one is bound
+// by its pulls' gathers, as level by level (2^24: 973 -> 450 us; the compactions
 // between the levels are gone).
 //
 // The frontier is two unordered queues: vertices of degree <= kSmallDeg, four

@@ -1,4 +1,5 @@
-// One-sweep radix sort: the digit counts of every pass are taken in one read of
+// One-sweep radix sort (Adinets and Merrill 2022; the look-back is Merrill and
+// Garland's single-pass scan, 2016): the digit counts of every pass are taken in one read of
 // the keys; each pass then reads and writes every key once.  A tile of kTile
 // keys ranks its keys per warp, publishes its digit counts, learns how many
 // equal digits lie in earlier tiles by looking back over what those published,
