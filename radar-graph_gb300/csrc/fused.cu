@@ -147,7 +147,7 @@ __device__ __forceinline__ Slot read_slot(const Slot* s) {
 // The barrier's wait, after a first look.  0: it ran out.  (Out of line: what it needs
 // of shared memory is read beside the polls, off the path of a wait that ends.)
 __device__ __noinline__ int poll(Shared* sh, const Team& t) {
-  unsigned left = t.target / t.ctas > sh->from ? sh->polls : kPolls;
+  unsigned left = t.target > (unsigned long long)sh->from * t.ctas ? sh->polls : kPolls;
   do {
     if (left-- == 0) {
       *sh->gave_up = 1;
@@ -431,12 +431,30 @@ __device__ __noinline__ uint32_t read_on(const uint32_t* adj, const uint32_t* vi
   return kNone;
 }
 
+// What a pulled level has put off.
+__device__ __noinline__ void read_rest(const BfsArgs& A, uint32_t pieces, const uint32_t* vis, uint32_t* nvis,
+                                       int32_t level, Shared* sh) {
+  const uint32_t nwarps = gridDim.x * kFWarps;
+  for (uint32_t i = blockIdx.x * kFWarps + (threadIdx.x >> 5); i < pieces; i += nwarps) {
+    const uint4 it = A.rest[i];
+    if (__any_sync(kAll, (__ldcg(nvis + (it.x >> 5)) >> (it.x & 31)) & 1u)) continue;  // found by another piece
+    const uint32_t f = first_visited(A.in.adj, vis, it.y, it.z);
+    const uint32_t bit = 1u << (it.x & 31);
+    if (f != kNone && (threadIdx.x & 31) == 0 && !(atomicOr(nvis + (it.x >> 5), bit) & bit)) {
+      A.depth[it.x] = level;
+      if (A.parents) A.parents[it.x] = f;
+      atomicAdd(&sh->count, 1u);
+      atomicAdd(&sh->degsum, (unsigned long long)(A.out.off[it.x + 1] - A.out.off[it.x]));
+    }
+  }
+}
+
 // A push level claims vertices with an atomicOr on the visited bitmap; a pull
 // level reads one bitmap and writes the other (a visited in-neighbour of an
 // unvisited vertex is in the frontier, so visited is all a pull has to test) and, on
 // a symmetric graph, marks vertices without edges visited, so that later pulls pass
 // them by.
-__global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
+__global__ void __launch_bounds__(kFT, 1) bfs_fused(const __grid_constant__ BfsArgs A) {
   __shared__ Shared sh;
   __shared__ Member buf[kFWarps][kBuf];
   Grid grid;
@@ -573,18 +591,7 @@ __global__ void __launch_bounds__(kFT, 1) bfs_fused(BfsArgs A) {
       if (!grid.sync(ns)) return;
       const uint32_t put_off = sh.slot.heavy;
       if (!put_off) continue;
-      for (uint32_t i = warp; i < put_off; i += nwarps) {
-        const uint4 it = A.rest[i];
-        if (__any_sync(kAll, (__ldcg(nvis + (it.x >> 5)) >> (it.x & 31)) & 1u)) continue;  // found by another piece
-        const uint32_t f = first_visited(A.in.adj, vis, it.y, it.z);
-        const uint32_t bit = 1u << (it.x & 31);
-        if (f != kNone && lane == 0 && !(atomicOr(nvis + (it.x >> 5), bit) & bit)) {
-          A.depth[it.x] = level;
-          if (A.parents) A.parents[it.x] = f;
-          atomicAdd(&sh.count, 1u);
-          atomicAdd(&sh.degsum, (unsigned long long)(A.out.off[it.x + 1] - A.out.off[it.x]));
-        }
-      }
+      read_rest(A, put_off, vis, nvis, level, &sh);
     } else {
       if (!queued) {  // after a pull: the frontier is what it added to the bitmap
         const uint32_t* old = A.vis[cv ^ 1];
